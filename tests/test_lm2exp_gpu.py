@@ -652,3 +652,23 @@ def test_batches_beyond_the_grid_limit():
         tb.check_status()
         _assert_close(got.cpu(), a, b, "3xtf32")
     assert torch.equal(tb.colmax(b.cuda()).cpu(), b.amax(dim=1).clamp(-1e38, 1e38))
+
+
+@pytest.mark.parametrize("precision, variant", [("tf32", 2567), ("tf32", 2566), ("tf32", 2564), ("3xtf32", 402564)])
+def test_pair_kernels_back_to_back(precision, variant):
+    """Hundreds of launches without a wait in between, on a shape with an odd number of k-blocks and a partly filled row
+    tile: the CTAs of a pair start and leave at different times, and nothing one of them does may touch the other
+    before it runs or after it has left (allocation, commits and deallocation of a pair are such accesses)."""
+    import triturus_b200 as tb
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = torch.rand(78, 186, 224, generator=g, device="cuda")
+    b = torch.randn(78, 224, 3328, generator=g, device="cuda")
+    first = tb.lm2exp(a, b, precision=precision, variant=variant)
+    for _ in range(400):
+        out = tb.lm2exp(a, b, precision=precision, variant=variant)
+    tb.check_status()
+    assert torch.equal(first, out)
+    want = orc.lm2exp_fp64(a[5:6].cpu(), b[5:6].cpu())
+    res = orc.compare_logspace(out[5:6], want, ATOL[precision])
+    assert res["ok"], res

@@ -24,7 +24,7 @@
 //   warp 2      TMA producer of ring 2: this CTA's 128 columns of b (no swizzle).
 //   warp 3      watches the a tiles land and says so on the leader's xf_done barriers.
 //   warps 4-7   epilogue (TMEM lane quarter = warp % 4).
-//   warps 8-15  transform: NG = two groups of four warps (one per lane quarter) take alternate k-blocks (three
+//   warps 8-15  transform: NG = two groups of four warps (one per lane quarter) take alternate tiles of b (three
 //               groups, 20 warps at 96 registers, ran 5 % slower; ring depths 6+6, 5+7, 7+5 instead of 8+4 the same).
 #pragma once
 
@@ -401,7 +401,14 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ transform: b tile -> E^T in tensor memory
     const int q = warp & 3;         // TMEM lane quarter this warp may write
-    const int grp = (warp - 8) >> 2;  // this warp's group takes the k-blocks with kb % NG == grp
+    // This warp's group takes every NG-th tile of ring 2, counted over the whole launch and not per output tile: a
+    // slot of the ring (NSB is a multiple of NG) then always belongs to the same group, which has waited for the
+    // slot's previous tile before it waits for the next one.  A wait by parity is only meaningful under that
+    // condition: counted per output tile, an odd number of k-blocks swapped the groups' slots at every tile, a group
+    // could look at a slot whose previous load (the other group's) had not landed, take the phase before that for its
+    // own, and hand the slot back twice.
+    const int grp = (warp - 8) >> 2;
+    static_assert(NSB % Cfg::NG == 0, "a ring-2 slot belongs to one transform group");
     const int kl = q * 32 + lane;
     const uint32_t ebase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + Cfg::E_COL0;
     const uint32_t xf_done_leader0 = map_to_cta(smem_u32(&xf_done[0]), 0);
@@ -415,12 +422,15 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       // A column past K reads zero-filled values; the stabiliser +inf turns them into exact zeros.
       float m = INFINITY;
       if (!Cfg::SLOTS && kcol < p.K) m = clamp_stab(__ldg(p.m_ws + static_cast<int64_t>(r) * p.K + kcol));
+      const auto first_kb = [&](uint32_t itb_tile) -> int {  // this group's first k-block of a pass that starts at ring-2 tile itb_tile
+        return (grp + Cfg::NG - static_cast<int>(itb_tile % Cfg::NG)) % Cfg::NG;
+      };
       const uint32_t mslot = (tcount & 1) * 4 + q;
       float* mdst = m_tile + (tcount & 1) * BM + kl;
       if (Cfg::FUSED) {
         // ---- max pass: running maximum of this lane's column over the k-blocks of this group
         float mx = -INFINITY;
-        for (int kb = grp; kb < KB; kb += Cfg::NG) {
+        for (int kb = first_kb(itb0); kb < KB; kb += Cfg::NG) {
           const uint32_t itb = itb0 + static_cast<uint32_t>(kb);
           const int sb = itb % NSB;
           if (!(ok = mbar_wait_warp(&b_full[sb], (itb / NSB) & 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
@@ -454,9 +464,10 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         }
       }
       // The group of k-block 0 publishes the tile's stabilisers; the other groups pick them up.  In the optimistic
-      // instance that is done after the loads of the group's own first k-block are in flight (the first group
+      // instance that is done after the loads of the group's own first k-block are in flight (that group
       // publishes as soon as it holds k-block 0, i.e. at about the same time), not before them.
-      bool need_m = Cfg::SLOTS && grp != 0;
+      const int kb_first = first_kb(itb0);
+      bool need_m = Cfg::SLOTS && (Cfg::OPT ? kb_first != 0 : grp != 0);
       auto fetch_m = [&]() -> bool {
         if (!mbar_wait_warp(&m_ready[mslot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_TRANSFORM)) return false;
         m = *mdst;
@@ -468,7 +479,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (need_m && Cfg::FUSED) {
         if (!(ok = fetch_m())) break;
       }
-      for (int kb = grp; kb < KB; kb += Cfg::NG) {
+      for (int kb = kb_first; kb < KB; kb += Cfg::NG) {
         const uint32_t it = it0 + static_cast<uint32_t>(kb);
         const int s = it % NS;
         const uint32_t ph = (it / NS) & 1;
@@ -485,7 +496,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (!(ok = fetch_m())) break;
         }
         if (Cfg::OPT && kb == 0) {
-          // (grp == 0) stabiliser = maximum over the first k-block; the slot's readers of two tiles ago are done
+          // stabiliser = maximum over the first k-block; the slot's readers of two tiles ago are done
           float mx = -INFINITY;
 #pragma unroll
           for (int x = 0; x < 32; ++x) mx = fmaxf(mx, x < jrem ? v[x] : -INFINITY);

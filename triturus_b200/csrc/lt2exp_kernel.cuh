@@ -586,7 +586,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
     const int tt = threadIdx.x - 8 * 32;
     const int n = tt % BN;       // column of the tile owned by this thread
     constexpr int NG = Cfg::NGROUPS;
-    const int grp = tt / BN;     // this thread's group takes k-blocks with i % NGROUPS == grp
+    const int grp = tt / BN;     // this thread's group takes every NGROUPS-th k-block
     uint32_t it = 0, tcount = 0;
     bool ok = true;
     LtWork work(p, KBT);
@@ -662,9 +662,13 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
         for (int x = 0; x < 32; ++x) eb[x] = exp_shifted(eb[x], mb);
         // Raw a values of this group's next PF k-blocks.
         float apf[PF];
+        // Groups alternate over the stage counter, not over i: a group's consecutive stages are then NG apart whatever
+        // the row counts of the chunks, so that a stage it waits for by parity is never two uses behind (with NS = 2
+        // or 3 stages and odd row counts it could be, counted over i).
+        const int g0 = (grp + NG - static_cast<int>(it % NG)) % NG;
 #pragma unroll
         for (int x = 0; x < PF; ++x) {
-          const int i = grp + x * NG;  // row within the slice
+          const int i = g0 + x * NG;  // row within the slice
           apf[x] = (col_ok && i < In) ? __ldg(a_sl + static_cast<int64_t>(i) * p.a_s1) : -INFINITY;
         }
         for (int ib = 0; ok && ib < In; ib += PF * NG) {
@@ -672,12 +676,12 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
 #pragma unroll
           for (int x = 0; x < PF; ++x) {
             acur[x] = apf[x];
-            const int i = ib + PF * NG + grp + x * NG;
+            const int i = ib + PF * NG + g0 + x * NG;
             apf[x] = (col_ok && i < In) ? __ldg(a_sl + static_cast<int64_t>(i) * p.a_s1) : -INFINITY;
           }
 #pragma unroll
           for (int x = 0; x < PF; ++x) {
-            const int i = ib + grp + x * NG;
+            const int i = ib + g0 + x * NG;
             if (i >= In) break;
             const uint32_t my_it = it + static_cast<uint32_t>(i);  // stage counter of k-block (jc, i_lo + i)
             const int s = my_it % NS;

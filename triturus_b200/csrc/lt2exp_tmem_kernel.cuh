@@ -277,7 +277,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     // ------------------------------------------------------------------ transform: operand generator
     const int tt = threadIdx.x - 8 * 32;
     const int n = tt % BN;   // column of the tile = TMEM lane owned by this thread
-    const int grp = tt / BN; // this thread's group takes k-blocks with (i - i_lo) % 2 == grp
+    const int grp = tt / BN; // this thread's group takes every NGROUPS-th k-block
     constexpr int NG = Cfg::NGROUPS;
     // TMEM lane quarter of this warp; with two column blocks per tile the upper four warps write the second
     // block's operand columns.
@@ -352,9 +352,13 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
 #pragma unroll
         for (int x = 0; x < 32; ++x) eb[x] = exp_shifted(eb[x], mb);
         float apf[PF];
+        // Groups alternate over the stage counter, not over i: a group's consecutive stages are then NG apart whatever
+        // the row counts of the chunks, so that a stage it waits for by parity is never two uses behind (with NS = 2
+        // or 3 stages and odd row counts it could be, counted over i).
+        const int g0 = (grp + NG - static_cast<int>(it % NG)) % NG;
 #pragma unroll
         for (int x = 0; x < PF; ++x) {
-          const int i = grp + x * NG;
+          const int i = g0 + x * NG;
           apf[x] = (col_ok && i < In) ? __ldg(a_sl + static_cast<int64_t>(i) * p.a_s1) : -INFINITY;
         }
         for (int ib = 0; ok && ib < In; ib += PF * NG) {
@@ -362,12 +366,12 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
 #pragma unroll
           for (int x = 0; x < PF; ++x) {
             acur[x] = apf[x];
-            const int i = ib + PF * NG + grp + x * NG;
+            const int i = ib + PF * NG + g0 + x * NG;
             apf[x] = (col_ok && i < In) ? __ldg(a_sl + static_cast<int64_t>(i) * p.a_s1) : -INFINITY;
           }
 #pragma unroll
           for (int x = 0; x < PF; ++x) {
-            const int i = ib + grp + x * NG;
+            const int i = ib + g0 + x * NG;
             if (i >= In) break;
             const uint32_t my_it = it + static_cast<uint32_t>(i);
             const int s = my_it % NS;
