@@ -111,12 +111,16 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     tma_prefetch_desc(&tmap_b);
     if (p.out_tma) tma_prefetch_desc(&tmap_out);
   }
+  // Both CTAs run and have initialised their barriers before anything crosses between them.  The pair allocation
+  // below is such a crossing (it takes both CTAs' tensor memory): the CTAs of a cluster do not start at the same
+  // instant, and an allocation by the first one before the second exists is an access to an absent block.
+  cluster_sync_all();
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish_pair();
   }
   for (int c = threadIdx.x; c < 2 * BN; c += Cfg::NTHREADS) colbuf[c] = NEG_INF_BITS;
-  // Both CTAs must have initialised their barriers before either one signals across.
+  // The leader's MMAs write both CTAs' tensor memory: both allocations are done before the roles start.
   tc_fence_before_sync();
   cluster_sync_all();
   tc_fence_after_sync();
@@ -163,6 +167,9 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             tma_load_3d(b_tile(s, 0) + g * Cfg::B_BOX, &tmap_b, &full[s], my_n0 + g * 32, kb * BK, r);
         }
       }
+      // The leader's commits arrive on both CTAs' stage_empty barriers: this CTA stays until the last ones are in.
+      for (uint32_t d = ok ? min(it, static_cast<uint32_t>(NS)) : 0u; ok && d > 0; --d)
+        ok = mbar_wait(&stage_empty[(it - d) % NS], ((it - d) / NS) & 1, ctl, STATUS_TIMEOUT_PRODUCER);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -463,6 +470,7 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
   }
+  cluster_sync_all();  // (the pair deallocation involves both CTAs: neither leaves before the other has done it)
 }
 
 }  // namespace tb200

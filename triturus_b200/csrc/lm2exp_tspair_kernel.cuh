@@ -178,11 +178,15 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     tma_prefetch_desc(&tmap_b);
     if (p.out_tma) tma_prefetch_desc(&tmap_out);
   }
+  // Both CTAs run and have initialised their barriers before anything crosses between them.  The pair allocation
+  // below is such a crossing (it takes both CTAs' tensor memory): the CTAs of a cluster do not start at the same
+  // instant, and an allocation by the first one before the second exists is an access to an absent block.
+  cluster_sync_all();
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
     tmem_relinquish_pair();
   }
-  // Both CTAs must have initialised their barriers before either one signals across.
+  // The leader's MMAs write both CTAs' tensor memory: both allocations are done before the roles start.
   tc_fence_before_sync();
   cluster_sync_all();
   tc_fence_after_sync();
@@ -220,6 +224,9 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           tma_load_3d(a_tile(s), &tmap_a, &a_full[s], kb * BK, my_i0, r);
         }
       }
+      // The leader's commits arrive on both CTAs' stage_empty barriers: this CTA stays until the last ones are in.
+      for (uint32_t d = ok ? min(it, static_cast<uint32_t>(NS)) : 0u; ok && d > 0; --d)
+        ok = mbar_wait(&stage_empty[(it - d) % NS], ((it - d) / NS) & 1, ctl, STATUS_TIMEOUT_PRODUCER);
     }
     __syncwarp();
   } else if (warp == 2) {
@@ -554,6 +561,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     tc_fence_after_sync();
     tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
   }
+  cluster_sync_all();  // (the pair deallocation involves both CTAs: neither leaves before the other has done it)
   if (Cfg::FUSED && p.reset_flag != nullptr && threadIdx.x == 0) {
     // A conditional launch that ran: every CTA read the flag when it started, so the CTA that finishes last may
     // put it down (the word behind it counts the finished CTAs; the optimistic launch before this one cleared it).
