@@ -672,3 +672,35 @@ def test_pair_kernels_back_to_back(precision, variant):
     want = orc.lm2exp_fp64(a[5:6].cpu(), b[5:6].cpu())
     res = orc.compare_logspace(out[5:6], want, ATOL[precision])
     assert res["ok"], res
+
+
+@pytest.mark.parametrize("shape", [(2, 129, 1, 200), (2, 256, 32, 256), (2, 300, 127, 260), (3, 257, 129, 516),
+                                   (1, 1000, 250, 1000), (2, 200, 1025, 129), (1, 500, 4096, 300)])
+@pytest.mark.parametrize("dist", ["normal", "offset", "huge"])
+def test_3xtf32_on_the_tmem_operand_pair_kernel(shape, dist):
+    """3xTF32 on pair tiles: hi * hi in tf32, the corrections in bf16.  One to more k-blocks than there are operand
+    stages (four), partial last k-blocks, rows past I, columns past K, isolated and whole-column -inf, weights near the
+    largest float on values that stay above 2^-114 of their column's largest (below it a correction is subnormal, which the
+    tensor core drops).  Tolerance: 2^-17 for the split (four bf16 roundings of 2^-9 on terms of 2^-10 or less), the tensor
+    core's truncating additions (two per eight terms, half an ulp each: 1.2e-8 per term), the rounding of the exponent's
+    argument (2^-23 of the up to 80 that a column spans) and of the result."""
+    R, I, J, K = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 6.0
+    if dist == "offset":
+        b += 200.0 * torch.randn(R, 1, K, generator=g)
+        b[torch.rand(R, J, K, generator=g) < 0.01] = float("-inf")
+        b[0, :, 3] = float("-inf")
+        a[:, :, 0] += 1e-3  # (J = 1: no zero weights)
+    elif dist == "huge":
+        a = a * 1e-6
+        a[:, :, J // 2] = 3.4028e38
+        b[:, J // 2] -= 25.0
+        b.clamp_(-55.0, 24.0)
+    got = _run(a, b, precision="3xtf32", variant=102564)
+    want = orc.lm2exp_fp64(a, b)
+    assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
+    fin = torch.isfinite(want)
+    tol = 2.0**-17 + 1.2e-8 * J + 80 * 2.0**-23 + 2.0**-22 * want[fin].abs()
+    assert ((got[fin].double() - want[fin]).abs() <= tol).all()

@@ -337,6 +337,7 @@ static int launch_lm2exp_pair(const CUtensorMap& ta, const CUtensorMap& tb, cons
 //                                  NS NSB groups optimistic
 using LmTsPair = Lm2expTsPairCfg<8, 4, 2>;
 using LmTsPairOpt = Lm2expTsPairCfg<8, 4, 2, true>;
+using LmTsPairX = Lm2expTsPairCfg<4, 4, 2, false, false, 1>;  // 3xTF32
 using LmTsPairFused = Lm2expTsPairCfg<8, 4, 2, false, true>;  // exact max pass inside: the conditional launch behind Opt
 
 // The CTA-pair kernel with the generated operand in tensor memory (plain TF32, a with j contiguous).
@@ -750,7 +751,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   // The TMEM-operand pair kernel takes a with j contiguous and does not fold column maxima of the result; other
   // calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
   // columns k, unswizzled (only the transform threads read them).
-  const bool use_ts = plan.tspair && !a_mn && out_colmax == nullptr;
+  const bool use_ts = (plan.tspair || (pair && precision == TRITURUS_B200_PRECISION_3XTF32)) && !a_mn && out_colmax == nullptr;
   CUtensorMap tb_plain;
   if (use_ts) {
     const int64_t dims[3] = {K, J, R};
@@ -777,7 +778,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     p.reset_flag = flag;
     return launch_lm2exp_tspair<LmTsPairFused>(ta, tb_plain, to, p, st, true);
   }
-  if (pair && !use_ts && plan.optimistic_prepass && prepass && ws_flags && out_colmax == nullptr) {
+  if (pair && plan.optimistic_prepass && prepass && ws_flags && out_colmax == nullptr) {
     // Pre-pass over the first 32 rows of b only; the contraction raises the flag if a result overflowed, and the
     // full pre-pass and the contraction with its maxima follow as launches that return at once unless it did.
     int* flag = static_cast<int*>(workspace);
@@ -785,13 +786,15 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     if (rc != TRITURUS_B200_OK) return rc;
     Lm2expParams po = p;
     po.opt_flag = flag;
-    rc = precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, po, st, true)
-                                                      : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
+    rc = use_ts ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, po, st, true)
+         : precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, po, st, true)
+                                                       : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
     if (rc != TRITURUS_B200_OK) return rc;
     rc = colmax_run(b, m_buf, R, J, K, bstr, stream, flag, flag + 1);
     if (rc != TRITURUS_B200_OK) return rc;
     p.only_if = flag + 1;
     p.reset_flag = flag;
+    if (use_ts) return launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, true);
     return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, p, st, true)
                                                         : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, true);
   }
@@ -806,7 +809,9 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     if (rc != TRITURUS_B200_OK) return rc;
   }
   const bool dep = prepass;
-  if (use_ts) return launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
+  if (use_ts)
+    return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, dep)
+                                                        : launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
   if (pair) {
     return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, p, st, dep)
                                                         : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, dep);

@@ -52,13 +52,18 @@ __device__ long long g_timeline[16 * 256];
 // (1-2 us from L2 / HBM) -> transform -> MMA -> commit" is several thousand cycles long, so the number of
 // k-blocks in flight, not any pipe, bounds a single ring of six stages (measured 1 100 cycles per k-block for
 // 512 cycles of MMAs); two rings put 8 + 5 tiles in flight in the same shared memory.
-template <int NS_, int NSB_, int NG_ = 2, bool OPT_ = false, bool FUSED_ = false>
+template <int NS_, int NSB_, int NG_ = 2, bool OPT_ = false, bool FUSED_ = false, int PREC_ = 0>
 struct Lm2expTsPairCfg {
   static constexpr int BM = 128;   // columns k per CTA (256 per pair): TMEM lanes
   static constexpr int BN = 256;   // rows i per pair tile (N of the MMA), 128 per CTA's shared memory
   static constexpr int BK = 32, NG = NG_, NTW = 4 * NG_, NS = NS_, NSB = NSB_;
   static constexpr int A_TILE = 128 * BK * 4;  // this CTA's rows of a: 16 KB
   static constexpr int B_TILE = BK * BM * 4;   // this CTA's columns of b: 32 rows j x 128 k = 16 KB
+  // PREC (3xTF32): a ring-1 stage also holds the packed bf16 words of the corrections (tf32_split_pack_rn in ptx.cuh), of
+  // a in a second 16 KB tile and of E^T in 32 more TMEM columns.
+  static constexpr int PREC = PREC_;
+  static constexpr int A_STAGE = (PREC ? 2 : 1) * A_TILE;
+  static constexpr int E_COLS = (PREC ? 2 : 1) * BK;  // TMEM columns of an operand stage
   static constexpr int ACC_COLS = BN;
   static constexpr int E_COL0 = ACC_COLS;  // first TMEM column of the operand stages
   static constexpr int TMEM_COLS = 512;
@@ -77,10 +82,11 @@ struct Lm2expTsPairCfg {
   static constexpr bool FUSED = FUSED_;
   static constexpr bool SLOTS = OPT || FUSED;  // stabilisers handed from the transform warps to the other roles
   static_assert(!(OPT && FUSED), "one or the other");
+  static_assert(!PREC || !SLOTS, "3xTF32 takes its stabilisers from a pre-pass");
   static constexpr int NBAR = 3 * NS + 2 * NSB + 2 + (SLOTS ? 16 : 0) + (FUSED ? 4 * (NG - 1) : 0);
   static constexpr int M_TILE_BYTES = (SLOTS ? 2 * BM * 4 : 0) + (FUSED ? (NG - 1) * BM * 4 : 0);
-  static constexpr int SMEM_BYTES = 1024 + NS * A_TILE + NSB * B_TILE + EPI_STAGE + M_TILE_BYTES + NBAR * 8 + 64;
-  static_assert(E_COL0 + NS * BK <= TMEM_COLS, "TMEM capacity");
+  static constexpr int SMEM_BYTES = 1024 + NS * A_STAGE + NSB * B_TILE + EPI_STAGE + M_TILE_BYTES + NBAR * 8 + 64;
+  static_assert(E_COL0 + NS * E_COLS <= TMEM_COLS, "TMEM capacity");
   static_assert(SMEM_BYTES <= 232448, "shared memory capacity");
 };
 
@@ -93,6 +99,19 @@ __device__ __forceinline__ void umma_tf32_ts_pair(uint32_t d_tmem, uint32_t a_tm
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same with bf16 operands, 16 contraction values per MMA: a 32-bit TMEM column of A and a 32-bit word of B hold two.
+__device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                  uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
@@ -123,7 +142,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* a_base = smem;                     // ring 1: NS tiles of a
-  uint8_t* b_base = smem + NS * Cfg::A_TILE;  // ring 2: NSB tiles of b
+  uint8_t* b_base = smem + NS * Cfg::A_STAGE;  // ring 2: NSB tiles of b
   uint8_t* epi_stage = b_base + NSB * Cfg::B_TILE;  // 4 warps x 4 KB staging boxes, 1024-byte aligned
   float* m_tile = reinterpret_cast<float*>(epi_stage + Cfg::EPI_STAGE);  // OPT: [2][BM] stabilisers of two tiles
   uint64_t* bars = reinterpret_cast<uint64_t*>(epi_stage + Cfg::EPI_STAGE + Cfg::M_TILE_BYTES);
@@ -148,14 +167,14 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   const bool leader = rank == 0;
   const AbortCtl ctl{abort_flag, p.status};
 
-  auto a_tile = [&](int s) -> uint8_t* { return a_base + s * Cfg::A_TILE; };
+  auto a_tile = [&](int s) -> uint8_t* { return a_base + s * Cfg::A_STAGE; };
   auto b_tile = [&](int s) -> uint8_t* { return b_base + s * Cfg::B_TILE; };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < NS; ++s) {
       mbar_init(&a_full[s], 1);
-      mbar_init(&xf_done[s], 2 * 4 + 2);  // four transform warps (one per lane quarter) and the a-tile watcher, in each CTA
+      mbar_init(&xf_done[s], 2 * 4 + (Cfg::PREC ? 0 : 2));  // four transform warps (one per lane quarter) and the a-tile watcher, in each CTA
       mbar_init(&stage_empty[s], 1);
     }
     for (int s = 0; s < NSB; ++s) {
@@ -256,7 +275,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (leader && lane == 0) {
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
       constexpr uint32_t idesc = umma_idesc_tf32(2 * BM, BN);
-      constexpr uint32_t STAGE_ENC = Cfg::A_TILE >> 4;
+      constexpr uint32_t STAGE_ENC = Cfg::A_STAGE >> 4;
       const uint64_t db0 = umma_desc_k_sw128(smem_u32(a_tile(0)));
       const uint32_t d = tmem_base;
       uint32_t s = 0, ph = 0, tcount = 0;
@@ -271,10 +290,16 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           TB200_TL(0, tcount * KB + kb);
           tc_fence_after_sync();
           const uint64_t db = db0 + s * STAGE_ENC;
-          const uint32_t ea = tmem_base + Cfg::E_COL0 + s * BK;
+          const uint32_t ea = tmem_base + Cfg::E_COL0 + s * Cfg::E_COLS;
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks)
             umma_tf32_ts_pair(d, ea + ks * 8, db + 2 * ks, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+          if (Cfg::PREC) {
+            // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands
+#pragma unroll
+            for (int ks = 0; ks < BK / 8; ++ks)
+              umma_bf16_ts_pair(d, ea + BK + ks * 8, db + (Cfg::A_TILE >> 4) + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
+          }
           // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
           umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
           TB200_TL(1, tcount * KB + kb);
@@ -287,8 +312,9 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       }
     }
     __syncwarp();
-  } else if (warp == 3) {
+  } else if (warp == 3 && !Cfg::PREC) {
     // ------------------------------------------------------------------ a-tile watcher
+    // (3xTF32: the transform warps read the tile of a themselves)
     // The leader's MMA thread reads both CTAs' tiles of a and waits only on xf_done: this lane adds "this CTA's
     // tile of a has landed" to that barrier, so that the transform warps need not wait for it in their chain.
     if (lane == 0) {
@@ -315,7 +341,8 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     pdl_wait();  // m comes from the pre-pass, which may still be running when this kernel starts
     uint32_t tcount = 0;
     bool ok = true;
-    uint32_t acc_max = 0;  // OPT: largest accumulator bit pattern of this lane (sums of non-negative products, so
+    const bool opt = Cfg::OPT || (Cfg::PREC && p.opt_flag != nullptr);  // PREC: pre-pass over the first 32 rows only
+    uint32_t acc_max = 0;  // opt: largest accumulator bit pattern of this lane (sums of non-negative products, so
                            // +inf and NaN are exactly the patterns >= 0x7f800000 read as unsigned)
     for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
       int r, n0, i0;
@@ -375,8 +402,9 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
               __syncwarp();
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
-                const float o = m + lg2_approx(__uint_as_float(v[h][e])) * LN2_F;
-                if (Cfg::OPT) acc_max = max(acc_max, v[h][e]);
+                const float acc = __uint_as_float(v[h][e]);
+                const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
+                if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
                 *reinterpret_cast<float*>(stg + sw128_offset(e, lane)) = o;
               }
               fence_proxy_async_smem();
@@ -391,8 +419,9 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
               const int nrows = min(32, p.I - ib);
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
-                const float o = m + lg2_approx(__uint_as_float(v[h][e])) * LN2_F;
-                if (Cfg::OPT) acc_max = max(acc_max, v[h][e]);
+                const float acc = __uint_as_float(v[h][e]);
+                const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
+                if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
                 if (col_ok && e < nrows) orow[static_cast<int64_t>(e) * p.out_s1] = o;
               }
             }
@@ -402,7 +431,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (warp == 4 && lane == 0) TB200_TL(8, tcount);
     }
     if (use_tma && lane == 0) tma_store_wait_all();  // shared memory must outlive the last box
-    if (Cfg::OPT) {
+    if (opt) {
       if (__any_sync(0xffffffffu, acc_max >= 0x7f800000u) && lane == 0) *p.opt_flag = 1;
     }
   } else if (warp >= 8) {
@@ -516,7 +545,12 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (lane == 0) mbar_arrive(&m_ready[mslot]);
         }
         uint32_t e[32];
-        if (jrem >= BK) {
+        uint32_t pk[Cfg::PREC ? 32 : 1];
+        if (Cfg::PREC) {
+#pragma unroll
+          for (int x = 0; x < 32; ++x)
+            tf32_split_pack_rn(exp_shifted(x < jrem ? v[x] : -INFINITY, m), e[x], pk[Cfg::PREC ? x : 0]);
+        } else if (jrem >= BK) {
 #pragma unroll
           for (int x = 0; x < 32; ++x) e[x] = tf32_round_bits(exp_shifted(v[x], m));
         } else {
@@ -532,7 +566,21 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (!(ok = mbar_wait_warp(&stage_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
         if (warp == 8 && lane == 0) TB200_TL(4, it);
         tc_fence_after_sync();
-        tmem_st_32x32(ebase + s * BK, e);
+        tmem_st_32x32(ebase + s * Cfg::E_COLS, e);
+        if constexpr (Cfg::PREC != 0) {
+          tmem_st_32x32(ebase + s * Cfg::E_COLS + BK, pk);
+          // the tile of a stays as it is (the tensor core drops the low 13 bits); its corrections go to the second tile
+          if (!(ok = mbar_wait_warp(&a_full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+          const float4* raw = reinterpret_cast<const float4*>(a_tile(s)) + kl;
+          uint4* pack = reinterpret_cast<uint4*>(a_tile(s) + Cfg::A_TILE) + kl;
+#pragma unroll
+          for (int c = 0; c < Cfg::A_TILE / 16 / 128; ++c) {
+            const float4 w = raw[c * 128];
+            pack[c * 128] = make_uint4(tf32_corrections_trunc(w.x), tf32_corrections_trunc(w.y),
+                                       tf32_corrections_trunc(w.z), tf32_corrections_trunc(w.w));
+          }
+          fence_proxy_async_smem();
+        }
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
