@@ -748,10 +748,10 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   p.fused_max = fused ? 1 : 0;
   p.status = status_dev;
 
-  // The TMEM-operand pair kernel takes a with j contiguous and does not fold column maxima of the result; other
-  // calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
+  // The TMEM-operand pair kernel takes a with j contiguous and, in plain TF32, does not fold column maxima of the result;
+  // other calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
   // columns k, unswizzled (only the transform threads read them).
-  const bool use_ts = (plan.tspair || (pair && precision == TRITURUS_B200_PRECISION_3XTF32)) && !a_mn && out_colmax == nullptr;
+  const bool use_ts = !a_mn && ((plan.tspair && out_colmax == nullptr) || (pair && precision == TRITURUS_B200_PRECISION_3XTF32));
   CUtensorMap tb_plain;
   if (use_ts) {
     const int64_t dims[3] = {K, J, R};

@@ -353,6 +353,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       float m = 0.f;
       if (!Cfg::SLOTS && col_ok) m = clamp_stab(__ldg(p.m_ws + static_cast<int64_t>(r) * p.K + kcol));
       float* ocol = p.out + static_cast<int64_t>(r) * p.out_s0 + kcol;
+      float cmx = -INFINITY;  // PREC: largest result of this lane's column in the tile, for the next layer of a chain
       if (!(ok = mbar_wait_warp(acc_full, tcount & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
       if (warp == 4 && lane == 0) TB200_TL(7, tcount);
       tc_fence_after_sync();
@@ -405,6 +406,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 const float acc = __uint_as_float(v[h][e]);
                 const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
                 if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
+                if (Cfg::PREC) cmx = fmaxf(cmx, o);  // (rows past I hold log 0 = -inf)
                 *reinterpret_cast<float*>(stg + sw128_offset(e, lane)) = o;
               }
               fence_proxy_async_smem();
@@ -422,6 +424,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 const float acc = __uint_as_float(v[h][e]);
                 const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
                 if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
+                if (Cfg::PREC) cmx = fmaxf(cmx, o);  // (rows past I hold log 0 = -inf)
                 if (col_ok && e < nrows) orow[static_cast<int64_t>(e) * p.out_s1] = o;
               }
             }
@@ -429,6 +432,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         }
       }
       if (warp == 4 && lane == 0) TB200_TL(8, tcount);
+      if (Cfg::PREC && p.out_max != nullptr && col_ok) red_max_f32(p.out_max + static_cast<int64_t>(r) * p.K + kcol, cmx);
     }
     if (use_tma && lane == 0) tma_store_wait_all();  // shared memory must outlive the last box
     if (opt) {
