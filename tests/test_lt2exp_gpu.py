@@ -441,3 +441,28 @@ def test_strided_views_of_a_and_b_are_read_in_place(precision, variant):
     tb.check_status()
     res = orc.compare_logspace(got.cpu(), orc.lt2exp_fp64(w, a_v.cpu().contiguous(), b_b.cpu().contiguous()), ATOL[precision])
     assert res["ok"], res
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 128, 31, 20, 128), (2, 130, 32, 32, 129), (1, 127, 33, 33, 200),
+                                   (2, 40, 7, 300, 90), (1, 200, 100, 64, 260), (1, 128, 256, 256, 130)])
+@pytest.mark.parametrize("split", [1, 3, 9998])
+def test_3xtf32_on_the_tmem_operand_kernel(shape, split):
+    """3xTF32 with the generated operand in tensor memory (hi * hi in tf32, the corrections in bf16): k-blocks around the
+    chunks of 32 after which the accumulator is re-summed, rows and columns around the 128 of a tile, whole tiles, added
+    slices and parts completed through scratch memory.  Tolerance: 2^-17 for the split, 1.2e-8 per term of a chunk of 1 024
+    for the tensor core's truncating additions, the rounding of two exponents' arguments (2^-23 of about 30 each)
+    and of the result."""
+    R, S, I, J, K = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    w = torch.rand(R, S, I, J, generator=g) + 1e-3
+    a = torch.randn(R, I, K, generator=g) * 4.0 + 50.0 * torch.randn(R, 1, K, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0
+    if K > 1:
+        a[torch.rand(R, I, K, generator=g) < 0.02] = float("-inf")
+        b[0, :, K // 2] = float("-inf")
+    got = _run(w, a, b, precision="3xtf32", variant=split * 10000 + 1281)
+    want = orc.lt2exp_fp64(w, a, b, chunk=1)
+    assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
+    fin = torch.isfinite(want)
+    tol = 2.0**-17 + 1.2e-8 * 1024 + 60 * 2.0**-23 + 2.0**-22 * want[fin].abs()
+    assert ((got[fin].double() - want[fin]).abs() <= tol).all()

@@ -291,7 +291,6 @@ using LmPlainT = Lm2expCfg<128, 2, 0, 4, false, true>;
 using LmPlainX = Lm2expCfg<128, 2, 1, 2, true, true>;
 
 using LmPairT = Lm2expPairCfg<0, 6>;
-using LmPairX = Lm2expPairCfg<1, 3>;
 
 // Launch on CTA pairs: a cluster of two CTAs per 256 x 256 tile.
 template <class Cfg>
@@ -748,10 +747,10 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   p.fused_max = fused ? 1 : 0;
   p.status = status_dev;
 
-  // The TMEM-operand pair kernel takes a with j contiguous and, in plain TF32, does not fold column maxima of the result;
-  // other calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
+  // The TMEM-operand pair kernel in plain TF32 takes a with j contiguous only and does not fold column maxima of the
+  // result; other calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
   // columns k, unswizzled (only the transform threads read them).
-  const bool use_ts = !a_mn && ((plan.tspair && out_colmax == nullptr) || (pair && precision == TRITURUS_B200_PRECISION_3XTF32));
+  const bool use_ts = (plan.tspair && !a_mn && out_colmax == nullptr) || (pair && precision == TRITURUS_B200_PRECISION_3XTF32);
   CUtensorMap tb_plain;
   if (use_ts) {
     const int64_t dims[3] = {K, J, R};
@@ -787,16 +786,14 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     Lm2expParams po = p;
     po.opt_flag = flag;
     rc = use_ts ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, po, st, true)
-         : precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, po, st, true)
-                                                       : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
+                : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
     if (rc != TRITURUS_B200_OK) return rc;
     rc = colmax_run(b, m_buf, R, J, K, bstr, stream, flag, flag + 1);
     if (rc != TRITURUS_B200_OK) return rc;
     p.only_if = flag + 1;
     p.reset_flag = flag;
-    if (use_ts) return launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, true);
-    return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, p, st, true)
-                                                        : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, true);
+    return use_ts ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, true)
+                  : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, true);
   }
   if (prepass && b_km) {
     for (int64_t r0 = 0; r0 < R; r0 += 65535) {  // (R <= 65535 here: one round)
@@ -812,10 +809,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   if (use_ts)
     return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, dep)
                                                         : launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
-  if (pair) {
-    return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_pair<LmPairX>(ta, tb, to, p, st, dep)
-                                                        : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, dep);
-  }
+  if (pair) return launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, dep);
   auto single = [&](const Lm2expParams& q, bool dependent) -> int {
     if (b_km || gen_a || gen_b) {
       if (precision == TRITURUS_B200_PRECISION_3XTF32) {
@@ -1148,23 +1142,24 @@ static int launch_lt2exp(const CUtensorMap& tw, Lt2expParams p, const LtLaunch& 
   return launch_lt2exp_with<Cfg, lt2exp_kernel<Cfg>, true>(tw, p, L);
 }
 
-// (the kernels that keep the generated operand in tensor memory complete shared tiles with additions only)
+// (of the kernels that keep the generated operand in tensor memory, those in plain TF32 complete shared tiles with
+// additions only)
 template <class Cfg>
 static int launch_lt2exp_tmem(const CUtensorMap& tw, Lt2expParams p, const LtLaunch& L) {
-  return launch_lt2exp_with<Cfg, lt2exp_tmem_kernel<Cfg>, false>(tw, p, L);
+  return launch_lt2exp_with<Cfg, lt2exp_tmem_kernel<Cfg>, Cfg::PREC != 0>(tw, p, L);
 }
 
 //                              MT NS   (generated operand in TMEM, 128 columns k per tile, TF32)
 using LtM_1 = Lt2expTmemCfg<1, 8>;
 using LtM_2 = Lt2expTmemCfg<2, 6>;
 using LtM_1x2 = Lt2expTmemCfg<1, 4, 2>;  // 128 rows x two 128-column blocks sharing each w tile
+using LtMX_1 = Lt2expTmemCfg<1, 4, 1, 1>;  // 3xTF32, 128 x 128
 
 //                          BN   MT PREC NS NTW
 using LtT_128_1 = Lt2expCfg<128, 1, 0, 6, 8>;
 using LtT_128_2 = Lt2expCfg<128, 2, 0, 4, 8>;
 using LtT_256_1 = Lt2expCfg<256, 1, 0, 4, 8>;
 using LtT_256_2 = Lt2expCfg<256, 2, 0, 3, 8>;
-using LtX_128_1 = Lt2expCfg<128, 1, 1, 3, 8>;
 using LtX_128_2 = Lt2expCfg<128, 2, 1, 2, 8>;
 using LtX_256_1 = Lt2expCfg<256, 1, 1, 2, 8>;
 // plain TF32 with chunked re-summation of the accumulator (contractions of more than 32 K terms)
@@ -1189,6 +1184,7 @@ static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int6
     // 128 rows x 256 columns in TF32: the kernel that keeps the generated operand in TMEM moves a third of
     // the shared-memory bytes per k-block (measured 8 % faster on such tiles).
     if (tile == 2561 && precision == TRITURUS_B200_PRECISION_TF32 && !long_tf) tile = 1285;
+    if (precision == TRITURUS_B200_PRECISION_3XTF32) tile = 1281;
   }
   *bn = tile / 10;
   *mt = tile % 10;
@@ -1224,7 +1220,7 @@ static int lt2exp_dispatch(int precision, int bn, int mt, bool promote, Args... 
   }
   if (precision == TRITURUS_B200_PRECISION_3XTF32) {
     if (bn == 256 && mt == 1) return launch_lt2exp<LtX_256_1>(args...);
-    return mt == 2 ? launch_lt2exp<LtX_128_2>(args...) : launch_lt2exp<LtX_128_1>(args...);
+    return mt == 2 ? launch_lt2exp<LtX_128_2>(args...) : launch_lt2exp_tmem<LtMX_1>(args...);
   }
   if (bn == 256) return mt == 2 ? launch_lt2exp<LtT_256_2>(args...) : launch_lt2exp<LtT_256_1>(args...);
   return mt == 2 ? launch_lt2exp<LtT_128_2>(args...) : launch_lt2exp<LtT_128_1>(args...);

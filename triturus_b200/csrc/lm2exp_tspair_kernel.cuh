@@ -67,7 +67,8 @@ struct Lm2expTsPairCfg {
   static constexpr int ACC_COLS = BN;
   static constexpr int E_COL0 = ACC_COLS;  // first TMEM column of the operand stages
   static constexpr int TMEM_COLS = 512;
-  static constexpr int NTHREADS = (8 + NTW) * 32;
+  static constexpr int NPW = PREC_ ? 4 : 0;  // PREC: warps that write the packed words of a (behind the transform warps)
+  static constexpr int NTHREADS = (8 + NTW + NPW) * 32;
   static constexpr int EPI_STAGE = 4 * 2 * 32 * 128;  // per epilogue warp two 32 x 32 fp32 boxes
   // OPT: no stabiliser pre-pass.  The stabiliser of a column is the maximum over its first k-block (32 rows j),
   // found by the transform warp that handles that k-block and handed to the other roles through shared memory
@@ -115,6 +116,20 @@ __device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tm
       "}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// pack_tile_corrections (ptx.cuh) for a transposed a: the tile holds four boxes of 32 i x 32 j, i contiguous; the packed
+// words are written K-major like those of an ordinary tile.  Thread t of 128 takes row i = t.
+__device__ __forceinline__ void pack_tile_corrections_mn(const uint8_t* tile, uint8_t* packed, int t) {
+  const uint8_t* box = tile + (t >> 5) * 4096 + (t & 3) * 4;
+#pragma unroll 2
+  for (int g = 0; g < 8; ++g) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      w[e] = tf32_corrections_trunc(*reinterpret_cast<const float*>(box + sw128_base32_offset(g * 4 + e, (t & 31) >> 2)));
+    *reinterpret_cast<uint4*>(packed + sw128_offset(t, g * 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 template <class Cfg>
@@ -174,7 +189,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     *abort_flag = 0;
     for (int s = 0; s < NS; ++s) {
       mbar_init(&a_full[s], 1);
-      mbar_init(&xf_done[s], 2 * 4 + (Cfg::PREC ? 0 : 2));  // four transform warps (one per lane quarter) and the a-tile watcher, in each CTA
+      mbar_init(&xf_done[s], 2 * 4 + 2 * (Cfg::PREC ? Cfg::NPW : 1));  // four transform warps (one per lane quarter) and the a-tile watcher (PREC: the packing warps), in each CTA
       mbar_init(&stage_empty[s], 1);
     }
     for (int s = 0; s < NSB; ++s) {
@@ -240,7 +255,12 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (!(ok = mbar_wait(&stage_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_PRODUCER))) break;
           TB200_TL(9, it);
           mbar_arrive_expect_tx(&a_full[s], Cfg::A_TILE);
-          tma_load_3d(a_tile(s), &tmap_a, &a_full[s], kb * BK, my_i0, r);
+          if (Cfg::PREC && p.a_mn) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) tma_load_3d(a_tile(s) + g * 4096, &tmap_a, &a_full[s], my_i0 + g * 32, kb * BK, r);
+          } else {
+            tma_load_3d(a_tile(s), &tmap_a, &a_full[s], kb * BK, my_i0, r);
+          }
         }
       }
       // The leader's commits arrive on both CTAs' stage_empty barriers: this CTA stays until the last ones are in.
@@ -274,9 +294,13 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     // ------------------------------------------------------------------ pair MMA issuer (leader CTA only)
     if (leader && lane == 0) {
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
-      constexpr uint32_t idesc = umma_idesc_tf32(2 * BM, BN);
+      // PREC takes a transposed a too: MN-major for the tf32 MMAs (bit 16), while its packed words are always K-major.
+      const bool a_mn = Cfg::PREC && p.a_mn != 0;
+      const uint32_t idesc = umma_idesc_tf32(2 * BM, BN) | (a_mn ? 1u << 16 : 0u);
+      const uint32_t a_step = a_mn ? 64u : 2u;  // encoded address step per 8 contraction values
       constexpr uint32_t STAGE_ENC = Cfg::A_STAGE >> 4;
-      const uint64_t db0 = umma_desc_k_sw128(smem_u32(a_tile(0)));
+      const uint64_t db0 = a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0)), 4096) : umma_desc_k_sw128(smem_u32(a_tile(0)));
+      const uint64_t dbp0 = umma_desc_k_sw128(smem_u32(a_tile(0)) + Cfg::A_TILE);
       const uint32_t d = tmem_base;
       uint32_t s = 0, ph = 0, tcount = 0;
       bool ok = true;
@@ -293,12 +317,12 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           const uint32_t ea = tmem_base + Cfg::E_COL0 + s * Cfg::E_COLS;
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks)
-            umma_tf32_ts_pair(d, ea + ks * 8, db + 2 * ks, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+            umma_tf32_ts_pair(d, ea + ks * 8, db + a_step * ks, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
           if (Cfg::PREC) {
             // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands
 #pragma unroll
             for (int ks = 0; ks < BK / 8; ++ks)
-              umma_bf16_ts_pair(d, ea + BK + ks * 8, db + (Cfg::A_TILE >> 4) + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
+              umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + s * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
           }
           // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
           umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
@@ -314,7 +338,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     __syncwarp();
   } else if (warp == 3 && !Cfg::PREC) {
     // ------------------------------------------------------------------ a-tile watcher
-    // (3xTF32: the transform warps read the tile of a themselves)
+    // (3xTF32: the packing warps wait for the tile of a)
     // The leader's MMA thread reads both CTAs' tiles of a and waits only on xf_done: this lane adds "this CTA's
     // tile of a has landed" to that barrier, so that the transform warps need not wait for it in their chain.
     if (lane == 0) {
@@ -438,6 +462,24 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     if (opt) {
       if (__any_sync(0xffffffffu, acc_max >= 0x7f800000u) && lane == 0) *p.opt_flag = 1;
     }
+  } else if (Cfg::PREC && warp >= 8 + Cfg::NTW) {
+    // ------------------------------------------------------------------ packing: the corrections of the tile of a
+    // The tile itself stays as it is (the tensor core drops the low 13 bits).
+    const int t = threadIdx.x - (8 + Cfg::NTW) * 32;
+    const uint32_t xf_done_leader0 = map_to_cta(smem_u32(&xf_done[0]), 0);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = pair; ok && tile < p.num_tiles; tile += npairs) {
+      for (int kb = 0; kb < KB; ++kb, ++it) {
+        const int s = it % NS;
+        if (!(ok = mbar_wait_warp(&a_full[s], (it / NS) & 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+        if (p.a_mn) pack_tile_corrections_mn(a_tile(s), a_tile(s) + Cfg::A_TILE, t);
+        else pack_tile_corrections(a_tile(s), a_tile(s) + Cfg::A_TILE, t);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(xf_done_leader0 + static_cast<uint32_t>(s) * 8u);
+      }
+    }
   } else if (warp >= 8) {
     // ------------------------------------------------------------------ transform: b tile -> E^T in tensor memory
     const int q = warp & 3;         // TMEM lane quarter this warp may write
@@ -549,11 +591,11 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (lane == 0) mbar_arrive(&m_ready[mslot]);
         }
         uint32_t e[32];
-        uint32_t pk[Cfg::PREC ? 32 : 1];
         if (Cfg::PREC) {
+          // (the exps stay in fp32 until the stage is free and are split there, 16 at a time: both words of all 32 do not
+          // fit in the 96 registers of a thread)
 #pragma unroll
-          for (int x = 0; x < 32; ++x)
-            tf32_split_pack_rn(exp_shifted(x < jrem ? v[x] : -INFINITY, m), e[x], pk[Cfg::PREC ? x : 0]);
+          for (int x = 0; x < 32; ++x) e[x] = __float_as_uint(exp_shifted(x < jrem ? v[x] : -INFINITY, m));
         } else if (jrem >= BK) {
 #pragma unroll
           for (int x = 0; x < 32; ++x) e[x] = tf32_round_bits(exp_shifted(v[x], m));
@@ -570,20 +612,17 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (!(ok = mbar_wait_warp(&stage_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
         if (warp == 8 && lane == 0) TB200_TL(4, it);
         tc_fence_after_sync();
-        tmem_st_32x32(ebase + s * Cfg::E_COLS, e);
         if constexpr (Cfg::PREC != 0) {
-          tmem_st_32x32(ebase + s * Cfg::E_COLS + BK, pk);
-          // the tile of a stays as it is (the tensor core drops the low 13 bits); its corrections go to the second tile
-          if (!(ok = mbar_wait_warp(&a_full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-          const float4* raw = reinterpret_cast<const float4*>(a_tile(s)) + kl;
-          uint4* pack = reinterpret_cast<uint4*>(a_tile(s) + Cfg::A_TILE) + kl;
 #pragma unroll
-          for (int c = 0; c < Cfg::A_TILE / 16 / 128; ++c) {
-            const float4 w = raw[c * 128];
-            pack[c * 128] = make_uint4(tf32_corrections_trunc(w.x), tf32_corrections_trunc(w.y),
-                                       tf32_corrections_trunc(w.z), tf32_corrections_trunc(w.w));
+          for (int h = 0; h < 2; ++h) {
+            uint32_t hi[16], pk[16];
+#pragma unroll
+            for (int x = 0; x < 16; ++x) tf32_split_pack_rn(__uint_as_float(e[h * 16 + x]), hi[x], pk[x]);
+            tmem_st_32x16(ebase + s * Cfg::E_COLS + h * 16, hi);
+            tmem_st_32x16(ebase + s * Cfg::E_COLS + BK + h * 16, pk);
           }
-          fence_proxy_async_smem();
+        } else {
+          tmem_st_32x32(ebase + s * Cfg::E_COLS, e);
         }
         tmem_st_wait();
         tc_fence_before_sync();

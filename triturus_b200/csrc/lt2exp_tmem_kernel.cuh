@@ -33,49 +33,73 @@
 
 namespace tb200 {
 
-template <int MT_, int NS_, int NB_ = 1>
+// PREC (3xTF32): hi * hi as tf32 MMAs and the two corrections as bf16 MMAs at twice the rate on packed words
+// (tf32_split_pack_rn in ptx.cuh).  The w tile serves the tf32 MMAs as it lies in shared memory (the tensor core
+// truncates); four packing warps (16-19) write its packed words to a second tile, the transform warps P^T and its packed
+// words to 64 TMEM columns.  (With the packing in the transform warps a k-block took 960 cycles: their chain of waits,
+// arithmetic and fences was what bounded it, tensor pipe 53 % and shared-memory pipe 60 % active.)
+// Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the packing, 32 KB read by the tensor
+// core = 640 cycles of the shared-memory pipe next to 512 of the tensor pipe (all operands in shared memory and three
+// tf32 products: 1 400 next to 768).
+// Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
+// master copy in shared memory (see "Accumulator promotion" in lt2exp_kernel.cuh; TMEM has no room for a third).
+template <int MT_, int NS_, int NB_ = 1, int PREC_ = 0>
 struct Lt2expTmemCfg {
   static constexpr int BM = 128, BK = 32;  // BM: rows s per w box
   static constexpr int NB = NB_;           // 128-column blocks per tile: each is one M = 128 MMA on the same w tile
   static constexpr int BN = 128 * NB;      // columns k per tile
-  static constexpr int MT = MT_, NS = NS_, PREC = 0, NTW = 8;
-  static constexpr bool PROMOTE = false;  // no chunked re-summation of the accumulator in these kernels
-  static constexpr int CHUNK = 1 << 30;
+  static constexpr int MT = MT_, NS = NS_, PREC = PREC_, NTW = 8;
+  static constexpr bool PROMOTE = PREC != 0;  // chunked re-summation of the accumulator
+  static constexpr int CHUNK = PROMOTE ? 32 : 1 << 30;
   static constexpr int W_TILE = BM * BK * 4;
-  static constexpr int STAGE = MT * W_TILE;
+  static constexpr int W_BYTES = MT * W_TILE;             // what TMA brings per stage
+  static constexpr int STAGE = (PREC ? 2 : 1) * W_BYTES;  // ... and the packed words of it
   static constexpr int BLK_COLS = MT * BM;        // accumulator columns of one column block
   static constexpr int ACC_COLS = NB * BLK_COLS;
-  static constexpr int P_STAGE = NB * BK;         // operand columns per stage
+  static constexpr int P_STAGE = NB * (PREC ? 2 : 1) * BK;  // operand columns per stage
   static constexpr int NBUF = (2 * ACC_COLS + NS * P_STAGE <= 512) ? 2 : 1;
   static constexpr int P_COL0 = NBUF * ACC_COLS;  // first operand column
   static constexpr int TMEM_USED = P_COL0 + NS * P_STAGE;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int NTHREADS = (8 + NTW) * 32;
+  static constexpr int NPW = PREC ? 4 : 0;  // packing warps
+  static constexpr int NTHREADS = (8 + NTW + NPW) * 32;
   static constexpr int NTT = NTW * 32;
   static constexpr int NGROUPS = NTT / BN;
   static constexpr int CQ = BN / 4;
   static constexpr int RG = NTT / CQ;
   static constexpr int MPART = 2 * RG * BN;
   static constexpr int NBAR = 3 * NS + 7;
-  static constexpr int SMEM_BYTES = 1024 + NS * STAGE + 2 * BN * 4 + 2 * MPART * 4 + NBAR * 8 + 64;
+  static constexpr int MASTER = PROMOTE ? MT * BM * BN * 4 : 0;
+  static_assert(!PREC || (MT == 1 && NB == 1 && NBUF == 2), "3xTF32: 128 x 128 tiles, two accumulators");
+  static constexpr int SMEM_BYTES = 1024 + NS * STAGE + MASTER + 2 * BN * 4 + 2 * MPART * 4 + NBAR * 8 + 64;
   static_assert(TMEM_USED <= 512, "TMEM capacity");
   static_assert(NGROUPS * NB == 2, "eight transform warps: two groups on one column block, or one group on two");
   static_assert(SMEM_BYTES <= 232448, "shared memory capacity");
 };
 
+__device__ __forceinline__ void add_quad(uint32_t (&v)[32], int g, float4 x) {
+  v[g * 4 + 0] = __float_as_uint(__uint_as_float(v[g * 4 + 0]) + x.x);
+  v[g * 4 + 1] = __float_as_uint(__uint_as_float(v[g * 4 + 1]) + x.y);
+  v[g * 4 + 2] = __float_as_uint(__uint_as_float(v[g * 4 + 2]) + x.z);
+  v[g * 4 + 3] = __float_as_uint(__uint_as_float(v[g * 4 + 3]) + x.w);
+}
+
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::NTHREADS, 1)
 lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, MT = Cfg::MT, NS = Cfg::NS;
-  constexpr int PF = 8;  // prefetch distance (own k-blocks) for the a values
+  constexpr int PF = Cfg::PREC ? 4 : 8;  // prefetch distance (own k-blocks) for the a values
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stage_base = smem;
-  float* msum = reinterpret_cast<float*>(smem + NS * Cfg::STAGE);  // [2][BN]: ma + mb of the tile's columns
+  // PROMOTE: [BM / 4 row quads][128 columns][4] master copy of the accumulator, each thread its own column
+  float4* master = reinterpret_cast<float4*>(smem + NS * Cfg::STAGE);
+  float* msum = reinterpret_cast<float*>(smem + NS * Cfg::STAGE + Cfg::MASTER);  // [2][BN]: ma + mb of the tile's columns
   float* mpart = msum + 2 * BN;                                    // [2][2][RG][BN] partial column maxima
   uint64_t* bars = reinterpret_cast<uint64_t*>(mpart + 2 * Cfg::MPART);
   uint64_t* full = bars;                 // [NS] w tile landed (TMA bytes) and operand stage written to TMEM
+  uint64_t* w_full = bars + NS;          // PREC [NS] w tile landed (the packing warps wait for it)
   uint64_t* opnd_empty = bars + 2 * NS;  // [NS] MMAs reading the stage (shared memory and TMEM) retired
   uint64_t* acc_full = bars + 3 * NS;    // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
@@ -91,7 +115,9 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int s = 0; s < NS; ++s) {
-      mbar_init(&full[s], 1 + Cfg::NTW / Cfg::NGROUPS);  // the producer and the warps that write the operand stage
+      if (Cfg::PREC) mbar_init(&w_full[s], 1);
+      // the producer (PREC: the packing warps instead) and the warps that write the operand stage
+      mbar_init(&full[s], (Cfg::PREC ? Cfg::NPW : 1) + Cfg::NTW / Cfg::NGROUPS);
       mbar_init(&opnd_empty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -114,7 +140,8 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
 
   const int JC = (p.J + BK - 1) / BK;
   const int KBT = JC * p.I;  // k-blocks per output tile
-  const bool split_mode = p.nsplit > 1 || p.stream != 0;
+  const bool parking = Cfg::PROMOTE && p.stream != 0 && p.park != nullptr;  // shared tiles are completed through scratch memory
+  const bool split_mode = (p.nsplit > 1 || p.stream != 0) && !parking;
 
   // Output tile -> (r, n0 = first column k, s0 = first row s); the items of a CTA come from LtWork.
   auto decode = [&](int tile, int& r, int& n0, int& s0) {
@@ -141,10 +168,11 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
             const int s = it % NS;
             const uint32_t ph = (it / NS) & 1;
             if (!(ok = mbar_wait(&opnd_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_PRODUCER))) break;
-            mbar_arrive_expect_tx(&full[s], Cfg::STAGE);
+            uint64_t* landed = Cfg::PREC ? &w_full[s] : &full[s];
+            mbar_arrive_expect_tx(landed, Cfg::W_BYTES);
 #pragma unroll
             for (int t = 0; t < MT; ++t)
-              tma_load_4d(stage_base + s * Cfg::STAGE + t * Cfg::W_TILE, &tmap_w, &full[s], jc * BK, i, s0 + t * BM, r);
+              tma_load_4d(stage_base + s * Cfg::STAGE + t * Cfg::W_TILE, &tmap_w, landed, jc * BK, i, s0 + t * BM, r);
           }
         }
       }
@@ -160,19 +188,21 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     {
       constexpr uint32_t idesc = umma_idesc_tf32(128, BM * MT);  // M = 128 columns k, N = rows s
       const uint32_t stage0 = smem_u32(stage_base);
-      uint32_t tcount = 0;
+      uint32_t ccount = 0;  // accumulation chunks issued so far (one per work item unless PROMOTE)
       int s = 0;
       uint32_t ph = 0;
       bool ok = true, ready = false;
       LtWork work(p, KBT);
-      for (LtItem w; ok && work.next(w); ++tcount) {
-        const int KB = w.kb_hi - w.kb_lo;
-        const int buf = tcount % Cfg::NBUF;
-        const uint32_t aph = (tcount / Cfg::NBUF) & 1;
+      for (LtItem w; ok && work.next(w);) {
+       const int KB = w.kb_hi - w.kb_lo;
+       for (int kb = 0; ok && kb < KB; ++ccount) {
+        const int kb0 = kb, kb_end = Cfg::PROMOTE ? min(KB, kb0 + Cfg::CHUNK) : KB;
+        const int buf = ccount % Cfg::NBUF;
+        const uint32_t aph = (ccount / Cfg::NBUF) & 1;
         if (!(ok = mbar_wait_warp(&acc_empty[buf], aph ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * Cfg::ACC_COLS;
-        for (int kb = 0; kb < KB; ++kb) {
+        for (; kb < kb_end; ++kb) {
           if (!ready) {
             if (!(ok = mbar_wait_warp(&full[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
           }
@@ -188,7 +218,13 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
 #pragma unroll
               for (int ks = 0; ks < BK / 8; ++ks)
                 umma_tf32_ts(d + blk * Cfg::BLK_COLS, pa + blk * BK + ks * 8, dw + 2 * ks, idesc,
-                             (kb > 0 || ks > 0) ? 1u : 0u);
+                             (kb > kb0 || ks > 0) ? 1u : 0u);
+            }
+            if (Cfg::PREC) {
+              // p_lo * w_hi + p_hi * w_lo: 64 bf16 values in rows of 128 bytes like the tf32 operands
+#pragma unroll
+              for (int ks = 0; ks < BK / 8; ++ks)
+                umma_bf16_ts(d, pa + BK + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, umma_idesc_bf16(128, BM * MT), 1u);
             }
             umma_commit(&opnd_empty[s]);
           }
@@ -198,6 +234,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
         }
         if (ok && elect_one_sync()) umma_commit(&acc_full[buf]);
         __syncwarp();
+       }
       }
     }
   } else if (warp >= 4 && warp < 8) {
@@ -207,6 +244,106 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     uint32_t tcount = 0;
     bool ok = true;
     LtWork work(p, KBT);
+    if constexpr (Cfg::PROMOTE) {
+      uint32_t ccount = 0;
+      const int kl = q * 32 + lane;  // this lane's column of the tile
+      for (LtItem w; ok && work.next(w); ++tcount) {
+        int r, n0, s0;
+        decode(w.tile, r, n0, s0);
+        const int kcol = n0 + kl;
+        const bool col_ok = kcol < p.K;
+        float* out_col = p.out + static_cast<int64_t>(r) * p.out_s0 + kcol;
+        const int slot = tcount & 1;
+        const int nch = (w.kb_hi - w.kb_lo + Cfg::CHUNK - 1) / Cfg::CHUNK;
+        const bool park_it = parking && w.park_slot >= 0;
+        const bool collect = parking && w.ncollect > 0;
+        constexpr int PARK_TILE = BM * BN;  // floats per parked tile, in the order of `master`
+        float cmx = -INFINITY;  // running maximum of this lane's column over the rows of the tile
+        for (int ch = 0; ok && ch < nch; ++ch, ++ccount) {
+          const int buf = ccount % Cfg::NBUF;
+          const bool first = ch == 0, last = ch == nch - 1;
+          if (!(ok = mbar_wait_warp(&acc_full[buf], (ccount / Cfg::NBUF) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
+          tc_fence_after_sync();
+          if (last && collect) {
+            // The other parts of the tile run at the same time on other CTAs and end about now.  (Not earlier: while
+            // this warp waits, no chunk is drained.)
+            for (int cc = 0; ok && cc < w.ncollect; ++cc) {
+              const long long t0 = clock64();
+              while (ld_acquire_gpu(p.park_flags + w.slot0 + cc) < 4) {
+                if (*ctl.flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
+                  raise_abort(ctl, STATUS_TIMEOUT_EPILOGUE);
+                  ok = false;
+                  break;
+                }
+              }
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+          }
+          const float m = msum[slot * BN + kl];
+#pragma unroll 1
+          for (int c = 0; c < BM / 32; ++c) {
+            const int sb = s0 + c * 32;
+            if (sb >= p.S) break;
+            uint32_t v[32];
+            tmem_ld_32x32(lane_base + buf * Cfg::ACC_COLS + c * 32, v);
+            float4* mst = master + c * 8 * 128 + kl;
+            tmem_ld_wait();
+            if (!first) {
+#pragma unroll
+              for (int g = 0; g < 8; ++g) add_quad(v, g, mst[g * 128]);
+            }
+            if (!last || park_it) {
+              float4* dst = last ? reinterpret_cast<float4*>(p.park + static_cast<int64_t>(w.park_slot) * PARK_TILE) + c * 8 * 128 + kl : mst;
+#pragma unroll
+              for (int g = 0; g < 8; ++g)
+                dst[g * 128] = make_float4(__uint_as_float(v[g * 4]), __uint_as_float(v[g * 4 + 1]),
+                                           __uint_as_float(v[g * 4 + 2]), __uint_as_float(v[g * 4 + 3]));
+              continue;
+            }
+            if (collect) {
+              for (int cc = 0; cc < w.ncollect; ++cc) {
+                const float4* src = reinterpret_cast<const float4*>(p.park + static_cast<int64_t>(w.slot0 + cc) * PARK_TILE) + c * 8 * 128 + kl;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) add_quad(v, g, __ldcg(src + g * 128));  // written during this launch: not through the read-only path
+              }
+            }
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              float* dst = out_col + static_cast<int64_t>(sb + e) * p.out_s1;
+              const bool valid = col_ok && sb + e < p.S;
+              const float acc = __uint_as_float(v[e]);
+              if (split_mode) {
+                if (valid) atomicAdd(dst, acc);
+              } else {
+                const float o = m + logf(acc);
+                if (valid) {
+                  *dst = o;
+                  cmx = fmaxf(cmx, o);
+                }
+              }
+            }
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&acc_empty[buf]);
+            if (last) mbar_arrive(&msum_empty[slot]);
+          }
+          if (park_it && last) {
+            // This warp's columns of the partial sums are written: publish them (one count per epilogue warp).
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) add_release_gpu(p.park_flags + w.park_slot, 1);
+          }
+        }
+        if (ok && p.out_max != nullptr && !split_mode && !park_it && col_ok) {
+          float* dst = p.out_max + static_cast<int64_t>(r) * p.K + kcol;
+          if (p.tiles_m == 1) *dst = cmx;
+          else red_max_f32(dst, cmx);
+        }
+      }
+    } else
     for (LtItem w; ok && work.next(w); ++tcount) {
       int r, n0, s0;
       decode(w.tile, r, n0, s0);
@@ -271,6 +408,26 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       if (lane == 0) {
         mbar_arrive(&acc_empty[buf]);
         mbar_arrive(&msum_empty[slot]);
+      }
+    }
+  } else if (Cfg::PREC && warp >= 8 + Cfg::NTW) {
+    // ------------------------------------------------------------------ packing: the corrections of the w tile
+    const int t = threadIdx.x - (8 + Cfg::NTW) * 32;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    LtWork work(p, KBT);
+    for (LtItem w; ok && work.next(w);) {
+      for (int kb = w.kb_lo; kb < w.kb_hi; ++kb) {
+        if (!(ok = mbar_wait_warp(&w_full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+        pack_tile_corrections(stage_base + s * Cfg::STAGE, stage_base + s * Cfg::STAGE + Cfg::W_BYTES, t);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[s]);
+        if (++s == NS) {
+          s = 0;
+          ph ^= 1;
+        }
       }
     }
   } else if (warp >= 8) {
@@ -377,6 +534,23 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
             const int s = my_it % NS;
             const uint32_t ph = (my_it / NS) & 1;
             const float ea = exp_shifted(acur[x], ma);
+            if constexpr (Cfg::PREC != 0) {
+              if (!(ok = mbar_wait_warp(&opnd_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+              tc_fence_after_sync();
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {  // 16 of the 32 terms at a time: both words of all 32 do not fit in registers
+                uint32_t hi[16], pk[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) tf32_split_pack_rn(ea * eb[h * 16 + e], hi[e], pk[e]);
+                tmem_st_32x16(lane_base + s * Cfg::P_STAGE + h * 16, hi);
+                tmem_st_32x16(lane_base + s * Cfg::P_STAGE + BK + h * 16, pk);
+              }
+              tmem_st_wait();
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&full[s]);
+              continue;
+            }
             uint32_t pv[32];
 #pragma unroll
             for (int e = 0; e < 32; ++e) pv[e] = tf32_round_bits(ea * eb[e]);

@@ -311,6 +311,16 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v
       : "memory");
 }
 
+// The same for 16 columns.
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -426,6 +436,19 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
       : "memory");
 }
 
+// The same with bf16 operands, two per 32-bit TMEM column of A and word of B, 16 contraction values per MMA.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Arrive on `bar` once every MMA issued so far by this thread has finished (implies
 // tcgen05.fence::before_thread_sync).
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -484,6 +507,19 @@ __device__ __forceinline__ uint32_t tf32_corrections_trunc(float w) {
   const float hi = __uint_as_float(__float_as_uint(w) & 0xFFFFE000u);
   return pack_bf16x2(w - hi, hi);
 }
+// Packed corrections of a 16 KB operand tile, word for word: thread t of 128.
+__device__ __forceinline__ void pack_tile_corrections(const uint8_t* tile, uint8_t* packed, int t) {
+  const float4* src = reinterpret_cast<const float4*>(tile) + t;
+  uint4* dst = reinterpret_cast<uint4*>(packed) + t;
+  float4 v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = src[c * 128];
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    dst[c * 128] = make_uint4(tf32_corrections_trunc(v[c].x), tf32_corrections_trunc(v[c].y), tf32_corrections_trunc(v[c].z),
+                              tf32_corrections_trunc(v[c].w));
+}
+
 __device__ __forceinline__ void tf32_split_trunc(float x, float& hi, float& lo) {
   hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
   lo = x - hi;
