@@ -704,3 +704,29 @@ def test_3xtf32_on_the_tmem_operand_pair_kernel(shape, dist):
     fin = torch.isfinite(want)
     tol = 2.0**-17 + 1.2e-8 * J + 80 * 2.0**-23 + 2.0**-22 * want[fin].abs()
     assert ((got[fin].double() - want[fin]).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 3e-45, 0.0])
+def test_logarithm_of_the_3xtf32_epilogue(scale):
+    """The epilogue's logarithm against float64 on sums of one product (b = 0, J = 1, so that the sum is the weight):
+    normal floats over their whole range, values around 1, and blocks that hold subnormals and zeros.  Tolerance: 2 ulp of
+    the result and, for subnormal weights, whose low bits the operand split drops, 2^-10 of the value per lost bit: not
+    compared below 2^-126 except for -inf."""
+    import triturus_b200 as tb
+
+    g = torch.Generator().manual_seed(5)
+    x = torch.exp(torch.empty(4, 384, 1).uniform_(-80.0, 80.0, generator=g))
+    x[1] = torch.empty(384, 1).uniform_(0.7, 1.42, generator=g)
+    x[2, ::7] *= scale
+    x[3] = 1.0
+    # tf32 weights: the sum is the weight exactly
+    x = (x.view(torch.int32) & ~0x1FFF).view(torch.float32)
+    b = torch.zeros(4, 1, 256)
+    for variant in (0, 102564, 1281):
+        got = tb.lm2exp(x.cuda(), b.cuda(), precision="3xtf32", variant=variant).cpu()
+        tb.check_status()
+        want = x.double().log().expand(4, 384, 256)
+        assert torch.equal(got[(x == 0).expand_as(got)] == float("-inf"), torch.ones_like(got[(x == 0).expand_as(got)]).bool())
+        cmp = (x >= 2.0**-126).expand_as(got)
+        ulp = torch.finfo(torch.float32).eps * want[cmp].abs().clamp_min(1e-30)
+        assert ((got[cmp].double() - want[cmp]).abs() <= 2 * ulp).all()

@@ -416,6 +416,11 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
               if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
             }
             const int ib = i0 + c * 32;
+            if (Cfg::PREC) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e) acc_max = max(acc_max, v[h][e]);
+              log_block(v[h]);
+            }
             // Register e of this lane is row ib + e, column kcol of the result.  The 32 x 32 block goes through a
             // staging box (row e at byte e * 128 in the 128-byte swizzle, the 32 lanes of a store fill one row)
             // and from there as one TMA store: per-row stores straight from the registers ran at ~70 cycles per
@@ -428,8 +433,8 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
                 const float acc = __uint_as_float(v[h][e]);
-                const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
-                if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
+                const float o = m + (Cfg::PREC ? acc : lg2_approx(acc) * LN2_F);
+                if (Cfg::OPT) acc_max = max(acc_max, v[h][e]);
                 if (Cfg::PREC) cmx = fmaxf(cmx, o);  // (rows past I hold log 0 = -inf)
                 *reinterpret_cast<float*>(stg + sw128_offset(e, lane)) = o;
               }
@@ -446,8 +451,8 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
               for (int e = 0; e < 32; ++e) {
                 const float acc = __uint_as_float(v[h][e]);
-                const float o = m + (Cfg::PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
-                if (Cfg::OPT || Cfg::PREC) acc_max = max(acc_max, v[h][e]);
+                const float o = m + (Cfg::PREC ? acc : lg2_approx(acc) * LN2_F);
+                if (Cfg::OPT) acc_max = max(acc_max, v[h][e]);
                 if (Cfg::PREC) cmx = fmaxf(cmx, o);  // (rows past I hold log 0 = -inf)
                 if (col_ok && e < nrows) orow[static_cast<int64_t>(e) * p.out_s1] = o;
               }
