@@ -730,3 +730,21 @@ def test_logarithm_of_the_3xtf32_epilogue(scale):
         cmp = (x >= 2.0**-126).expand_as(got)
         ulp = torch.finfo(torch.float32).eps * want[cmp].abs().clamp_min(1e-30)
         assert ((got[cmp].double() - want[cmp]).abs() <= 2 * ulp).all()
+
+
+@pytest.mark.parametrize("variant", [2566, 2567])
+@pytest.mark.parametrize("shape", [(3, 129, 32, 130), (2, 200, 256, 300), (2, 256, 255, 257), (80, 321, 225, 260), (2, 448, 257, 256)])
+def test_accumulator_in_halves_of_the_tmem_operand_pair_kernel(shape, variant):
+    """Up to eight k-blocks (J <= 256) the pair kernel fills and drains its accumulator in two halves of 64 rows of each
+    CTA: rows that end inside each of the four 64-row parts, several tiles per pair, odd numbers of k-blocks, and the first
+    J beyond the rule.  The arithmetic is that of the shared-memory pair kernel in the same order: bit for bit, except
+    that the optimistic stabiliser of 2567 is another one (the tolerance of plain TF32 then)."""
+    R, I, J, K = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 6.0
+    b[0, :, 3] = float("-inf")
+    got = _run(a, b, precision="tf32", variant=variant)
+    _assert_close(got[:3], a[:3], b[:3], "tf32")
+    if variant == 2566:
+        assert torch.equal(got, _run(a, b, precision="tf32", variant=2564))

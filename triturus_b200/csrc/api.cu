@@ -336,6 +336,9 @@ static int launch_lm2exp_pair(const CUtensorMap& ta, const CUtensorMap& tb, cons
 //                                  NS NSB groups optimistic
 using LmTsPair = Lm2expTsPairCfg<8, 4, 2>;
 using LmTsPairOpt = Lm2expTsPairCfg<8, 4, 2, true>;
+// ... with the accumulator in halves, for contractions whose k-blocks fit the eight operand stages
+using LmTsPairH = Lm2expTsPairCfg<8, 4, 2, false, false, 0, true>;
+using LmTsPairOptH = Lm2expTsPairCfg<8, 4, 2, true, false, 0, true>;
 using LmTsPairX = Lm2expTsPairCfg<4, 4, 2, false, false, 1>;  // 3xTF32
 using LmTsPairFused = Lm2expTsPairCfg<8, 4, 2, false, true>;  // exact max pass inside: the conditional launch behind Opt
 
@@ -759,6 +762,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     rc = make_tmap(&tb_plain, b, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != TRITURUS_B200_OK) return rc;
   }
+  const bool ts_halves = J <= 32 * LmTsPair::NS;
   const int64_t bstr[3] = {gen_b ? bs_raw[0] : bs0, gen_b ? bs_raw[1] : bs1, gen_b ? bs_raw[2] : 1};
   if (use_ts && plan.optimistic && prepass && ws_flags) {
     // No pre-pass: the contraction takes each column's stabiliser from its first 32 rows and raises the flag
@@ -769,7 +773,8 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     Lm2expParams po = p;
     po.m_ws = nullptr;
     po.opt_flag = flag;
-    rc = launch_lm2exp_tspair<LmTsPairOpt>(ta, tb_plain, to, po, st, false);
+    rc = ts_halves ? launch_lm2exp_tspair<LmTsPairOptH>(ta, tb_plain, to, po, st, false)
+                   : launch_lm2exp_tspair<LmTsPairOpt>(ta, tb_plain, to, po, st, false);
     if (rc != TRITURUS_B200_OK) return rc;
     // (the exact column maxima are found inside the conditional kernel: one launch behind the optimistic one)
     p.m_ws = nullptr;
@@ -808,7 +813,8 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   const bool dep = prepass;
   if (use_ts)
     return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, dep)
-                                                        : launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
+           : ts_halves ? launch_lm2exp_tspair<LmTsPairH>(ta, tb_plain, to, p, st, dep)
+                       : launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
   if (pair) return launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, dep);
   auto single = [&](const Lm2expParams& q, bool dependent) -> int {
     if (b_km || gen_a || gen_b) {

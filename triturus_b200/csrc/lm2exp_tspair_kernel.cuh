@@ -52,7 +52,7 @@ __device__ long long g_timeline[16 * 256];
 // (1-2 us from L2 / HBM) -> transform -> MMA -> commit" is several thousand cycles long, so the number of
 // k-blocks in flight, not any pipe, bounds a single ring of six stages (measured 1 100 cycles per k-block for
 // 512 cycles of MMAs); two rings put 8 + 5 tiles in flight in the same shared memory.
-template <int NS_, int NSB_, int NG_ = 2, bool OPT_ = false, bool FUSED_ = false, int PREC_ = 0>
+template <int NS_, int NSB_, int NG_ = 2, bool OPT_ = false, bool FUSED_ = false, int PREC_ = 0, bool HALVES_ = false>
 struct Lm2expTsPairCfg {
   static constexpr int BM = 128;   // columns k per CTA (256 per pair): TMEM lanes
   static constexpr int BN = 256;   // rows i per pair tile (N of the MMA), 128 per CTA's shared memory
@@ -83,8 +83,15 @@ struct Lm2expTsPairCfg {
   static constexpr bool FUSED = FUSED_;
   static constexpr bool SLOTS = OPT || FUSED;  // stabilisers handed from the transform warps to the other roles
   static_assert(!(OPT && FUSED), "one or the other");
+  // HALVES, for short contractions (KB <= NS, all k-blocks of a tile in the operand stages at once): the accumulator is
+  // filled in two halves of 128 rows which the MMA issuer and the epilogue hand over separately, so that the epilogue of one
+  // half runs under the MMAs of the other (R128 I256 J256 K8192: 482 -> 447 us).  Not beyond: N = 128 MMAs read the operand
+  // in TMEM twice, and the main loop then loses more than the borders of the tiles gain (R32 1024^3: 160 -> 174 us).
+  static constexpr bool HALVES = HALVES_;
+  static constexpr int NH = HALVES ? 2 : 1;
+  static_assert(!PREC || !HALVES, "not instantiated");
   static_assert(!PREC || !SLOTS, "3xTF32 takes its stabilisers from a pre-pass");
-  static constexpr int NBAR = 3 * NS + 2 * NSB + 2 + (SLOTS ? 16 : 0) + (FUSED ? 4 * (NG - 1) : 0);
+  static constexpr int NBAR = 3 * NS + 2 * NSB + 4 + (SLOTS ? 16 : 0) + (FUSED ? 4 * (NG - 1) : 0);
   static constexpr int M_TILE_BYTES = (SLOTS ? 2 * BM * 4 : 0) + (FUSED ? (NG - 1) * BM * 4 : 0);
   static constexpr int SMEM_BYTES = 1024 + NS * A_STAGE + NSB * B_TILE + EPI_STAGE + M_TILE_BYTES + NBAR * 8 + 64;
   static_assert(E_COL0 + NS * E_COLS <= TMEM_COLS, "TMEM capacity");
@@ -166,13 +173,13 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   uint64_t* stage_empty = bars + 2 * NS;  // [NS] pair MMAs reading ring-1 stage retired (committed by the leader)
   uint64_t* b_full = bars + 3 * NS;       // [NSB] this CTA's tile of b landed
   uint64_t* b_empty = b_full + NSB;       // [NSB] the four transform warps of the k-block hold it in registers
-  uint64_t* acc_full = b_empty + NSB;     // [1] accumulator complete (committed by the leader)
-  uint64_t* acc_empty = acc_full + 1;     // [1] (leader's copy is used) epilogues of both CTAs drained it
-  uint64_t* m_ready = acc_empty + 1;      // SLOTS [2][4] slot, lane quarter: stabilisers written
+  uint64_t* acc_full = b_empty + NSB;     // [NH] accumulator (half) complete (committed by the leader)
+  uint64_t* acc_empty = acc_full + 2;     // [NH] (leader's copy is used) epilogues of both CTAs drained it
+  uint64_t* m_ready = acc_empty + 2;      // SLOTS [2][4] slot, lane quarter: stabilisers written
   uint64_t* m_free = m_ready + 8;         // SLOTS [2][4] every reader of the quarter (epilogue warp, other groups) is done
   uint64_t* part_ready = m_free + 8;      // FUSED [NG - 1][4] group g > 0, lane quarter: its partial maxima written
   float* m_part = m_tile + 2 * BM;        // FUSED [NG - 1][BM] partial column maxima of the groups other than the first
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1 + (Cfg::SLOTS ? 16 : 0) +
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2 + (Cfg::SLOTS ? 16 : 0) +
                                                     (Cfg::FUSED ? 4 * (Cfg::NG - 1) : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -196,8 +203,10 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       mbar_init(&b_full[s], 1);
       mbar_init(&b_empty[s], 4);
     }
-    mbar_init(acc_full, 1);
-    mbar_init(acc_empty, 8);
+    for (int h = 0; h < Cfg::NH; ++h) {
+      mbar_init(&acc_full[h], 1);
+      mbar_init(&acc_empty[h], 8);
+    }
     if (Cfg::SLOTS) {
       for (int i = 0; i < 8; ++i) {
         mbar_init(&m_ready[i], 1);
@@ -296,43 +305,75 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
       // PREC takes a transposed a too: MN-major for the tf32 MMAs (bit 16), while its packed words are always K-major.
       const bool a_mn = Cfg::PREC && p.a_mn != 0;
-      const uint32_t idesc = umma_idesc_tf32(2 * BM, BN) | (a_mn ? 1u << 16 : 0u);
+      const uint32_t idesc = umma_idesc_tf32(2 * BM, BN / Cfg::NH) | (a_mn ? 1u << 16 : 0u);
       const uint32_t a_step = a_mn ? 64u : 2u;  // encoded address step per 8 contraction values
+      constexpr uint32_t HALF_ENC = (64 * BK * 4) >> 4;  // 64 rows of a further
       constexpr uint32_t STAGE_ENC = Cfg::A_STAGE >> 4;
       const uint64_t db0 = a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0)), 4096) : umma_desc_k_sw128(smem_u32(a_tile(0)));
       const uint64_t dbp0 = umma_desc_k_sw128(smem_u32(a_tile(0)) + Cfg::A_TILE);
-      const uint32_t d = tmem_base;
       uint32_t s = 0, ph = 0, tcount = 0;
       bool ok = true;
-      for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
-        TB200_TL(11, tcount);
-        if (!(ok = mbar_wait(acc_empty, (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
-        TB200_TL(12, tcount);
-        tc_fence_after_sync();
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
-          TB200_TL(0, tcount * KB + kb);
-          tc_fence_after_sync();
-          const uint64_t db = db0 + s * STAGE_ENC;
-          const uint32_t ea = tmem_base + Cfg::E_COL0 + s * Cfg::E_COLS;
+      auto advance = [&]() {
+        if (++s == NS) {
+          s = 0;
+          ph ^= 1;
+        }
+      };
+      // One k-block: all 256 rows, or (HALVES) rows h * 64 .. + 63 of both CTAs into accumulator half h.
+      auto issue = [&](uint32_t st, uint32_t h, bool accumulate) {
+        const uint32_t d = tmem_base + h * (BN / 2);
+        const uint64_t db = db0 + st * STAGE_ENC + h * HALF_ENC;
+        const uint32_t ea = tmem_base + Cfg::E_COL0 + st * Cfg::E_COLS;
+#pragma unroll
+        for (int ks = 0; ks < BK / 8; ++ks)
+          umma_tf32_ts_pair(d, ea + ks * 8, db + a_step * ks, idesc, (accumulate || ks > 0) ? 1u : 0u);
+        if (Cfg::PREC) {
+          // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks)
-            umma_tf32_ts_pair(d, ea + ks * 8, db + a_step * ks, idesc, (kb > 0 || ks > 0) ? 1u : 0u);
-          if (Cfg::PREC) {
-            // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands
-#pragma unroll
-            for (int ks = 0; ks < BK / 8; ++ks)
-              umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + s * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
-          }
-          // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
-          umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
-          TB200_TL(1, tcount * KB + kb);
-          if (++s == NS) {
-            s = 0;
-            ph ^= 1;
-          }
+            umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + st * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
         }
-        if (ok) umma_commit_pair_mcast(smem_u32(acc_full), 3);
+      };
+      for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
+        TB200_TL(11, tcount);
+        if (!(ok = mbar_wait(&acc_empty[0], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
+        TB200_TL(12, tcount);
+        tc_fence_after_sync();
+        if (Cfg::HALVES) {
+          // The first half of the accumulator takes all k-blocks of the tile (they fit the operand stages) as soon as the
+          // epilogue of the previous tile has drained it, the second half when it is drained too.
+          const uint32_t s_first = s;
+          for (int kb = 0; kb < KB; ++kb) {
+            if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
+            TB200_TL(0, tcount * KB + kb);
+            tc_fence_after_sync();
+            issue(s, 0, kb > 0);
+            advance();
+          }
+          if (!ok) break;
+          umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
+          if (!(ok = mbar_wait(&acc_empty[1], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
+          tc_fence_after_sync();
+          for (int kb = 0; kb < KB; ++kb) {
+            const uint32_t st = s_first + kb < NS ? s_first + kb : s_first + kb - NS;
+            issue(st, 1, kb > 0);
+            // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
+            umma_commit_pair_mcast(smem_u32(&stage_empty[st]), 3);
+            TB200_TL(1, tcount * KB + kb);
+          }
+          umma_commit_pair_mcast(smem_u32(&acc_full[1]), 3);
+        } else {
+          for (int kb = 0; kb < KB; ++kb) {
+            if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
+            TB200_TL(0, tcount * KB + kb);
+            tc_fence_after_sync();
+            issue(s, 0, kb > 0);
+            umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
+            TB200_TL(1, tcount * KB + kb);
+            advance();
+          }
+          if (ok) umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
+        }
       }
     }
     __syncwarp();
@@ -360,7 +401,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     uint8_t* stg2 = epi_stage + q * 8192;  // two boxes: one is filled while the TMA unit still reads the other
     uint32_t nbox = 0;
     const bool use_tma = p.out_tma != 0;
-    const uint32_t acc_empty_leader = map_to_cta(smem_u32(acc_empty), 0);
+    const uint32_t acc_empty_leader0 = map_to_cta(smem_u32(acc_empty), 0);
     const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     pdl_wait();  // m comes from the pre-pass, which may still be running when this kernel starts
     uint32_t tcount = 0;
@@ -378,10 +419,15 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (!Cfg::SLOTS && col_ok) m = clamp_stab(__ldg(p.m_ws + static_cast<int64_t>(r) * p.K + kcol));
       float* ocol = p.out + static_cast<int64_t>(r) * p.out_s0 + kcol;
       float cmx = -INFINITY;  // PREC: largest result of this lane's column in the tile, for the next layer of a chain
-      if (!(ok = mbar_wait_warp(acc_full, tcount & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
+      // Accumulator column c holds row i0 + c; in halves, columns 128 hf + (0 .. 63) the leader's rows of a, i0 + 64 hf on,
+      // and the 64 behind them the other CTA's, i0 + 128 + 64 hf on.
+#pragma unroll 1
+      for (int hf = 0; ok && hf < Cfg::NH; ++hf) {
+      const uint32_t acc_empty_leader = acc_empty_leader0 + static_cast<uint32_t>(hf) * 8u;
+      if (!(ok = mbar_wait_warp(&acc_full[hf], tcount & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
       if (warp == 4 && lane == 0) TB200_TL(7, tcount);
       tc_fence_after_sync();
-      if (Cfg::SLOTS) {
+      if (Cfg::SLOTS && hf == 0) {
         // the stabilisers this tile was computed with (written long before the accumulator completed)
         const uint32_t slot = (tcount & 1) * 4 + q;
         if (!(ok = mbar_wait_warp(&m_ready[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
@@ -390,7 +436,10 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         __syncwarp();
         if (lane == 0) mbar_arrive(&m_free[slot]);
       }
-      const int nchunks = (k0 < p.K) ? min(BN / 32, (p.I - i0 + 31) / 32) : 0;
+      const int row0 = i0 + hf * 64;
+      const int nchunks = k0 >= p.K ? 0
+                          : Cfg::HALVES ? min(2, max(0, (p.I - row0 + 31) / 32)) + min(2, max(0, (p.I - row0 - 128 + 31) / 32))
+                                        : min(BN / 32, (p.I - i0 + 31) / 32);
       if (nchunks == 0) {
         // nothing to store (this warp's columns are padding): release the accumulator right away
         tc_fence_before_sync();
@@ -399,7 +448,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         continue;
       }
       uint32_t v[2][32];
-      tmem_ld_32x32(tbase, v[0]);
+      tmem_ld_32x32(tbase + hf * (BN / 2), v[0]);
 #pragma unroll 1
       for (int idx = 0; idx < nchunks; idx += 2) {
 #pragma unroll
@@ -408,14 +457,14 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (c < nchunks) {
             tmem_ld_wait();  // chunk c is in v[h]
             if (c + 1 < nchunks) {
-              tmem_ld_32x32(tbase + (c + 1) * 32, v[h ^ 1]);
+              tmem_ld_32x32(tbase + hf * (BN / 2) + (c + 1) * 32, v[h ^ 1]);
             } else {
-              // the whole accumulator is in registers: hand it back to the MMA issuer
+              // all of it is in registers: hand it back to the MMA issuer
               tc_fence_before_sync();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
             }
-            const int ib = i0 + c * 32;
+            const int ib = row0 + c * 32 + (Cfg::HALVES && c >= 2 ? 64 : 0);
             if (Cfg::PREC) {
 #pragma unroll
               for (int e = 0; e < 32; ++e) acc_max = max(acc_max, v[h][e]);
@@ -461,7 +510,8 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         }
       }
       if (warp == 4 && lane == 0) TB200_TL(8, tcount);
-      if (Cfg::PREC && p.out_max != nullptr && col_ok) red_max_f32(p.out_max + static_cast<int64_t>(r) * p.K + kcol, cmx);
+      }
+      if (Cfg::PREC && ok && p.out_max != nullptr && col_ok) red_max_f32(p.out_max + static_cast<int64_t>(r) * p.K + kcol, cmx);
     }
     if (use_tma && lane == 0) tma_store_wait_all();  // shared memory must outlive the last box
     if (opt) {
