@@ -183,9 +183,9 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                                                     (Cfg::FUSED ? 4 * (Cfg::NG - 1) : 0));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();  // 0 = leader
+  const uint32_t rank = warp_uniform(cluster_ctarank());  // 0 = leader
   const bool leader = rank == 0;
   const AbortCtl ctl{abort_flag, p.status};
 
@@ -233,7 +233,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   tc_fence_before_sync();
   cluster_sync_all();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   const int KB = (p.J + BK - 1) / BK;
   const int npairs = gridDim.x >> 1;
@@ -301,7 +301,10 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ pair MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    // The whole warp runs the loop and one elected lane issues: control flow and descriptors are uniform and stay in uniform
+    // registers.  (One lane in a branch of its own took 80 - 100 cycles per MMA for moving them there, more than the 64 to
+    // 128 of the MMA itself: 750 cycles per k-block in plain TF32, 1 300 in 3xTF32.)
+    if (leader) {
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
       // PREC takes a transposed a too: MN-major for the tf32 MMAs (bit 16), while its packed words are always K-major.
       const bool a_mn = Cfg::PREC && p.a_mn != 0;
@@ -336,7 +339,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       };
       for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
         TB200_TL(11, tcount);
-        if (!(ok = mbar_wait(&acc_empty[0], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
+        if (!(ok = mbar_wait_warp(&acc_empty[0], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
         TB200_TL(12, tcount);
         tc_fence_after_sync();
         if (Cfg::HALVES) {
@@ -344,35 +347,42 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           // epilogue of the previous tile has drained it, the second half when it is drained too.
           const uint32_t s_first = s;
           for (int kb = 0; kb < KB; ++kb) {
-            if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
+            if (!(ok = mbar_wait_warp(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
             TB200_TL(0, tcount * KB + kb);
             tc_fence_after_sync();
-            issue(s, 0, kb > 0);
+            if (elect_one_sync()) issue(s, 0, kb > 0);
+            __syncwarp();
             advance();
           }
           if (!ok) break;
-          umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
-          if (!(ok = mbar_wait(&acc_empty[1], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
+          if (elect_one_sync()) umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
+          if (!(ok = mbar_wait_warp(&acc_empty[1], (tcount & 1) ^ 1, ctl, STATUS_TIMEOUT_MMA))) break;
           tc_fence_after_sync();
           for (int kb = 0; kb < KB; ++kb) {
             const uint32_t st = s_first + kb < NS ? s_first + kb : s_first + kb - NS;
-            issue(st, 1, kb > 0);
-            // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
-            umma_commit_pair_mcast(smem_u32(&stage_empty[st]), 3);
+            if (elect_one_sync()) {
+              issue(st, 1, kb > 0);
+              // free the stage (shared memory and TMEM) in both CTAs once these MMAs retire
+              umma_commit_pair_mcast(smem_u32(&stage_empty[st]), 3);
+            }
+            __syncwarp();
             TB200_TL(1, tcount * KB + kb);
           }
-          umma_commit_pair_mcast(smem_u32(&acc_full[1]), 3);
+          if (elect_one_sync()) umma_commit_pair_mcast(smem_u32(&acc_full[1]), 3);
         } else {
           for (int kb = 0; kb < KB; ++kb) {
-            if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
+            if (!(ok = mbar_wait_warp(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
             TB200_TL(0, tcount * KB + kb);
             tc_fence_after_sync();
-            issue(s, 0, kb > 0);
-            umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
+            if (elect_one_sync()) {
+              issue(s, 0, kb > 0);
+              umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
+            }
+            __syncwarp();
             TB200_TL(1, tcount * KB + kb);
             advance();
           }
-          if (ok) umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
+          if (ok && elect_one_sync()) umma_commit_pair_mcast(smem_u32(&acc_full[0]), 3);
         }
       }
     }

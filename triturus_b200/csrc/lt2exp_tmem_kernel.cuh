@@ -108,7 +108,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mx_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_uniform(threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const AbortCtl ctl{abort_flag, p.status};
 
@@ -136,7 +136,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   const int JC = (p.J + BK - 1) / BK;
   const int KBT = JC * p.I;  // k-blocks per output tile

@@ -64,6 +64,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same value in every lane, as the compiler can see it too: what depends on it may live in uniform registers.
+template <class T>
+__device__ __forceinline__ T warp_uniform(T x) {
+  return __shfl_sync(0xffffffffu, x, 0);
+}
+
 // True in exactly one lane of a fully converged warp (the same lane on every call).  Code that the whole warp
 // runs with uniform control flow and that issues its single-thread instructions under this predicate keeps
 // its addresses and descriptors in uniform registers.
