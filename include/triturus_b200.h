@@ -217,6 +217,13 @@ int triturus_b200_lt2exp_chain_f32(const float* w, const float* a, const float* 
 int triturus_b200_colmax_f32(const float* x, float* m, int64_t R, int64_t J, int64_t K, const int64_t x_strides[3],
                              void* stream);
 
+/* padded[r, y, 0 .. n) = x[r, y, 0 .. n) for y < rows, with rows of round_up(n, 4) floats back to back (16-byte aligned,
+ * the rest of a row zero): what the tensor maps of the entry points need of an operand whose row pitch is no multiple of
+ * 16 bytes.  s0 and s1 are x's element strides of r and y; consecutive values of a row are adjacent.  x needs 4-byte,
+ * padded 16-byte alignment; padded holds R * rows * round_up(n, 4) floats. */
+int triturus_b200_pad_rows_f32(const float* x, float* padded, int64_t R, int64_t rows, int64_t n, int64_t s0, int64_t s1,
+                               void* stream);
+
 /*
  * Plain matrix product out[M,N] = a[M,K] * b[K,N] through the same pipeline with the log-space steps switched off.
  * Replaces triturus/mm.py:181-214 (wrapper) and :91-178 (_ker_mm).  precision TF32: both operands rounded to the

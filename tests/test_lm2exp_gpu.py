@@ -748,3 +748,20 @@ def test_accumulator_in_halves_of_the_tmem_operand_pair_kernel(shape, variant):
     _assert_close(got[:3], a[:3], b[:3], "tf32")
     if variant == 2566:
         assert torch.equal(got, _run(a, b, precision="tf32", variant=2564))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 5, 7), (2, 33, 101), (1, 1, 4099), (5, 700, 203), (2, 3, 5, 50), (1, 4099),
+                                   (70000, 2, 3)])
+def test_padded_copy_of_rows(shape):
+    """The rows of an operand that the tensor maps cannot describe, copied to a pitch of whole 16 bytes: bit for bit, from
+    a base that is only 4-byte aligned, from rows of a wider tensor, and broadcast (stride 0) over the first dimension."""
+    from triturus_b200 import _native
+
+    n = 1
+    for s in shape:
+        n *= s
+    x = torch.randn(n + 1, device="cuda")[1:].view(shape)
+    wide = torch.randn(*shape[:-1], 2 * shape[-1] + 1, device="cuda")[..., 1 : shape[-1] + 1]
+    for t in (x, wide, x[:1].expand(shape)):
+        got = _native._tma_ready(t)
+        assert _native._tma_ok(got) and torch.equal(got, t)

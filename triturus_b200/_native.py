@@ -32,6 +32,7 @@ EXPORTED_SYMBOLS = (
     "triturus_b200_lt2exp_ws_f32",
     "triturus_b200_lt2exp_chain_f32",
     "triturus_b200_colmax_f32",
+    "triturus_b200_pad_rows_f32",
     "triturus_b200_selftest_wait_timeout",
     "triturus_b200_mm_f32",
     "triturus_b200_lm2exp_static_max_columns",
@@ -136,6 +137,8 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
                                          c_int, c_void_p, c_void_p]  # fmt: skip
     lib.triturus_b200_colmax_f32.restype = c_int
     lib.triturus_b200_colmax_f32.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_int64, i64p, c_void_p]
+    lib.triturus_b200_pad_rows_f32.restype = c_int
+    lib.triturus_b200_pad_rows_f32.argtypes = [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p]
     return lib
 
 
@@ -229,8 +232,31 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     padded = (inner + 3) // 4 * 4
     buf = torch.empty(*t.shape[:-1], padded, dtype=t.dtype, device=t.device)
     view = buf[..., :inner]
-    view.copy_(t)
+    if not _pad_rows(t, buf):
+        view.copy_(t)
     return view
+
+
+def _pad_rows(t: torch.Tensor, buf: torch.Tensor) -> bool:
+    """Fill `buf` with the rows of `t` through the library's own kernel, which streams rows of consecutive floats whatever
+    their pitch and base; False where it does not apply (the caller then copies with torch)."""
+    if not t.is_cuda or t.dtype != torch.float32 or t.stride(-1) != 1 or t.data_ptr() % 4 or not 2 <= t.dim() <= 4:
+        return False
+    shape, stride = t.shape, t.stride()
+    if t.dim() == 4:  # the two middle dimensions as one sequence of rows
+        if shape[1] > 1 and stride[1] != shape[2] * stride[2]:
+            return False
+        R, rows, s0, s1 = shape[0], shape[1] * shape[2], stride[0], stride[2]
+    elif t.dim() == 3:
+        R, rows, s0, s1 = shape[0], shape[1], stride[0], stride[1]
+    else:
+        R, rows, s0, s1 = 1, shape[0], 0, stride[0]
+    if buf.numel() == 0 or buf.numel() >= 1 << 33:
+        return False
+    with _on_device(t.device) as idx:
+        rc = LIB.triturus_b200_pad_rows_f32(t.data_ptr(), buf.data_ptr(), R, rows, shape[-1], s0, s1, _raw_stream(idx))
+    _check(rc, "triturus_b200_pad_rows_f32")
+    return True
 
 
 # Problems up to this many FLOP take operands that break the tensor-map rules in place (the single-CTA kernel then
