@@ -709,9 +709,9 @@ def test_3xtf32_on_the_tmem_operand_pair_kernel(shape, dist):
 @pytest.mark.parametrize("scale", [1.0, 1e-30, 3e-45, 0.0])
 def test_logarithm_of_the_3xtf32_epilogue(scale):
     """The epilogue's logarithm against float64 on sums of one product (b = 0, J = 1, so that the sum is the weight):
-    normal floats over their whole range, values around 1, and blocks that hold subnormals and zeros.  Tolerance: 2 ulp of
-    the result and, for subnormal weights, whose low bits the operand split drops, 2^-10 of the value per lost bit: not
-    compared below 2^-126 except for -inf."""
+    normal floats over their whole range, values around 1, and blocks that hold subnormals and zeros.  Tolerance: 2^-22 of a
+    binary logarithm (lg2.approx around 1) and 2 ulp of the result; subnormal weights, whose low bits the operand split
+    drops, are not compared except for -inf."""
     import triturus_b200 as tb
 
     g = torch.Generator().manual_seed(5)
@@ -729,7 +729,7 @@ def test_logarithm_of_the_3xtf32_epilogue(scale):
         assert torch.equal(got[(x == 0).expand_as(got)] == float("-inf"), torch.ones_like(got[(x == 0).expand_as(got)]).bool())
         cmp = (x >= 2.0**-126).expand_as(got)
         ulp = torch.finfo(torch.float32).eps * want[cmp].abs().clamp_min(1e-30)
-        assert ((got[cmp].double() - want[cmp]).abs() <= 2 * ulp).all()
+        assert ((got[cmp].double() - want[cmp]).abs() <= 2 * ulp + 2.0**-22 * 0.6932).all()
 
 
 @pytest.mark.parametrize("variant", [2566, 2567])

@@ -327,15 +327,16 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const uint32_t d = tmem_base + h * (BN / 2);
         const uint64_t db = db0 + st * STAGE_ENC + h * HALF_ENC;
         const uint32_t ea = tmem_base + Cfg::E_COL0 + st * Cfg::E_COLS;
-#pragma unroll
-        for (int ks = 0; ks < BK / 8; ++ks)
-          umma_tf32_ts_pair(d, ea + ks * 8, db + a_step * ks, idesc, (accumulate || ks > 0) ? 1u : 0u);
         if (Cfg::PREC) {
-          // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands
+          // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands.  First,
+          // while the accumulator of a tile is empty: the sum of the first k-block's corrections is not truncated then.
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks)
-            umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + st * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), 1u);
+            umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + st * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), (accumulate || ks > 0) ? 1u : 0u);
         }
+#pragma unroll
+        for (int ks = 0; ks < BK / 8; ++ks)
+          umma_tf32_ts_pair(d, ea + ks * 8, db + a_step * ks, idesc, (Cfg::PREC || accumulate || ks > 0) ? 1u : 0u);
       };
       for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
         TB200_TL(11, tcount);

@@ -213,18 +213,20 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
           if (elect_one_sync()) {
             const uint64_t dw = umma_desc_k_sw128(stage0 + s * Cfg::STAGE);
             const uint32_t pa = tmem_base + Cfg::P_COL0 + s * Cfg::P_STAGE;
+            if (Cfg::PREC) {
+              // p_lo * w_hi + p_hi * w_lo: 64 bf16 values in rows of 128 bytes like the tf32 operands.  First, while
+              // the accumulator of a chunk is empty and does not truncate them
+#pragma unroll
+              for (int ks = 0; ks < BK / 8; ++ks)
+                umma_bf16_ts(d, pa + BK + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, umma_idesc_bf16(128, BM * MT),
+                             (kb > kb0 || ks > 0) ? 1u : 0u);
+            }
 #pragma unroll
             for (int blk = 0; blk < Cfg::NB; ++blk) {  // the column blocks share the w tile
 #pragma unroll
               for (int ks = 0; ks < BK / 8; ++ks)
                 umma_tf32_ts(d + blk * Cfg::BLK_COLS, pa + blk * BK + ks * 8, dw + 2 * ks, idesc,
-                             (kb > kb0 || ks > 0) ? 1u : 0u);
-            }
-            if (Cfg::PREC) {
-              // p_lo * w_hi + p_hi * w_lo: 64 bf16 values in rows of 128 bytes like the tf32 operands
-#pragma unroll
-              for (int ks = 0; ks < BK / 8; ++ks)
-                umma_bf16_ts(d, pa + BK + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, umma_idesc_bf16(128, BM * MT), 1u);
+                             (Cfg::PREC || kb > kb0 || ks > 0) ? 1u : 0u);
             }
             umma_commit(&opnd_empty[s]);
           }

@@ -466,40 +466,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 
 constexpr float LOG2E_F = 1.4426950408889634f;
 constexpr float LN2_F = 0.6931471805599453f;
-// Natural logarithm of a positive normal float: x = 2^k (1 + f) with 1 + f in [sqrt(1/2), sqrt(2)), k ln 2 + f + f^2 Q(f)
-// with Q of degree 7, least squares reweighted towards the smallest largest relative error (3e-8).  At most 1.15 ulp off
-// over all normal floats, 0.3 ulp in the root mean square.
-__device__ __forceinline__ float log_normal(uint32_t bits) {
-  const int32_t k = static_cast<int32_t>(bits - 0x3f3504f3u) >> 23;
-  const float f = __uint_as_float(bits - (static_cast<uint32_t>(k) << 23)) - 1.0f;
-  float q = 0x1.65c680p-4f;
-  q = fmaf(q, f, -0x1.25046ap-3f);
-  q = fmaf(q, f, 0x1.31853ap-3f);
-  q = fmaf(q, f, -0x1.535d38p-3f);
-  q = fmaf(q, f, 0x1.98d2bep-3f);
-  q = fmaf(q, f, -0x1.00049ap-2f);
-  q = fmaf(q, f, 0x1.5556f4p-2f);
-  q = fmaf(q, f, -0x1.fffffap-2f);
-  const float kf = __int_as_float(0x4b400000 + k) - 12582912.0f;  // k as a float, past the conversion unit
-  return fmaf(kf, 0x1.62e430p-1f, fmaf(f * f, q, f));
-}
-// Replaces 32 accumulator values by their logarithms.  Straight-line code when every value of the warp is a positive normal
-// float; zeros, subnormals, infinities, negative values and NaN take logf for all 32.  (logf alone, with its own handling
-// of those cases per value, took 3 700 cycles per block in the epilogue of the 3xTF32 pair kernel: R32 1024^3 292 -> 275 us,
-// R64 512x512x256 69.9 -> 63.7 us.  The kernels whose tiles are few keep logf: the second path through the code costs them
-// more instruction fetches than it saves, R24 150x101x203 39.2 -> 41.0 us.)
-__device__ __forceinline__ void log_block(uint32_t (&v)[32]) {
-  uint32_t odd = 0;
-#pragma unroll
-  for (int e = 0; e < 32; ++e) odd = max(odd, v[e] - 0x00800000u);
-  if (__any_sync(0xffffffffu, odd >= 0x7f000000u)) {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(logf(__uint_as_float(v[e])));
-  } else {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(log_normal(v[e]));
-  }
-}
 constexpr float STAB_CLAMP = 1e38f;  // the reference clamps the stabiliser to +-1e38 (baselines/lm2exp.py:12)
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -516,6 +482,32 @@ __device__ __forceinline__ float lg2_approx(float x) {
 
 // exp(v - m) with the subtraction done first, as the reference does (baselines/lm2exp.py:13).
 __device__ __forceinline__ float exp_shifted(float v, float m) { return ex2_approx((v - m) * LOG2E_F); }
+
+// Natural logarithm of a positive normal float: x = 2^k m with m in [0.75, 1.5), ln 2 (k + log2 m).  lg2.approx is off by
+// at most 2^-22 there, half of what the exps of the sum's terms are.
+__device__ __forceinline__ float log_normal(uint32_t bits) {
+  const uint32_t k23 = (bits - 0x3f400000u) & 0xff800000u;  // k << 23
+  const float l = lg2_approx(__uint_as_float(bits - k23));
+  const float k = __int_as_float(0x4b400000 + (static_cast<int32_t>(k23) >> 23)) - 12582912.0f;  // past the conversion unit
+  return fmaf(k, LN2_F, l * LN2_F);
+}
+// Replaces 32 accumulator values by their logarithms.  Straight-line code when every value of the warp is a positive normal
+// float; zeros, subnormals, infinities, negative values and NaN take logf for all 32.  (logf alone, with its own handling
+// of those cases per value, took 3 700 cycles per block in the epilogue of the 3xTF32 pair kernel: with the
+// registers of one block only, R32 1024^3 292 -> 239 us, R64 512x512x256 69.9 -> 51.4 us.  The kernels whose tiles are few keep logf: the second path through the code costs them
+// more instruction fetches than it saves, R24 150x101x203 39.2 -> 41.0 us.)
+__device__ __forceinline__ void log_block(uint32_t (&v)[32]) {
+  uint32_t odd = 0;
+#pragma unroll
+  for (int e = 0; e < 32; ++e) odd = max(odd, v[e] - 0x00800000u);
+  if (__any_sync(0xffffffffu, odd >= 0x7f000000u)) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(logf(__uint_as_float(v[e])));
+  } else {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(log_normal(v[e]));
+  }
+}
 
 // Round an fp32 in [0, +inf) to the nearest tf32 (ties away), as raw bits.  The tensor core drops the low
 // 13 mantissa bits of its operands, so adding half a tf32 ulp beforehand turns that truncation into
