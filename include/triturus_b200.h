@@ -85,7 +85,8 @@ const char* triturus_b200_strerror(int code);
  * The single-CTA kernel has the same form for its fused max pass (STAB = 3; automatic for plain TF32 when one
  * 128-row block covers I, the contraction has four k-blocks or more, the launch more than one wave of tiles and
  * 2e10 FLOP): the pass scans one k-block instead of the whole slab, and the same kernel with the full pass
- * follows as the conditional launch.  The shared-memory pair kernel (tile 2564; the automatic choice in 3xTF32,
+ * follows as the conditional launch.  Tile 2564 (the automatic choice in 3xTF32, where it runs on the
+ * kernel that keeps the generated operand in tensor memory,
  * with the same size rule) has it as STAB = 4: the pre-pass launch scans 32 rows instead of J, then the
  * contraction and two conditional launches (full pre-pass, contraction), 4 in all.  None of the three is used
  * when column maxima of the result are requested or a stabiliser is supplied.  The reference finds the exact

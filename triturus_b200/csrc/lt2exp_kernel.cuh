@@ -330,6 +330,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
   const int KBT = JC * p.I;            // k-blocks per output tile
   const bool parking = p.stream != 0 && p.park != nullptr;  // shared tiles are completed through scratch memory
   const bool split_mode = (p.nsplit > 1 || p.stream != 0) && !parking;  // partial sums are added into the zero-filled output
+  if (split_mode) pdl_launch_dependents();  // the log pass takes its column maxima meanwhile
 
   // Output tile -> (r, n0 = first column, s0 = first row).
   auto decode = [&](int tile, int& r, int& n0, int& s0) {
@@ -420,6 +421,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
     const int q = warp & 3;
     const bool vec_ok = ((p.K & 3) == 0) && ((p.out_s1 & 3) == 0) && ((p.out_s0 & 3) == 0) &&
                         ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    if (split_mode) pdl_wait();  // the zero-filled result
     uint32_t tcount = 0, ccount = 0;
     bool ok = true;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -754,7 +756,10 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
 }
 
 // Zero-fills the (possibly strided) output before a split launch accumulates into it.
+// (The contraction is launched as its programmatic dependent and waits for it only before its first addition; the log pass
+// as the contraction's, waiting before it reads the sums.)
 __global__ void lt2exp_zero_kernel(float* out, int64_t out_s0, int64_t out_s1, int R, int S, int K) {
+  pdl_launch_dependents();
   const int64_t total = static_cast<int64_t>(R) * S * K;
   for (int64_t x = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; x < total;
        x += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -811,6 +816,7 @@ __global__ void __launch_bounds__(256) lt2exp_finish_kernel(const Lt2expParams p
     msum[tid] = clamp_stab(ma) + clamp_stab(mb);
   }
   __syncthreads();
+  pdl_wait();  // the sums
   const int n = tid & 127;
   if (k0 + n >= p.K) return;
   const float m = msum[n];

@@ -142,6 +142,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   const int KBT = JC * p.I;  // k-blocks per output tile
   const bool parking = Cfg::PROMOTE && p.stream != 0 && p.park != nullptr;  // shared tiles are completed through scratch memory
   const bool split_mode = (p.nsplit > 1 || p.stream != 0) && !parking;
+  if (split_mode) pdl_launch_dependents();  // the log pass takes its column maxima meanwhile
 
   // Output tile -> (r, n0 = first column k, s0 = first row s); the items of a CTA come from LtWork.
   auto decode = [&](int tile, int& r, int& n0, int& s0) {
@@ -243,6 +244,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     // ------------------------------------------------------------------ epilogue
     const int q = warp & 3;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    if (split_mode) pdl_wait();  // the zero-filled result
     uint32_t tcount = 0;
     bool ok = true;
     LtWork work(p, KBT);
