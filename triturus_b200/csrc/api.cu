@@ -319,7 +319,7 @@ using LmPo_128_2 = Lm2expCfg<128, 2, 0, 4, true, false, true>;
 using LmPlainT = Lm2expCfg<128, 2, 0, 4, false, true>;
 using LmPlainX = Lm2expCfg<128, 2, 1, 2, true, true>;
 
-using LmPairT = Lm2expPairCfg<0, 6>;
+using LmPairT = Lm2expPairCfg<6>;
 
 // Launch on CTA pairs: a cluster of two CTAs per 256 x 256 tile.
 template <class Cfg>

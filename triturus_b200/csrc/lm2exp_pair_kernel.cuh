@@ -20,19 +20,19 @@
 
 namespace tb200 {
 
-template <int PREC_, int NS_>
+// (plain TF32 only: 3xTF32 on pair tiles runs lm2exp_tspair_kernel.cuh)
+template <int NS_>
 struct Lm2expPairCfg {
   static constexpr int BM = 128;   // rows per CTA (256 per pair)
   static constexpr int BN = 256;   // columns per pair tile
   static constexpr int BNH = 128;  // columns whose operand this CTA builds
   static constexpr int BK = 32, NTW = 8;
-  static constexpr int PREC = PREC_, NS = NS_;
-  static constexpr int NCOPY = PREC ? 2 : 1;
+  static constexpr int NS = NS_;
   static constexpr int A_TILE = BM * BK * 4;  // 16 KB
   static constexpr int B_BOX = 32 * BK * 4;   // 4 KB
   static constexpr int NGRP = BNH / 32;
   static constexpr int B_TILE = NGRP * B_BOX;  // 16 KB
-  static constexpr int STAGE = NCOPY * (A_TILE + B_TILE);
+  static constexpr int STAGE = A_TILE + B_TILE;
   static constexpr int RP = NTW / NGRP;
   static constexpr int ROWS_PER_WARP = BK / RP;
   static constexpr int ACC_COLS = BN;
@@ -52,7 +52,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg::NTHREADS, 1)
 lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_out, const Lm2expParams p) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BNH = Cfg::BNH, BK = Cfg::BK, NS = Cfg::NS;
-  constexpr int PREC = Cfg::PREC, NTW = Cfg::NTW, NGRP = Cfg::NGRP;
+  constexpr int NTW = Cfg::NTW, NGRP = Cfg::NGRP;
 
   // A conditional launch: runs only if the launch before it left the word up (same value for every thread of
   // both CTAs, read before any barrier or allocation exists).
@@ -85,10 +85,8 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const bool leader = rank == 0;
   const AbortCtl ctl{abort_flag, p.status};
 
-  auto a_tile = [&](int s, int c) -> uint8_t* { return stage_base + s * Cfg::STAGE + c * Cfg::A_TILE; };
-  auto b_tile = [&](int s, int c) -> uint8_t* {
-    return stage_base + s * Cfg::STAGE + Cfg::NCOPY * Cfg::A_TILE + c * Cfg::B_TILE;
-  };
+  auto a_tile = [&](int s) -> uint8_t* { return stage_base + s * Cfg::STAGE; };
+  auto b_tile = [&](int s) -> uint8_t* { return stage_base + s * Cfg::STAGE + Cfg::A_TILE; };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -158,13 +156,13 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           if (p.a_mn) {
 #pragma unroll
             for (int g = 0; g < BM / 32; ++g)
-              tma_load_3d(a_tile(s, 0) + g * 4096, &tmap_a, &full[s], my_i0 + g * 32, kb * BK, r);
+              tma_load_3d(a_tile(s) + g * 4096, &tmap_a, &full[s], my_i0 + g * 32, kb * BK, r);
           } else {
-            tma_load_3d(a_tile(s, 0), &tmap_a, &full[s], kb * BK, my_i0, r);
+            tma_load_3d(a_tile(s), &tmap_a, &full[s], kb * BK, my_i0, r);
           }
 #pragma unroll
           for (int g = 0; g < NGRP; ++g)
-            tma_load_3d(b_tile(s, 0) + g * Cfg::B_BOX, &tmap_b, &full[s], my_n0 + g * 32, kb * BK, r);
+            tma_load_3d(b_tile(s) + g * Cfg::B_BOX, &tmap_b, &full[s], my_n0 + g * 32, kb * BK, r);
         }
       }
       // The leader's commits arrive on both CTAs' stage_empty barriers: this CTA stays until the last ones are in.
@@ -182,12 +180,9 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       // of stage 0 are built once (stage s adds s * STAGE / 16 to the encoded address), one barrier wait
       // (the transform warps waited for the TMA bytes before they arrived), one multicast commit.
       constexpr uint32_t STAGE_ENC = Cfg::STAGE >> 4;
-      const uint64_t da_hi0 = p.a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0, 0)), 4096)
-                                     : umma_desc_k_sw128(smem_u32(a_tile(0, 0)));
-      const uint64_t da_lo0 = p.a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0, PREC ? 1 : 0)), 4096)
-                                     : umma_desc_k_sw128(smem_u32(a_tile(0, PREC ? 1 : 0)));
-      const uint64_t db_hi0 = umma_desc_mn_sw128_base32(smem_u32(b_tile(0, 0)), Cfg::B_BOX);
-      const uint64_t db_lo0 = umma_desc_mn_sw128_base32(smem_u32(b_tile(0, PREC ? 1 : 0)), Cfg::B_BOX);
+      const uint64_t da_hi0 = p.a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0)), 4096)
+                                     : umma_desc_k_sw128(smem_u32(a_tile(0)));
+      const uint64_t db_hi0 = umma_desc_mn_sw128_base32(smem_u32(b_tile(0)), Cfg::B_BOX);
       uint32_t s = 0, ph = 0, tcount = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < p.num_tiles; tile += npairs, ++tcount) {
@@ -200,17 +195,10 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           if (!(ok = mbar_wait(&xf_done[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
           tc_fence_after_sync();
           const uint64_t da_hi = da_hi0 + s * STAGE_ENC, db_hi = db_hi0 + s * STAGE_ENC;
-          const uint64_t da_lo = da_lo0 + s * STAGE_ENC, db_lo = db_lo0 + s * STAGE_ENC;
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks) {
             const uint32_t acc = (kb > 0 || ks > 0) ? 1u : 0u;
-            if (PREC) {
-              umma_tf32_ss_pair(d, da_hi + a_step * ks, db_lo + 64 * ks, idesc, acc);
-              umma_tf32_ss_pair(d, da_lo + a_step * ks, db_hi + 64 * ks, idesc, 1u);
-              umma_tf32_ss_pair(d, da_hi + a_step * ks, db_hi + 64 * ks, idesc, 1u);
-            } else {
-              umma_tf32_ss_pair(d, da_hi + a_step * ks, db_hi + 64 * ks, idesc, acc);
-            }
+            umma_tf32_ss_pair(d, da_hi + a_step * ks, db_hi + 64 * ks, idesc, acc);
           }
           // free the stage in both CTAs once these MMAs retire
           umma_commit_pair_mcast(smem_u32(&stage_empty[s]), 3);
@@ -280,7 +268,7 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             for (int e = 0; e < 32; ++e) {
               const float m_e = __shfl_sync(0xffffffffu, m_lane, e);
               const float acc = __uint_as_float(v[h][e]);
-              o[e] = m_e + (PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
+              o[e] = m_e + lg2_approx(acc) * LN2_F;
             }
             if (opt) {
 #pragma unroll
@@ -372,7 +360,6 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     const int rp = wv / NGRP;
     const int c = lane & 7;
     const int jsub = lane >> 3;
-    const int tt = threadIdx.x - 8 * 32;
     uint32_t it = 0;
     bool ok = true;
     pdl_wait();  // m comes from the pre-pass (the producer warp is already loading operand tiles meanwhile)
@@ -392,8 +379,7 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int s = it % NS;
         const uint32_t ph = (it / NS) & 1;
         if (!(ok = mbar_wait_warp(&full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-        uint8_t* box_hi = b_tile(s, 0) + grp * Cfg::B_BOX;
-        uint8_t* box_lo = b_tile(s, PREC ? 1 : 0) + grp * Cfg::B_BOX;
+        uint8_t* box = b_tile(s) + grp * Cfg::B_BOX;
         const int jrem = p.J - kb * BK;
         constexpr int NLD = Cfg::ROWS_PER_WARP / 4;
         // loads, then arithmetic, then stores (the stores overwrite what the loads read)
@@ -401,10 +387,9 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll
         for (int x = 0; x < NLD; ++x) {
           const int j = rp * Cfg::ROWS_PER_WARP + 4 * x + jsub;
-          v[x] = *reinterpret_cast<const float4*>(box_hi + sw128_base32_offset(j, c));
+          v[x] = *reinterpret_cast<const float4*>(box + sw128_base32_offset(j, c));
         }
         uint4 hi[NLD];
-        float4 lo[NLD];
 #pragma unroll
         for (int x = 0; x < NLD; ++x) {
           const int j = rp * Cfg::ROWS_PER_WARP + 4 * x + jsub;
@@ -415,38 +400,13 @@ lm2exp_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           e[1] = exp_shifted((rowv && colv[1]) ? v[x].y : -INFINITY, m4[1]);
           e[2] = exp_shifted((rowv && colv[2]) ? v[x].z : -INFINITY, m4[2]);
           e[3] = exp_shifted((rowv && colv[3]) ? v[x].w : -INFINITY, m4[3]);
-          if (PREC) {
-            float4 h;
-            tf32_split_rn(e[0], h.x, lo[x].x);
-            tf32_split_rn(e[1], h.y, lo[x].y);
-            tf32_split_rn(e[2], h.z, lo[x].z);
-            tf32_split_rn(e[3], h.w, lo[x].w);
-            hi[x] = make_uint4(__float_as_uint(h.x), __float_as_uint(h.y), __float_as_uint(h.z), __float_as_uint(h.w));
-          } else {
-            hi[x] = make_uint4(tf32_round_bits(e[0]), tf32_round_bits(e[1]), tf32_round_bits(e[2]),
+          hi[x] = make_uint4(tf32_round_bits(e[0]), tf32_round_bits(e[1]), tf32_round_bits(e[2]),
                                tf32_round_bits(e[3]));
-          }
         }
 #pragma unroll
         for (int x = 0; x < NLD; ++x) {
           const int j = rp * Cfg::ROWS_PER_WARP + 4 * x + jsub;
-          const uint32_t off = sw128_base32_offset(j, c);
-          *reinterpret_cast<uint4*>(box_hi + off) = hi[x];
-          if (PREC) *reinterpret_cast<float4*>(box_lo + off) = lo[x];
-        }
-        if (PREC) {
-          float4* ah = reinterpret_cast<float4*>(a_tile(s, 0));
-          float4* al = reinterpret_cast<float4*>(a_tile(s, 1));
-          for (int ch = tt; ch < Cfg::A_TILE / 16; ch += Cfg::NTT) {
-            const float4 w = ah[ch];
-            float4 h, l;
-            tf32_split_trunc(w.x, h.x, l.x);
-            tf32_split_trunc(w.y, h.y, l.y);
-            tf32_split_trunc(w.z, h.z, l.z);
-            tf32_split_trunc(w.w, h.w, l.w);
-            ah[ch] = h;
-            al[ch] = l;
-          }
+          *reinterpret_cast<uint4*>(box + sw128_base32_offset(j, c)) = hi[x];
         }
         fence_proxy_async_smem();
         __syncwarp();
