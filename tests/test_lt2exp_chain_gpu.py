@@ -103,3 +103,34 @@ def test_argument_checks():
     with pytest.raises(ValueError):
         tb.lt2exp(w.cuda(), a.cuda(), b.cuda(), a_colmax=torch.zeros(1, 31, device="cuda"),
                   b_colmax=torch.zeros(1, 31, device="cuda"))
+
+
+@pytest.mark.parametrize("variant, precision", [(11281, "tf32"), (11282, "tf32"), (11283, "tf32"), (11284, "tf32"), (0, "tf32"),
+                                                (0, "3xtf32"), (11282, "3xtf32"), (99981281, "tf32"), (99981281, "3xtf32")])
+@pytest.mark.parametrize("I, J", [(1, 17), (1, 40), (3, 32), (2, 20)])
+def test_items_of_one_to_three_k_blocks(I, J, variant, precision):
+    """Several tiles per CTA whose contraction is one to three k-blocks (one, 2, 3 and 2 here; one per part in the
+    end-to-end form), few rows and columns at very different levels: a tile may be built by either transform group alone, and
+    the epilogue must see that tile's stabilisers and not those of two tiles before, with a scan of a and b and
+    with supplied maxima (nothing then holds the groups together)."""
+    import triturus_b200 as tb
+
+    R, S, K = 37, 20, 2052
+    g = torch.Generator().manual_seed(I * 100 + J)
+    w = torch.rand(R, S, I, J, generator=g) + 0.01
+    a = torch.randn(R, I, K, generator=g) + 100.0 * torch.randn(R, 1, K, generator=g)
+    b = torch.randn(R, J, K, generator=g) + 100.0 * torch.randn(R, 1, K, generator=g)
+    want = orc.lt2exp_fp64(w, a, b)
+    wd, ad, bd = w.cuda(), a.cuda(), b.cuda()
+    ma, mb = ad.amax(dim=1), bd.amax(dim=1)
+    scanned = tb.lt2exp(wd, ad, bd, precision=precision, variant=variant)
+    res = orc.compare_logspace(scanned.cpu(), want, ATOL[precision])
+    assert res["ok"], res
+    for _ in range(20):
+        out, m = tb.lt2exp(wd, ad, bd, precision=precision, variant=variant, a_colmax=ma, b_colmax=mb, return_colmax=True)
+        assert torch.equal(m, out.amax(dim=1))
+        res = orc.compare_logspace(out.cpu(), want, ATOL[precision])
+        assert res["ok"], res
+        out = tb.lt2exp(wd, ad, bd, precision=precision, variant=variant)
+        assert torch.equal(out, scanned)  # (whole tiles, or parked parts added in a fixed order)
+    tb.check_status()

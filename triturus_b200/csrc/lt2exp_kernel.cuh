@@ -641,10 +641,12 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
       ma = clamp_stab(ma);
       mb = clamp_stab(mb);
       const int slot = tcount & 1;
-      if (grp == 0) {
-        if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-        msum[slot * BN + n] = ma + mb;
-      }
+      // The group that builds the item's first k-block hands the epilogue its stabilisers: the write precedes that
+      // group's arrival on the stage, and stage -> MMA -> accumulator -> epilogue orders it before the read.  (A fixed
+      // group may have no k-block in the item at all: one k-block and an odd stage counter.)  Every group waits
+      // for the slot, since the writer changes from item to item and a wait by parity must not skip a use.
+      if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+      if (grp == static_cast<int>(it % NG)) msum[slot * BN + n] = ma + mb;
 
       for (int jc = w.kb_lo / p.I; ok && jc * p.I < w.kb_hi; ++jc) {
         const int i_lo = lt_row_lo(w, jc, p.I);

@@ -493,10 +493,10 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       ma = clamp_stab(ma);
       mb = clamp_stab(mb);
       const int slot = tcount & 1;
-      if (grp == 0) {
-        if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-        msum[slot * BN + n] = ma + mb;
-      }
+      // Written by the group that builds the item's first k-block, after every group has waited for the slot (see
+      // lt2exp_kernel.cuh).
+      if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+      if (grp == static_cast<int>(it % NG)) msum[slot * BN + n] = ma + mb;
 
       for (int jc = w.kb_lo / p.I; ok && jc * p.I < w.kb_hi; ++jc) {
         const int i_lo = lt_row_lo(w, jc, p.I);
