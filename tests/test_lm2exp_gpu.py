@@ -654,6 +654,21 @@ def test_batches_beyond_the_grid_limit():
     assert torch.equal(tb.colmax(b.cuda()).cpu(), b.amax(dim=1).clamp(-1e38, 1e38))
 
 
+def _tol_3xtf32(a, b, want, terms=None):
+    """Largest error of lm2exp in 3xTF32, per result.  Of a term: its split (weights truncated to 11 bits, low parts of
+    both factors truncated to 11 bits, product of the low parts dropped: 2^-20 + 2^-21 + 2^-21), ex2.approx (2^-22) and the
+    rounding of the exponent's argument (2^-23 of it, weighted with the term's share of the sum).  Of the sum: three
+    truncating additions of the last products (2^-23 each) and 2e-8 for each of the `terms` before (measured: 1.65e-5
+    at 1 024 terms).  Of the result: the logarithm (2^-22) and rounding beside the stabiliser (2^-23)."""
+    a64, b64 = a.double(), b.double()
+    m = b64.amax(dim=1, keepdim=True).clamp(-1e38, 1e38)
+    e = (b64 - m).exp()
+    x = (m - b64).clamp(max=100.0)  # (beyond that e is zero in fp32)
+    arg = torch.bmm(a64, e * x) / torch.bmm(a64, e)
+    terms = a.shape[2] if terms is None else terms
+    return 2.0**-19 + 2 * 2.0**-22 + 2.0**-23 * arg + 3 * 2.0**-23 + 2e-8 * terms + 2.0**-23 * (want.abs() + m.abs())
+
+
 @pytest.mark.parametrize("precision, variant", [("tf32", 2567), ("tf32", 2566), ("tf32", 2564), ("3xtf32", 402564)])
 def test_pair_kernels_back_to_back(precision, variant):
     """Hundreds of launches without a wait in between, on a shape with an odd number of k-blocks and a partly filled row
@@ -678,12 +693,9 @@ def test_pair_kernels_back_to_back(precision, variant):
                                    (1, 1000, 250, 1000), (2, 200, 1025, 129), (1, 500, 4096, 300)])
 @pytest.mark.parametrize("dist", ["normal", "offset", "huge"])
 def test_3xtf32_on_the_tmem_operand_pair_kernel(shape, dist):
-    """3xTF32 on pair tiles: hi * hi in tf32, the corrections in bf16.  One to more k-blocks than there are operand
+    """3xTF32 on pair tiles: hi * hi and both corrections as tf32 products.  One to more k-blocks than there are operand
     stages (four), partial last k-blocks, rows past I, columns past K, isolated and whole-column -inf, weights near the
-    largest float on values that stay above 2^-114 of their column's largest (below it a correction is subnormal, which the
-    tensor core drops).  Tolerance: 2^-17 for the split (four bf16 roundings of 2^-9 on terms of 2^-10 or less), the tensor
-    core's truncating additions (two per eight terms, half an ulp each: 1.2e-8 per term), the rounding of the exponent's
-    argument (2^-23 of the up to 80 that a column spans) and of the result."""
+    largest float.  Tolerance: _tol_3xtf32."""
     R, I, J, K = shape
     g = torch.Generator().manual_seed(sum(shape))
     a = torch.rand(R, I, J, generator=g)
@@ -702,8 +714,26 @@ def test_3xtf32_on_the_tmem_operand_pair_kernel(shape, dist):
     want = orc.lm2exp_fp64(a, b)
     assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
     fin = torch.isfinite(want)
-    tol = 2.0**-17 + 1.2e-8 * J + 80 * 2.0**-23 + 2.0**-22 * want[fin].abs()
-    assert ((got[fin].double() - want[fin]).abs() <= tol).all()
+    assert ((got.double() - want).abs() <= _tol_3xtf32(a, b, want))[fin].all()
+
+
+@pytest.mark.parametrize("variant", [102564, 402564, 1281, 1282])
+@pytest.mark.parametrize("J", [1, 2, 8, 40, 200])
+def test_3xtf32_sums_of_one_term(J, variant):
+    """What does not average out: each result is one product of a weight of 24 bits with exp(b - m), all other weights
+    of the row being zero.  b within 1 of its column's maximum, so that the exponential's own error stays small.  (With
+    corrections of 8 significant bits, as bf16 has, some of them are off by three times the tolerance.)"""
+    g = torch.Generator().manual_seed(J)
+    R, I, K = 3, 700, 300
+    b = -torch.rand(R, J, K, generator=g)
+    a = torch.zeros(R, I, J)
+    a.scatter_(2, torch.randint(0, J, (R, I, 1), generator=g), 0.5 + 1.5 * torch.rand(R, I, 1, generator=g))
+    if variant == 402564:  # (the optimistic pre-pass takes its stabiliser from the first 32 rows)
+        b[:, J // 2:] += 0.25
+    got = _run(a, b, precision="3xtf32", variant=variant)
+    want = orc.lm2exp_fp64(a, b)
+    err = (got.double() - want).abs()
+    assert (err <= _tol_3xtf32(a, b, want, terms=1)).all(), err.max()
 
 
 @pytest.mark.parametrize("scale", [1.0, 1e-30, 3e-45, 0.0])

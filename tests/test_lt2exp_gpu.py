@@ -443,15 +443,31 @@ def test_strided_views_of_a_and_b_are_read_in_place(precision, variant):
     assert res["ok"], res
 
 
+def _tol_3xtf32(w, a, b, want, terms=None):
+    """Largest error of lt2exp in 3xTF32, per result: as for lm2exp (test_lm2exp_gpu.py), with two exponentials and the
+    rounding of their product (2^-24) per term, and the tensor core's truncating additions over at most a chunk of 1 024
+    terms, after which the accumulator is re-summed with rounded additions (2^-24 each)."""
+    R, S, I, J = w.shape
+    tol = []
+    for r in range(R):
+        a64, b64, w64 = a[r].double(), b[r].double(), w[r].double().view(S, I * J)
+        ma, mb = a64.amax(dim=0).clamp(-1e38, 1e38), b64.amax(dim=0).clamp(-1e38, 1e38)
+        xa, xb = (ma - a64).clamp(max=100.0), (mb - b64).clamp(max=100.0)
+        e = ((a64 - ma).exp()[:, None] * (b64 - mb).exp()[None]).view(I * J, -1)
+        arg = (w64 @ (e * (xa[:, None] + xb[None]).view(I * J, -1))) / (w64 @ e)
+        n = I * J if terms is None else terms
+        tol.append(2.0**-19 + 3 * 2.0**-22 + 2.0**-24 + 2.0**-23 * arg + 3 * 2.0**-23 + 2e-8 * min(n, 1024)
+                   + 2.0**-24 * (n // 1024) + 2.0**-23 * (want[r].abs() + ma.abs() + mb.abs()))
+    return torch.stack(tol)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 128, 31, 20, 128), (2, 130, 32, 32, 129), (1, 127, 33, 33, 200),
                                    (2, 40, 7, 300, 90), (1, 200, 100, 64, 260), (1, 128, 256, 256, 130)])
 @pytest.mark.parametrize("split", [1, 3, 9998])
 def test_3xtf32_on_the_tmem_operand_kernel(shape, split):
-    """3xTF32 with the generated operand in tensor memory (hi * hi in tf32, the corrections in bf16): k-blocks around the
-    chunks of 32 after which the accumulator is re-summed, rows and columns around the 128 of a tile, whole tiles, added
-    slices and parts completed through scratch memory.  Tolerance: 2^-17 for the split, 1.2e-8 per term of a chunk of 1 024
-    for the tensor core's truncating additions, the rounding of two exponents' arguments (2^-23 of about 30 each)
-    and of the result."""
+    """3xTF32 with the generated operand in tensor memory (hi * hi and both corrections as tf32 products): k-blocks around
+    the chunks of 32 after which the accumulator is re-summed, rows and columns around the 128 of a tile, whole tiles, added
+    slices and parts completed through scratch memory.  Tolerance: _tol_3xtf32."""
     R, S, I, J, K = shape
     g = torch.Generator().manual_seed(sum(shape))
     w = torch.rand(R, S, I, J, generator=g) + 1e-3
@@ -464,5 +480,21 @@ def test_3xtf32_on_the_tmem_operand_kernel(shape, split):
     want = orc.lt2exp_fp64(w, a, b, chunk=1)
     assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
     fin = torch.isfinite(want)
-    tol = 2.0**-17 + 1.2e-8 * 1024 + 60 * 2.0**-23 + 2.0**-22 * want[fin].abs()
-    assert ((got[fin].double() - want[fin]).abs() <= tol).all()
+    assert ((got.double() - want).abs() <= _tol_3xtf32(w, a, b, want))[fin].all()
+
+
+@pytest.mark.parametrize("variant", [11281, 11282, 12561, 21281])
+@pytest.mark.parametrize("I, J", [(1, 1), (1, 8), (3, 20), (8, 33)])
+def test_3xtf32_sums_of_one_term(I, J, variant):
+    """What does not average out: each result is one product of a weight of 24 bits with the two exponentials, all other
+    weights of the row being zero (see the test of the same name for lm2exp)."""
+    g = torch.Generator().manual_seed(10 * I + J)
+    R, S, K = 2, 600, 260
+    a, b = -torch.rand(R, I, K, generator=g), -torch.rand(R, J, K, generator=g)
+    w = torch.zeros(R, S, I * J)
+    w.scatter_(2, torch.randint(0, I * J, (R, S, 1), generator=g), 0.5 + 1.5 * torch.rand(R, S, 1, generator=g))
+    w = w.view(R, S, I, J)
+    got = _run(w, a, b, precision="3xtf32", variant=variant)
+    want = orc.lt2exp_fp64(w, a, b)
+    err = (got.double() - want).abs()
+    assert (err <= _tol_3xtf32(w, a, b, want, terms=1)).all(), err.max()

@@ -59,15 +59,18 @@ struct Lm2expTsPairCfg {
   static constexpr int BK = 32, NG = NG_, NTW = 4 * NG_, NS = NS_, NSB = NSB_;
   static constexpr int A_TILE = 128 * BK * 4;  // this CTA's rows of a: 16 KB
   static constexpr int B_TILE = BK * BM * 4;   // this CTA's columns of b: 32 rows j x 128 k = 16 KB
-  // PREC (3xTF32): a ring-1 stage also holds the packed bf16 words of the corrections (tf32_split_pack_rn in ptx.cuh), of
-  // a in a second 16 KB tile and of E^T in 32 more TMEM columns.
+  // PREC (3xTF32): e_lo * a_hi + e_hi * a_lo + e_hi * a_hi, all as tf32 MMAs.  A ring-1 stage also holds the low parts, of
+  // a in a second 16 KB tile and of E^T in 32 more TMEM columns.  (The two corrections as bf16 MMAs of twice the rate,
+  // both factors of a term packed into one word, ran R32 1024^3 in 234 us instead of 298 and R64
+  // 512x512x256 in 51 instead of 58.  But bf16 has 8 significant bits: a single term was off by up to 7.1e-6 of itself
+  // instead of 1.1e-6, and that does not average out where one term dominates a sum.)
   static constexpr int PREC = PREC_;
   static constexpr int A_STAGE = (PREC ? 2 : 1) * A_TILE;
   static constexpr int E_COLS = (PREC ? 2 : 1) * BK;  // TMEM columns of an operand stage
   static constexpr int ACC_COLS = BN;
   static constexpr int E_COL0 = ACC_COLS;  // first TMEM column of the operand stages
   static constexpr int TMEM_COLS = 512;
-  static constexpr int NPW = PREC_ ? 4 : 0;  // PREC: warps that write the packed words of a (behind the transform warps)
+  static constexpr int NPW = PREC_ ? 4 : 0;  // PREC: warps that write the low parts of a (behind the transform warps)
   static constexpr int NTHREADS = (8 + NTW + NPW) * 32;
   static constexpr int EPI_STAGE = 4 * 2 * 32 * 128;  // per epilogue warp two 32 x 32 fp32 boxes
   // OPT: no stabiliser pre-pass.  The stabiliser of a column is the maximum over its first k-block (32 rows j),
@@ -110,33 +113,6 @@ __device__ __forceinline__ void umma_tf32_ts_pair(uint32_t d_tmem, uint32_t a_tm
       "}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-
-// The same with bf16 operands, 16 contraction values per MMA: a 32-bit TMEM column of A and a 32-bit word of B hold two.
-__device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                  uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// pack_tile_corrections (ptx.cuh) for a transposed a: the tile holds four boxes of 32 i x 32 j, i contiguous; the packed
-// words are written K-major like those of an ordinary tile.  Thread t of 128 takes row i = t.
-__device__ __forceinline__ void pack_tile_corrections_mn(const uint8_t* tile, uint8_t* packed, int t) {
-  const uint8_t* box = tile + (t >> 5) * 4096 + (t & 3) * 4;
-#pragma unroll 2
-  for (int g = 0; g < 8; ++g) {
-    uint32_t w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      w[e] = tf32_corrections_trunc(*reinterpret_cast<const float*>(box + sw128_base32_offset(g * 4 + e, (t & 31) >> 2)));
-    *reinterpret_cast<uint4*>(packed + sw128_offset(t, g * 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
 }
 
 template <class Cfg>
@@ -196,7 +172,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     *abort_flag = 0;
     for (int s = 0; s < NS; ++s) {
       mbar_init(&a_full[s], 1);
-      mbar_init(&xf_done[s], 2 * 4 + 2 * (Cfg::PREC ? Cfg::NPW : 1));  // four transform warps (one per lane quarter) and the a-tile watcher (PREC: the packing warps), in each CTA
+      mbar_init(&xf_done[s], 2 * 4 + 2 * (Cfg::PREC ? Cfg::NPW : 1));  // four transform warps (one per lane quarter) and the a-tile watcher (PREC: the splitting warps), in each CTA
       mbar_init(&stage_empty[s], 1);
     }
     for (int s = 0; s < NSB; ++s) {
@@ -306,14 +282,13 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     // 128 of the MMA itself: 750 cycles per k-block in plain TF32, 1 300 in 3xTF32.)
     if (leader) {
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
-      // PREC takes a transposed a too: MN-major for the tf32 MMAs (bit 16), while its packed words are always K-major.
+      // PREC takes a transposed a too: MN-major (bit 16), its low parts in the same layout.
       const bool a_mn = Cfg::PREC && p.a_mn != 0;
       const uint32_t idesc = umma_idesc_tf32(2 * BM, BN / Cfg::NH) | (a_mn ? 1u << 16 : 0u);
       const uint32_t a_step = a_mn ? 64u : 2u;  // encoded address step per 8 contraction values
       constexpr uint32_t HALF_ENC = (64 * BK * 4) >> 4;  // 64 rows of a further
       constexpr uint32_t STAGE_ENC = Cfg::A_STAGE >> 4;
       const uint64_t db0 = a_mn ? umma_desc_mn_sw128_base32(smem_u32(a_tile(0)), 4096) : umma_desc_k_sw128(smem_u32(a_tile(0)));
-      const uint64_t dbp0 = umma_desc_k_sw128(smem_u32(a_tile(0)) + Cfg::A_TILE);
       uint32_t s = 0, ph = 0, tcount = 0;
       bool ok = true;
       auto advance = [&]() {
@@ -328,11 +303,14 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const uint64_t db = db0 + st * STAGE_ENC + h * HALF_ENC;
         const uint32_t ea = tmem_base + Cfg::E_COL0 + st * Cfg::E_COLS;
         if (Cfg::PREC) {
-          // e_lo * a_hi + e_hi * a_lo: 64 bf16 values per k-block, in rows of 128 bytes like the tf32 operands.  First,
-          // while the accumulator of a tile is empty: the sum of the first k-block's corrections is not truncated then.
+          // The corrections first, while the accumulator of a tile is empty: the sum of the first k-block's is not
+          // truncated to the bits of the whole sum then.
 #pragma unroll
           for (int ks = 0; ks < BK / 8; ++ks)
-            umma_bf16_ts_pair(d, ea + BK + ks * 8, dbp0 + st * STAGE_ENC + 2 * ks, umma_idesc_bf16(2 * BM, BN), (accumulate || ks > 0) ? 1u : 0u);
+            umma_tf32_ts_pair(d, ea + BK + ks * 8, db + a_step * ks, idesc, (accumulate || ks > 0) ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < BK / 8; ++ks)
+            umma_tf32_ts_pair(d, ea + ks * 8, db + (Cfg::A_TILE >> 4) + a_step * ks, idesc, 1u);
         }
 #pragma unroll
         for (int ks = 0; ks < BK / 8; ++ks)
@@ -390,7 +368,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     __syncwarp();
   } else if (warp == 3 && !Cfg::PREC) {
     // ------------------------------------------------------------------ a-tile watcher
-    // (3xTF32: the packing warps wait for the tile of a)
+    // (3xTF32: the splitting warps wait for the tile of a)
     // The leader's MMA thread reads both CTAs' tiles of a and waits only on xf_done: this lane adds "this CTA's
     // tile of a has landed" to that barrier, so that the transform warps need not wait for it in their chain.
     if (lane == 0) {
@@ -532,7 +510,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (__any_sync(0xffffffffu, acc_max >= 0x7f800000u) && lane == 0) *p.opt_flag = 1;
     }
   } else if (Cfg::PREC && warp >= 8 + Cfg::NTW) {
-    // ------------------------------------------------------------------ packing: the corrections of the tile of a
+    // ------------------------------------------------------------------ splitting: the low parts of the tile of a
     // The tile itself stays as it is (the tensor core drops the low 13 bits).
     const int t = threadIdx.x - (8 + Cfg::NTW) * 32;
     const uint32_t xf_done_leader0 = map_to_cta(smem_u32(&xf_done[0]), 0);
@@ -542,8 +520,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       for (int kb = 0; kb < KB; ++kb, ++it) {
         const int s = it % NS;
         if (!(ok = mbar_wait_warp(&a_full[s], (it / NS) & 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-        if (p.a_mn) pack_tile_corrections_mn(a_tile(s), a_tile(s) + Cfg::A_TILE, t);
-        else pack_tile_corrections(a_tile(s), a_tile(s) + Cfg::A_TILE, t);
+        write_tile_lo(a_tile(s), a_tile(s) + Cfg::A_TILE, t);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(xf_done_leader0 + static_cast<uint32_t>(s) * 8u);
@@ -684,11 +661,11 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if constexpr (Cfg::PREC != 0) {
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            uint32_t hi[16], pk[16];
+            float hi[16], lo[16];
 #pragma unroll
-            for (int x = 0; x < 16; ++x) tf32_split_pack_rn(__uint_as_float(e[h * 16 + x]), hi[x], pk[x]);
+            for (int x = 0; x < 16; ++x) tf32_split_rn(__uint_as_float(e[h * 16 + x]), hi[x], lo[x]);
             tmem_st_32x16(ebase + s * Cfg::E_COLS + h * 16, hi);
-            tmem_st_32x16(ebase + s * Cfg::E_COLS + BK + h * 16, pk);
+            tmem_st_32x16(ebase + s * Cfg::E_COLS + BK + h * 16, lo);
           }
         } else {
           tmem_st_32x32(ebase + s * Cfg::E_COLS, e);

@@ -33,14 +33,12 @@
 
 namespace tb200 {
 
-// PREC (3xTF32): hi * hi as tf32 MMAs and the two corrections as bf16 MMAs at twice the rate on packed words
-// (tf32_split_pack_rn in ptx.cuh).  The w tile serves the tf32 MMAs as it lies in shared memory (the tensor core
-// truncates); four packing warps (16-19) write its packed words to a second tile, the transform warps P^T and its packed
-// words to 64 TMEM columns.  (With the packing in the transform warps a k-block took 960 cycles: their chain of waits,
-// arithmetic and fences was what bounded it, tensor pipe 53 % and shared-memory pipe 60 % active.)
-// Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the packing, 32 KB read by the tensor
-// core = 640 cycles of the shared-memory pipe next to 512 of the tensor pipe (all operands in shared memory and three
-// tf32 products: 1 400 next to 768).
+// PREC (3xTF32): p_lo * w_hi + p_hi * w_lo + p_hi * w_hi, all as tf32 MMAs.  The w tile serves them as it lies in shared
+// memory (the tensor core truncates); four splitting warps (16-19) write its low parts to a second tile, the transform
+// warps both parts of P^T to 64 TMEM columns.  (The corrections as bf16 MMAs of twice the rate: R32 256^4 1 154 instead of
+// 1 298 us, but terms off by up to 7e-6, see lm2exp_tspair_kernel.cuh.)
+// Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the splitting, 48 KB read by the tensor
+// core = 768 cycles of the shared-memory pipe next to 768 of the tensor pipe (both operands in shared memory: 1 400).
 // Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
 // master copy in shared memory (see "Accumulator promotion" in lt2exp_kernel.cuh; TMEM has no room for a third).
 template <int MT_, int NS_, int NB_ = 1, int PREC_ = 0>
@@ -53,7 +51,7 @@ struct Lt2expTmemCfg {
   static constexpr int CHUNK = PROMOTE ? 32 : 1 << 30;
   static constexpr int W_TILE = BM * BK * 4;
   static constexpr int W_BYTES = MT * W_TILE;             // what TMA brings per stage
-  static constexpr int STAGE = (PREC ? 2 : 1) * W_BYTES;  // ... and the packed words of it
+  static constexpr int STAGE = (PREC ? 2 : 1) * W_BYTES;  // ... and the low parts of it
   static constexpr int BLK_COLS = MT * BM;        // accumulator columns of one column block
   static constexpr int ACC_COLS = NB * BLK_COLS;
   static constexpr int P_STAGE = NB * (PREC ? 2 : 1) * BK;  // operand columns per stage
@@ -61,7 +59,7 @@ struct Lt2expTmemCfg {
   static constexpr int P_COL0 = NBUF * ACC_COLS;  // first operand column
   static constexpr int TMEM_USED = P_COL0 + NS * P_STAGE;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int NPW = PREC ? 4 : 0;  // packing warps
+  static constexpr int NPW = PREC ? 4 : 0;  // splitting warps
   static constexpr int NTHREADS = (8 + NTW + NPW) * 32;
   static constexpr int NTT = NTW * 32;
   static constexpr int NGROUPS = NTT / BN;
@@ -99,7 +97,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   float* mpart = msum + 2 * BN;                                    // [2][2][RG][BN] partial column maxima
   uint64_t* bars = reinterpret_cast<uint64_t*>(mpart + 2 * Cfg::MPART);
   uint64_t* full = bars;                 // [NS] w tile landed (TMA bytes) and operand stage written to TMEM
-  uint64_t* w_full = bars + NS;          // PREC [NS] w tile landed (the packing warps wait for it)
+  uint64_t* w_full = bars + NS;          // PREC [NS] w tile landed (the splitting warps wait for it)
   uint64_t* opnd_empty = bars + 2 * NS;  // [NS] MMAs reading the stage (shared memory and TMEM) retired
   uint64_t* acc_full = bars + 3 * NS;    // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
@@ -116,7 +114,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     *abort_flag = 0;
     for (int s = 0; s < NS; ++s) {
       if (Cfg::PREC) mbar_init(&w_full[s], 1);
-      // the producer (PREC: the packing warps instead) and the warps that write the operand stage
+      // the producer (PREC: the splitting warps instead) and the warps that write the operand stage
       mbar_init(&full[s], (Cfg::PREC ? Cfg::NPW : 1) + Cfg::NTW / Cfg::NGROUPS);
       mbar_init(&opnd_empty[s], 1);
     }
@@ -215,12 +213,12 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
             const uint64_t dw = umma_desc_k_sw128(stage0 + s * Cfg::STAGE);
             const uint32_t pa = tmem_base + Cfg::P_COL0 + s * Cfg::P_STAGE;
             if (Cfg::PREC) {
-              // p_lo * w_hi + p_hi * w_lo: 64 bf16 values in rows of 128 bytes like the tf32 operands.  First, while
-              // the accumulator of a chunk is empty and does not truncate them
+              // the corrections first, while the accumulator of a chunk is empty and does not truncate them to its bits
 #pragma unroll
               for (int ks = 0; ks < BK / 8; ++ks)
-                umma_bf16_ts(d, pa + BK + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, umma_idesc_bf16(128, BM * MT),
-                             (kb > kb0 || ks > 0) ? 1u : 0u);
+                umma_tf32_ts(d, pa + BK + ks * 8, dw + 2 * ks, idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+              for (int ks = 0; ks < BK / 8; ++ks) umma_tf32_ts(d, pa + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, idesc, 1u);
             }
 #pragma unroll
             for (int blk = 0; blk < Cfg::NB; ++blk) {  // the column blocks share the w tile
@@ -415,7 +413,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       }
     }
   } else if (Cfg::PREC && warp >= 8 + Cfg::NTW) {
-    // ------------------------------------------------------------------ packing: the corrections of the w tile
+    // ------------------------------------------------------------------ splitting: the low parts of the w tile
     const int t = threadIdx.x - (8 + Cfg::NTW) * 32;
     int s = 0;
     uint32_t ph = 0;
@@ -424,7 +422,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     for (LtItem w; ok && work.next(w);) {
       for (int kb = w.kb_lo; kb < w.kb_hi; ++kb) {
         if (!(ok = mbar_wait_warp(&w_full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-        pack_tile_corrections(stage_base + s * Cfg::STAGE, stage_base + s * Cfg::STAGE + Cfg::W_BYTES, t);
+        write_tile_lo(stage_base + s * Cfg::STAGE, stage_base + s * Cfg::STAGE + Cfg::W_BYTES, t);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[s]);
@@ -543,11 +541,11 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
               tc_fence_after_sync();
 #pragma unroll
               for (int h = 0; h < 2; ++h) {  // 16 of the 32 terms at a time: both words of all 32 do not fit in registers
-                uint32_t hi[16], pk[16];
+                float hi[16], lo[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) tf32_split_pack_rn(ea * eb[h * 16 + e], hi[e], pk[e]);
+                for (int e = 0; e < 16; ++e) tf32_split_rn(ea * eb[h * 16 + e], hi[e], lo[e]);
                 tmem_st_32x16(lane_base + s * Cfg::P_STAGE + h * 16, hi);
-                tmem_st_32x16(lane_base + s * Cfg::P_STAGE + BK + h * 16, pk);
+                tmem_st_32x16(lane_base + s * Cfg::P_STAGE + BK + h * 16, lo);
               }
               tmem_st_wait();
               tc_fence_before_sync();

@@ -318,12 +318,12 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&v
 }
 
 // The same for 16 columns.
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const float (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+      "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
       : "memory");
 }
 
@@ -376,11 +376,6 @@ __device__ __forceinline__ uint32_t sw128_base32_offset(uint32_t j, uint32_t c) 
 __host__ __device__ constexpr uint32_t umma_idesc_tf32(int m, int n) {
   return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
          (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-// The same for A = B = bf16.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 // One MMA D[tmem] (+)= A[smem] * B[smem], issued by a single thread.
@@ -437,19 +432,6 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t"
-      "}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The same with bf16 operands, two per 32-bit TMEM column of A and word of B, 16 contraction values per MMA.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
@@ -519,37 +501,19 @@ __device__ __forceinline__ void tf32_split_rn(float x, float& hi, float& lo) {
   hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
   lo = x - hi;
 }
-// 3xTF32 with the corrections in bf16.  x = hi + lo with hi in tf32; hi_x * hi_y runs as tf32 MMAs, and
-// lo_x * hi_y + hi_x * lo_y, 2^-11 of it, as bf16 MMAs at twice the rate on words that hold both factors: the generated
-// operand has lo in the lower half and hi in the upper, the weights the reverse, so that a dot product over the halves
-// gives the two terms.  bf16 rounds a factor to 2^-9 of it, to nearest, i.e. the product to about 2^-20 without bias.
-// That is below what the all-tf32 form loses: the tensor core truncates there, the low parts to tf32 and the accumulator
-// at each of three additions per eight terms, of which this form needs two.
-__device__ __forceinline__ uint32_t pack_bf16x2(float upper, float lower) {
-  uint32_t d;  // (satfinite: rounding the largest floats up must not make an infinity of them)
-  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(upper), "f"(lower));
-  return d;
-}
-__device__ __forceinline__ void tf32_split_pack_rn(float x, uint32_t& hi, uint32_t& packed) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
-  packed = pack_bf16x2(__uint_as_float(hi), x - __uint_as_float(hi));
-}
-// (the weights enter the tf32 MMAs as they are, i.e. truncated)
-__device__ __forceinline__ uint32_t tf32_corrections_trunc(float w) {
-  const float hi = __uint_as_float(__float_as_uint(w) & 0xFFFFE000u);
-  return pack_bf16x2(w - hi, hi);
-}
-// Packed corrections of a 16 KB operand tile, word for word: thread t of 128.
-__device__ __forceinline__ void pack_tile_corrections(const uint8_t* tile, uint8_t* packed, int t) {
+// The weights' side of the 3xTF32 scheme where they enter the high products as they are, i.e. truncated by the tensor
+// core: lo = x - trunc(x), exact in fp32.
+__device__ __forceinline__ float tf32_lo_trunc(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
+// The low parts of a 16 KB operand tile, word for word in the same layout: thread t of 128.
+__device__ __forceinline__ void write_tile_lo(const uint8_t* tile, uint8_t* lo, int t) {
   const float4* src = reinterpret_cast<const float4*>(tile) + t;
-  uint4* dst = reinterpret_cast<uint4*>(packed) + t;
+  float4* dst = reinterpret_cast<float4*>(lo) + t;
   float4 v[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) v[c] = src[c * 128];
 #pragma unroll
   for (int c = 0; c < 8; ++c)
-    dst[c * 128] = make_uint4(tf32_corrections_trunc(v[c].x), tf32_corrections_trunc(v[c].y), tf32_corrections_trunc(v[c].z),
-                              tf32_corrections_trunc(v[c].w));
+    dst[c * 128] = make_float4(tf32_lo_trunc(v[c].x), tf32_lo_trunc(v[c].y), tf32_lo_trunc(v[c].z), tf32_lo_trunc(v[c].w));
 }
 
 __device__ __forceinline__ void tf32_split_trunc(float x, float& hi, float& lo) {
