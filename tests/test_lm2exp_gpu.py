@@ -762,6 +762,30 @@ def test_logarithm_of_the_3xtf32_epilogue(scale):
         assert ((got[cmp].double() - want[cmp]).abs() <= 2 * ulp + 2.0**-22 * 0.6932).all()
 
 
+@pytest.mark.parametrize("precision, variant", [("3xtf32", 102564), ("3xtf32", 402564), ("3xtf32", 101282), ("tf32", 2566), ("tf32", 102564)])
+def test_results_do_not_depend_on_their_neighbours(precision, variant):
+    """A column's and a row's results to the bit, whatever stands beside them: dead columns, rows of zero weights, rows
+    past the end of the result, and the columns alone (what a rank of a column-sharded call computes)."""
+    import triturus_b200 as tb
+
+    g = torch.Generator(device="cuda").manual_seed(11)
+    a = torch.rand(2, 320, 96, generator=g, device="cuda")
+    b = 3.0 * torch.randn(2, 96, 512, generator=g, device="cuda")
+    base = tb.lm2exp(a, b, precision=precision, variant=variant)
+    dead = b.clone()
+    dead[:, :, 5::32] = float("-inf")
+    zero = a.clone()
+    zero[:, 7::32] = 0.0
+    got = tb.lm2exp(zero, dead, precision=precision, variant=variant)
+    live_i = torch.arange(320, device="cuda") % 32 != 7
+    live_k = torch.arange(512, device="cuda") % 32 != 5
+    assert torch.equal(got[:, live_i][:, :, live_k], base[:, live_i][:, :, live_k])
+    assert (got[:, ~live_i] == float("-inf")).all() and (got[:, :, ~live_k] == float("-inf")).all()
+    assert torch.equal(tb.lm2exp(a[:, :301], b, precision=precision, variant=variant), base[:, :301])
+    assert torch.equal(tb.lm2exp(a, b[:, :, 100:360], precision=precision, variant=variant), base[:, :, 100:360])
+    tb.check_status()
+
+
 @pytest.mark.parametrize("variant", [2566, 2567])
 @pytest.mark.parametrize("shape", [(3, 129, 32, 130), (2, 200, 256, 300), (2, 256, 255, 257), (80, 321, 225, 260), (2, 448, 257, 256)])
 def test_accumulator_in_halves_of_the_tmem_operand_pair_kernel(shape, variant):
