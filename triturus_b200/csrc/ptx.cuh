@@ -465,40 +465,6 @@ __device__ __forceinline__ float lg2_approx(float x) {
 // exp(v - m) with the subtraction done first, as the reference does (baselines/lm2exp.py:13).
 __device__ __forceinline__ float exp_shifted(float v, float m) { return ex2_approx((v - m) * LOG2E_F); }
 
-// Natural logarithm of a positive normal float: x = 2^k m with m in [0.75, 1.5), ln 2 (k + log2 m).  lg2.approx is off by
-// at most 2^-22 there, half of what the exps of the sum's terms are.  `shift` is subtracted from k.
-__device__ __forceinline__ float log_normal(uint32_t bits, float shift = 0.f) {
-  const uint32_t k23 = (bits - 0x3f400000u) & 0xff800000u;  // k << 23
-  const float l = lg2_approx(__uint_as_float(bits - k23));
-  const float k = __int_as_float(0x4b400000 + (static_cast<int32_t>(k23) >> 23)) - (12582912.0f + shift);  // past the conversion unit
-  return fmaf(k, LN2_F, l * LN2_F);
-}
-// The same for any float: subnormals scaled by 2^24, zeros -inf, +inf itself, negative values and NaN NaN.  Bit for bit
-// log_normal on positive normal floats, so that which of the two a block takes does not show in its results.
-__device__ __forceinline__ float log_any(uint32_t bits) {
-  const float x = __uint_as_float(bits);
-  const bool sub = bits < 0x00800000u;
-  const float l = log_normal(sub ? __float_as_uint(x * 16777216.0f) : bits, sub ? 24.0f : 0.0f);
-  return x > 0.f ? (x < INFINITY ? l : x) : (x == 0.f ? -INFINITY : NAN);
-}
-// Replaces 32 accumulator values by their logarithms.  Straight-line code for normal floats only when every value of the
-// warp is one.  (logf, with its own handling of the other cases per value, took 3 700 cycles per block in the
-// epilogue of the 3xTF32 pair kernel: with the registers of one block only, R32 1024^3 292 -> 239 us, R64 512x512x256
-// 69.9 -> 51.4 us.  The kernels whose tiles are few keep logf: the second path through the code costs them more
-// instruction fetches than it saves, R24 150x101x203 39.2 -> 41.0 us.)
-__device__ __forceinline__ void log_block(uint32_t (&v)[32]) {
-  uint32_t odd = 0;
-#pragma unroll
-  for (int e = 0; e < 32; ++e) odd = max(odd, v[e] - 0x00800000u);
-  if (__any_sync(0xffffffffu, odd >= 0x7f000000u)) {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(log_any(v[e]));
-  } else {
-#pragma unroll
-    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(log_normal(v[e]));
-  }
-}
-
 // Round an fp32 in [0, +inf) to the nearest tf32 (ties away), as raw bits.  The tensor core drops the low
 // 13 mantissa bits of its operands, so adding half a tf32 ulp beforehand turns that truncation into
 // rounding.  Not valid for inf/nan.
