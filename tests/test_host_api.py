@@ -256,6 +256,14 @@ def test_operand_preparation_rules():
     assert not _native._in_place_small(b_odd.double(), 1e6, 0, False)
 
 
+def test_odd_operands_are_read_in_place_only_where_that_is_faster():
+    """Two to three times slower than the padded copy from 1e9 FLOP on, faster by the host's work for the copy at 1.5e8."""
+    b_odd = torch.zeros(2, 64, 97)
+    assert _native._lm2exp_b_operand(b_odd, 0, flop=1.5e8) is b_odd
+    got = _native._lm2exp_b_operand(b_odd, 0, flop=1e9)
+    assert got is not b_odd and _native._tma_ok(got) and torch.equal(got, b_odd)
+
+
 def test_automatic_plans_of_lm2exp():
     """What a call runs for the benchmark shapes and around the size rule of the optimistic stabilisers (the plan
     queries need no GPU: without one they assume 148 SMs)."""

@@ -260,10 +260,14 @@ def _pad_rows(t: torch.Tensor, buf: torch.Tensor) -> bool:
 
 
 # Problems up to this many FLOP take operands that break the tensor-map rules in place (the single-CTA kernel then
-# fetches them element by element, ~3x slower per k-block than through TMA); larger ones get the padded copy, which
-# is the cheaper of the two there.  Measured: R24 150x101x203 0.035 ms in place / 0.072 ms with the copy;
-# R32 1024x1024x1022 0.75 / 0.26 ms; R128 256x256x8190 1.20 / 1.60 ms in TF32 but 2.97 / 2.32 ms in 3xTF32.
-_IN_PLACE_MAX_FLOP = 8e9
+# fetches them element by element, about three times slower per k-block than through TMA); larger ones get the padded copy.
+# The line lies where a loop of calls takes equally long: below it the host's work for the copies (two allocations and
+# launches, 12 us or more per call) is what counts, above it the fetch.  Microseconds per call, in place / with
+# the copies, both operands odd: 1.5e8 (R24 150x101x203) 40 / 46 in 3xTF32 and 33 / 46 in TF32; 3.9e8 (R64, the same)
+# 61 / 46 and 45 / 47; 1.0e9 (R8 255x255x1001) 66 / 47 and 54 / 47; 1.1e9 (R4 511^3) 117 / 48 and 93 / 47; 4.0e9 (R2
+# 1001^3) 219 / 75 and 174 / 60; 8.6e9 (R128 64x64x8191) 777 / 812 and 534 / 507.  One odd operand, or an inner stride
+# of 2 (copied by torch): the same side of the line, except TF32 at 1.1e9 with an odd a alone, 31 / 33.
+_IN_PLACE_MAX_FLOP = 3e8
 
 
 def _in_place_small(t: torch.Tensor, flop: float, variant: int, want_colmax: bool) -> bool:
