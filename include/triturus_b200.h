@@ -139,7 +139,9 @@ int triturus_b200_lm2exp_chain_f32(const float* a, const float* b, float* out, i
  *   variant: 0 = automatic, otherwise SPLIT * 10000 + BN * 10 + MT with BN * 10 + MT as above (0 = automatic;
  *            additionally, TF32 only, the generated operand kept in tensor memory instead of shared memory:
  *            1283 / 1284 = tile of 128 columns x 128 / 256 rows, 1285 = 256 columns x 128 rows, which the
- *            automatic choice uses where it would otherwise take 2561)
+ *            automatic choice uses where it would otherwise take 2561; in 3xTF32 the codes 1281, 1282, 2561 and 2562
+ *            all run the one kernel of that precision, 128 columns x 128 rows with the generated operand in tensor
+ *            memory, and plans name it 1281)
  *            and SPLIT the number of slices the contraction over (i, j) of every output tile is cut into, the
  *            counterpart of the reference's NUM_SPLITS and mode argument (triturus/lt2exp.py:533-541):
  *            0 = automatic (slices when the output tiles would occupy fewer than half the SMs; when the last

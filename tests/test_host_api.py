@@ -256,6 +256,19 @@ def test_operand_preparation_rules():
     assert not _native._in_place_small(b_odd.double(), 1e6, 0, False)
 
 
+def test_lt2exp_tile_codes_in_3xtf32():
+    """All shared-memory tile codes run the one 3xTF32 kernel, with the split they ask for; the codes of the plain-TF32
+    kernels that keep the operand in tensor memory are refused."""
+    plan, ws = _native.LIB.triturus_b200_lt2exp_plan, _native.LIB.triturus_b200_lt2exp_workspace_bytes
+    shape = (8, 256, 128, 128, 4096)
+    for tile in (0, 1281, 1282, 2561, 2562):
+        assert plan(*shape, 1, 10000 + tile) == 11281 and plan(*shape, 1, 30000 + tile) == 31281
+        assert plan(*shape, 1, 99980000 + tile) == 99981281
+        assert ws(*shape, 1, 99980000 + tile) == ws(*shape, 1, 99981281) > 0
+    for tile in (1283, 1284, 1285):
+        assert plan(*shape, 1, 10000 + tile) < 0
+
+
 def test_odd_operands_are_read_in_place_only_where_that_is_faster():
     """Two to three times slower than the padded copy from 1e9 FLOP on, faster by the host's work for the copy at 1.5e8."""
     b_odd = torch.zeros(2, 64, 97)

@@ -1207,17 +1207,15 @@ using LtM_2 = Lt2expTmemCfg<2, 6>;
 using LtM_1x2 = Lt2expTmemCfg<1, 4, 2>;  // 128 rows x two 128-column blocks sharing each w tile
 using LtMX_1 = Lt2expTmemCfg<1, 4, 1, 1>;  // 3xTF32, 128 x 128
 
-//                          BN   MT PREC NS NTW
-using LtT_128_1 = Lt2expCfg<128, 1, 0, 6, 8>;
-using LtT_128_2 = Lt2expCfg<128, 2, 0, 4, 8>;
-using LtT_256_1 = Lt2expCfg<256, 1, 0, 4, 8>;
-using LtT_256_2 = Lt2expCfg<256, 2, 0, 3, 8>;
-using LtX_128_2 = Lt2expCfg<128, 2, 1, 2, 8>;
-using LtX_256_1 = Lt2expCfg<256, 1, 1, 2, 8>;
+//                          BN   MT NS NTW
+using LtT_128_1 = Lt2expCfg<128, 1, 6, 8>;
+using LtT_128_2 = Lt2expCfg<128, 2, 4, 8>;
+using LtT_256_1 = Lt2expCfg<256, 1, 4, 8>;
+using LtT_256_2 = Lt2expCfg<256, 2, 3, 8>;
 // plain TF32 with chunked re-summation of the accumulator (contractions of more than 32 K terms)
-using LtP_128_1 = Lt2expCfg<128, 1, 0, 6, 8, true>;
-using LtP_128_2 = Lt2expCfg<128, 2, 0, 4, 8, true>;
-using LtP_256_1 = Lt2expCfg<256, 1, 0, 4, 8, true>;
+using LtP_128_1 = Lt2expCfg<128, 1, 6, 8, true>;
+using LtP_128_2 = Lt2expCfg<128, 2, 4, 8, true>;
+using LtP_256_1 = Lt2expCfg<256, 1, 4, 8, true>;
 
 }  // namespace tb200
 
@@ -1231,17 +1229,21 @@ static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int6
   *split = variant / 10000;
   int tile = variant % 10000;
   const bool long_tf = precision == TRITURUS_B200_PRECISION_TF32 && I * ((J + 31) / 32 * 32) > tb200::kLongContraction;
-  if (tile == 0) {
+  if (precision == TRITURUS_B200_PRECISION_3XTF32) {
+    // One kernel, which keeps the generated operand in TMEM on 128 x 128 tiles; the codes of the other shared-memory tiles
+    // stay accepted and run it too.  (Their own instances, both operands and their low parts in shared memory with
+    // two stages, us on 1281 / 1282 / 2561: R32 256^4 1 154 / 3 180 / 2 603, R64 256x128x128x4096 8 480 / 11 740 / 9 590, R16
+    // 128x64x64x2048 148 / 425 / 160, R64 128x16x16x1024 69 / 136 / 68, R8 300x32x32x1000 55 / 67 / 52; 15 more shapes:
+    // 1281 the fastest.)
+    if (tile == 0 || tile == 1282 || tile == 2561 || tile == 2562) tile = 1281;
+  } else if (tile == 0) {
     tile = tb200::auto_variant(R, S, K, true, false, long_tf ? 256 : 512);
     // 128 rows x 256 columns in TF32: the kernel that keeps the generated operand in TMEM moves a third of
     // the shared-memory bytes per k-block (measured 8 % faster on such tiles).
-    if (tile == 2561 && precision == TRITURUS_B200_PRECISION_TF32 && !long_tf) tile = 1285;
-    if (precision == TRITURUS_B200_PRECISION_3XTF32) tile = 1281;
+    if (tile == 2561 && !long_tf) tile = 1285;
   }
   *bn = tile / 10;
   *mt = tile % 10;
-  // 3xTF32 keeps hi and lo copies of both operands: two row blocks leave room for 128 columns only
-  if (precision == TRITURUS_B200_PRECISION_3XTF32 && *bn == 256 && *mt == 2) *bn = 128;
   *promote = long_tf && (tile == 1281 || tile == 1282 || tile == 2561);
   // operand in TMEM: 128 columns x 128 / 256 rows (1283 / 1284), 256 columns x 128 rows (1285)
   if (*bn == 128 && (*mt == 3 || *mt == 4 || *mt == 5)) return TRITURUS_B200_OK;
@@ -1270,10 +1272,7 @@ static int lt2exp_dispatch(int precision, int bn, int mt, bool promote, Args... 
     if (mt == 5) return launch_lt2exp_tmem<LtM_1x2>(args...);
     return mt == 4 ? launch_lt2exp_tmem<LtM_2>(args...) : launch_lt2exp_tmem<LtM_1>(args...);
   }
-  if (precision == TRITURUS_B200_PRECISION_3XTF32) {
-    if (bn == 256 && mt == 1) return launch_lt2exp<LtX_256_1>(args...);
-    return mt == 2 ? launch_lt2exp<LtX_128_2>(args...) : launch_lt2exp_tmem<LtMX_1>(args...);
-  }
+  if (precision == TRITURUS_B200_PRECISION_3XTF32) return launch_lt2exp_tmem<LtMX_1>(args...);
   if (bn == 256) return mt == 2 ? launch_lt2exp<LtT_256_2>(args...) : launch_lt2exp<LtT_256_1>(args...);
   return mt == 2 ? launch_lt2exp<LtT_128_2>(args...) : launch_lt2exp<LtT_128_1>(args...);
 }

@@ -1,7 +1,8 @@
 // lt2exp:  out[r,s,k] = ma[r,k] + mb[r,k] + log( sum_{i,j} w[r,s,i,j] * exp(a[r,i,k]-ma[r,k]) * exp(b[r,j,k]-mb[r,k]) )
 //
 // Replaces the reference's Triton kernels _ker_lt2exp_unsplit / _ker_lt2exp_split
-// (triturus/lt2exp.py:227-357, 365-506) with one persistent, warp-specialised sm_100a kernel.
+// (triturus/lt2exp.py:227-357, 365-506) with one persistent, warp-specialised sm_100a kernel.  This file: plain TF32 with
+// the generated operand in shared memory, and what lt2exp_tmem_kernel.cuh (3xTF32, and some plain TF32 tiles) shares with it.
 // As a GEMM: D[M = s, N = k] = W[M, Kc = (i,j)] * P[Kc, N] with the Khatri-Rao operand
 // P[(i,j), k] = exp(a[i,k]-ma[k]) * exp(b[j,k]-mb[k]), which is generated tile by tile in shared memory and
 // never written to HBM (the reference's torch baseline materialises it, baselines/lt2exp.py:21-22, and its
@@ -27,14 +28,12 @@
 // epilogue adds its raw accumulator into the zero-filled output with red.global.add and
 // lt2exp_finish_kernel then turns the sums into (ma + mb) + log(sum) in place.
 //
-// Accumulator promotion (3xTF32 always; plain TF32 in the PROMOTE instances the launcher picks for contractions
-// of more than 32 K terms).  The tensor core adds into its fp32 accumulator with truncation, so a
+// Accumulator promotion (the PROMOTE instances the launcher picks for contractions of more than 32 K terms; the
+// 3xTF32 kernel always, see lt2exp_tmem_kernel.cuh).  The tensor core adds into its fp32 accumulator with truncation, so a
 // sum of positive terms drifts low by about half an ulp per MMA: ~3e-8 relative per 8 contraction terms,
-// 1e-4 after 32 K terms and 2.5e-3 after 256 K, far more than the 3xTF32 operand error.  In 3xTF32 mode
-// the MMA warp therefore starts a fresh TMEM accumulator every CHUNK k-blocks and the epilogue warps, idle
+// 1e-4 after 32 K terms and 2.5e-3 after 256 K.  The MMA warp therefore starts a fresh TMEM accumulator every CHUNK k-blocks and the epilogue warps, idle
 // during the main loop, add each finished chunk into a master copy kept in a further TMEM region with
-// round-to-nearest fp32 adds (tcgen05.ld, add, tcgen05.st).  Plain TF32 on shorter contractions keeps one chunk
-// per work item: the drift stays below 3e-4 there, well inside the 2e-3 tolerance of that mode.
+// round-to-nearest fp32 adds (tcgen05.ld, add, tcgen05.st).  Shorter contractions keep one chunk per work item: the drift stays below 3e-4 there, well inside the 2e-3 tolerance of that mode.
 #pragma once
 
 #include "ptx.cuh"
@@ -191,19 +190,18 @@ __device__ __forceinline__ int lt_row_hi(const LtItem& w, int jc, int I) {
   return hi < I ? hi : I;
 }
 
-template <int BN_, int MT_, int PREC_, int NS_, int NTW_, bool PROMOTE_ = (PREC_ != 0)>
+template <int BN_, int MT_, int NS_, int NTW_, bool PROMOTE_ = false>
 struct Lt2expCfg {
   static constexpr int BM = 128, BK = 32;
-  static constexpr int BN = BN_, MT = MT_, PREC = PREC_, NS = NS_, NTW = NTW_;
-  static constexpr int NCOPY = PREC ? 2 : 1;
+  static constexpr int BN = BN_, MT = MT_, PREC = 0, NS = NS_, NTW = NTW_;
   static constexpr int A_TILE = BM * BK * 4;
   static constexpr int B_TILE = BN * BK * 4;
-  static constexpr int STAGE = NCOPY * (MT * A_TILE + B_TILE);
+  static constexpr int STAGE = MT * A_TILE + B_TILE;
   static constexpr int ACC_COLS = MT * BN;
   static constexpr bool PROMOTE = PROMOTE_;
-  // k-blocks (of 32 terms) accumulated by the tensor core before a promotion: 1 K terms keep the drift near
-  // 1e-5 for 3xTF32; plain TF32 (2e-3 budget, operand rounding ~1e-3) promotes every 4 K terms (~6e-5).
-  static constexpr int CHUNK = PREC ? 32 : 128;
+  // k-blocks (of 32 terms) accumulated by the tensor core before a promotion: plain TF32 (2e-3 budget, operand rounding
+  // ~1e-3) promotes every 4 K terms (~6e-5).
+  static constexpr int CHUNK = 128;
   // Accumulator buffers the MMA warp rotates through, and the master copy behind them when promoting.
   static constexpr int NBUF = PROMOTE ? ((3 * ACC_COLS <= 512) ? 2 : 1) : ((2 * ACC_COLS <= 512) ? 2 : 1);
   static constexpr int MASTER_COL = NBUF * ACC_COLS;
@@ -271,7 +269,6 @@ template <class Cfg>
 __global__ void __launch_bounds__(Cfg::NTHREADS, 1)
 lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, MT = Cfg::MT, NS = Cfg::NS;
-  constexpr int PREC = Cfg::PREC;
   constexpr int PF = 8;  // prefetch distance (own k-blocks) for the a values
 
   extern __shared__ uint8_t smem_raw[];
@@ -281,7 +278,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
   float* mpart = msum + 2 * BN;  // [2][2][RG][BN] partial column maxima (slot, a|b, row group, column)
   uint64_t* bars = reinterpret_cast<uint64_t*>(mpart + 2 * Cfg::MPART);
   uint64_t* a_full = bars;               // [NS] w tiles landed
-  uint64_t* b_full = bars + NS;          // [NS] P operand (and w split) written
+  uint64_t* b_full = bars + NS;          // [NS] P operand written
   uint64_t* opnd_empty = bars + 2 * NS;  // [NS] MMAs reading the stage retired
   uint64_t* acc_full = bars + 3 * NS;    // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
@@ -294,12 +291,8 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
   const int lane = threadIdx.x & 31;
   const AbortCtl ctl{abort_flag, p.status};
 
-  auto a_tile = [&](int s, int c, int t) -> uint8_t* {
-    return stage_base + s * Cfg::STAGE + (c * MT + t) * Cfg::A_TILE;
-  };
-  auto b_tile = [&](int s, int c) -> uint8_t* {
-    return stage_base + s * Cfg::STAGE + Cfg::NCOPY * MT * Cfg::A_TILE + c * Cfg::B_TILE;
-  };
+  auto a_tile = [&](int s, int t) -> uint8_t* { return stage_base + s * Cfg::STAGE + t * Cfg::A_TILE; };
+  auto b_tile = [&](int s) -> uint8_t* { return stage_base + s * Cfg::STAGE + MT * Cfg::A_TILE; };
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -360,7 +353,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
             mbar_arrive_expect_tx(&a_full[s], MT * Cfg::A_TILE);
 #pragma unroll
             for (int t = 0; t < MT; ++t)
-              tma_load_4d(a_tile(s, 0, t), &tmap_w, &a_full[s], jc * BK, i, s0 + t * BM, r);
+              tma_load_4d(a_tile(s, t), &tmap_w, &a_full[s], jc * BK, i, s0 + t * BM, r);
           }
         }
       }
@@ -390,24 +383,14 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
             if (!(ok = mbar_wait(&a_full[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
             if (!(ok = mbar_wait(&b_full[s], ph, ctl, STATUS_TIMEOUT_MMA))) break;
             tc_fence_after_sync();
-            const uint64_t db_hi = umma_desc_k_sw128(smem_u32(b_tile(s, 0)));
-            const uint64_t db_lo = PREC ? umma_desc_k_sw128(smem_u32(b_tile(s, 1))) : 0;
+            const uint64_t db = umma_desc_k_sw128(smem_u32(b_tile(s)));
 #pragma unroll
             for (int t = 0; t < MT; ++t) {
               const uint32_t d = tmem_base + buf * Cfg::ACC_COLS + t * BN;
-              const uint64_t da_hi = umma_desc_k_sw128(smem_u32(a_tile(s, 0, t)));
-              const uint64_t da_lo = PREC ? umma_desc_k_sw128(smem_u32(a_tile(s, 1, t))) : 0;
+              const uint64_t da = umma_desc_k_sw128(smem_u32(a_tile(s, t)));
 #pragma unroll
-              for (int ks = 0; ks < BK / 8; ++ks) {
-                const uint32_t acc = (kb > kb0 || ks > 0) ? 1u : 0u;
-                if (PREC) {
-                  umma_tf32_ss(d, da_hi + 2 * ks, db_lo + 2 * ks, idesc, acc);
-                  umma_tf32_ss(d, da_lo + 2 * ks, db_hi + 2 * ks, idesc, 1u);
-                  umma_tf32_ss(d, da_hi + 2 * ks, db_hi + 2 * ks, idesc, 1u);
-                } else {
-                  umma_tf32_ss(d, da_hi + 2 * ks, db_hi + 2 * ks, idesc, acc);
-                }
-              }
+              for (int ks = 0; ks < BK / 8; ++ks)
+                umma_tf32_ss(d, da + 2 * ks, db + 2 * ks, idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
             }
             umma_commit(&opnd_empty[s]);
           }
@@ -542,7 +525,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
             for (int e = 0; e < 32; ++e) {
               const float m_e = __shfl_sync(0xffffffffu, m_lane, e);
               const float acc = __uint_as_float(v[e]);
-              o[e] = m_e + (PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
+              o[e] = m_e + lg2_approx(acc) * LN2_F;
             }
             if (row < p.S) {
               if (vec_ok) {
@@ -692,45 +675,18 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
             const uint32_t ph = (my_it / NS) & 1;
             if (!(ok = mbar_wait_warp(&opnd_empty[s], ph ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
             const float ea = exp_shifted(acur[x], ma);  // acur = -inf past K: exact zero
-            uint8_t* bh = b_tile(s, 0);
-            uint8_t* bl = b_tile(s, PREC ? 1 : 0);
+            uint8_t* bt = b_tile(s);
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
               const uint32_t off = static_cast<uint32_t>(n) * 128u + ((static_cast<uint32_t>(g) ^ (n & 7u)) << 4);
               const float p0 = ea * eb[g * 4 + 0], p1 = ea * eb[g * 4 + 1];
               const float p2 = ea * eb[g * 4 + 2], p3 = ea * eb[g * 4 + 3];
-              if (PREC) {
-                float4 h, l;
-                tf32_split_rn(p0, h.x, l.x);
-                tf32_split_rn(p1, h.y, l.y);
-                tf32_split_rn(p2, h.z, l.z);
-                tf32_split_rn(p3, h.w, l.w);
-                *reinterpret_cast<float4*>(bh + off) = h;
-                *reinterpret_cast<float4*>(bl + off) = l;
-              } else {
-                uint4 u;
-                u.x = tf32_round_bits(p0);
-                u.y = tf32_round_bits(p1);
-                u.z = tf32_round_bits(p2);
-                u.w = tf32_round_bits(p3);
-                *reinterpret_cast<uint4*>(bh + off) = u;
-              }
-            }
-            if (PREC) {
-              // Split the w tiles in place (hi keeps the tf32 bits, lo = w - hi).
-              if (!(ok = mbar_wait_warp(&a_full[s], ph, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-              float4* ah = reinterpret_cast<float4*>(a_tile(s, 0, 0));
-              float4* al = reinterpret_cast<float4*>(a_tile(s, 1, 0));
-              for (int c = n; c < MT * Cfg::A_TILE / 16; c += BN) {
-                const float4 v = ah[c];
-                float4 h, l;
-                tf32_split_trunc(v.x, h.x, l.x);
-                tf32_split_trunc(v.y, h.y, l.y);
-                tf32_split_trunc(v.z, h.z, l.z);
-                tf32_split_trunc(v.w, h.w, l.w);
-                ah[c] = h;
-                al[c] = l;
-              }
+              uint4 u;
+              u.x = tf32_round_bits(p0);
+              u.y = tf32_round_bits(p1);
+              u.z = tf32_round_bits(p2);
+              u.w = tf32_round_bits(p3);
+              *reinterpret_cast<uint4*>(bt + off) = u;
             }
             fence_proxy_async_smem();
             __syncwarp();
