@@ -445,7 +445,7 @@ def test_strided_views_of_a_and_b_are_read_in_place(precision, variant):
 
 def _tol_3xtf32(w, a, b, want, terms=None):
     """Largest error of lt2exp in 3xTF32, per result: as for lm2exp (test_lm2exp_gpu.py), with two exponentials and the
-    rounding of their product (2^-24) per term, and the tensor core's truncating additions over at most a chunk of 1 024
+    rounding of their product (2^-24) per term, and the tensor core's truncating additions over at most a chunk of 768
     terms, after which the accumulator is re-summed with rounded additions (2^-24 each)."""
     R, S, I, J = w.shape
     tol = []
@@ -456,17 +456,17 @@ def _tol_3xtf32(w, a, b, want, terms=None):
         e = ((a64 - ma).exp()[:, None] * (b64 - mb).exp()[None]).view(I * J, -1)
         arg = (w64 @ (e * (xa[:, None] + xb[None]).view(I * J, -1))) / (w64 @ e)
         n = I * J if terms is None else terms
-        tol.append(2.0**-19 + 3 * 2.0**-22 + 2.0**-24 + 2.0**-23 * arg + 3 * 2.0**-23 + 2e-8 * min(n, 1024)
-                   + 2.0**-24 * (n // 1024) + 2.0**-23 * (want[r].abs() + ma.abs() + mb.abs()))
+        tol.append(2.0**-19 + 3 * 2.0**-22 + 2.0**-24 + 2.0**-23 * arg + 3 * 2.0**-23 + 2e-8 * min(n, 768)
+                   + 2.0**-24 * (n // 768) + 2.0**-23 * (want[r].abs() + ma.abs() + mb.abs()))
     return torch.stack(tol)
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 128, 31, 20, 128), (2, 130, 32, 32, 129), (1, 127, 33, 33, 200),
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 128, 31, 20, 128), (2, 130, 24, 32, 129), (1, 130, 25, 30, 129), (2, 130, 32, 32, 129), (1, 127, 33, 33, 200),
                                    (2, 40, 7, 300, 90), (1, 200, 100, 64, 260), (1, 128, 256, 256, 130)])
 @pytest.mark.parametrize("split", [1, 3, 9998])
 def test_3xtf32_on_the_tmem_operand_kernel(shape, split):
     """3xTF32 with the generated operand in tensor memory (hi * hi and both corrections as tf32 products): k-blocks around
-    the chunks of 32 after which the accumulator is re-summed, rows and columns around the 128 of a tile, whole tiles, added
+    the chunks of 24 after which the accumulator is re-summed, rows and columns around the 128 of a tile, whole tiles, added
     slices and parts completed through scratch memory.  Tolerance: _tol_3xtf32."""
     R, S, I, J, K = shape
     g = torch.Generator().manual_seed(sum(shape))

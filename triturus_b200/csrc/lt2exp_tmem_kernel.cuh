@@ -41,6 +41,9 @@ namespace tb200 {
 // core = 768 cycles of the shared-memory pipe next to 768 of the tensor pipe (both operands in shared memory: 1 400).
 // Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
 // master copy in shared memory (see "Accumulator promotion" in lt2exp_kernel.cuh; TMEM has no room for a third).
+// Chunks of 24 (768 terms): rms error of a long flat sum 1.2e-5.  16: 0.8e-5, but 1 to 9 % slower, the drain being no longer
+// hidden (R16 128x64x64x2048 150 -> 162 us, 1 x 256^4 71 -> 79); 32: 1.6e-5, at most 2 % faster (R64 256x128x128x4096 8 560 ->
+// 8 370 us, R32 256^4 1 163 -> 1 156).
 template <int MT_, int NS_, int NB_ = 1, int PREC_ = 0>
 struct Lt2expTmemCfg {
   static constexpr int BM = 128, BK = 32;  // BM: rows s per w box
@@ -48,7 +51,7 @@ struct Lt2expTmemCfg {
   static constexpr int BN = 128 * NB;      // columns k per tile
   static constexpr int MT = MT_, NS = NS_, PREC = PREC_, NTW = 8;
   static constexpr bool PROMOTE = PREC != 0;  // chunked re-summation of the accumulator
-  static constexpr int CHUNK = PROMOTE ? 32 : 1 << 30;
+  static constexpr int CHUNK = PROMOTE ? 24 : 1 << 30;  // k-blocks
   static constexpr int W_TILE = BM * BK * 4;
   static constexpr int W_BYTES = MT * W_TILE;             // what TMA brings per stage
   static constexpr int STAGE = (PREC ? 2 : 1) * W_BYTES;  // ... and the low parts of it
