@@ -219,9 +219,13 @@ def check_status(device=None) -> None:
 def _tma_ok(t: torch.Tensor) -> bool:
     """Innermost stride 1, other strides positive multiples of 4 elements, base 16-byte aligned: what a TMA
     tensor map needs."""
-    if t.data_ptr() % 16 != 0 or not (t.shape[-1] == 1 or t.stride(-1) == 1):
+    shape, stride = t.shape, t.stride()  # (asked of every operand of every call: 0.8 us here, 2.4 us through t.stride(d))
+    if t.data_ptr() % 16 or (stride[-1] != 1 and shape[-1] != 1):
         return False
-    return all(t.shape[d] == 1 or (t.stride(d) > 0 and t.stride(d) % 4 == 0) for d in range(t.dim() - 1))
+    for n, s in zip(shape[:-1], stride):
+        if (s % 4 or s <= 0) and n != 1:
+            return False
+    return True
 
 
 def _tma_ready(t: torch.Tensor) -> torch.Tensor:
@@ -261,30 +265,36 @@ def _pad_rows(t: torch.Tensor, buf: torch.Tensor) -> bool:
 
 # Problems up to this many FLOP take operands that break the tensor-map rules in place (the single-CTA kernel then
 # fetches them element by element, about three times slower per k-block than through TMA); larger ones get the padded copy.
-# The line lies where a loop of calls takes equally long: below it the host's work for the copies (two allocations and
-# launches, 12 us or more per call) is what counts, above it the fetch.  Microseconds per call, in place / with
-# the copies, both operands odd: 1.5e8 (R24 150x101x203) 40 / 46 in 3xTF32 and 33 / 46 in TF32; 3.9e8 (R64, the same)
-# 61 / 46 and 45 / 47; 1.0e9 (R8 255x255x1001) 66 / 47 and 54 / 47; 1.1e9 (R4 511^3) 117 / 48 and 93 / 47; 4.0e9 (R2
-# 1001^3) 219 / 75 and 174 / 60; 8.6e9 (R128 64x64x8191) 777 / 812 and 534 / 507.  One odd operand, or an inner stride
-# of 2 (copied by torch): the same side of the line, except TF32 at 1.1e9 with an odd a alone, 31 / 33.
-_IN_PLACE_MAX_FLOP = 3e8
+# Rows of consecutive floats, which triturus_b200_pad_rows_f32 copies: from the line on no form was faster in place.
+# Microseconds per call of a loop, in place / with the copies, both operands odd: R24 150x101x203 (1.5e8 FLOP) 40 / 46 in
+# 3xTF32 and 33 / 46 in TF32; R64 the same (3.9e8) 61 / 46 and 45 / 47; R8 255x255x1001 (1.0e9) 66 / 47 and 54 / 47, but
+# with an odd a alone in TF32 31 / 33; R4 511^3 (1.1e9) 117 / 48 and 93 / 47, an odd a alone 50 / 34; R2 1001^3 (4.0e9)
+# 219 / 75 and 174 / 60.  Below the line the host's work for the copies (two allocations and launches, 12 us or
+# more) can be what counts.
+_IN_PLACE_MAX_FLOP = 1.1e9
+# Other views, which torch would copy: R64 64x64x8192 with a transposed b of odd pitch (4.3e9) 374 / 447 in 3xTF32, R128
+# 256x256x8190 (1.4e11) 1 200 / 1 600 in TF32 but 2 970 / 2 320 in 3xTF32.
+_IN_PLACE_MAX_FLOP_STRIDED = 8e9
 
 
 def _in_place_small(t: torch.Tensor, flop: float, variant: int, want_colmax: bool) -> bool:
     """True when `t` should go to the library as it is although a tensor map cannot describe it."""
     tile = int(variant) % 100000
-    return (flop <= _IN_PLACE_MAX_FLOP and not want_colmax and tile in _SINGLE_CTA_TILES
+    limit = _IN_PLACE_MAX_FLOP if t.stride(-1) == 1 else _IN_PLACE_MAX_FLOP_STRIDED
+    return (flop <= limit and not want_colmax and tile in _SINGLE_CTA_TILES
             and t.dtype == torch.float32 and t.data_ptr() % 4 == 0)
 
 
-def _lm2exp_a_operand(a: torch.Tensor, K: int) -> torch.Tensor:
-    """`a` [R,I,J] as the library takes it: unchanged when j is contiguous and the TMA rules hold; a
-    transposed view (i contiguous, the other strides multiples of 4 elements, base 16-byte aligned) can be
-    read in place as an MN-major tensor-core operand; otherwise a padded copy.
+def _lm2exp_a_operand(a: torch.Tensor, K: int, variant: int = 0, flop: float = float("inf"), want_colmax: bool = False) -> torch.Tensor:
+    """`a` [R,I,J] as the library takes it: unchanged when j is contiguous and the TMA rules hold, and when the problem
+    is small (`_in_place_small`); a transposed view (i contiguous, the other strides multiples of 4 elements, base
+    16-byte aligned) can be read in place as an MN-major tensor-core operand; otherwise a padded copy.
 
     Reading the view in place makes the contraction kernel about 16 % slower (four TMA boxes per tile and the
     MN-major operand fetch; measured 13 % on R32 x 1024^3, 18 % on R128 I=J=256 K=8192), a transposing copy
     runs at about 0.9 TB/s of `a`: the cheaper of the two is taken from a rough estimate of the kernel time."""
+    if _tma_ok(a) or _in_place_small(a, flop, variant, want_colmax):
+        return a
     R, I, J = a.shape
     if J > 1 and a.stride(2) != 1 and (I == 1 or a.stride(1) == 1) and a.data_ptr() % 16 == 0:
         if a.stride(2) > 0 and a.stride(2) % 4 == 0 and (R == 1 or (a.stride(0) > 0 and a.stride(0) % 4 == 0)):
@@ -357,7 +367,7 @@ def _lm2exp_impl(a: torch.Tensor, b: torch.Tensor, precision: int, variant: int)
     R, I, J = a.shape
     K = b.shape[2]
     flop = 2.0 * R * I * J * K
-    a = a if _in_place_small(a, flop, variant, False) else _lm2exp_a_operand(a, K)
+    a = _lm2exp_a_operand(a, K, variant, flop, False)
     b = _lm2exp_b_operand(b, variant, flop, False)
     out = torch.empty((R, I, K), dtype=torch.float32, device=a.device)
     ws_bytes = int(LIB.triturus_b200_lm2exp_workspace_bytes(R, I, J, K))
@@ -382,7 +392,7 @@ def _lm2exp_chain_impl(
     R, I, J = a.shape
     K = b.shape[2]
     flop = 2.0 * R * I * J * K
-    a = a if _in_place_small(a, flop, variant, want_colmax) else _lm2exp_a_operand(a, K)
+    a = _lm2exp_a_operand(a, K, variant, flop, want_colmax)
     b = _lm2exp_b_operand(b, variant, flop, want_colmax)
     out = torch.empty((R, I, K), dtype=torch.float32, device=a.device)
     out_colmax = torch.empty((R, K) if want_colmax else (0,), dtype=torch.float32, device=a.device)
