@@ -215,7 +215,7 @@ struct Lt2expCfg {
   static constexpr int CQ = BN / 4;
   static constexpr int RG = NTT / CQ;
   static constexpr int MPART = 2 * RG * BN;  // floats per slot: partial maxima of a and of b
-  static constexpr int NBAR = 3 * NS + 7;
+  static constexpr int NBAR = 3 * NS + 9;
   static constexpr int SMEM_BYTES = 1024 + NS * STAGE + 2 * BN * 4 + 2 * MPART * 4 + NBAR * 8 + 64;
   static_assert(NTT % CQ == 0 && RG >= NGROUPS, "column-maximum thread mapping");
   static_assert(NTT % BN == 0 && NGROUPS >= 1, "transform thread mapping");
@@ -282,7 +282,8 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
   uint64_t* opnd_empty = bars + 2 * NS;  // [NS] MMAs reading the stage retired
   uint64_t* acc_full = bars + 3 * NS;    // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
-  uint64_t* msum_empty = acc_empty + 2;  // [2] epilogue finished reading msum[slot]
+  uint64_t* msum_full = acc_empty + 2;   // [2] (NGROUPS > 1) msum[slot] written
+  uint64_t* msum_empty = msum_full + 2;  // [2] epilogue finished reading msum[slot]
   uint64_t* mx_bar = msum_empty + 2;     // [1] every transform warp published its partial maxima
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mx_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -304,6 +305,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], 4);
+      mbar_init(&msum_full[s], Cfg::GROUP_WARPS);
       mbar_init(&msum_empty[s], 4);
     }
     mbar_init(mx_bar, Cfg::NTW);
@@ -440,6 +442,12 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
         const uint32_t aph = (ccount / Cfg::NBUF) & 1;
         const bool first = ch == 0, last = ch == nch - 1;
         if (!(ok = mbar_wait_warp(&acc_full[buf], aph, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
+        // With several transform groups the accumulator says nothing of msum: group 0, which writes it, may have no k-block
+        // in the item at all (one k-block and an odd stage counter).  With one group its arrival on the operand stage orders
+        // the write, and a barrier of its own would cost 2 to 3 % (1285: R16 128x64x64x2048 65.2 -> 66.4 us, R128
+        // 64x32x32x512 49.3 -> 50.8).  (The write by whichever group builds the first k-block, behind a wait of all
+        // groups for the slot, cost 1 % where CTAs take several parts: R9 96x224x64x1289 157.4 -> 159.0 us.)
+        if (Cfg::NGROUPS > 1 && first && !(ok = mbar_wait_warp(&msum_full[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
         tc_fence_after_sync();
 #pragma unroll 1
         for (int t = 0; t < MT; ++t) {
@@ -624,12 +632,14 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
       ma = clamp_stab(ma);
       mb = clamp_stab(mb);
       const int slot = tcount & 1;
-      // The group that builds the item's first k-block hands the epilogue its stabilisers: the write precedes that
-      // group's arrival on the stage, and stage -> MMA -> accumulator -> epilogue orders it before the read.  (A fixed
-      // group may have no k-block in the item at all: one k-block and an odd stage counter.)  Every group waits
-      // for the slot, since the writer changes from item to item and a wait by parity must not skip a use.
-      if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-      if (grp == static_cast<int>(it % NG)) msum[slot * BN + n] = ma + mb;
+      if (grp == 0) {
+        if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+        msum[slot * BN + n] = ma + mb;
+        if (NG > 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&msum_full[slot]);
+        }
+      }
 
       for (int jc = w.kb_lo / p.I; ok && jc * p.I < w.kb_hi; ++jc) {
         const int i_lo = lt_row_lo(w, jc, p.I);

@@ -69,7 +69,7 @@ struct Lt2expTmemCfg {
   static constexpr int CQ = BN / 4;
   static constexpr int RG = NTT / CQ;
   static constexpr int MPART = 2 * RG * BN;
-  static constexpr int NBAR = 3 * NS + 7;
+  static constexpr int NBAR = 3 * NS + 9;
   static constexpr int MASTER = PROMOTE ? MT * BM * BN * 4 : 0;
   static_assert(!PREC || (MT == 1 && NB == 1 && NBUF == 2), "3xTF32: 128 x 128 tiles, two accumulators");
   static constexpr int SMEM_BYTES = 1024 + NS * STAGE + MASTER + 2 * BN * 4 + 2 * MPART * 4 + NBAR * 8 + 64;
@@ -104,7 +104,8 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
   uint64_t* opnd_empty = bars + 2 * NS;  // [NS] MMAs reading the stage (shared memory and TMEM) retired
   uint64_t* acc_full = bars + 3 * NS;    // [2]
   uint64_t* acc_empty = acc_full + 2;    // [2]
-  uint64_t* msum_empty = acc_empty + 2;  // [2]
+  uint64_t* msum_full = acc_empty + 2;   // [2] (NGROUPS > 1, see lt2exp_kernel.cuh)
+  uint64_t* msum_empty = msum_full + 2;  // [2]
   uint64_t* mx_bar = msum_empty + 2;     // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mx_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -124,6 +125,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     for (int s = 0; s < 2; ++s) {
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], 4);
+      mbar_init(&msum_full[s], BN / 32);
       mbar_init(&msum_empty[s], 4);
     }
     mbar_init(mx_bar, Cfg::NTW);
@@ -268,6 +270,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
           const int buf = ccount % Cfg::NBUF;
           const bool first = ch == 0, last = ch == nch - 1;
           if (!(ok = mbar_wait_warp(&acc_full[buf], (ccount / Cfg::NBUF) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
+          if (Cfg::NGROUPS > 1 && first && !(ok = mbar_wait_warp(&msum_full[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
           tc_fence_after_sync();
           if (last && collect) {
             // The other parts of the tile run at the same time on other CTAs and end about now.  (Not earlier: while
@@ -356,6 +359,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       const uint32_t aph = (tcount / Cfg::NBUF) & 1;
       const int slot = tcount & 1;
       if (!(ok = mbar_wait_warp(&acc_full[buf], aph, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
+      if (Cfg::NGROUPS > 1 && !(ok = mbar_wait_warp(&msum_full[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
       tc_fence_after_sync();
 #pragma unroll 1
       for (int blk = 0; blk < Cfg::NB; ++blk) {  // column blocks of the tile: this lane's column in each
@@ -494,10 +498,14 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       ma = clamp_stab(ma);
       mb = clamp_stab(mb);
       const int slot = tcount & 1;
-      // Written by the group that builds the item's first k-block, after every group has waited for the slot (see
-      // lt2exp_kernel.cuh).
-      if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
-      if (grp == static_cast<int>(it % NG)) msum[slot * BN + n] = ma + mb;
+      if (grp == 0) {
+        if (!(ok = mbar_wait_warp(&msum_empty[slot], ((tcount >> 1) & 1) ^ 1, ctl, STATUS_TIMEOUT_TRANSFORM))) break;
+        msum[slot * BN + n] = ma + mb;
+        if (NG > 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&msum_full[slot]);
+        }
+      }
 
       for (int jc = w.kb_lo / p.I; ok && jc * p.I < w.kb_hi; ++jc) {
         const int i_lo = lt_row_lo(w, jc, p.I);
