@@ -147,7 +147,7 @@ int triturus_b200_lm2exp_chain_f32(const float* a, const float* b, float* out, i
  *            0 = automatic (slices when the output tiles would occupy fewer than half the SMs; when the last
  *            wave of tiles would be less than 90 % full and a tile's contraction is at least 8192 terms long,
  *            the full waves run as whole tiles and the contractions of the last wave's tiles are shared among
- *            all SMs), 1 = never (mode "unsplit"), n >= 2 = n slices (fewer if a slice would drop below 16
+ *            all SMs), 1 = never (mode "unsplit"), n >= 2 = n slices (fewer if a slice would drop below four
  *            k-blocks), 9998 = the shared last wave in any case, 9999 = as automatic but at least two slices
  *            (mode "split").  Plain TF32 over more than 32768 terms re-sums its accumulator every 4096
  *            terms with rounded adds (automatic tiles only leave room for that; an explicit 2562 / 128x tile is

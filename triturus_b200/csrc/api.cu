@@ -125,8 +125,9 @@ __global__ void __launch_bounds__(256) rowmax_kernel(const float* __restrict__ x
 
 // dst[r, y, 0 .. 4 q) = src[r, y, 0 .. n) and zeros behind: rows whose pitch or base breaks the 16-byte rule of tensor maps,
 // copied to a pitch of q quads.  One thread writes one quad and reads four consecutive values of the source, which is
-// only 4-byte aligned; kPadPerThread quads per thread, a block apart, keep 16 loads in flight.  (torch's copy before it: a drawn
-// lm2exp of odd widths 379 us in all, 313 us with this kernel.)
+// only 4-byte aligned; kPadPerThread quads per thread, a block apart, keep 16 loads in flight.  Bound by HBM where it is large:
+// 32 x 1023 x 1022 in 44.7 us = 5.99 TB/s (torch's copy 88.0), 128 x 255 x 8191 in 360 us (679), 4 x 1001 x 1001 in 5.6 us (10.1),
+// 24 x 150 x 101 in 2.1 us (2.3).
 constexpr int kPadPerThread = 4;
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, float4* __restrict__ dst, int64_t quads,
                                                        int rows, int n, int q, int64_t s0, int64_t s1) {
@@ -371,7 +372,8 @@ using LmTsPairOptH = Lm2expTsPairCfg<8, 4, 2, true, false, 0, true>;
 using LmTsPairX = Lm2expTsPairCfg<4, 4, 2, false, false, 1>;  // 3xTF32
 using LmTsPairFused = Lm2expTsPairCfg<8, 4, 2, false, true>;  // exact max pass inside: the conditional launch behind Opt
 
-// The CTA-pair kernel with the generated operand in tensor memory (plain TF32, a with j contiguous).
+// The CTA-pair kernel with the generated operand in tensor memory: plain TF32 with j of a contiguous, 3xTF32 with either
+// layout of a.
 template <class Cfg>
 static int launch_lm2exp_tspair(const CUtensorMap& ta, const CUtensorMap& tb_plain, const CUtensorMap& to,
                                 Lm2expParams p, cudaStream_t stream, bool after_prepass) {
@@ -438,7 +440,7 @@ struct Lm2expPlan {
   bool optimistic;  // ... without a pre-pass: stabiliser from the first k-block, exact passes as conditional launches (2567)
   bool fused;   // max pass inside the contraction kernel (no pre-pass launch)
   bool optimistic_fused;  // ... over the first k-block of each slab only, exact pass as a conditional launch
-  bool optimistic_prepass;  // pair tile in shared memory: pre-pass over the first 32 rows, exact passes conditional
+  bool optimistic_prepass;  // pair tile 2564: pre-pass over the first 32 rows, exact passes conditional
   bool colmax_exclusive;  // one row tile covers I: column maxima of the result are stored, not reduced
   bool promote_tf32;      // plain TF32 over more than kLongContraction terms: accumulator re-summed in chunks
 };
@@ -454,7 +456,7 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
                        bool have_m = false, bool b_km = false, bool single_cta = false) {
   if (variant < 0) return TRITURUS_B200_EINVAL;
   // 0 = automatic, 1 = pre-pass, 2 = fused max pass, 3 = fused max pass over the first k-block only (optimistic),
-  // 4 = pre-pass over the first 32 rows only (optimistic; shared-memory pair tile)
+  // 4 = pre-pass over the first 32 rows only (optimistic; pair tile 2564)
   const int stab_mode = variant / 100000;
   int tile_variant = variant % 100000;
   if (stab_mode > 4 || (have_m && stab_mode >= 2)) return TRITURUS_B200_EINVAL;
@@ -463,9 +465,9 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
     // pair moves the fewest shared-memory bytes per MAC.  With the optimistic stabilisers, which need no full
     // pre-pass, the pair kernels also win from two 128-row blocks on (cfg3, I = 256: 0.479 ms on the
     // TMEM-operand pair kernel against 0.508 ms on the single-CTA kernel with the optimistic fused max pass; in
-    // 3xTF32 1.14 against 1.30 ms).  Otherwise a single-CTA tile with the fused max pass.
+    // 3xTF32 0.91 against 1.31 ms).  Otherwise a single-CTA tile with the fused max pass.
     // (Not for 3xTF32 contractions longer than 4096, where the drift of the tensor core's truncating
-    // accumulator, ~1.2e-8 per term, would use up the 3xTF32 tolerance: only the single-CTA kernel re-sums
+    // accumulator, ~1.6e-8 per term, would use up the 3xTF32 tolerance: only the single-CTA kernel re-sums
     // its accumulator in chunks.)
     // The optimistic forms cost two or three launches more, which return at once on the device but take the host
     // some 7 us per call: below ~50 us of work a loop of calls would wait for the host (R64 256^3: 14.4 us per
@@ -522,7 +524,8 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
       out->fused && (stab_mode == 3 || (stab_mode == 0 && precision == TRITURUS_B200_PRECISION_TF32 && J >= 128 &&
                                         big_enough && tile_count(R, I, K, bn, mt) > sm_count()));
   out->colmax_exclusive = !pair && I <= 128 * mt;
-  // The shared-memory pair kernel, where it is the automatic choice (3xTF32): the pre-pass scans 32 rows instead of J.
+  // Pair tile 2564, where it is the automatic choice (3xTF32, on the TMEM-operand kernel): the pre-pass scans 32 rows
+  // instead of J (R32 1024^3 297 -> 275 us, R128 256x256x8192 1 006 -> 905).
   out->optimistic_prepass = pair && !tspair && !have_m && J >= 128 &&
                             (stab_mode == 4 || (stab_mode == 0 && variant % 100000 == 0 && big_enough));
   out->promote_tf32 = !pair && bn == 128 && precision == TRITURUS_B200_PRECISION_TF32 && J > kLongContraction;
@@ -1043,7 +1046,8 @@ struct LtSplit {
 // it the end-to-end form would have to add every partial sum into the result with atomics, which costs more
 // than the ragged wave it removes, so the automatic choice then keeps whole tiles.
 static LtSplit lt2exp_split(int64_t tiles, int I, int J, int request, bool auto_stream) {
-  // (16 k-blocks before: 1 x 128 64x64x128 30.7 -> 24.6 us in TF32, 41.6 -> 36.9 us in 3xTF32)
+  // Slices of four k-blocks, where 16 was the least before: a 1 x 128 x 128 result over 64 / 128 / 256 k-blocks takes 21.4 /
+  // 21.7 / 22.7 us on the device in TF32, 26.3 / 26.2 / 26.5 with 16, and 32.6 / 32.9 / 33.4 in 3xTF32, 38.8 / 38.3 / 38.4 with 16.
   constexpr int kMinSliceBlocks = 4;
   constexpr int kMinStreamBlocks = 256;
   const int JC = (J + 31) / 32;
@@ -1058,8 +1062,10 @@ static LtSplit lt2exp_split(int64_t tiles, int I, int J, int request, bool auto_
   int64_t want = request;
   if (request == 0 || request == 9999) {
     want = tiles * 2 > sms ? 1 : sms / tiles;
-    // Two more launches (zero-fill and log pass) cost about as much as 50 k-blocks of the main loop: a
-    // contraction shorter than that is left whole.
+    // Two more launches (zero-fill and log pass), chained behind one another, cost 8 us in TF32 and 11 in 3xTF32, and a
+    // k-block 0.38 and 0.47 us: on the device slices are level with whole tiles at 32 k-blocks (1 x 128 x 128: 21.3 / 22.6
+    // us in TF32, 32.7 / 32.9 in 3xTF32) and a third faster at 64 (21.6 / 34.6, 32.6 / 47.7).  The line is drawn at 64 and
+    // not where they are level, since the last bits of a split result depend on the order of arrival.
     if (request == 0 && kb < 64) want = 1;
     if (request == 9999 && want < 2) want = 2;
     if (want == 1 && tiles > sms / 2) {
@@ -1110,8 +1116,10 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
                        (L.query != nullptr || (L.ws != nullptr && L.ws_bytes >= park_need &&
                                                (reinterpret_cast<uintptr_t>(L.ws) & 255) == 0));
   // Not chosen automatically for a launch that re-sums its accumulator in chunks (3xTF32, long plain-TF32
-  // contractions): sharing tiles made those slower (R32 256^4: 1.32 against 0.81 ms in TF32, 2.87 against 1.68 ms
-  // in 3xTF32; R128: 2.75 against 2.40 ms), the explicit request 9998 still selects it.
+  // contractions): sharing tiles makes long plain-TF32 contractions slower (R32 256^4: 1.32 against 0.81 ms; R128: 2.75
+  // against 2.40 ms); the explicit request 9998 still selects it.  The 3xTF32 kernel would gain, whole / shared: R8
+  // 256x128x128x4096 1 478 / 1 009 us, R10 K2048 924 / 636, R128 256^4 5 228 / 4 869, R32 1 160 / 1 127, R16 256x128x128x4096
+  // 2 025 / 2 040.
   const bool chunked = Cfg::PROMOTE && static_cast<int64_t>((p.J + 31) / 32) * p.I > Cfg::CHUNK;
   const LtSplit sp = lt2exp_split(nt, p.I, p.J, L.split_request, have_ws && !chunked);
   p.nsplit = sp.nsplit;

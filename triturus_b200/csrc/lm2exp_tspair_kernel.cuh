@@ -1,4 +1,4 @@
-// lm2exp on CTA pairs with the generated operand in tensor memory (plain TF32).
+// lm2exp on CTA pairs with the generated operand in tensor memory (plain TF32, and 3xTF32 as the PREC instance).
 //
 // Same arithmetic as lm2exp_pair_kernel.cuh (replaces triturus/lm2exp.py:63-164), but the contraction is
 // written transposed, D^T[k, i] = sum_j E^T[k, j] * a[i, j] with E = exp(b - m): the generated operand E^T is the
@@ -15,17 +15,22 @@
 // One pair tile is 256 columns k (M, 128 per CTA = the CTA's TMEM lanes) x 256 rows i (N, 128 per CTA's
 // shared memory).  Tensor memory per CTA: columns [0, 256) accumulator D^T, [256, 256 + 32 * NS) the E^T stages.
 // The accumulator is single-buffered (a second one would leave no room for the operand), so the epilogue of a
-// tile is not hidden behind the next tile's MMAs; the transform warps run ahead by NS k-blocks meanwhile.
+// tile is not hidden behind the next tile's MMAs; the transform warps run ahead by NS k-blocks meanwhile.  (Short
+// contractions fill and drain it in two halves, see HALVES below.  3xTF32, R32 1024^3: 1 533 cycles per k-block in the main
+// loop, which is the tensor core's 1 536, and 14 400 of the 62 900 cycles of a tile in the epilogue.)
 // In the transposed result a lane owns a column k, so the stabiliser m[k] is a lane constant; a 32 x 32 block of
 // results is staged in shared memory (the 32 lanes of a store fill one row) and written by one TMA store; two boxes per warp alternate.
 //
 //   warp 0      TMA producer of ring 1: this CTA's 128 rows of a (128B swizzle).
-//   warp 1      TMEM allocation; in the leader CTA one lane issues the pair MMAs.
+//   warp 1      TMEM allocation; in the leader CTA the warp walks the k-blocks and one elected lane issues the pair MMAs.
 //   warp 2      TMA producer of ring 2: this CTA's 128 columns of b (no swizzle).
-//   warp 3      watches the a tiles land and says so on the leader's xf_done barriers.
+//   warp 3      watches the a tiles land and says so on the leader's xf_done barriers (3xTF32: idle).
 //   warps 4-7   epilogue (TMEM lane quarter = warp % 4).
 //   warps 8-15  transform: NG = two groups of four warps (one per lane quarter) take alternate tiles of b (three
 //               groups, 20 warps at 96 registers, ran 5 % slower; ring depths 6+6, 5+7, 7+5 instead of 8+4 the same).
+//   warps 16-19 3xTF32: wait for the tiles of a, write their low parts to a second tile and say so on xf_done.
+// 3xTF32 has four stages of 2 x 16 KB (a and its low parts) and 64 TMEM columns (both parts of E^T), takes a transposed a as
+// well (MN-major tiles) and folds column maxima of the result.
 #pragma once
 
 #include "lm2exp_kernel.cuh"
@@ -279,7 +284,7 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     // ------------------------------------------------------------------ pair MMA issuer (leader CTA only)
     // The whole warp runs the loop and one elected lane issues: control flow and descriptors are uniform and stay in uniform
     // registers.  (One lane in a branch of its own took 80 - 100 cycles per MMA for moving them there, more than the 64 to
-    // 128 of the MMA itself: 750 cycles per k-block in plain TF32, 1 300 in 3xTF32.)
+    // 128 of the MMA itself: 750 cycles per k-block in plain TF32.)
     if (leader) {
       // M = 256 columns k over the pair (A from TMEM), N = 256 rows i (B = a, K-major, 128 rows per CTA)
       // PREC takes a transposed a too: MN-major (bit 16), its low parts in the same layout.
@@ -444,8 +449,8 @@ lm2exp_tspair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         for (int h = 0; h < (Cfg::PREC ? 1 : 2); ++h) {
           const int c = idx + h;
           if (c < nchunks) {
-            // (PREC: one buffer, the logarithms want the registers of the second: R64 512x512x256 63.5 -> 55.3 us, R32 1024^3
-            // 272 -> 252 us)
+            // (PREC: one buffer, the logarithms want the registers of the second: R64 512x512x256 72.5 -> 63.6 us, R32 1024^3
+            // 349 -> 321 us)
             if (Cfg::PREC && c > 0) tmem_ld_32x32(tbase + hf * (BN / 2) + c * 32, v[Cfg::PREC ? 0 : h]);
             tmem_ld_wait();  // chunk c is in v[h]
             if (!Cfg::PREC && c + 1 < nchunks) {

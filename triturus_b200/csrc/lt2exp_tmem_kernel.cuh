@@ -1,4 +1,4 @@
-// lt2exp with the generated operand in TENSOR MEMORY (TF32).
+// lt2exp with the generated operand in TENSOR MEMORY (some plain TF32 tiles, and all of 3xTF32 as the PREC instance).
 //
 // Same contraction as lt2exp_kernel.cuh (which replaces triturus/lt2exp.py:227-357 and :365-506), computed
 // transposed:
@@ -22,11 +22,14 @@
 // Stage s of shared memory (w) and operand stage s of TMEM are released together by one tcgen05.commit.
 //
 //   warp 0      TMA producer: w boxes {32 j, 1 i, 128 s, 1 r}, 128-byte swizzle.
-//   warp 1      TMEM allocation; one lane issues tcgen05.mma.kind::tf32 with A in TMEM (M = 128, N = 128*MT, K = 8).
+//   warp 1      TMEM allocation; the warp walks the k-blocks and one elected lane issues tcgen05.mma.kind::tf32 with A in TMEM
+//               (M = 128, N = 128*MT, K = 8).
 //   warps 4-7   epilogue: tcgen05.ld, out[s, k] = m[k] + log(acc), coalesced 128-byte stores (or fp32 reductions
-//               into the zero-filled result when the contraction is split, see lt2exp_kernel.cuh).
+//               into the zero-filled result when the contraction is split, see lt2exp_kernel.cuh); 3xTF32: re-summation of
+//               finished chunks meanwhile.
 //   warps 8-15  transform: warp w writes TMEM lane quarter w % 4; the two warps of a quarter take alternate
 //               k-blocks.  Column maxima first (cooperative, as in lt2exp_kernel.cuh).
+//   warps 16-19 3xTF32: the low parts of the w tiles.
 #pragma once
 
 #include "lt2exp_kernel.cuh"
@@ -39,6 +42,8 @@ namespace tb200 {
 // 1 298 us, but terms off by up to 7e-6, see lm2exp_tspair_kernel.cuh.)
 // Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the splitting, 48 KB read by the tensor
 // core = 768 cycles of the shared-memory pipe next to 768 of the tensor pipe (both operands in shared memory: 1 400).
+// Measured 1 030 cycles per k-block (R32 256^4): the four stages' chain of TMA, splitting, MMA and commit bounds it.
+// At 96 registers a thread (20 warps) 92 bytes are spilled, outside the loops over k-blocks: 40 loads and 44 stores per CTA.
 // Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
 // master copy in shared memory (see "Accumulator promotion" in lt2exp_kernel.cuh; TMEM has no room for a third).
 // Chunks of 24 (768 terms): rms error of a long flat sum 1.2e-5.  16: 0.8e-5, but 1 to 9 % slower, the drain being no longer
