@@ -43,7 +43,8 @@ namespace tb200 {
 // Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the splitting, 48 KB read by the tensor
 // core = 768 cycles of the shared-memory pipe next to 768 of the tensor pipe (both operands in shared memory: 1 400).
 // Measured 1 030 cycles per k-block (R32 256^4): the four stages' chain of TMA, splitting, MMA and commit bounds it.
-// At 96 registers a thread (20 warps) 92 bytes are spilled, outside the loops over k-blocks: 40 loads and 44 stores per CTA.
+// At 96 registers a thread (20 warps) 92 bytes are spilled, outside the loops over k-blocks: 68 loads and 52 stores per
+// CTA of one tile.
 // Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
 // master copy in shared memory (see "Accumulator promotion" in lt2exp_kernel.cuh; TMEM has no room for a third).
 // Chunks of 24 (768 terms): rms error of a long flat sum 1.2e-5.  16: 0.8e-5, but 1 to 9 % slower, the drain being no longer
