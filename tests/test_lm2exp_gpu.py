@@ -838,3 +838,40 @@ def test_padded_copy_of_rows(shape):
     for t in (x, wide, x[:1].expand(shape)):
         got = _native._tma_ready(t)
         assert _native._tma_ok(got) and torch.equal(got, t)
+
+
+@pytest.mark.parametrize("variant", [102564, 402564])
+@pytest.mark.parametrize("shape", [
+    (40, 289, 70, 260),    # ten row units of 32, the last with one row; groups of two pairs, shares that cross entries
+    (80, 257, 33, 130),    # one 256-column slab with 126 columns of padding, two k-blocks of which the second has one row
+    (26, 320, 129, 600),   # three slabs: 72 of the 74 pairs; five k-blocks
+    (9, 260, 40, 2051),    # nine slabs, rows that a TMA store cannot write
+    (1, 300, 40, 19200),   # more slabs than pairs: tiles round robin
+], ids=str)  # fmt: skip
+def test_3xtf32_pair_tiles_with_two_accumulators(shape, variant):
+    """Shapes that the 3xTF32 kernel with two accumulators takes (several waves of 256-row tiles, or one that is mostly
+    padding): at the edges of its tiles, row units and shares, for both layouts of a, with impossible states, and with the
+    column maxima of the result."""
+    import triturus_b200 as tb
+
+    R, I, J, K = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    b[torch.rand(R, J, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K - 1] = float("-inf")
+    a[R - 1, I - 1] = 0.0
+    want = orc.lm2exp_fp64(a, b)
+    ad, bd = a.cuda(), b.cuda()
+    got = tb.lm2exp(ad, bd, precision="3xtf32", variant=variant)
+    views = [ad.transpose(1, 2).contiguous().transpose(1, 2)]
+    outs = [got.cpu(), *(tb.lm2exp(v, bd, precision="3xtf32", variant=variant).cpu() for v in views)]
+    out, m = tb.lm2exp(ad, bd, precision="3xtf32", variant=variant, return_colmax=True)
+    tb.check_status()
+    outs.append(out.cpu())
+    assert torch.equal(m, out.amax(1))
+    fin = torch.isfinite(want)
+    tol = _tol_3xtf32(a, b, want)
+    for o in outs:
+        assert torch.equal(o == float("-inf"), want == float("-inf")) and not torch.isnan(o).any()
+        assert ((o.double() - want).abs() <= tol)[fin].all()

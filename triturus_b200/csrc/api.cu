@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -13,6 +14,7 @@
 #include "lm2exp_kernel.cuh"
 #include "lm2exp_pair_kernel.cuh"
 #include "lm2exp_tspair_kernel.cuh"
+#include "lm2exp_pair3x_kernel.cuh"
 #include "lt2exp_kernel.cuh"
 #include "lt2exp_tmem_kernel.cuh"
 
@@ -417,6 +419,81 @@ static int launch_lm2exp_tspair(const CUtensorMap& ta, const CUtensorMap& tb_pla
                                 after_prepass, ta, tb_plain, to, p);
 }
 
+// 3xTF32 with two accumulators: see lm2exp_pair3x_kernel.cuh.
+//
+// Cost of the `units` row units (of 32 rows) of one batch entry on a pair, in units of 32 rows' MMAs: even tiles of at most six
+// units, of which those under five take as long as five (the transform warps bound them: 950 cycles per k-block, against
+// 192 per unit).
+static int64_t pair3x_cost(int64_t units) {
+  if (units <= 0) return 0;
+  const int64_t nt = (units + Lm2expPair3xCfg::UNITS - 1) / Lm2expPair3xCfg::UNITS;
+  return std::max(units, 5 * nt);
+}
+
+struct Pair3xPlan {
+  int groups;       // groups of tiles_n pairs with equal contiguous shares of the rows, or 0: tiles round robin
+  int64_t busiest;  // cost of the busiest pair
+};
+
+// Shares or round robin: whichever keeps the busiest pair busy for less.  (R32 1024^3: 58 units against 66.)
+static Pair3xPlan pair3x_plan(int64_t R, int64_t I, int64_t K, int64_t pairs) {
+  const int64_t units = (I + 31) / 32, tiles_n = (K + 2 * Lm2expPair3xCfg::BM - 1) / (2 * Lm2expPair3xCfg::BM);
+  const int64_t nt = (units + Lm2expPair3xCfg::UNITS - 1) / Lm2expPair3xCfg::UNITS;
+  const int64_t robin = (R * tiles_n * nt + pairs - 1) / pairs * std::max<int64_t>((units + nt - 1) / nt, 5);
+  const int64_t total = R * units;
+  const int64_t groups = std::min(pairs / tiles_n, total);
+  if (groups < 1) return {0, robin};
+  int64_t busiest = 0;
+  for (int64_t g = 0; g < groups; ++g) {
+    const int64_t lo = total * g / groups, hi = total * (g + 1) / groups;
+    const int64_t r0 = lo / units, r1 = (hi - 1) / units;  // first and last batch entry of the share
+    const int64_t cost = r0 == r1 ? pair3x_cost(hi - lo)
+                                  : pair3x_cost((r0 + 1) * units - lo) + (r1 - r0 - 1) * pair3x_cost(units) + pair3x_cost(hi - r1 * units);
+    busiest = std::max(busiest, cost);
+  }
+  return busiest <= robin ? Pair3xPlan{static_cast<int>(groups), busiest} : Pair3xPlan{0, robin};
+}
+
+// Tiles of 192 rows with two accumulators, or of 256 with one?  Cycles of the busiest pair: the second leaves 14 400 of every
+// tile to the epilogue and its tiles come in whole waves; in the first a unit takes 1.1 times its MMAs, or the 2 500 of its
+// epilogue where the contraction is short, and the last epilogue 8 000 alone.  us, one / two accumulators: R48 260x1000x300 129 /
+// 82, R40 1000x700x700 212 / 175, R12 768^3 75 / 58, R64 320x128x512 57 / 40, R8 384x256x2048 39.6 / 30.1, R64 512x512x256 62.6 / 55.8,
+// R24 512x256x1024 59.2 / 52.9, R16 1024x1024x512 95 / 87; R1 2048^3 89 / 91 and R100 512x64x256 38.3 / 39.6, which the
+// estimate leaves to one accumulator.
+// A launch of more than about 130 us runs at the power limit, where regenerating the operand for more tiles costs what the
+// overlap gains (R32 1024^3 316 / 324): there only a quarter less of cycles counts.
+static bool pair3x_wins(int64_t R, int64_t I, int64_t J, int64_t K) {
+  const int64_t pairs = sm_count() / 2, kb = (J + 31) / 32;
+  const double one = static_cast<double>((R * ((I + 255) / 256) * ((K + 255) / 256) + pairs - 1) / pairs) * (kb * 1536.0 + 14400.0);
+  const double busiest = static_cast<double>(pair3x_plan(R, I, K, pairs).busiest);
+  const double two = busiest * 1.1 * std::max(kb * 192.0, 2300.0) + 8000.0;
+  return two < (busiest * kb * 192.0 < 250e3 ? 0.9 : 0.75) * one;
+}
+
+static int launch_lm2exp_pair3x(const CUtensorMap& ta, const CUtensorMap& tb_plain, const CUtensorMap& to, Lm2expParams p,
+                                cudaStream_t stream, bool after_prepass) {
+  using Cfg = Lm2expPair3xCfg;
+  static std::once_flag once[64];
+  static cudaError_t attr_rc[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return TRITURUS_B200_ELAUNCH;
+  std::call_once(once[dev], [&] {
+    attr_rc[dev] = cudaFuncSetAttribute(lm2exp_pair3x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+  });
+  if (attr_rc[dev] != cudaSuccess) return TRITURUS_B200_ELAUNCH;
+  const int64_t pairs = sm_count() / 2;
+  p.tiles_m = (p.I + 31) / 32;
+  p.tiles_n = (p.K + 2 * Cfg::BM - 1) / (2 * Cfg::BM);
+  const int64_t nt = static_cast<int64_t>(p.R) * p.tiles_n * ((p.tiles_m + Cfg::UNITS - 1) / Cfg::UNITS);
+  if (nt > INT32_MAX) return TRITURUS_B200_EINVAL;
+  p.num_tiles = static_cast<int>(nt);
+  p.pair_groups = pair3x_plan(p.R, p.I, p.K, pairs).groups;
+  const int64_t clusters = p.pair_groups > 0 ? static_cast<int64_t>(p.pair_groups) * p.tiles_n : std::min(nt, pairs);
+  return launch_maybe_dependent(lm2exp_pair3x_kernel, dim3(static_cast<unsigned>(2 * clusters)), Cfg::NTHREADS, Cfg::SMEM_BYTES,
+                                stream, after_prepass, ta, tb_plain, to, p);
+}
+
 static int64_t tile_count(int64_t R, int64_t rows, int64_t cols, int bn, int mt) {
   return R * ((rows + 128 * mt - 1) / (128 * mt)) * ((cols + bn - 1) / bn);
 }
@@ -746,6 +823,12 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   // Every tensor map is encoded before the pre-pass is launched: the contraction kernel then follows it
   // directly in the stream, which its launch as a programmatic dependent requires.
   const bool prepass = !fused && b_colmax == nullptr;
+  // The TMEM-operand pair kernels in plain TF32 take a with j contiguous only and do not fold column maxima of the
+  // result; other calls run on the pair kernel that keeps the operand in shared memory.
+  const bool prec_3x = precision == TRITURUS_B200_PRECISION_3XTF32;
+  const bool use_ts = (plan.tspair && !a_mn && out_colmax == nullptr) || (pair && prec_3x);
+  const bool ts_halves = use_ts && !prec_3x && J <= 32 * LmTsPair::NS;
+  const bool pair3x = use_ts && prec_3x && pair3x_wins(R, I, J, K);
 
   CUtensorMap ta, tb;
   memset(&ta, 0, sizeof(ta));
@@ -761,7 +844,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   } else {
     const int64_t dims[3] = {J, I, R};
     const int64_t strides[3] = {1, as1, as0};
-    const uint32_t box[3] = {32, 128, 1};
+    const uint32_t box[3] = {32, pair3x ? static_cast<uint32_t>(Lm2expPair3xCfg::BN / 2) : 128u, 1};
     rc = make_tmap(&ta, a, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != TRITURUS_B200_OK) return rc;
   }
@@ -818,10 +901,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   p.fused_max = fused ? 1 : 0;
   p.status = status_dev;
 
-  // The TMEM-operand pair kernel in plain TF32 takes a with j contiguous only and does not fold column maxima of the
-  // result; other calls run on the pair kernel that keeps the operand in shared memory.  Its b tiles are 32 rows j x 128
-  // columns k, unswizzled (only the transform threads read them).
-  const bool use_ts = (plan.tspair && !a_mn && out_colmax == nullptr) || (pair && precision == TRITURUS_B200_PRECISION_3XTF32);
+  // The b tiles of the TMEM-operand kernels: 32 rows j x 128 columns k, unswizzled (only the transform threads read them).
   CUtensorMap tb_plain;
   if (use_ts) {
     const int64_t dims[3] = {K, J, R};
@@ -830,7 +910,10 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     rc = make_tmap(&tb_plain, b, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc != TRITURUS_B200_OK) return rc;
   }
-  const bool ts_halves = J <= 32 * LmTsPair::NS;
+  auto launch_3x = [&](const Lm2expParams& q, bool dependent) -> int {
+    return pair3x ? launch_lm2exp_pair3x(ta, tb_plain, to, q, st, dependent)
+                  : launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, q, st, dependent);
+  };
   const int64_t bstr[3] = {gen_b ? bs_raw[0] : bs0, gen_b ? bs_raw[1] : bs1, gen_b ? bs_raw[2] : 1};
   if (use_ts && plan.optimistic && prepass && ws_flags) {
     // No pre-pass: the contraction takes each column's stabiliser from its first 32 rows and raises the flag
@@ -858,15 +941,13 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
     if (rc != TRITURUS_B200_OK) return rc;
     Lm2expParams po = p;
     po.opt_flag = flag;
-    rc = use_ts ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, po, st, true)
-                : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
+    rc = use_ts ? launch_3x(po, true) : launch_lm2exp_pair<LmPairT>(ta, tb, to, po, st, true);
     if (rc != TRITURUS_B200_OK) return rc;
     rc = colmax_run(b, m_buf, R, J, K, bstr, stream, flag, flag + 1);
     if (rc != TRITURUS_B200_OK) return rc;
     p.only_if = flag + 1;
     p.reset_flag = flag;
-    return use_ts ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, true)
-                  : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, true);
+    return use_ts ? launch_3x(p, true) : launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, true);
   }
   if (prepass && b_km) {
     for (int64_t r0 = 0; r0 < R; r0 += 65535) {  // (R <= 65535 here: one round)
@@ -880,7 +961,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   }
   const bool dep = prepass;
   if (use_ts)
-    return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_tspair<LmTsPairX>(ta, tb_plain, to, p, st, dep)
+    return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_3x(p, dep)
            : ts_halves ? launch_lm2exp_tspair<LmTsPairH>(ta, tb_plain, to, p, st, dep)
                        : launch_lm2exp_tspair<LmTsPair>(ta, tb_plain, to, p, st, dep);
   if (pair) return launch_lm2exp_pair<LmPairT>(ta, tb, to, p, st, dep);

@@ -40,6 +40,7 @@ struct Lm2expParams {
   int64_t out_s0, out_s1;  // element strides of out (innermost stride is 1)
   int R, I, J, K;
   int tiles_m, tiles_n, num_tiles;
+  int pair_groups = 0;      // lm2exp_pair3x_kernel: groups of pairs with equal shares of the rows (tiles_m: units of 32 rows)
   int fused_max;
   int out_tma;              // out meets the TMA rules: the epilogue stores through tmap_out
   int a_mn;                 // a is stored with i contiguous (a transposed view): MN-major A operand, loaded as

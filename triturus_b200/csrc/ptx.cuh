@@ -465,6 +465,24 @@ __device__ __forceinline__ float lg2_approx(float x) {
 // exp(v - m) with the subtraction done first, as the reference does (baselines/lm2exp.py:13).
 __device__ __forceinline__ float exp_shifted(float v, float m) { return ex2_approx((v - m) * LOG2E_F); }
 
+// The same of two values: the subtractions and the products as one instruction each (the same roundings).
+__device__ __forceinline__ void exp_shifted_x2(float v0, float v1, float m, float& e0, float& e1) {
+  float t0, t1;
+  asm("{\n\t"
+      ".reg .b64 v, m, l;\n\t"
+      "mov.b64 v, {%2, %3};\n\t"
+      "mov.b64 m, {%4, %4};\n\t"
+      "mov.b64 l, {%5, %5};\n\t"
+      "add.rn.f32x2 v, v, m;\n\t"
+      "mul.rn.f32x2 v, v, l;\n\t"
+      "mov.b64 {%0, %1}, v;\n\t"
+      "}"
+      : "=f"(t0), "=f"(t1)
+      : "f"(v0), "f"(v1), "f"(-m), "f"(LOG2E_F));
+  e0 = ex2_approx(t0);
+  e1 = ex2_approx(t1);
+}
+
 // Round an fp32 in [0, +inf) to the nearest tf32 (ties away), as raw bits.  The tensor core drops the low
 // 13 mantissa bits of its operands, so adding half a tf32 ulp beforehand turns that truncation into
 // rounding.  Not valid for inf/nan.
