@@ -98,6 +98,11 @@ size_t triturus_b200_lm2exp_workspace_bytes(int64_t R, int64_t I, int64_t J, int
  * 4 (optimistic 32-row pre-pass, contraction, and two conditional launches; a with j contiguous and a full-size
  * workspace assumed); negative on invalid arguments.  The reference has no counterpart (its launch count is Triton's business, triturus/lm2exp.py:186-205). */
 int triturus_b200_lm2exp_launches(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant);
+/* Small calls.  An automatic call (variant 0) whose time would be latency runs one launch of lm2exp_direct_kernel (mma.sync
+ * on 32 x 32 tiles) instead of the plan that triturus_b200_lm2exp_plan and _launches name, which an explicit variant still
+ * runs: 1 when a call with these arguments does (`odd`: a or b cannot be described by a tensor map), else 0; negative on invalid arguments.
+ * Results agree with the plan's kernels to rounding.  Such a call touches neither the workspace nor the status word. */
+int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd);
 int triturus_b200_lm2exp_f32(const float* a, const float* b, float* out, int64_t R, int64_t I, int64_t J, int64_t K,
                              const int64_t a_strides[3], const int64_t b_strides[3], const int64_t out_strides[3],
                              int precision, int variant, void* workspace, size_t workspace_bytes,
@@ -160,6 +165,17 @@ int triturus_b200_lm2exp_chain_f32(const float* a, const float* b, float* out, i
 /* Number of kernels one triturus_b200_lt2exp_f32 call launches for these arguments on the current device
  * (1, or 3 when the contraction is split); negative on invalid arguments. */
 int triturus_b200_lt2exp_launches(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant);
+/* Small calls, as for lm2exp: 1 when an automatic or unsplit call (variant 0 or 10000) with these arguments runs one launch of
+ * lt2exp_direct_kernel instead of its plan (`odd_w`: the rows of w can only be fetched 4 bytes at a time: J odd, or strides or base odd).
+ * Deterministic, also where the plan would split the contraction. */
+int triturus_b200_lt2exp_direct(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd_w);
+/* That kernel by itself, for w of any strides as well: the other entry points want w to meet the tensor-map rules.
+ * I and J at most 128 each and (I + J) * 160 + J * 2048 bytes of shared memory within 200 KB (TRITURUS_B200_EINVAL else).
+ * a_colmax, b_colmax, out_colmax as in triturus_b200_lt2exp_chain_f32 (all may be NULL). */
+int triturus_b200_lt2exp_direct_f32(const float* w, const float* a, const float* b, float* out, int64_t R, int64_t S, int64_t I,
+                                    int64_t J, int64_t K, const int64_t w_strides[4], const int64_t a_strides[3],
+                                    const int64_t b_strides[3], const int64_t out_strides[3], int precision, const float* a_colmax,
+                                    const float* b_colmax, float* out_colmax, void* stream);
 /* What a triturus_b200_lt2exp_f32 call with these arguments runs on the current device, as the explicit variant
  * code that pins it: SPLIT * 10000 + BN * 10 + MT with SPLIT = 1 (whole tiles), the slice count, or 9998 (last
  * wave shared).  The counterpart of reading the reference's autotuner choice (triturus/lt2exp.py:9-75,78-222); negative

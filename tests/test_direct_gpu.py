@@ -1,0 +1,117 @@
+"""The kernels for small calls (mma.sync on 32 x 32 tiles) against float64: at the edges of their tiles, for every layout of the
+operands that they fetch, with impossible states, supplied and returned column maxima, and against the tcgen05 kernels."""
+
+import pytest
+import torch
+
+from oracle import logspace_oracle as orc
+from triturus_b200 import _native
+
+# Plain TF32 rounds both operands of a product to nearest at 10 fraction bits: off by 2^-11 of themselves at most each, and
+# exp(b - m) by ulps.  3xTF32: sums of at most 512 (lm2exp) or 128 (lt2exp) terms; the products' low parts are cut at 2^-11 of
+# 2^-11, and a sum of 64 MMAs, each truncated, in eight partial sums drifts by 8 * 2^-23.
+TOL = {"tf32": 2 * 2.0**-11 + 1e-5, "3xtf32": 1e-5}
+# The tcgen05 kernels round one operand and truncate the other, 2^-11 + 2^-10, and the above on this side.
+TOL_BOTH = {"tf32": 2.0**-11 + 2.0**-10 + TOL["tf32"], "3xtf32": 1.1e-4}
+
+
+def _views(t):
+    """`t` in the layouts that a caller may pass: contiguous, the last two dimensions swapped in memory, every second element of
+    a wider tensor, at an odd base, and with an odd row pitch."""
+    wide = torch.zeros(*t.shape[:-1], 2 * t.shape[-1], device=t.device)
+    wide[..., ::2] = t
+    shifted = torch.zeros(t.numel() + 1, device=t.device)
+    shifted[1:] = t.flatten()
+    pitched = torch.zeros(*t.shape[:-1], t.shape[-1] + 1 + t.shape[-1] % 2, device=t.device)
+    pitched[..., : t.shape[-1]] = t
+    return [t, t.transpose(-1, -2).contiguous().transpose(-1, -2), wide[..., ::2], shifted[1:].view(t.shape), pitched[..., : t.shape[-1]]]
+
+
+def _check(got, want, tol):
+    assert torch.equal(got.cpu() == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
+    fin = torch.isfinite(want)
+    err = (got.cpu().double() - want).abs()[fin]
+    tol = tol + 2.0**-22 * want.abs()[fin]
+    assert (err <= tol).all(), (err - tol).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (2, 33, 9, 31), (3, 32, 8, 64), (2, 31, 7, 33), (1, 64, 64, 96), (5, 40, 130, 44),
+                                   (1, 70, 511, 66), (1, 32, 512, 32)], ids=str)  # fmt: skip
+def test_lm2exp(shape, precision):
+    import triturus_b200 as tb
+
+    R, I, J, K = shape
+    for odd in (0, 1):
+        assert _native.LIB.triturus_b200_lm2exp_direct(*shape, int(precision == "3xtf32"), 0, odd) == 1
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    b[torch.rand(R, J, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K - 1] = float("-inf")
+    a[R - 1, I - 1] = 0.0
+    want = orc.lm2exp_fp64(a, b)
+    first = None
+    for av in _views(a.cuda()):
+        for bv in _views(b.cuda()):
+            got = tb.lm2exp(av, bv, precision=precision)
+            first = got if first is None else first
+            assert torch.equal(got, first)  # the layout does not matter, bit for bit
+    _check(first, want, TOL[precision])
+    ad, bd = a.cuda(), b.cuda()
+    m = bd.amax(1)
+    out, top = tb.lm2exp(ad, bd, precision=precision, b_colmax=m, return_colmax=True)
+    assert torch.equal(out, first) and torch.equal(top, out.amax(1))
+    if R > 1:
+        same = tb.lm2exp(ad[:1].expand(R, I, J), bd[:1].expand(R, J, K), precision=precision)  # stride 0
+        assert torch.equal(same, first[:1].expand(R, I, K))
+    ref = tb.lm2exp(ad, bd, precision=precision, variant=1281)
+    _check(ref, first.cpu().double(), TOL_BOTH[precision])
+    tb.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1, 1), (2, 33, 3, 9, 31), (1, 32, 9, 8, 64), (2, 31, 17, 7, 33), (1, 40, 65, 33, 36), (1, 64, 50, 50, 100),
+                                   (1, 20, 128, 16, 32), (3, 75, 50, 50, 100)], ids=str)  # fmt: skip
+def test_lt2exp(shape, precision):
+    import triturus_b200 as tb
+
+    R, S, I, J, K = shape
+    for odd in (0, 1):
+        assert _native.LIB.triturus_b200_lt2exp_direct(*shape, int(precision == "3xtf32"), 0, odd) == 1
+    g = torch.Generator().manual_seed(sum(shape))
+    w = torch.rand(R, S, I, J, generator=g)
+    a = torch.randn(R, I, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    a[torch.rand(R, I, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K - 1] = float("-inf")
+    w[R - 1, S - 1] = 0.0
+    want = orc.lt2exp_fp64(w, a, b)
+    wd, ad, bd = w.cuda(), a.cuda(), b.cuda()
+    first = tb.lt2exp(wd, ad, bd, precision=precision)
+    _check(first, want, TOL[precision])
+    for av, bv in zip(_views(ad), reversed(_views(bd))):
+        assert torch.equal(tb.lt2exp(wd, av, bv, precision=precision), first)
+    flat = torch.zeros(w.numel() + 1, device="cuda")
+    flat[1:] = wd.flatten()
+    assert torch.equal(tb.lt2exp(flat[1:].view(w.shape), ad, bd, precision=precision, mode="unsplit"), first)
+    out, top = tb.lt2exp(wd, ad, bd, precision=precision, a_colmax=ad.amax(1), b_colmax=bd.amax(1), return_colmax=True)
+    assert torch.equal(out, first) and torch.equal(top, out.amax(1))
+    ref = tb.lt2exp(wd, ad, bd, precision=precision, variant=11281)
+    _check(ref, first.cpu().double(), TOL_BOTH[precision])
+    tb.check_status()
+
+
+def test_which_calls_are_small():
+    """Explicit variants run what they name, and the rules keep to sizes that the kernels can hold."""
+    lm, lt = _native.LIB.triturus_b200_lm2exp_direct, _native.LIB.triturus_b200_lt2exp_direct
+    assert lm(4, 256, 256, 256, 0, 0, 0) == 1 and lm(4, 256, 256, 256, 0, 201281, 0) == 0
+    assert lm(32, 1024, 1024, 1024, 1, 0, 0) == 0 and lm(1, 1, 513, 1, 0, 0, 0) == 0
+    assert lm(24, 150, 101, 203, 1, 0, 1) == 1 and lm(0, 1, 1, 1, 0, 0, 0) < 0
+    assert lt(3, 75, 50, 50, 100, 1, 0, 1) == 1 and lt(3, 75, 50, 50, 100, 1, 10000, 1) == 1
+    assert lt(3, 75, 50, 50, 100, 1, 99990000, 1) == 0 and lt(3, 75, 50, 50, 100, 1, 11281, 1) == 0
+    assert lt(1, 256, 256, 256, 256, 1, 0, 0) == 0 and lt(1, 1, 128, 128, 1, 0, 0, 0) == 0
+    for shape in ((1, 1, 129, 1, 1), (1, 1, 1, 129, 1)):
+        assert lt(*shape, 0, 0, 0) == 0

@@ -23,6 +23,9 @@ EXPORTED_SYMBOLS = (
     "triturus_b200_lm2exp_launches",
     "triturus_b200_lt2exp_launches",
     "triturus_b200_lt2exp_plan",
+    "triturus_b200_lm2exp_direct",
+    "triturus_b200_lt2exp_direct",
+    "triturus_b200_lt2exp_direct_f32",
     "triturus_b200_lm2exp_plan",
     "triturus_b200_lm2exp_f32",
     "triturus_b200_lm2exp_chain_launches",
@@ -92,6 +95,15 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.triturus_b200_lt2exp_launches.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int]
     lib.triturus_b200_lt2exp_plan.restype = c_int
     lib.triturus_b200_lt2exp_plan.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int]
+    lib.triturus_b200_lm2exp_direct.restype = c_int
+    lib.triturus_b200_lm2exp_direct.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int, c_int, c_int]
+    lib.triturus_b200_lt2exp_direct.restype = c_int
+    lib.triturus_b200_lt2exp_direct.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int, c_int]
+    lib.triturus_b200_lt2exp_direct_f32.restype = c_int
+    lib.triturus_b200_lt2exp_direct_f32.argtypes = [
+        c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
+        i64p, i64p, i64p, i64p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+    ]  # fmt: skip
     lib.triturus_b200_lm2exp_plan.restype = c_int
     lib.triturus_b200_lm2exp_plan.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int, c_int]
     lib.triturus_b200_lm2exp_f32.restype = c_int
@@ -420,11 +432,35 @@ def _lm2exp_chain_impl(
     return out, out_colmax
 
 
+def _lt2exp_direct_odd(w: torch.Tensor, K: int, precision: int, variant: int) -> bool:
+    """True when a call with a w that breaks the tensor-map rules is small enough for the kernel that takes any strides."""
+    R, S, I, J = w.shape
+    odd = (w.data_ptr() // 4 | J | w.stride(0) | w.stride(1) | w.stride(2)) & 1 != 0 or w.stride(3) != 1
+    return LIB.triturus_b200_lt2exp_direct(R, S, I, J, K, int(precision), int(variant), int(odd)) == 1
+
+
+def _lt2exp_direct(w, a, b, a_colmax, b_colmax, out_colmax, precision: int) -> torch.Tensor:
+    R, S, I, J = w.shape
+    K = a.shape[2]
+    out = torch.empty((R, S, K), dtype=torch.float32, device=a.device)
+    with _on_device(a.device) as idx:
+        rc = LIB.triturus_b200_lt2exp_direct_f32(
+            w.data_ptr(), a.data_ptr(), b.data_ptr(), out.data_ptr(), R, S, I, J, K,
+            _i64(w.stride()), _i64(a.stride()), _i64(b.stride()), _i64(out.stride()), int(precision),
+            *(None if t is None else t.data_ptr() for t in (a_colmax, b_colmax, out_colmax)), _raw_stream(idx),
+        )  # fmt: skip
+    _check(rc, "triturus_b200_lt2exp_direct_f32")
+    return out
+
+
 def _lt2exp_impl(w: torch.Tensor, a: torch.Tensor, b: torch.Tensor, precision: int, variant: int) -> torch.Tensor:
     _require_cuda(w, a, b)
     R, S, I, J = w.shape
     K = a.shape[2]
-    w = _tma_ready(w)
+    if not _tma_ok(w):
+        if _lt2exp_direct_odd(w, K, precision, variant):
+            return _lt2exp_direct(w, a, b, None, None, None, precision)
+        w = _tma_ready(w)
     # a and b are read with ordinary loads and go in as they are, whatever their strides (16-byte loads when they
     # allow it; a view with a k stride other than 1 is read 4 bytes at a time, uncoalesced but without a copy)
     out = torch.empty((R, S, K), dtype=torch.float32, device=a.device)
@@ -478,9 +514,13 @@ def _lt2exp_chain_impl(
     _require_cuda(w, a, b)
     R, S, I, J = w.shape
     K = a.shape[2]
-    w = _tma_ready(w)
     a_colmax = _colmax_arg(a_colmax, R, K, a, "a_colmax")
     b_colmax = _colmax_arg(b_colmax, R, K, a, "b_colmax")
+    if not _tma_ok(w):
+        if _lt2exp_direct_odd(w, K, precision, variant):
+            out_colmax = torch.empty((R, K) if want_colmax else (0,), dtype=torch.float32, device=a.device)
+            return _lt2exp_direct(w, a, b, a_colmax, b_colmax, out_colmax if want_colmax else None, precision), out_colmax
+        w = _tma_ready(w)
     out = torch.empty((R, S, K), dtype=torch.float32, device=a.device)
     out_colmax = torch.empty((R, K) if want_colmax else (0,), dtype=torch.float32, device=a.device)
     with _on_device(a.device) as idx:

@@ -17,6 +17,7 @@
 #include "lm2exp_pair3x_kernel.cuh"
 #include "lt2exp_kernel.cuh"
 #include "lt2exp_tmem_kernel.cuh"
+#include "direct_kernels.cuh"
 
 namespace tb200 {
 
@@ -744,6 +745,78 @@ size_t triturus_b200_lm2exp_workspace_bytes(int64_t R, int64_t I, int64_t J, int
   return kLm2expFlagBytes + static_cast<size_t>(R) * static_cast<size_t>(K) * sizeof(float);
 }
 
+}  // extern "C"
+
+// ----------------------------------------------------------------------------- small problems
+
+namespace tb200 {
+
+// Floats per copy of rows of `n` consecutive values: 4 or 2 where base, row length and the strides of the other dimensions
+// are multiples of it, else 1.
+static int direct_width(const float* base, int64_t n, int64_t inner, int64_t s0, int64_t s1, int64_t s2 = 0) {
+  if (inner != 1) return 1;
+  const uint64_t bits = (reinterpret_cast<uintptr_t>(base) >> 2) | static_cast<uint64_t>(n) | static_cast<uint64_t>(s0) |
+                        static_cast<uint64_t>(s1) | static_cast<uint64_t>(s2);
+  return (bits & 3) == 0 ? 4 : (bits & 1) == 0 ? 2 : 1;
+}
+
+// Does an automatic call of lm2exp run lm2exp_direct_kernel?  Estimates in us, of device time in a graph.  Direct: 3 and, per 32 x 32
+// tile, 5 ns and 0.034 per contraction value (more where shared memory leaves one or two blocks per SM, and with the third
+// product); else what one wave of the tcgen05 kernels takes, 2.5 times that where they fetch an operand element by
+// element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 512^3 24.0 / 11.2, 1 x 1024x128x1024 11.7 / 11.4,
+// 16 x 256^3 15.8 / 17.0, 64 x 128x128x512 17.0 / 39.5; odd: 100 x 65x33x70 19.5 / 8.5, 64 x 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50.
+// 3xTF32: 1 x 64^3 11.1 / 3.2, 8 x 128^3 17.4 / 3.8, 1 x 512^3 33.3 / 13.6, 16 x 256^3 23.1 / 19.8, 32 x 256^3 23.4 / 36.3; odd: 24 x
+// 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58.
+static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd) {
+  if (J > 512 || R > 65535 || (I + 31) / 32 > 65535) return false;
+  const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
+  const double tiles = static_cast<double>(R) * ((I + 31) / 32) * ((K + 31) / 32);
+  const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? 1.4 : 1.0) * (odd ? 1.3 : 1.0);
+  const double tcgen = (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
+  return direct <= tcgen;
+}
+
+// Raises the shared-memory limit of a kernel once per device.
+template <auto Kern>
+static bool direct_smem_limit(int bytes) {
+  static std::once_flag once[64];
+  static cudaError_t attr_rc[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return false;
+  std::call_once(once[dev], [&] { attr_rc[dev] = cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+  return attr_rc[dev] == cudaSuccess;
+}
+
+template <int PREC>
+static int launch_lm2exp_direct(const DirectLmParams& p, int64_t R, cudaStream_t stream) {
+  if (!direct_smem_limit<lm2exp_direct_kernel<PREC>>(direct_lm_smem(512))) return TRITURUS_B200_ELAUNCH;
+  const dim3 grid(static_cast<unsigned>((p.K + 31) / 32), static_cast<unsigned>((p.I + 31) / 32), static_cast<unsigned>(R));
+  lm2exp_direct_kernel<PREC><<<grid, DIRECT_THREADS, direct_lm_smem(p.J), stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? TRITURUS_B200_OK : TRITURUS_B200_ELAUNCH;
+}
+
+static int lm2exp_direct(const float* a, const float* b, float* out, int64_t R, int64_t I, int64_t J, int64_t K, const int64_t as[3],
+                         const int64_t bs[3], const int64_t os[3], int precision, const float* b_colmax, float* out_colmax, cudaStream_t stream) {
+  DirectLmParams p;
+  p.a = a, p.b = b, p.out = out, p.m_in = b_colmax, p.out_max = out_colmax;
+  p.a_s0 = as[0], p.a_s1 = as[1], p.a_s2 = as[2];
+  p.b_s0 = bs[0], p.b_s1 = bs[1], p.b_s2 = bs[2];
+  p.out_s0 = os[0], p.out_s1 = os[1];
+  p.I = static_cast<int>(I), p.J = static_cast<int>(J), p.K = static_cast<int>(K);
+  p.width_a = direct_width(a, J, as[2], as[0], as[1]);
+  p.width_b = direct_width(b, K, bs[2], bs[0], bs[1]);
+  if (out_colmax != nullptr) {
+    const int64_t blocks = (R * K + 255) / 256;
+    fill_neg_inf_kernel<<<static_cast<int>(blocks < 1184 ? blocks : 1184), 256, 0, stream>>>(out_colmax, R * K);
+  }
+  return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lm2exp_direct<1>(p, R, stream) : launch_lm2exp_direct<0>(p, R, stream);
+}
+
+}  // namespace tb200
+
+extern "C" {
+
 // Shared body of the lm2exp entry points.  b_colmax (optional): [R, K] column maxima of b supplied by the
 // caller, which replace the stabiliser pass.  out_colmax (optional): [R, K] receives max_i out[r, i, k].
 static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t R, int64_t I, int64_t J, int64_t K,
@@ -796,6 +869,9 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   if (gen_b) b_km = false;
   // (the element-wise loader takes the place of the warps that fold the column maxima of the result)
   if ((gen_a || gen_b) && out_colmax != nullptr) return TRITURUS_B200_EALIGN;
+  if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b))
+    return lm2exp_direct(a, b, out, R, I, J, K, a_strides, b_strides, out_strides, precision, b_colmax, out_colmax,
+                         static_cast<cudaStream_t>(stream));
 
   Lm2expPlan plan;
   {
@@ -1031,6 +1107,12 @@ static int lm2exp_run(const float* a, const float* b, float* out, int64_t R, int
     if (rc != TRITURUS_B200_OK) return rc;
   }
   return TRITURUS_B200_OK;
+}
+
+int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd) {
+  if (R <= 0 || I <= 0 || J <= 0 || K <= 0) return TRITURUS_B200_EINVAL;
+  if (precision != TRITURUS_B200_PRECISION_TF32 && precision != TRITURUS_B200_PRECISION_3XTF32) return TRITURUS_B200_EINVAL;
+  return variant == 0 && direct_lm_wins(R, I, J, K, precision, odd != 0) ? 1 : 0;
 }
 
 int triturus_b200_mm_f32(const float* a, const float* b, float* out, int64_t M, int64_t K, int64_t N,
@@ -1432,6 +1514,67 @@ extern "C" size_t triturus_b200_lt2exp_workspace_bytes(int64_t R, int64_t S, int
   return rc == TRITURUS_B200_OK ? q.ws_bytes : 0;
 }
 
+// Does an automatic call of lt2exp that never splits, or is free to, run lt2exp_direct_kernel?  Estimate in us as for lm2exp: 4
+// and, per 32 x 32 tile (37 tiles at least: 296 blocks in clusters of eight), 12 ns and 0.035 per term, 1.6 times that for
+// rows of w that only 4-byte copies can fetch; the third product a quarter more.  The tcgen05 kernel takes 19 - 24 us for
+// such calls in TF32 and 29 - 35 in 3xTF32.  tcgen05 / direct, TF32: 1 x 32 32x32x64 19.9 / 5.7, 1 x 128 64x64x256 22.8 / 8.9, 16 x 32
+// 32x32x512 20.8 / 18.6, 8 x 128 32x32x512 22.2 / 27.0; 3xTF32: 1 x 64 64x64x128 29.8 / 7.7, 3 x 75 50x50x100 34.7 / 17.0, 16 x 32 32x32x512
+// 29.2 / 21.7, 8 x 128 32x32x512 32.6 / 35.1.
+static bool direct_lt_wins(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant, bool odd) {
+  if ((variant != 0 && variant != 10000) || R > 65535 || (S + 31) / 32 > 65535 || J > 128 || I > 128) return false;
+  if (tb200::direct_lt_smem(static_cast<int>(I), static_cast<int>(J), 2) > 200 * 1024) return false;
+  const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
+  const double tiles = std::max(static_cast<double>(R) * ((S + 31) / 32) * ((K + 31) / 32), 37.0);
+  const double terms = static_cast<double>(I) * ((J + 7) / 8 * 8);
+  return (4.0 + tiles * (0.012 + 0.035e-3 * terms * (odd ? 1.6 : 1.0))) * (x3 ? 1.25 : 1.0) <= (x3 ? 27.0 : 17.0);
+}
+
+template <int PREC>
+static int launch_lt2exp_direct(const tb200::DirectLtParams& p, int64_t R, cudaStream_t stream) {
+  using namespace tb200;
+  if (!direct_smem_limit<lt2exp_direct_kernel<PREC>>(200 * 1024)) return TRITURUS_B200_ELAUNCH;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((p.K + 31) / 32 * p.parts), static_cast<unsigned>((p.S + 31) / 32), static_cast<unsigned>(R));
+  cfg.blockDim = dim3(DIRECT_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>(direct_lt_smem(p.I, p.J, p.nbuf));
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = static_cast<unsigned>(p.parts);
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, lt2exp_direct_kernel<PREC>, p) == cudaSuccess ? TRITURUS_B200_OK : TRITURUS_B200_ELAUNCH;
+}
+
+static int lt2exp_direct(const float* w, const float* a, const float* b, float* out, int64_t R, int64_t S, int64_t I, int64_t J, int64_t K,
+                         const int64_t ws[4], const int64_t as[3], const int64_t bs[3], const int64_t os[3], int precision,
+                         const float* a_colmax, const float* b_colmax, float* out_colmax, cudaStream_t stream) {
+  using namespace tb200;
+  DirectLtParams p;
+  p.w = w, p.a = a, p.b = b, p.out = out, p.ma_in = a_colmax, p.mb_in = b_colmax, p.out_max = out_colmax;
+  p.w_s0 = ws[0], p.w_s1 = ws[1], p.w_s2 = ws[2], p.w_s3 = ws[3];
+  p.a_s0 = as[0], p.a_s1 = as[1], p.a_s2 = as[2];
+  p.b_s0 = bs[0], p.b_s1 = bs[1], p.b_s2 = bs[2];
+  p.out_s0 = os[0], p.out_s1 = os[1];
+  p.S = static_cast<int>(S), p.I = static_cast<int>(I), p.J = static_cast<int>(J), p.K = static_cast<int>(K);
+  p.width_w = direct_width(w, J, ws[3], ws[0], ws[1], ws[2]);
+  p.width_a = direct_width(a, K, as[2], as[0], as[1]);
+  p.width_b = direct_width(b, K, bs[2], bs[0], bs[1]);
+  // Blocks that share a tile's rows i: enough to fill the GPU, each with at least one row per warp.
+  const int64_t tiles = R * ((S + 31) / 32) * ((K + 31) / 32);
+  int parts = 1;
+  while (parts < 8 && tiles * parts < 2 * sm_count() && I > 8 * parts) parts *= 2;
+  p.parts = parts;
+  p.nbuf = I > 8 * parts ? 2 : 1;
+  if (out_colmax != nullptr) {
+    const int64_t blocks = (R * K + 255) / 256;
+    fill_neg_inf_kernel<<<static_cast<int>(blocks < 1184 ? blocks : 1184), 256, 0, stream>>>(out_colmax, R * K);
+  }
+  return precision == TRITURUS_B200_PRECISION_3XTF32 ? launch_lt2exp_direct<1>(p, R, stream) : launch_lt2exp_direct<0>(p, R, stream);
+}
+
 // Shared body of the lt2exp entry points.  a_colmax / b_colmax (optional, both or neither): [R, K] column
 // maxima of a and b, which replace the scan at the start of every tile.  out_colmax (optional): [R, K] receives
 // max_s out[r, s, k].
@@ -1464,6 +1607,9 @@ static int lt2exp_run_block(const float* w, const float* a, const float* b, floa
   if (!fix_stride(I, ws2, j4) || !fix_stride(S, ws1, j4 * I) || !fix_stride(R, ws0, j4 * I * S))
     return TRITURUS_B200_EALIGN;
   if ((S > 1 && os1 <= 0) || (R > 1 && os0 <= 0)) return TRITURUS_B200_EALIGN;
+  if (direct_lt_wins(R, S, I, J, K, precision, variant, tb200::direct_width(w, J, w_strides[3], w_strides[0], w_strides[1], w_strides[2]) == 1))
+    return lt2exp_direct(w, a, b, out, R, S, I, J, K, w_strides, a_strides, b_strides, out_strides, precision, a_colmax, b_colmax,
+                         out_colmax, static_cast<cudaStream_t>(stream));
 
   int bn, mt, split;
   bool promote;
@@ -1554,6 +1700,34 @@ extern "C" int triturus_b200_lt2exp_ws_f32(const float* w, const float* a, const
                                            size_t workspace_bytes, int32_t* status_dev, void* stream) {
   return lt2exp_run(w, a, b, out, R, S, I, J, K, w_strides, a_strides, b_strides, out_strides, precision, variant,
                     nullptr, nullptr, nullptr, workspace, workspace_bytes, status_dev, stream);
+}
+
+extern "C" int triturus_b200_lt2exp_direct(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant,
+                                           int odd_w) {
+  const int rc = lt2exp_check_dims(R, S, I, J, K, precision);
+  if (rc != TRITURUS_B200_OK) return rc;
+  return direct_lt_wins(R, S, I, J, K, precision, variant, odd_w != 0) ? 1 : 0;
+}
+
+extern "C" int triturus_b200_lt2exp_direct_f32(const float* w, const float* a, const float* b, float* out, int64_t R, int64_t S,
+                                               int64_t I, int64_t J, int64_t K, const int64_t w_strides[4], const int64_t a_strides[3],
+                                               const int64_t b_strides[3], const int64_t out_strides[3], int precision,
+                                               const float* a_colmax, const float* b_colmax, float* out_colmax, void* stream) {
+  if (w == nullptr || a == nullptr || b == nullptr || out == nullptr || w_strides == nullptr || a_strides == nullptr ||
+      b_strides == nullptr || out_strides == nullptr)
+    return TRITURUS_B200_EINVAL;
+  if ((a_colmax == nullptr) != (b_colmax == nullptr)) return TRITURUS_B200_EINVAL;
+  if (out_colmax != nullptr && (out_colmax == a_colmax || out_colmax == b_colmax)) return TRITURUS_B200_EINVAL;
+  const int rc = lt2exp_check_dims(R, S, I, J, K, precision);
+  if (rc != TRITURUS_B200_OK) return rc;
+  if (R > 65535 || (S + 31) / 32 > 65535 || J > 128 || I > 128 ||
+      tb200::direct_lt_smem(static_cast<int>(I), static_cast<int>(J), 2) > 200 * 1024)
+    return TRITURUS_B200_EINVAL;
+  if (((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(out)) & 3) != 0)
+    return TRITURUS_B200_EALIGN;
+  if ((K > 1 && out_strides[2] != 1) || (S > 1 && out_strides[1] <= 0) || (R > 1 && out_strides[0] <= 0)) return TRITURUS_B200_EALIGN;
+  return lt2exp_direct(w, a, b, out, R, S, I, J, K, w_strides, a_strides, b_strides, out_strides, precision, a_colmax, b_colmax, out_colmax,
+                       static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int triturus_b200_lt2exp_chain_f32(const float* w, const float* a, const float* b, float* out, int64_t R,
