@@ -115,3 +115,55 @@ def test_which_calls_are_small():
     assert lt(1, 256, 256, 256, 256, 1, 0, 0) == 0 and lt(1, 1, 128, 128, 1, 0, 0, 0) == 0
     for shape in ((1, 1, 129, 1, 1), (1, 1, 1, 129, 1)):
         assert lt(*shape, 0, 0, 0) == 0
+
+
+@pytest.mark.gpu
+def test_calls_that_the_extension_leaves_to_python():
+    """Small calls take the extension module; what it does not recognise behaves as without it: checks, modes, other streams
+    and subclasses."""
+    import triturus_b200 as tb
+
+    g = torch.Generator().manual_seed(3)
+    a, b = torch.rand(2, 40, 24, generator=g).cuda(), torch.randn(2, 24, 50, generator=g).cuda()
+    w, x, y = torch.rand(2, 20, 6, 7, generator=g).cuda(), torch.randn(2, 6, 50, generator=g).cuda(), torch.randn(2, 7, 50, generator=g).cuda()
+    host = _native.HOST
+    out, lt = tb.lm2exp(a, b), tb.lt2exp(w, x, y)
+    assert torch.equal(host.lm2exp(a, b, 1, 0), out) and torch.equal(host.lt2exp(w, x, y, 1, 0), lt)
+    assert host.lm2exp(a, b, 1, 1281) is None and host.lm2exp(a, b, -1, 0) is None and host.lt2exp(w, x, y, 1, 11281) is None
+    assert host.lm2exp(a, b[:, :23], 1, 0) is None and host.lm2exp(a.double(), b.double(), 1, 0) is None
+    assert host.lm2exp(a.cpu(), b.cpu(), 1, 0) is None and host.lm2exp(a, None, 1, 0) is None
+    assert host.lm2exp(a[:, :0], b, 1, 0) is None
+    assert host.lm2exp(torch.rand(64, 512, 256, device="cuda"), torch.rand(64, 256, 512, device="cuda"), 1, 0) is None
+    with pytest.raises(AssertionError):
+        tb.lm2exp(a, b[:, :23])
+    with pytest.raises(ValueError):
+        tb.lm2exp(a, b, precision="fp32")
+    with pytest.raises(RuntimeError):  # I and J are no single dimension
+        tb.lt2exp(torch.rand(2, 20, 7, 6, device="cuda").transpose(2, 3), x, y)
+    assert torch.equal(tb.lm2exp(a.requires_grad_(), b), out) and not tb.lm2exp(a, b).requires_grad
+    with torch.inference_mode():
+        assert torch.equal(tb.lm2exp(a * 1, b * 1), out)
+    with torch.device("cuda"):  # a function mode: through Python
+        assert host.lm2exp(a, b, 1, 0) is None and torch.equal(tb.lm2exp(a, b), out)
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert host.lm2exp(b.as_subclass(Sub), b, 1, 0) is None
+    with pytest.raises(Exception):
+        torch.vmap(lambda u: tb.lm2exp(u, b))(torch.stack([a, a]))
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        again = tb.lm2exp(a, b)
+    torch.cuda.synchronize()
+    assert torch.equal(again, out)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = tb.lm2exp(a, b)
+        held_lt = tb.lt2exp(w, x, y)
+    held.zero_(), held_lt.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(held, out) and torch.equal(held_lt, lt)
+    tb.check_status()

@@ -24,6 +24,7 @@ EXPORTED_SYMBOLS = (
     "triturus_b200_lt2exp_launches",
     "triturus_b200_lt2exp_plan",
     "triturus_b200_lm2exp_direct",
+    "triturus_b200_lm2exp_small_f32",
     "triturus_b200_lt2exp_direct",
     "triturus_b200_lt2exp_direct_f32",
     "triturus_b200_lm2exp_plan",
@@ -155,6 +156,28 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
 
 
 LIB = _load()
+
+
+def _load_host():
+    """The extension module that makes small calls of the library (csrc/host.cpp), built first where it is missing or stale;
+    like the library, an existing one is used as it is where it cannot be rebuilt."""
+    if _build.host_is_stale():
+        try:
+            _build.build_host()
+        except Exception as exc:  # noqa: BLE001
+            if not _build.HOST_PATH.exists():
+                raise NativeLibraryError(f"{_build.HOST_PATH} is missing and could not be built ({exc})") from exc
+    try:
+        from . import _host
+    except ImportError:
+        # built against another torch or interpreter: once more from its source
+        _build.build_host(force=True)
+        from . import _host
+    _host.set_error_class(NativeLibraryError)
+    return _host
+
+
+HOST = _load_host()
 
 
 def strerror(code: int) -> str:

@@ -776,6 +776,29 @@ static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int preci
   return direct <= tcgen;
 }
 
+// How each operand of lm2exp reaches shared memory.  a with j contiguous is a K-major tensor-core operand, a transposed
+// view (i contiguous) an MN-major one; b with k contiguous is MN-major, a transposed view (j contiguous)
+// K-major (single-CTA kernel only).  All four go through tensor maps when base and strides meet the TMA rules (true);
+// an operand that does not (row pitch not a multiple of 16 bytes, innermost stride other than 1, base not
+// 16-byte aligned) is fetched element by element by the single-CTA kernel or the direct one.  Strides of dimensions of size one
+// become what a tensor map takes.
+static bool lm2exp_a_layout(const float* a, int64_t R, int64_t I, int64_t J, int64_t& s0, int64_t& s1, int64_t& s2, bool& mn) {
+  mn = J > 1 && s2 != 1;
+  bool tma = aligned16(a);
+  if (tma && mn) tma = (I == 1 || s1 == 1) && fix_stride(J, s2, round_up4(I)) && fix_stride(R, s0, round_up4(I) * J);
+  else if (tma) tma = fix_stride(I, s1, round_up4(J)) && fix_stride(R, s0, round_up4(J) * I);
+  mn = mn && tma;
+  return tma;
+}
+static bool lm2exp_b_layout(const float* b, int64_t R, int64_t J, int64_t K, int64_t& s0, int64_t& s1, int64_t& s2, bool& km) {
+  km = K > 1 && s2 != 1;
+  bool tma = aligned16(b);
+  if (tma && km) tma = (J == 1 || s1 == 1) && fix_stride(K, s2, round_up4(J)) && fix_stride(R, s0, round_up4(J) * K);
+  else if (tma) tma = fix_stride(J, s1, round_up4(K)) && fix_stride(R, s0, round_up4(K) * J);
+  km = km && tma;
+  return tma;
+}
+
 // Raises the shared-memory limit of a kernel once per device.
 template <auto Kern>
 static bool direct_smem_limit(int bytes) {
@@ -844,29 +867,9 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   if (I > 1 && os1 <= 0) return TRITURUS_B200_EALIGN;
   if (R > 1 && os0 <= 0) return TRITURUS_B200_EALIGN;
   if ((reinterpret_cast<uintptr_t>(a) & 3) != 0 || (reinterpret_cast<uintptr_t>(b) & 3) != 0) return TRITURUS_B200_EALIGN;
-  // How each operand reaches shared memory.  a with j contiguous is a K-major tensor-core operand, a transposed
-  // view (i contiguous) an MN-major one; b with k contiguous is MN-major, a transposed view (j contiguous)
-  // K-major (single-CTA kernel only).  All four go through tensor maps when base and strides meet the TMA rules;
-  // an operand that does not (row pitch not a multiple of 16 bytes, innermost stride other than 1, base not
-  // 16-byte aligned) is fetched element by element by the single-CTA kernel instead (gen_a / gen_b).
   const int64_t as_raw[3] = {as0, as1, as2}, bs_raw[3] = {bs0, bs1, bs2};
-  bool a_mn = J > 1 && as2 != 1;
-  bool a_tma = aligned16(a);
-  if (a_tma && a_mn) {
-    a_tma = (I == 1 || as1 == 1) && fix_stride(J, as2, round_up4(I)) && fix_stride(R, as0, round_up4(I) * J);
-  } else if (a_tma) {
-    a_tma = fix_stride(I, as1, round_up4(J)) && fix_stride(R, as0, round_up4(J) * I);
-  }
-  bool b_km = K > 1 && bs2 != 1;
-  bool b_tma = aligned16(b);
-  if (b_tma && b_km) {
-    b_tma = (J == 1 || bs1 == 1) && fix_stride(K, bs2, round_up4(J)) && fix_stride(R, bs0, round_up4(J) * K);
-  } else if (b_tma) {
-    b_tma = fix_stride(J, bs1, round_up4(K)) && fix_stride(R, bs0, round_up4(K) * J);
-  }
-  const bool gen_a = !a_tma, gen_b = !b_tma;
-  if (gen_a) a_mn = false;
-  if (gen_b) b_km = false;
+  bool a_mn, b_km;
+  const bool gen_a = !lm2exp_a_layout(a, R, I, J, as0, as1, as2, a_mn), gen_b = !lm2exp_b_layout(b, R, J, K, bs0, bs1, bs2, b_km);
   // (the element-wise loader takes the place of the warps that fold the column maxima of the result)
   if ((gen_a || gen_b) && out_colmax != nullptr) return TRITURUS_B200_EALIGN;
   if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b))
@@ -1107,6 +1110,26 @@ static int lm2exp_run(const float* a, const float* b, float* out, int64_t R, int
     if (rc != TRITURUS_B200_OK) return rc;
   }
   return TRITURUS_B200_OK;
+}
+
+int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, int64_t R, int64_t I, int64_t J, int64_t K,
+                                   const int64_t a_strides[3], const int64_t b_strides[3], const int64_t out_strides[3], int precision,
+                                   void* stream) {
+  if (a == nullptr || b == nullptr || a_strides == nullptr || b_strides == nullptr || R <= 0 || I <= 0 || J <= 0 || K <= 0)
+    return TRITURUS_B200_EINVAL;
+  if (precision != TRITURUS_B200_PRECISION_TF32 && precision != TRITURUS_B200_PRECISION_3XTF32) return TRITURUS_B200_EINVAL;
+  if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) != 0) return TRITURUS_B200_EALIGN;
+  int64_t as[3] = {a_strides[0], a_strides[1], a_strides[2]}, bs[3] = {b_strides[0], b_strides[1], b_strides[2]};
+  bool mn, km;
+  const bool odd = !lm2exp_a_layout(a, R, I, J, as[0], as[1], as[2], mn) | !lm2exp_b_layout(b, R, J, K, bs[0], bs[1], bs[2], km);
+  const bool small = direct_lm_wins(R, I, J, K, precision, odd);
+  if (out == nullptr) return small ? 1 : 0;
+  if (!small || out_strides == nullptr) return TRITURUS_B200_EINVAL;
+  if ((reinterpret_cast<uintptr_t>(out) & 3) != 0 || (K > 1 && out_strides[2] != 1) || (I > 1 && out_strides[1] <= 0) ||
+      (R > 1 && out_strides[0] <= 0))
+    return TRITURUS_B200_EALIGN;
+  return lm2exp_direct(a, b, out, R, I, J, K, a_strides, b_strides, out_strides, precision, nullptr, nullptr,
+                       static_cast<cudaStream_t>(stream));
 }
 
 int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd) {

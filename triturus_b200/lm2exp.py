@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from . import _native
-from .utils import resolve_precision
+from .utils import precision_code, resolve_precision
 
 
 def lm2exp(
@@ -30,6 +30,10 @@ def lm2exp(
     `b` skips that call's stabiliser pass.  `b_colmax` must hold the column maxima of `b` over its middle
     dimension (float32 [R,K]).
     """
+    if b_colmax is None and not return_colmax and not torch.compiler.is_compiling():
+        out = _native.HOST.lm2exp(a, b, precision_code(precision), variant)  # None: not an ordinary call of a small problem
+        if out is not None:
+            return out
     assert len(a.shape) == len(b.shape) == 3
     assert a.shape[0] == b.shape[0]
     assert a.shape[2] == b.shape[1]

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from . import _native
-from .utils import resolve_precision
+from .utils import precision_code, resolve_precision
 
 _MODES = ("auto", "split", "unsplit")
 
@@ -39,6 +39,11 @@ def lt2exp(
     column maxima of `a` and `b` over their middle dimension, e.g. as returned by the calls that produced
     them, and replace the scan; `return_colmax=True` returns `(out, m)` with `m[r,k] = max_s out[r,s,k]`.
     """
+    if a_colmax is None and b_colmax is None and not return_colmax and mode in ("auto", "unsplit") and not torch.compiler.is_compiling():
+        # (None: not an ordinary call of a small problem, which has one launch and one order of additions in either mode)
+        out = _native.HOST.lt2exp(w, a, b, precision_code(precision), variant)
+        if out is not None:
+            return out
     assert len(w.shape) == 4
     assert len(a.shape) == len(b.shape) == 3
     assert w.shape[0] == a.shape[0] == b.shape[0]

@@ -58,6 +58,13 @@ def is_triturus_tf32_enabled() -> bool:
     return _TRITURUS_TF32_ENABLED
 
 
+def precision_code(precision: str | None) -> int:
+    """`resolve_precision` without the exception: -1 for a name that it would refuse."""
+    if precision is None:
+        return 0 if _TRITURUS_TF32_ENABLED else 1
+    return 0 if precision == "tf32" else 1 if precision == "3xtf32" else -1
+
+
 def resolve_precision(precision: str | None) -> int:
     """Map an explicit precision name, or the global flag when None, to the C-ABI precision code."""
     if precision is None:
