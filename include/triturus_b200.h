@@ -202,8 +202,9 @@ int triturus_b200_lt2exp_f32(const float* w, const float* a, const float* b, flo
  * k-blocks adds them to its own and writes the finished results.  The order of those additions is fixed, so
  * the results do not depend on timing.  triturus_b200_lt2exp_f32 (no workspace) never chooses the shared last
  * wave by itself and, when asked for it, falls back to additions into the zero-filled result.
- *   workspace: triturus_b200_lt2exp_workspace_bytes(...) bytes, 256-byte aligned (0 bytes: may be NULL); its
- *   first 1024 bytes are cleared by a cudaMemsetAsync on `stream` in every call that uses it.  The queries
+ *   A contraction cut into slices takes the column maxima of a and b from it: 2 * R * K floats that its first launch writes.
+ *   workspace: triturus_b200_lt2exp_workspace_bytes(...) bytes, 256-byte aligned (0 bytes: may be NULL); for parked tiles
+ *   its first 1024 bytes are cleared by a cudaMemsetAsync on `stream` in every call that uses it.  The queries
  *   triturus_b200_lt2exp_launches / _plan describe calls of this entry point with that workspace.
  *   The CTAs of such a launch wait for one another (with the usual bound), so the launch takes the whole GPU:
  *   on a device that another kernel shares at the same time, a CTA may start late and a wait may run out

@@ -1367,13 +1367,14 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
     p.lw_main = 0;
   }
   const bool parked = sp.stream != 0 && have_ws;             // shared tiles completed through the scratch memory
+  const size_t stab_need = 2 * static_cast<size_t>(p.R) * static_cast<size_t>(p.K) * sizeof(float);  // maxima of a and b
   const bool split = (sp.nsplit > 1 || sp.stream != 0) && !parked;  // ... or with additions into the zero-filled result
-  // the log pass of a split launch runs on a (K / 128, S / 64, R) grid
+  // (the log pass of a split launch once ran on a (K / 128, S / 64, R) grid; calls it refused stay refused)
   if (split && (p.S + 63) / 64 > 65535) return TRITURUS_B200_EINVAL;
   if (L.query != nullptr) {
     L.query->launches = split ? 3 : 1;
     L.query->split_code = sp.stream ? 9998 : sp.nsplit;
-    L.query->ws_bytes = parked ? park_need : 0;
+    L.query->ws_bytes = parked ? park_need : sp.nsplit > 1 ? stab_need : 0;
     return TRITURUS_B200_OK;
   }
   std::call_once(once[dev], [&] {
@@ -1382,6 +1383,7 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   if (attr_rc[dev] != cudaSuccess) return TRITURUS_B200_ELAUNCH;
   p.park = nullptr;
   p.park_flags = nullptr;
+  p.ma_wait = 0;
   if (parked) {
     p.park_flags = static_cast<int*>(L.ws);
     p.park = reinterpret_cast<float*>(static_cast<uint8_t*>(L.ws) + kParkHeader);
@@ -1390,14 +1392,24 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   if (split) {
     const int64_t total = static_cast<int64_t>(p.R) * p.S * p.K;
     const int64_t zb = (total + 255) / 256;
-    lt2exp_zero_kernel<<<static_cast<int>(zb < 4 * sm_count() ? zb : 4 * sm_count()), 256, 0, L.stream>>>(
-        p.out, p.out_s0, p.out_s1, p.R, p.S, p.K);
+    const int zgrid = static_cast<int>(zb < 4 * sm_count() ? zb : 4 * sm_count());
+    const int64_t mblocks = 2 * static_cast<int64_t>(p.R) * ((p.K + 31) / 32);
+    if (p.ma_in == nullptr && L.ws != nullptr && L.ws_bytes >= stab_need && (reinterpret_cast<uintptr_t>(L.ws) & 255) == 0 &&
+        mblocks <= (1 << 20)) {
+      float* m = static_cast<float*>(L.ws);
+      lt2exp_prepare_kernel<<<zgrid + static_cast<int>(mblocks), 256, 0, L.stream>>>(p, m, static_cast<int>(mblocks));
+      p.ma_in = m;
+      p.mb_in = m + static_cast<int64_t>(p.R) * p.K;
+      p.ma_wait = 1;
+    } else {
+      lt2exp_zero_kernel<<<zgrid, 256, 0, L.stream>>>(p.out, p.out_s0, p.out_s1, p.R, p.S, p.K);
+    }
   }
   const int grid = (sp.stream || p.num_items >= sm_count()) ? sm_count() : p.num_items;
   const int rc = launch_maybe_dependent(kern, dim3(static_cast<unsigned>(grid)), Cfg::NTHREADS, Cfg::SMEM_BYTES, L.stream, split, tw, p);
   if (rc != TRITURUS_B200_OK) return rc;
   if (split) {
-    const dim3 fgrid((p.K + 127) / 128, (p.S + 63) / 64, p.R);
+    const dim3 fgrid((p.K + 127) / 128, std::min((p.S + FINISH_ROWS - 1) / FINISH_ROWS, 65535), p.R);
     const int frc = launch_maybe_dependent(lt2exp_finish_kernel<Cfg::PREC>, fgrid, 256, 0, L.stream, true, p);
     if (frc != TRITURUS_B200_OK) return frc;
   }

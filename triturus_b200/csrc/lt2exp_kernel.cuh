@@ -69,6 +69,7 @@ struct Lt2expParams {
   // -inf first.
   const float* ma_in;
   const float* mb_in;
+  int ma_wait;  // the maxima come from the launch before this one (lt2exp_prepare_kernel): wait for it
   float* out_max;
 };
 
@@ -582,6 +583,7 @@ lt2exp_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParams p) 
     const int grp = tt / BN;     // this thread's group takes every NGROUPS-th k-block
     uint32_t it = 0, tcount = 0;
     bool ok = true;
+    if (p.ma_wait) pdl_wait();
     LtWork work(p, KBT);
     for (LtItem w; ok && work.next(w); ++tcount) {
       int r, n0, s0;
@@ -737,10 +739,61 @@ __global__ void lt2exp_zero_kernel(float* out, int64_t out_s0, int64_t out_s1, i
   }
 }
 
+// The same, and the column maxima of a and b into m[2][R, K], which the contraction and the log pass then take instead of
+// scanning a and b in every block: the first `mblocks` blocks take 32 columns of a or of b each, eight loads in flight per
+// thread, the others fill.
+__global__ void __launch_bounds__(256) lt2exp_prepare_kernel(const Lt2expParams p, float* m, int mblocks) {
+  pdl_launch_dependents();
+  if (static_cast<int>(blockIdx.x) >= mblocks) {
+    const int64_t total = static_cast<int64_t>(p.R) * p.S * p.K;
+    const int64_t step = static_cast<int64_t>(gridDim.x - mblocks) * blockDim.x;
+    for (int64_t x = (static_cast<int64_t>(blockIdx.x) - mblocks) * blockDim.x + threadIdx.x; x < total; x += step) {
+      const int k = static_cast<int>(x % p.K);
+      const int64_t rs = x / p.K;
+      p.out[(rs / p.S) * p.out_s0 + (rs % p.S) * p.out_s1 + k] = 0.0f;
+    }
+    return;
+  }
+  __shared__ float part[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nbx = (p.K + 31) / 32;
+  const int which = blockIdx.x & 1, item = blockIdx.x >> 1;
+  const int r = item / nbx, k = (item % nbx) * 32 + lane;
+  const int rows = which ? p.J : p.I;
+  const int64_t s1 = which ? p.b_s1 : p.a_s1;
+  const float* x = which ? p.b + static_cast<int64_t>(r) * p.b_s0 + static_cast<int64_t>(k) * p.b_s2
+                         : p.a + static_cast<int64_t>(r) * p.a_s0 + static_cast<int64_t>(k) * p.a_s2;
+  float mx = -INFINITY;
+  if (k < p.K) {
+    for (int j0 = warp; j0 < rows; j0 += 64) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int j = j0 + u * 8;
+        v[u] = __ldg(x + static_cast<int64_t>(j < rows ? j : j0) * s1);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) mx = fmaxf(mx, v[u]);
+    }
+  }
+  part[warp][lane] = mx;
+  __syncthreads();
+  if (warp == 0 && k < p.K) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, part[w][lane]);
+    m[static_cast<int64_t>(which) * p.R * p.K + static_cast<int64_t>(r) * p.K + k] = mx;
+  }
+}
+
 // Second pass of a split launch: out[r,s,k] = (ma[r,k] + mb[r,k]) + log(out[r,s,k]) in place, with the same
-// clamped column maxima the main kernel used.  Block = 128 columns x 64 rows of out, 256 threads; the
+// clamped column maxima the main kernel used.  Block = 128 columns x FINISH_ROWS rows of out, 256 threads; the
 // maxima are taken as in the main kernel (32 column quads x 8 row groups with 16-byte loads, or 128 columns x
-// 2 row groups).  Grid = (K / 128, S / 64, R).
+// 2 row groups), while the main kernel runs; what counts is the time from its last addition to the last result: all sums of
+// a thread are loaded at once, and the blocks are short.  With that and lt2exp_prepare_kernel instead of blocks of 64 rows, one
+// sum after the other, and a scan of a and b in every block of both passes, us: 1 x 256^4 3xTF32 77.7 -> 64.1, TF32 57.0 -> 49.2; 1 x
+// 128^4 TF32 25.7 -> 17.3; 2 x 100 100x100x200 3xTF32 38.7 -> 27.6.
+// Grid = (K / 128, S / FINISH_ROWS, R).
+constexpr int FINISH_ROWS = 16;
 template <int PREC>
 __global__ void __launch_bounds__(256) lt2exp_finish_kernel(const Lt2expParams p) {
   __shared__ float part[2][8][128];
@@ -749,6 +802,7 @@ __global__ void __launch_bounds__(256) lt2exp_finish_kernel(const Lt2expParams p
   const int r = blockIdx.z;
   const int tid = threadIdx.x;
   int nparts = 0;
+  if (p.ma_wait) pdl_wait();  // (the contraction has waited for the maxima; the sums come with it)
   if (p.ma_in != nullptr) {
     if (tid < 128 && k0 + tid < p.K) {
       part[0][0][tid] = __ldg(p.ma_in + static_cast<int64_t>(r) * p.K + k0 + tid);
@@ -788,14 +842,21 @@ __global__ void __launch_bounds__(256) lt2exp_finish_kernel(const Lt2expParams p
   const int n = tid & 127;
   if (k0 + n >= p.K) return;
   const float m = msum[n];
-  const int s_end = min(p.S, (static_cast<int>(blockIdx.y) + 1) * 64);
   float cmx = -INFINITY;  // maximum of this thread's results: its column, every second row of the block
-  for (int s = blockIdx.y * 64 + (tid >> 7); s < s_end; s += 2) {
-    float* o = p.out + static_cast<int64_t>(r) * p.out_s0 + static_cast<int64_t>(s) * p.out_s1 + k0 + n;
-    const float acc = *o;
-    const float res = m + (PREC ? logf(acc) : lg2_approx(acc) * LN2_F);
-    *o = res;
-    cmx = fmaxf(cmx, res);
+  float* o = p.out + static_cast<int64_t>(r) * p.out_s0 + k0 + n;
+  for (int64_t s0 = static_cast<int64_t>(blockIdx.y) * FINISH_ROWS + (tid >> 7); s0 < p.S; s0 += static_cast<int64_t>(gridDim.y) * FINISH_ROWS) {
+    float acc[FINISH_ROWS / 2];
+#pragma unroll
+    for (int x = 0; x < FINISH_ROWS / 2; ++x)
+      if (s0 + 2 * x < p.S) acc[x] = o[(s0 + 2 * x) * p.out_s1];
+#pragma unroll
+    for (int x = 0; x < FINISH_ROWS / 2; ++x) {
+      if (s0 + 2 * x < p.S) {
+        const float res = m + (PREC ? logf(acc[x]) : lg2_approx(acc[x]) * LN2_F);
+        o[(s0 + 2 * x) * p.out_s1] = res;
+        cmx = fmaxf(cmx, res);
+      }
+    }
   }
   if (p.out_max != nullptr) red_max_f32(p.out_max + static_cast<int64_t>(r) * p.K + k0 + n, cmx);
 }

@@ -457,6 +457,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
                                (Cfg::NB == 2 ? static_cast<uint32_t>((tt / 128) * BK) : 0u);
     uint32_t it = 0, tcount = 0;
     bool ok = true;
+    if (p.ma_wait) pdl_wait();
     LtWork work(p, KBT);
     for (LtItem w; ok && work.next(w); ++tcount) {
       int r, n0, s0;
