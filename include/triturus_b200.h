@@ -204,9 +204,10 @@ int triturus_b200_lt2exp_f32(const float* w, const float* a, const float* b, flo
  * wave by itself and, when asked for it, falls back to additions into the zero-filled result.
  *   A contraction cut into slices takes the column maxima of a and b from it: 2 * R * K floats that its first launch writes.
  *   workspace: triturus_b200_lt2exp_workspace_bytes(...) bytes, 256-byte aligned (0 bytes: may be NULL); for parked tiles
- *   its first 1024 bytes are cleared by a cudaMemsetAsync on `stream` in every call that uses it.  The queries
+ *   its first 4096 bytes are cleared by a cudaMemsetAsync on `stream` in every call that uses it.  The queries
  *   triturus_b200_lt2exp_launches / _plan describe calls of this entry point with that workspace.
- *   The CTAs of such a launch wait for one another (with the usual bound), so the launch takes the whole GPU:
+ *   In 3xTF32 whichever part ends last adds the parked sums up, in the order of the parts, and nobody waits.
+ *   In plain TF32 the CTAs of such a launch wait for one another (with the usual bound), so the launch takes the whole GPU:
  *   on a device that another kernel shares at the same time, a CTA may start late and a wait may run out
  *   (reported through status_dev, never a hang).
  */

@@ -1288,6 +1288,48 @@ static LtSplit lt2exp_split(int64_t tiles, int I, int J, int request, bool auto_
   return sp;
 }
 
+// How the tiles of a last, partly filled wave are shared among all CTAs (LtWork in lt2exp_kernel.cuh): equal parts, or mains and tails.
+struct LtShare {
+  int first, parts, main;  // first tile of the wave; equal parts per tile (0: mains and tails); k-blocks of a main
+};
+constexpr int64_t kItemBlocks = 32;  // a work item's prologue and epilogue, in k-blocks (25 us per tail of a 256 x 256 tile
+                                     // against 0.73 us per k-block)
+static LtShare lt2exp_share(int64_t nt, int64_t kbt) {
+  const int G = sm_count();
+  const int64_t waves = (nt + G - 1) / G;
+  LtShare sh{static_cast<int>((waves - 1) * G), 1, static_cast<int>(kbt)};
+  const int rem = static_cast<int>(nt - sh.first);
+  if (rem * 2 <= G) {
+    int64_t parts = G / rem;
+    if (parts > 8) parts = 8;  // shorter parts are mostly prologue and epilogue
+    if (parts > kbt) parts = kbt;
+    sh.parts = static_cast<int>(parts < 1 ? 1 : parts);
+  } else if (rem < G && kbt >= 2) {
+    // mains and tails: a CTA with the most tails (q of them) is busy as long as a main part, counting for
+    // every work item a prologue and epilogue: q * (kbt - x + o) = x + o
+    const int h = G - rem;
+    const int64_t q = (rem + h - 1) / h;
+    int64_t x = ((q * (kbt + kItemBlocks) - kItemBlocks) / (q + 1)) & ~int64_t(7);
+    if (x < 1) x = 1;
+    if (x > kbt - 1) x = kbt - 1;
+    sh.parts = 0;
+    sh.main = static_cast<int>(x);
+  }
+  return sh;
+}
+
+// 3xTF32: is sharing the last wave worth it?  By at least 3 % of the launch, counting the parking and adding up of a part as 28
+// k-blocks more than an item's own.  us, whole / shared: R10 128x128x128x2048 538 / 360, R40 64x90x200x500 669 / 409, R6
+// 200x100x100x1000 225 / 178, R30 60x100x100x1000 420 / 365, R8 256x128x128x4096 1 136 / 1 068, R32 256^4 1 320 / 1 249; R90
+// 128x128x32x128 88.9 / 91.6 and R128 128x100x100x128 334 / 341, which the estimate leaves whole.
+static bool lt2exp_share_wins(int64_t nt, int64_t kbt) {
+  const int64_t G = sm_count(), waves = (nt + G - 1) / G, item = kbt + kItemBlocks;
+  const LtShare sh = lt2exp_share(nt, kbt);
+  if (waves > 8 || sh.parts == 1) return false;
+  const int64_t longest = sh.parts > 0 ? kbt / sh.parts : sh.main;
+  return static_cast<double>((waves - 1) * item + longest + kItemBlocks + 28) < 0.97 * static_cast<double>(waves * item);
+}
+
 // What a launch function is asked to do: launch, or (query != nullptr) only report what it would launch.
 struct LtQuery {
   int launches;     // kernels per call
@@ -1302,7 +1344,7 @@ struct LtLaunch {
   size_t ws_bytes;
 };
 
-constexpr size_t kParkHeader = 1024;  // flags (one int per CTA) ahead of the parked tiles
+constexpr size_t kParkHeader = 4096;  // flags (one int per CTA, in 3xTF32 four per shared tile) ahead of the parked tiles
 
 template <class Cfg, void (*Kern)(const CUtensorMap, const Lt2expParams), bool CAN_PARK>
 static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLaunch& L) {
@@ -1318,17 +1360,18 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   if (nt > INT32_MAX) return TRITURUS_B200_EINVAL;
   p.num_tiles = static_cast<int>(nt);
   // Scratch memory for the end-to-end form: one parked tile per CTA behind the flags.
-  const size_t park_need = kParkHeader + static_cast<size_t>(sm_count()) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
-  const bool have_ws = CAN_PARK && sm_count() * sizeof(int) <= kParkHeader &&
+  // (3xTF32: every part parks, up to two per tile of a last wave that fills more than half of the SMs.)
+  const size_t park_need = kParkHeader + static_cast<size_t>(sm_count()) * (Cfg::PREC ? 2 : 1) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
+  const bool have_ws = CAN_PARK && sm_count() * sizeof(int) * (Cfg::PREC ? 4 : 1) <= kParkHeader &&
                        (L.query != nullptr || (L.ws != nullptr && L.ws_bytes >= park_need &&
                                                (reinterpret_cast<uintptr_t>(L.ws) & 255) == 0));
-  // Not chosen automatically for a launch that re-sums its accumulator in chunks (3xTF32, long plain-TF32
-  // contractions): sharing tiles makes long plain-TF32 contractions slower (R32 256^4: 1.32 against 0.81 ms; R128: 2.75
-  // against 2.40 ms); the explicit request 9998 still selects it.  The 3xTF32 kernel would gain, whole / shared: R8
-  // 256x128x128x4096 1 478 / 1 009 us, R10 K2048 924 / 636, R128 256^4 5 228 / 4 869, R32 1 160 / 1 127, R16 256x128x128x4096
-  // 2 025 / 2 040.
+  // Not chosen automatically for long plain-TF32 contractions, which re-sum their accumulator in chunks: sharing tiles makes
+  // those slower (R32 256^4: 1.32 against 0.81 ms; R128: 2.75 against 2.40 ms); the explicit request 9998 still selects it.
+  // 3xTF32 has a rule of its own (lt2exp_share).
   const bool chunked = Cfg::PROMOTE && static_cast<int64_t>((p.J + 31) / 32) * p.I > Cfg::CHUNK;
-  const LtSplit sp = lt2exp_split(nt, p.I, p.J, L.split_request, have_ws && !chunked);
+  LtSplit sp = lt2exp_split(nt, p.I, p.J, L.split_request, have_ws && !chunked);
+  if (Cfg::PREC && have_ws && L.split_request == 0 && sp.nsplit == 1 && lt2exp_share_wins(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I))
+    sp.stream = 1;
   p.nsplit = sp.nsplit;
   p.stream = sp.stream;
   const int64_t items = nt * sp.nsplit;
@@ -1336,31 +1379,10 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   p.num_items = static_cast<int>(items);
   if (sp.stream) {
     // Whole waves first, then the tiles of the last wave shared among all CTAs (LtWork in lt2exp_kernel.cuh).
-    const int G = sm_count();
-    const int64_t kbt = static_cast<int64_t>((p.J + 31) / 32) * p.I;
-    const int64_t waves = (nt + G - 1) / G;
-    p.lw_first = static_cast<int>((waves - 1) * G);
-    const int rem = static_cast<int>(nt - p.lw_first);
-    p.lw_parts = 1;
-    p.lw_main = static_cast<int>(kbt);
-    if (rem * 2 <= G) {
-      int64_t parts = G / rem;
-      if (parts > 8) parts = 8;  // shorter parts are mostly prologue and epilogue
-      if (parts > kbt) parts = kbt;
-      p.lw_parts = static_cast<int>(parts < 1 ? 1 : parts);
-    } else if (rem < G && kbt >= 2) {
-      // mains and tails: a CTA with the most tails (q of them) is busy as long as a main part, counting for
-      // every work item a prologue and epilogue worth kItemBlocks k-blocks (measured: 25 us per tail of a
-      // 256 x 256 tile against 0.73 us per k-block): q * (kbt - x + o) = x + o
-      constexpr int64_t kItemBlocks = 32;
-      const int h = G - rem;
-      const int64_t q = (rem + h - 1) / h;
-      int64_t x = ((q * (kbt + kItemBlocks) - kItemBlocks) / (q + 1)) & ~int64_t(7);
-      if (x < 1) x = 1;
-      if (x > kbt - 1) x = kbt - 1;
-      p.lw_parts = 0;
-      p.lw_main = static_cast<int>(x);
-    }
+    const LtShare sh = lt2exp_share(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I);
+    p.lw_first = sh.first;
+    p.lw_parts = sh.parts;
+    p.lw_main = sh.main;
   } else {
     p.lw_first = p.num_tiles;
     p.lw_parts = 1;

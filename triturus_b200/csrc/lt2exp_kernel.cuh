@@ -58,7 +58,7 @@ struct Lt2expParams {
   // ([slot][MT * BN / 32 chunks][8 column quads][128 rows][4] floats: the 32 lanes of a store write 512
   // consecutive bytes) and then raises park_flags[slot] (zeroed by the launcher)
   // by one per epilogue warp; the CTA with the first part adds the parked sums to its own, in slot order, and
-  // writes the finished results.
+  // writes the finished results.  (3xTF32: nobody waits, see lt2exp_tmem_kernel.cuh.)
   float* park;
   int* park_flags;
   int vec_ab;            // a and b allow 16-byte loads along k (alignment, strides and K multiples of 4)
@@ -80,6 +80,7 @@ struct Lt2expParams {
 struct LtItem {
   int tile, kb_lo, kb_hi;
   int park_slot, slot0, ncollect;
+  int part;  // which part of the contraction of its tile (0: the first, or all of it)
 };
 
 // The work items of one CTA, in the order every role of the CTA walks them.
@@ -118,6 +119,7 @@ struct LtWork {
     w.park_slot = -1;
     w.slot0 = 0;
     w.ncollect = 0;
+    w.part = 0;
     if (!stream) {
       if (q >= nq) return false;
       w.tile = q / nsplit;
@@ -144,6 +146,7 @@ struct LtWork {
       phase = 2;
       const int j = c / lw_rem, t = c - j * lw_rem;
       if (j >= lw_parts) return false;
+      w.part = j;
       w.tile = lw_first + t;
       w.kb_lo = static_cast<int>(static_cast<int64_t>(j) * kb_tile / lw_parts);
       w.kb_hi = static_cast<int>(static_cast<int64_t>(j + 1) * kb_tile / lw_parts);
@@ -175,6 +178,7 @@ struct LtWork {
     w.tile = lw_first + tail_next;
     w.kb_lo = lw_main;
     w.kb_hi = kb_tile;
+    w.part = 1;
     w.park_slot = tail_next;
     tail_next += static_cast<int>(gridDim.x) - lw_rem;
     return true;

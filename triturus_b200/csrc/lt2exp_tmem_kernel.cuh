@@ -268,9 +268,14 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
         float* out_col = p.out + static_cast<int64_t>(r) * p.out_s0 + kcol;
         const int slot = tcount & 1;
         const int nch = (w.kb_hi - w.kb_lo + Cfg::CHUNK - 1) / Cfg::CHUNK;
-        const bool park_it = parking && w.park_slot >= 0;
-        const bool collect = parking && w.ncollect > 0;
+        // A tile of the shared last wave: every part parks its sums, and the warp that parks the last part of its columns
+        // adds them up, in the order of the parts whoever it is.  No CTA waits for another, which need not have started
+        // where a second kernel shares the GPU.
+        const int shared_parts = p.lw_parts > 0 ? p.lw_parts : p.lw_main < KBT ? 2 : 1;
+        const bool park_it = parking && w.tile >= p.lw_first && shared_parts > 1;
+        const int shared_tile = w.tile - p.lw_first;
         constexpr int PARK_TILE = BM * BN;  // floats per parked tile, in the order of `master`
+        float4* const parked = reinterpret_cast<float4*>(p.park + static_cast<int64_t>(shared_tile) * shared_parts * PARK_TILE) + kl;
         float cmx = -INFINITY;  // running maximum of this lane's column over the rows of the tile
         for (int ch = 0; ok && ch < nch; ++ch, ++ccount) {
           const int buf = ccount % Cfg::NBUF;
@@ -278,22 +283,6 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
           if (!(ok = mbar_wait_warp(&acc_full[buf], (ccount / Cfg::NBUF) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
           if (Cfg::NGROUPS > 1 && first && !(ok = mbar_wait_warp(&msum_full[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
           tc_fence_after_sync();
-          if (last && collect) {
-            // The other parts of the tile run at the same time on other CTAs and end about now.  (Not earlier: while
-            // this warp waits, no chunk is drained.)
-            for (int cc = 0; ok && cc < w.ncollect; ++cc) {
-              const long long t0 = clock64();
-              while (ld_acquire_gpu(p.park_flags + w.slot0 + cc) < 4) {
-                if (*ctl.flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                  raise_abort(ctl, STATUS_TIMEOUT_EPILOGUE);
-                  ok = false;
-                  break;
-                }
-              }
-            }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-          }
           const float m = msum[slot * BN + kl];
 #pragma unroll 1
           for (int c = 0; c < BM / 32; ++c) {
@@ -308,19 +297,12 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
               for (int g = 0; g < 8; ++g) add_quad(v, g, mst[g * 128]);
             }
             if (!last || park_it) {
-              float4* dst = last ? reinterpret_cast<float4*>(p.park + static_cast<int64_t>(w.park_slot) * PARK_TILE) + c * 8 * 128 + kl : mst;
+              float4* dst = last ? parked + w.part * (PARK_TILE / 4) + c * 8 * 128 : mst;
 #pragma unroll
               for (int g = 0; g < 8; ++g)
                 dst[g * 128] = make_float4(__uint_as_float(v[g * 4]), __uint_as_float(v[g * 4 + 1]),
                                            __uint_as_float(v[g * 4 + 2]), __uint_as_float(v[g * 4 + 3]));
               continue;
-            }
-            if (collect) {
-              for (int cc = 0; cc < w.ncollect; ++cc) {
-                const float4* src = reinterpret_cast<const float4*>(p.park + static_cast<int64_t>(w.slot0 + cc) * PARK_TILE) + c * 8 * 128 + kl;
-#pragma unroll
-                for (int g = 0; g < 8; ++g) add_quad(v, g, __ldcg(src + g * 128));  // written during this launch: not through the read-only path
-              }
             }
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
@@ -345,16 +327,39 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
             if (last) mbar_arrive(&msum_empty[slot]);
           }
           if (park_it && last) {
-            // This warp's columns of the partial sums are written: publish them (one count per epilogue warp).
-            __threadfence();
+            __threadfence();  // this lane's sums are visible ...
             __syncwarp();
-            if (lane == 0) add_release_gpu(p.park_flags + w.park_slot, 1);
+            int before = 0;
+            if (lane == 0) before = atomicAdd(p.park_flags + shared_tile * 4 + q, 1);  // ... before they are counted
+            if (__shfl_sync(0xffffffffu, before, 0) == shared_parts - 1) {
+              __threadfence();
+#pragma unroll 1
+              for (int c = 0; c < BM / 32; ++c) {
+                const int sb = s0 + c * 32;
+                if (sb >= p.S) break;
+                uint32_t v[32] = {};
+#pragma unroll 1
+                for (int part = 0; part < shared_parts; ++part) {
+                  const float4* src = parked + part * (PARK_TILE / 4) + c * 8 * 128;
+#pragma unroll
+                  for (int g = 0; g < 8; ++g) add_quad(v, g, __ldcg(src + g * 128));  // written during this launch: not through the read-only path
+                }
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                  const float o = m + logf(__uint_as_float(v[e]));
+                  if (col_ok && sb + e < p.S) {
+                    out_col[static_cast<int64_t>(sb + e) * p.out_s1] = o;
+                    cmx = fmaxf(cmx, o);
+                  }
+                }
+              }
+            }
           }
         }
-        if (ok && p.out_max != nullptr && !split_mode && !park_it && col_ok) {
+        if (ok && p.out_max != nullptr && !split_mode && col_ok) {
           float* dst = p.out_max + static_cast<int64_t>(r) * p.K + kcol;
-          if (p.tiles_m == 1) *dst = cmx;
-          else red_max_f32(dst, cmx);
+          if (!park_it && p.tiles_m == 1) *dst = cmx;
+          else red_max_f32(dst, cmx);  // (a part that did not complete its tile: -inf)
         }
       }
     } else
