@@ -17,6 +17,7 @@
 #include "lm2exp_pair3x_kernel.cuh"
 #include "lt2exp_kernel.cuh"
 #include "lt2exp_tmem_kernel.cuh"
+#include "lt2exp_duo_kernel.cuh"
 #include "direct_kernels.cuh"
 
 namespace tb200 {
@@ -1453,7 +1454,6 @@ static int launch_lt2exp_tmem(const CUtensorMap& tw, Lt2expParams p, const LtLau
 //                              MT NS   (generated operand in TMEM, 128 columns k per tile, TF32)
 using LtM_1 = Lt2expTmemCfg<1, 8>;
 using LtM_2 = Lt2expTmemCfg<2, 6>;
-using LtM_1x2 = Lt2expTmemCfg<1, 4, 2>;  // 128 rows x two 128-column blocks sharing each w tile
 using LtMX_1 = Lt2expTmemCfg<1, 4, 1, 1>;  // 3xTF32, 128 x 128
 
 //                          BN   MT NS NTW
@@ -1518,7 +1518,7 @@ static int lt2exp_dispatch(int precision, int bn, int mt, bool promote, Args... 
   }
   if (mt == 3 || mt == 4 || mt == 5) {
     if (precision != TRITURUS_B200_PRECISION_TF32) return TRITURUS_B200_EINVAL;
-    if (mt == 5) return launch_lt2exp_tmem<LtM_1x2>(args...);
+    if (mt == 5) return launch_lt2exp_with<Lt2expDuoCfg, lt2exp_duo_kernel, false>(args...);
     return mt == 4 ? launch_lt2exp_tmem<LtM_2>(args...) : launch_lt2exp_tmem<LtM_1>(args...);
   }
   if (precision == TRITURUS_B200_PRECISION_3XTF32) return launch_lt2exp_tmem<LtMX_1>(args...);
@@ -1705,6 +1705,18 @@ static int lt2exp_run_block(const float* w, const float* a, const float* b, floa
   p.vec_ab = (K % 4 == 0 && as2 == 1 && bs2 == 1 && aligned16(a) && aligned16(b) && as0 % 4 == 0 && as1 % 4 == 0 &&
               bs0 % 4 == 0 && bs1 % 4 == 0) ? 1 : 0;
   p.status = status_dev;
+  memset(&p.tmap_out, 0, sizeof(p.tmap_out));
+  if (bn == 128 && mt == 5) {  // lt2exp_duo_kernel stores through TMA where the result meets the tensor-map rules
+    int64_t t0 = os0, t1 = os1;
+    if (aligned16(out) && (K & 3) == 0 && fix_stride(S, t1, round_up4(K)) && fix_stride(R, t0, round_up4(K) * S)) {
+      const int64_t dims[3] = {K, S, R};
+      const int64_t strides[3] = {1, t1, t0};
+      const uint32_t box[3] = {32, 32, 1};
+      const int rc = make_tmap(&p.tmap_out, out, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc != TRITURUS_B200_OK) return rc;
+      p.out_tma = 1;
+    }
+  }
   p.ma_in = a_colmax;
   p.mb_in = b_colmax;
   p.out_max = out_colmax;

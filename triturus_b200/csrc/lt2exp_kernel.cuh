@@ -41,6 +41,8 @@
 namespace tb200 {
 
 struct Lt2expParams {
+  CUtensorMap tmap_out;  // out in 32 x 32 boxes where out_tma (lt2exp_duo_kernel)
+  int out_tma = 0;
   const float* a;  // [R, I, K]
   const float* b;  // [R, J, K]
   float* out;      // [R, S, K]
