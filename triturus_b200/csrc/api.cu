@@ -1454,7 +1454,7 @@ static int launch_lt2exp_tmem(const CUtensorMap& tw, Lt2expParams p, const LtLau
 //                              MT NS   (generated operand in TMEM, 128 columns k per tile, TF32)
 using LtM_1 = Lt2expTmemCfg<1, 8>;
 using LtM_2 = Lt2expTmemCfg<2, 6>;
-using LtMX_1 = Lt2expTmemCfg<1, 4, 1, 1>;  // 3xTF32, 128 x 128
+using LtMX_1 = Lt2expTmemCfg<1, 4, 1>;  // 3xTF32, 128 x 128
 
 //                          BN   MT NS NTW
 using LtT_128_1 = Lt2expCfg<128, 1, 6, 8>;

@@ -50,20 +50,18 @@ namespace tb200 {
 // Chunks of 24 (768 terms): rms error of a long flat sum 1.2e-5.  16: 0.8e-5, but 1 to 9 % slower, the drain being no longer
 // hidden (R16 128x64x64x2048 150 -> 162 us, 1 x 256^4 71 -> 79); 32: 1.6e-5, at most 2 % faster (R64 256x128x128x4096 8 560 ->
 // 8 370 us, R32 256^4 1 163 -> 1 156).
-template <int MT_, int NS_, int NB_ = 1, int PREC_ = 0>
+template <int MT_, int NS_, int PREC_ = 0>
 struct Lt2expTmemCfg {
   static constexpr int BM = 128, BK = 32;  // BM: rows s per w box
-  static constexpr int NB = NB_;           // 128-column blocks per tile: each is one M = 128 MMA on the same w tile
-  static constexpr int BN = 128 * NB;      // columns k per tile
+  static constexpr int BN = 128;           // columns k per tile
   static constexpr int MT = MT_, NS = NS_, PREC = PREC_, NTW = 8;
   static constexpr bool PROMOTE = PREC != 0;  // chunked re-summation of the accumulator
   static constexpr int CHUNK = PROMOTE ? 24 : 1 << 30;  // k-blocks
   static constexpr int W_TILE = BM * BK * 4;
   static constexpr int W_BYTES = MT * W_TILE;             // what TMA brings per stage
   static constexpr int STAGE = (PREC ? 2 : 1) * W_BYTES;  // ... and the low parts of it
-  static constexpr int BLK_COLS = MT * BM;        // accumulator columns of one column block
-  static constexpr int ACC_COLS = NB * BLK_COLS;
-  static constexpr int P_STAGE = NB * (PREC ? 2 : 1) * BK;  // operand columns per stage
+  static constexpr int ACC_COLS = MT * BM;
+  static constexpr int P_STAGE = (PREC ? 2 : 1) * BK;  // operand columns per stage
   static constexpr int NBUF = (2 * ACC_COLS + NS * P_STAGE <= 512) ? 2 : 1;
   static constexpr int P_COL0 = NBUF * ACC_COLS;  // first operand column
   static constexpr int TMEM_USED = P_COL0 + NS * P_STAGE;
@@ -77,10 +75,10 @@ struct Lt2expTmemCfg {
   static constexpr int MPART = 2 * RG * BN;
   static constexpr int NBAR = 3 * NS + 9;
   static constexpr int MASTER = PROMOTE ? MT * BM * BN * 4 : 0;
-  static_assert(!PREC || (MT == 1 && NB == 1 && NBUF == 2), "3xTF32: 128 x 128 tiles, two accumulators");
+  static_assert(!PREC || (MT == 1 && NBUF == 2), "3xTF32: 128 x 128 tiles, two accumulators");
   static constexpr int SMEM_BYTES = 1024 + NS * STAGE + MASTER + 2 * BN * 4 + 2 * MPART * 4 + NBAR * 8 + 64;
   static_assert(TMEM_USED <= 512, "TMEM capacity");
-  static_assert(NGROUPS * NB == 2, "eight transform warps: two groups on one column block, or one group on two");
+  static_assert(NGROUPS == 2, "eight transform warps: two groups");
   static_assert(SMEM_BYTES <= 232448, "shared memory capacity");
 };
 
@@ -218,12 +216,11 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
           }
           const int sn = (s + 1 == NS) ? 0 : s + 1;
           const uint32_t phn = (s + 1 == NS) ? ph ^ 1 : ph;
-          const bool peek = mbar_try_wait(&full[sn], phn);
           tc_fence_after_sync();
-          if (elect_one_sync()) {
-            const uint64_t dw = umma_desc_k_sw128(stage0 + s * Cfg::STAGE);
-            const uint32_t pa = tmem_base + Cfg::P_COL0 + s * Cfg::P_STAGE;
-            if (Cfg::PREC) {
+          const uint64_t dw = umma_desc_k_sw128(stage0 + s * Cfg::STAGE);
+          const uint32_t pa = tmem_base + Cfg::P_COL0 + s * Cfg::P_STAGE;
+          if (Cfg::PREC) {
+            if (elect_one_sync()) {
               // the corrections first, while the accumulator of a chunk is empty and does not truncate them to its bits
 #pragma unroll
               for (int ks = 0; ks < BK / 8; ++ks)
@@ -231,13 +228,14 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
 #pragma unroll
               for (int ks = 0; ks < BK / 8; ++ks) umma_tf32_ts(d, pa + ks * 8, dw + (Cfg::W_BYTES >> 4) + 2 * ks, idesc, 1u);
             }
+          }
+          // The tensor core takes the next MMA only when it is about done with the one before, so what this warp does between
+          // two stages is lost to it: 3xTF32 asks for the next stage in the middle of this one.
+          const bool peek = mbar_try_wait(&full[sn], phn);
+          if (elect_one_sync()) {
 #pragma unroll
-            for (int blk = 0; blk < Cfg::NB; ++blk) {  // the column blocks share the w tile
-#pragma unroll
-              for (int ks = 0; ks < BK / 8; ++ks)
-                umma_tf32_ts(d + blk * Cfg::BLK_COLS, pa + blk * BK + ks * 8, dw + 2 * ks, idesc,
-                             (Cfg::PREC || kb > kb0 || ks > 0) ? 1u : 0u);
-            }
+            for (int ks = 0; ks < BK / 8; ++ks)
+              umma_tf32_ts(d, pa + ks * 8, dw + 2 * ks, idesc, (Cfg::PREC || kb > kb0 || ks > 0) ? 1u : 0u);
             umma_commit(&opnd_empty[s]);
           }
           ready = __all_sync(0xffffffffu, peek);
@@ -372,12 +370,11 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
       if (!(ok = mbar_wait_warp(&acc_full[buf], aph, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
       if (Cfg::NGROUPS > 1 && !(ok = mbar_wait_warp(&msum_full[slot], (tcount >> 1) & 1, ctl, STATUS_TIMEOUT_EPILOGUE))) break;
       tc_fence_after_sync();
-#pragma unroll 1
-      for (int blk = 0; blk < Cfg::NB; ++blk) {  // column blocks of the tile: this lane's column in each
-        const int kcol = n0 + blk * 128 + q * 32 + lane;
+      {
+        const int kcol = n0 + q * 32 + lane;
         const bool col_ok = kcol < p.K;
         float* out_col = p.out + static_cast<int64_t>(r) * p.out_s0 + kcol;
-        const float m = msum[slot * BN + blk * 128 + q * 32 + lane];
+        const float m = msum[slot * BN + q * 32 + lane];
         float cmx = -INFINITY;  // running maximum of this lane's column over the rows of the tile
         // One chunk = 32 rows s for this lane's column.  The loop stays rolled (two chunks per trip, the
         // next one loading while the current one is finished): unrolled, every chunk was straight-line code
@@ -400,18 +397,18 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
             }
           }
         };
-        const uint32_t acc0 = lane_base + buf * Cfg::ACC_COLS + blk * Cfg::BLK_COLS;
+        const uint32_t acc0 = lane_base + buf * Cfg::ACC_COLS;
         uint32_t v0[32], v1[32];
         tmem_ld_32x32(acc0, v0);
 #pragma unroll 1
-        for (int c = 0; c < Cfg::BLK_COLS / 32; c += 2) {
+        for (int c = 0; c < Cfg::ACC_COLS / 32; c += 2) {
           const int sb = s0 + c * 32;
           if (sb >= p.S) break;
           tmem_ld_wait();
           tmem_ld_32x32(acc0 + (c + 1) * 32, v1);
           finish(v0, sb);
           tmem_ld_wait();
-          if (c + 2 < Cfg::BLK_COLS / 32) tmem_ld_32x32(acc0 + (c + 2) * 32, v0);
+          if (c + 2 < Cfg::ACC_COLS / 32) tmem_ld_32x32(acc0 + (c + 2) * 32, v0);
           if (sb + 32 < p.S) finish(v1, sb + 32);
         }
         tmem_ld_wait();
@@ -456,10 +453,7 @@ lt2exp_tmem_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expParam
     const int n = tt % BN;   // column of the tile = TMEM lane owned by this thread
     const int grp = tt / BN; // this thread's group takes every NGROUPS-th k-block
     constexpr int NG = Cfg::NGROUPS;
-    // TMEM lane quarter of this warp; with two column blocks per tile the upper four warps write the second
-    // block's operand columns.
-    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Cfg::P_COL0 +
-                               (Cfg::NB == 2 ? static_cast<uint32_t>((tt / 128) * BK) : 0u);
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Cfg::P_COL0;
     uint32_t it = 0, tcount = 0;
     bool ok = true;
     if (p.ma_wait) pdl_wait();
