@@ -498,3 +498,36 @@ def test_3xtf32_sums_of_one_term(I, J, variant):
     want = orc.lt2exp_fp64(w, a, b)
     err = (got.double() - want).abs()
     assert (err <= _tol_3xtf32(w, a, b, want, terms=1)).all(), err.max()
+
+
+@pytest.mark.parametrize("shape, split", [
+    ((74, 161, 3, 33, 250), 1),     # a tile per pair, six row units of which the last has one row, six columns of padding
+    ((80, 190, 2, 20, 256), 1),     # a second tile for a few pairs, two k-blocks each
+    ((1, 385, 128, 64, 512), 0),    # tiles of four, four and five row units; slices that begin and end inside a row of k-blocks
+    ((1, 385, 128, 64, 512), 7),
+    ((1, 64, 60, 70, 1000), 9998),  # parts of four column tiles, parked and added up; the last tile has 24 columns in its second half
+    ((40, 60, 50, 50, 512), 0),     # a last wave of few tiles: equal parts
+    ((60, 60, 100, 100, 512), 0),   # ... of more: mains and tails
+], ids=str)  # fmt: skip
+def test_3xtf32_on_pair_tiles(shape, split):
+    """Shapes that the 3xTF32 kernel of CTA pairs takes (tiles of 256 columns and up to six units of 32 rows), at the edges of its
+    tiles and work items, with impossible states and the column maxima of the result.  Tolerance: _tol_3xtf32."""
+    import triturus_b200 as tb
+
+    R, S, I, J, K = shape
+    g = torch.Generator().manual_seed(sum(shape))
+    w = torch.rand(R, S, I, J, generator=g) + 1e-3
+    a = torch.randn(R, I, K, generator=g) * 4.0 + 50.0 * torch.randn(R, 1, K, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0
+    a[torch.rand(R, I, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K // 2] = float("-inf")
+    variant = split * 10000 + 1281
+    got, m = tb.lt2exp(w.cuda(), a.cuda(), b.cuda(), precision="3xtf32", variant=variant, return_colmax=True)
+    tb.check_status()
+    assert torch.equal(m, got.amax(1))
+    some = sorted({0, R // 2, R - 1})
+    got, w, a, b = got[some].cpu(), w[some], a[some], b[some]
+    want = orc.lt2exp_fp64(w, a, b, chunk=1)
+    assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
+    fin = torch.isfinite(want)
+    assert ((got.double() - want).abs() <= _tol_3xtf32(w, a, b, want))[fin].all()

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/triturus_b200.h"
 #include "lm2exp_kernel.cuh"
@@ -18,6 +19,7 @@
 #include "lt2exp_kernel.cuh"
 #include "lt2exp_tmem_kernel.cuh"
 #include "lt2exp_duo_kernel.cuh"
+#include "lt2exp_pair3x_kernel.cuh"
 #include "direct_kernels.cuh"
 
 namespace tb200 {
@@ -1253,14 +1255,13 @@ struct LtSplit {
 // auto_stream: the launch can complete shared tiles through scratch memory (see Lt2expParams::park); without
 // it the end-to-end form would have to add every partial sum into the result with atomics, which costs more
 // than the ragged wave it removes, so the automatic choice then keeps whole tiles.
-static LtSplit lt2exp_split(int64_t tiles, int I, int J, int request, bool auto_stream) {
+static LtSplit lt2exp_split(int64_t tiles, int I, int J, int request, bool auto_stream, int sms) {
   // Slices of four k-blocks, where 16 was the least before: a 1 x 128 x 128 result over 64 / 128 / 256 k-blocks takes 21.4 /
   // 21.7 / 22.7 us on the device in TF32, 26.3 / 26.2 / 26.5 with 16, and 32.6 / 32.9 / 33.4 in 3xTF32, 38.8 / 38.3 / 38.4 with 16.
   constexpr int kMinSliceBlocks = 4;
   constexpr int kMinStreamBlocks = 256;
   const int JC = (J + 31) / 32;
   const int64_t kb = static_cast<int64_t>(JC) * I;
-  const int sms = sm_count();
   LtSplit sp{1, 0};
   if (request == 1) return sp;
   if (request == 9998) {
@@ -1295,8 +1296,7 @@ struct LtShare {
 };
 constexpr int64_t kItemBlocks = 32;  // a work item's prologue and epilogue, in k-blocks (25 us per tail of a 256 x 256 tile
                                      // against 0.73 us per k-block)
-static LtShare lt2exp_share(int64_t nt, int64_t kbt) {
-  const int G = sm_count();
+static LtShare lt2exp_share(int64_t nt, int64_t kbt, int G) {
   const int64_t waves = (nt + G - 1) / G;
   LtShare sh{static_cast<int>((waves - 1) * G), 1, static_cast<int>(kbt)};
   const int rem = static_cast<int>(nt - sh.first);
@@ -1323,9 +1323,9 @@ static LtShare lt2exp_share(int64_t nt, int64_t kbt) {
 // k-blocks more than an item's own.  us, whole / shared: R10 128x128x128x2048 538 / 360, R40 64x90x200x500 669 / 409, R6
 // 200x100x100x1000 225 / 178, R30 60x100x100x1000 420 / 365, R8 256x128x128x4096 1 136 / 1 068, R32 256^4 1 320 / 1 249; R90
 // 128x128x32x128 88.9 / 91.6 and R128 128x100x100x128 334 / 341, which the estimate leaves whole.
-static bool lt2exp_share_wins(int64_t nt, int64_t kbt) {
-  const int64_t G = sm_count(), waves = (nt + G - 1) / G, item = kbt + kItemBlocks;
-  const LtShare sh = lt2exp_share(nt, kbt);
+static bool lt2exp_share_wins(int64_t nt, int64_t kbt, int G) {
+  const int64_t waves = (nt + G - 1) / G, item = kbt + kItemBlocks;
+  const LtShare sh = lt2exp_share(nt, kbt, G);
   if (waves > 8 || sh.parts == 1) return false;
   const int64_t longest = sh.parts > 0 ? kbt / sh.parts : sh.main;
   return static_cast<double>((waves - 1) * item + longest + kItemBlocks + 28) < 0.97 * static_cast<double>(waves * item);
@@ -1347,6 +1347,16 @@ struct LtLaunch {
 
 constexpr size_t kParkHeader = 4096;  // flags (one int per CTA, in 3xTF32 four per shared tile) ahead of the parked tiles
 
+// CTAs that work on one tile.
+template <class Cfg, class = void>
+struct LtCtas {
+  static constexpr int value = 1;
+};
+template <class Cfg>
+struct LtCtas<Cfg, std::void_t<decltype(Cfg::CTAS)>> {
+  static constexpr int value = Cfg::CTAS;
+};
+
 template <class Cfg, void (*Kern)(const CUtensorMap, const Lt2expParams), bool CAN_PARK>
 static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLaunch& L) {
   auto kern = Kern;
@@ -1360,9 +1370,11 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   const int64_t nt = static_cast<int64_t>(p.R) * p.tiles_m * p.tiles_n;
   if (nt > INT32_MAX) return TRITURUS_B200_EINVAL;
   p.num_tiles = static_cast<int>(nt);
+  constexpr int CTAS = LtCtas<Cfg>::value;
+  const int workers = sm_count() / CTAS;  // CTAs, or pairs of them
   // Scratch memory for the end-to-end form: one parked tile per CTA behind the flags.
   // (3xTF32: every part parks, up to two per tile of a last wave that fills more than half of the SMs.)
-  const size_t park_need = kParkHeader + static_cast<size_t>(sm_count()) * (Cfg::PREC ? 2 : 1) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
+  const size_t park_need = kParkHeader + static_cast<size_t>(workers) * (Cfg::PREC ? 2 : 1) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
   const bool have_ws = CAN_PARK && sm_count() * sizeof(int) * (Cfg::PREC ? 4 : 1) <= kParkHeader &&
                        (L.query != nullptr || (L.ws != nullptr && L.ws_bytes >= park_need &&
                                                (reinterpret_cast<uintptr_t>(L.ws) & 255) == 0));
@@ -1370,8 +1382,8 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   // those slower (R32 256^4: 1.32 against 0.81 ms; R128: 2.75 against 2.40 ms); the explicit request 9998 still selects it.
   // 3xTF32 has a rule of its own (lt2exp_share).
   const bool chunked = Cfg::PROMOTE && static_cast<int64_t>((p.J + 31) / 32) * p.I > Cfg::CHUNK;
-  LtSplit sp = lt2exp_split(nt, p.I, p.J, L.split_request, have_ws && !chunked);
-  if (Cfg::PREC && have_ws && L.split_request == 0 && sp.nsplit == 1 && lt2exp_share_wins(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I))
+  LtSplit sp = lt2exp_split(nt, p.I, p.J, L.split_request, have_ws && !chunked, workers);
+  if (Cfg::PREC && have_ws && L.split_request == 0 && sp.nsplit == 1 && lt2exp_share_wins(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I, workers))
     sp.stream = 1;
   p.nsplit = sp.nsplit;
   p.stream = sp.stream;
@@ -1380,7 +1392,7 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   p.num_items = static_cast<int>(items);
   if (sp.stream) {
     // Whole waves first, then the tiles of the last wave shared among all CTAs (LtWork in lt2exp_kernel.cuh).
-    const LtShare sh = lt2exp_share(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I);
+    const LtShare sh = lt2exp_share(nt, static_cast<int64_t>((p.J + 31) / 32) * p.I, workers);
     p.lw_first = sh.first;
     p.lw_parts = sh.parts;
     p.lw_main = sh.main;
@@ -1428,7 +1440,7 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
       lt2exp_zero_kernel<<<zgrid, 256, 0, L.stream>>>(p.out, p.out_s0, p.out_s1, p.R, p.S, p.K);
     }
   }
-  const int grid = (sp.stream || p.num_items >= sm_count()) ? sm_count() : p.num_items;
+  const int grid = CTAS * ((sp.stream || p.num_items >= workers) ? workers : p.num_items);
   const int rc = launch_maybe_dependent(kern, dim3(static_cast<unsigned>(grid)), Cfg::NTHREADS, Cfg::SMEM_BYTES, L.stream, split, tw, p);
   if (rc != TRITURUS_B200_OK) return rc;
   if (split) {
@@ -1456,6 +1468,35 @@ using LtM_1 = Lt2expTmemCfg<1, 8>;
 using LtM_2 = Lt2expTmemCfg<2, 6>;
 using LtMX_1 = Lt2expTmemCfg<1, 4, 1>;  // 3xTF32, 128 x 128
 
+// Cycles of the busiest of `workers` CTAs (or pairs of them) over `nt` tiles in 3xTF32, as launch_lt2exp_with shares them out.  A
+// slice costs 39 000 besides its k-blocks, the launches before and after among them.
+static double lt2exp_busiest(int64_t nt, int I, int J, int workers, double per_kb, double per_item) {
+  const int64_t kbt = static_cast<int64_t>((J + 31) / 32) * I, waves = (nt + workers - 1) / workers;
+  const int64_t nsplit = lt2exp_split(nt, I, J, 0, false, workers).nsplit;
+  if (nsplit > 1) return static_cast<double>((kbt + nsplit - 1) / nsplit) * per_kb + 39000.0;
+  const double item = static_cast<double>(kbt) * per_kb + per_item;
+  if (!lt2exp_share_wins(nt, kbt, workers)) return static_cast<double>(waves) * item;
+  const LtShare sh = lt2exp_share(nt, kbt, workers);
+  const int64_t longest = sh.parts > 0 ? kbt / sh.parts : sh.main;
+  return static_cast<double>(waves - 1) * item + static_cast<double>(longest) * per_kb + per_item + 28000.0;
+}
+
+// 3xTF32: pairs of CTAs on 256 columns (lt2exp_pair3x_kernel), or CTAs on 128 x 128 (lt2exp_tmem_kernel)?  A k-block is 1 000
+// cycles of a CTA, and of a pair 192 per 32 rows, from 700 on; an item's prologue and epilogue 25 000 and 30 000.  Fitted to 65
+// shapes of 32 ... 384 rows and widths and 64 ... 4096 columns: no pair that this chooses takes longer by more than 1 %.  us, 128 x 128
+// / pairs: R15 160x126x163x480 458 / 315, R148 192x8x32x256 76.3 / 50.3, R64 32x64x64x1024 262 / 211, R40 64x90x200x500 407 / 341, R32
+// 256^4 1 105 / 1 044, R1 256^4 65.9 / 59.3; and where pairs would have columns of padding or fill the GPU unevenly, R90
+// 128x128x32x128 92.3 / 130, R25 92x155x80x524 254 / 285, R2 384x128x128x384 62.3 / 67.4.
+static bool lt2exp_pair3x_wins(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K) {
+  const int64_t units = (S + 31) / 32, row_tiles = (units + Lt2expPair3xCfg::UNITS - 1) / Lt2expPair3xCfg::UNITS;
+  const double per_kb = std::max(192.0 * static_cast<double>((units + row_tiles - 1) / row_tiles), 700.0);
+  const double one = lt2exp_busiest(R * ((S + 127) / 128) * ((K + 127) / 128), static_cast<int>(I), static_cast<int>(J), sm_count(), 1000.0,
+                                    25000.0);
+  const double two = lt2exp_busiest(R * row_tiles * ((K + 255) / 256), static_cast<int>(I), static_cast<int>(J), sm_count() / 2, per_kb,
+                                    30000.0);
+  return two < 0.92 * one;
+}
+
 //                          BN   MT NS NTW
 using LtT_128_1 = Lt2expCfg<128, 1, 6, 8>;
 using LtT_128_2 = Lt2expCfg<128, 2, 4, 8>;
@@ -1468,6 +1509,8 @@ using LtP_256_1 = Lt2expCfg<256, 1, 4, 8, true>;
 
 }  // namespace tb200
 
+constexpr int kPair3xTile = 9;  // (`mt` of lt2exp_pair3x_kernel; plans name 3xTF32 tiles 1281)
+
 // Decodes SPLIT * 10000 + BN * 10 + MT, filling in the automatic tile shape.
 // *promote: plain TF32 over a contraction of more than kLongContraction terms on a tile whose accumulator
 // leaves room for a master copy in TMEM (the automatic choice is restricted to such tiles; an explicit
@@ -1479,8 +1522,8 @@ static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int6
   int tile = variant % 10000;
   const bool long_tf = precision == TRITURUS_B200_PRECISION_TF32 && I * ((J + 31) / 32 * 32) > tb200::kLongContraction;
   if (precision == TRITURUS_B200_PRECISION_3XTF32) {
-    // One kernel, which keeps the generated operand in TMEM on 128 x 128 tiles; the codes of the other shared-memory tiles
-    // stay accepted and run it too.  (Their own instances, both operands and their low parts in shared memory with
+    // The generated operand in TMEM, on 128 x 128 tiles or pairs of CTAs (below); the codes of the other shared-memory tiles
+    // stay accepted and run that too.  (Their own instances, both operands and their low parts in shared memory with
     // two stages, us on 1281 / 1282 / 2561: R32 256^4 1 154 / 3 180 / 2 603, R64 256x128x128x4096 8 480 / 11 740 / 9 590, R16
     // 128x64x64x2048 148 / 425 / 160, R64 128x16x16x1024 69 / 136 / 68, R8 300x32x32x1000 55 / 67 / 52; 15 more shapes:
     // 1281 the fastest.)
@@ -1494,6 +1537,10 @@ static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int6
   *bn = tile / 10;
   *mt = tile % 10;
   *promote = long_tf && (tile == 1281 || tile == 1282 || tile == 2561);
+  if (precision == TRITURUS_B200_PRECISION_3XTF32 && tile == 1281 && tb200::lt2exp_pair3x_wins(R, S, I, J, K)) {
+    *mt = kPair3xTile;
+    return TRITURUS_B200_OK;
+  }
   // operand in TMEM: 128 columns x 128 / 256 rows (1283 / 1284), 256 columns x 128 rows (1285)
   if (*bn == 128 && (*mt == 3 || *mt == 4 || *mt == 5)) return TRITURUS_B200_OK;
   if ((*bn != 128 && *bn != 256) || (*mt != 1 && *mt != 2)) return TRITURUS_B200_EINVAL;
@@ -1521,6 +1568,7 @@ static int lt2exp_dispatch(int precision, int bn, int mt, bool promote, Args... 
     if (mt == 5) return launch_lt2exp_with<Lt2expDuoCfg, lt2exp_duo_kernel, false>(args...);
     return mt == 4 ? launch_lt2exp_tmem<LtM_2>(args...) : launch_lt2exp_tmem<LtM_1>(args...);
   }
+  if (mt == kPair3xTile) return launch_lt2exp_with<Lt2expPair3xCfg, lt2exp_pair3x_kernel, true>(args...);
   if (precision == TRITURUS_B200_PRECISION_3XTF32) return launch_lt2exp_tmem<LtMX_1>(args...);
   if (bn == 256) return mt == 2 ? launch_lt2exp<LtT_256_2>(args...) : launch_lt2exp<LtT_256_1>(args...);
   return mt == 2 ? launch_lt2exp<LtT_128_2>(args...) : launch_lt2exp<LtT_128_1>(args...);
@@ -1543,7 +1591,7 @@ static int lt2exp_query(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, i
   CUtensorMap none{};
   const tb200::LtLaunch L{split, static_cast<cudaStream_t>(nullptr), q, nullptr, 0};
   rc = lt2exp_dispatch(precision, bn, mt, promote, none, p, L);
-  *tile_code = bn * 10 + mt;
+  *tile_code = bn * 10 + (mt == kPair3xTile ? 1 : mt);
   return rc;
 }
 
@@ -1676,10 +1724,13 @@ static int lt2exp_run_block(const float* w, const float* a, const float* b, floa
   }
 
   CUtensorMap tw;
+  uint32_t box_rows = 128;
   {
     const int64_t dims[4] = {J, I, S, R};
     const int64_t strides[4] = {1, ws2, ws1, ws0};
-    const uint32_t box[4] = {32, 1, 128, 1};
+    const int64_t units = (S + 31) / 32, nt = (units + tb200::Lt2expPair3xCfg::UNITS - 1) / tb200::Lt2expPair3xCfg::UNITS;
+    if (mt == kPair3xTile) box_rows = static_cast<uint32_t>((units + nt - 1) / nt * 16);
+    const uint32_t box[4] = {32, 1, box_rows, 1};
     const int rc = make_tmap(&tw, w, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc != TRITURUS_B200_OK) return rc;
   }
@@ -1705,6 +1756,7 @@ static int lt2exp_run_block(const float* w, const float* a, const float* b, floa
   p.vec_ab = (K % 4 == 0 && as2 == 1 && bs2 == 1 && aligned16(a) && aligned16(b) && as0 % 4 == 0 && as1 % 4 == 0 &&
               bs0 % 4 == 0 && bs1 % 4 == 0) ? 1 : 0;
   p.status = status_dev;
+  p.box_rows = static_cast<int>(box_rows);
   memset(&p.tmap_out, 0, sizeof(p.tmap_out));
   if (bn == 128 && mt == 5) {  // lt2exp_duo_kernel stores through TMA where the result meets the tensor-map rules
     int64_t t0 = os0, t1 = os1;

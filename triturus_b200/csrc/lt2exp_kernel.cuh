@@ -51,6 +51,7 @@ struct Lt2expParams {
   int64_t out_s0, out_s1;
   int R, S, I, J, K;
   int tiles_m, tiles_n, num_tiles;
+  int box_rows = 0;  // lt2exp_pair3x_kernel: rows of a box of w (half of the largest tile's)
   int nsplit;     // equal slices of the contraction per tile (1: whole tiles)
   int stream;     // 1: whole waves of tiles, then the tiles of the last wave shared among all CTAs (see LtWork)
   int num_items;  // num_tiles * nsplit (not used when stream == 1)
@@ -103,19 +104,22 @@ struct LtWork {
   int kb_tile, nsplit, stream;
   int lw_first, lw_rem, lw_parts, lw_main;  // last wave: first tile, tiles, parts per tile (0: mains and tails), main length
   int phase, tail_next;                     // stream: 0 = whole waves, 1 = last wave, 2 = done
-  __device__ LtWork(const Lt2expParams& p, int kb_tile_) {
+  int self, workers;                        // this CTA (or pair of CTAs) of how many
+  __device__ LtWork(const Lt2expParams& p, int kb_tile_, int self_ = blockIdx.x, int workers_ = gridDim.x) {
+    self = self_;
+    workers = workers_;
     kb_tile = kb_tile_;
     nsplit = p.nsplit;
     stream = p.stream;
-    q = blockIdx.x;
+    q = self;
     nq = stream ? p.lw_first : p.num_items;
-    step = gridDim.x;
+    step = workers;
     lw_first = p.lw_first;
     lw_rem = p.num_tiles - p.lw_first;
     lw_parts = p.lw_parts;
     lw_main = p.lw_main;
     phase = 0;
-    tail_next = static_cast<int>(blockIdx.x) - lw_rem;  // (mains and tails) first tail of a helper CTA
+    tail_next = self - lw_rem;  // (mains and tails) first tail of a helper CTA
   }
   __device__ bool next(LtItem& w) {
     w.park_slot = -1;
@@ -142,7 +146,7 @@ struct LtWork {
       phase = 1;
     }
     if (phase != 1) return false;
-    const int c = blockIdx.x;
+    const int c = self;
     if (lw_parts > 0) {
       // equal parts: part j of tile t on CTA t + j * rem
       phase = 2;
@@ -182,7 +186,7 @@ struct LtWork {
     w.kb_hi = kb_tile;
     w.part = 1;
     w.park_slot = tail_next;
-    tail_next += static_cast<int>(gridDim.x) - lw_rem;
+    tail_next += workers - lw_rem;
     return true;
   }
 };

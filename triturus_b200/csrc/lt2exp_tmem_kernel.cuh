@@ -42,7 +42,9 @@ namespace tb200 {
 // 1 298 us, but terms off by up to 7e-6, see lm2exp_tspair_kernel.cuh.)
 // Per k-block of a 128 x 128 tile: 16 KB TMA in, 16 KB read and 16 KB written by the splitting, 48 KB read by the tensor
 // core = 768 cycles of the shared-memory pipe next to 768 of the tensor pipe (both operands in shared memory: 1 400).
-// Measured 1 030 cycles per k-block (R32 256^4): the four stages' chain of TMA, splitting, MMA and commit bounds it.
+// Measured 1 000 cycles per k-block (R32 256^4, 1 030 before the issuer asked for the next stage in the middle of one): what it does
+// between two stages bounds it, and what the queue of the tensor core does not cover.  Calls that fill pairs of CTAs run
+// lt2exp_pair3x_kernel.cuh instead.
 // At 96 registers a thread (20 warps) 92 bytes are spilled, outside the loops over k-blocks: 68 loads and 52 stores per
 // CTA of one tile.
 // Every CHUNK k-blocks the MMA warp changes to the other accumulator and the epilogue warps add the finished one to a
