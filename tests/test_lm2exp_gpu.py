@@ -875,3 +875,40 @@ def test_3xtf32_pair_tiles_with_two_accumulators(shape, variant):
     for o in outs:
         assert torch.equal(o == float("-inf"), want == float("-inf")) and not torch.isnan(o).any()
         assert ((o.double() - want).abs() <= tol)[fin].all()
+
+
+@pytest.mark.parametrize("shape", [
+    (8, 64, 992, 160),    # one row block, 96 columns of padding, few tiles
+    (1, 177, 768, 640),   # six row units, the last with 17 rows; one entry
+    (2, 40, 1024, 64),    # a quarter of the columns of a tile, the longest contraction of the rule
+    (120, 33, 44, 1000),  # two k-blocks of which the second has 12 rows
+    (3, 256, 516, 132),   # a second slab of four columns
+], ids=str)  # fmt: skip
+def test_3xtf32_calls_of_up_to_1024_terms_run_on_pairs(shape):
+    """Automatic calls in 3xTF32 that CTA pairs take although a single-CTA kernel could: with impossible states, as a
+    transposed view, with column maxima of the result and with those of b supplied."""
+    import triturus_b200 as tb
+    from triturus_b200 import _native
+
+    R, I, J, K = shape
+    assert _native.LIB.triturus_b200_lm2exp_plan(R, I, J, K, 1, 0) == 102564
+    assert _native.LIB.triturus_b200_lm2exp_direct(R, I, J, K, 1, 0, 0) == 0
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    b[torch.rand(R, J, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K - 1] = float("-inf")
+    a[R - 1, I - 1] = 0.0
+    want = orc.lm2exp_fp64(a, b)
+    ad, bd = a.cuda(), b.cuda()
+    outs = [tb.lm2exp(ad, bd, precision="3xtf32"), tb.lm2exp(ad.transpose(1, 2).contiguous().transpose(1, 2), bd, precision="3xtf32")]
+    out, m = tb.lm2exp(ad, bd, precision="3xtf32", return_colmax=True)
+    assert torch.equal(m, out.amax(1))
+    outs += [out, tb.lm2exp(ad, bd, precision="3xtf32", b_colmax=bd.amax(1))]
+    tb.check_status()
+    fin = torch.isfinite(want)
+    tol = _tol_3xtf32(a, b, want)
+    for o in outs:
+        o = o.cpu()
+        assert torch.equal(o == float("-inf"), want == float("-inf")) and not torch.isnan(o).any()
+        assert ((o.double() - want).abs() <= tol)[fin].all()

@@ -575,9 +575,19 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
     const bool big = 2.0 * static_cast<double>(R) * I * J * K >= 2e10;
     const bool long_3x = precision == TRITURUS_B200_PRECISION_3XTF32 && J > 4096;
     const bool long_tf = precision == TRITURUS_B200_PRECISION_TF32 && J > kLongContraction;
-    const bool want_pair = !b_km && !single_cta && (stab_mode < 2 || stab_mode == 4) && !long_3x && !long_tf &&
+    const bool wide_pair = (stab_mode < 2 || stab_mode == 4) && !long_3x && !long_tf &&
                            (I > 256 || (I > 128 && J >= 128 && !have_m && stab_mode != 1 && big)) && K > 128 &&
                            tile_count(R, I, K, 256, 2) >= sm_count() / 4;
+    // 3xTF32 up to the 1024 terms that the single-CTA kernel sums without a break: its transform warps split three operands
+    // per stage through shared memory, which takes two to three times as long as the pair kernels' k-blocks, so that those
+    // win even with the launch of a pre-pass and with few or half-empty tiles.  us, single-CTA / pairs: R8 64x992x160 53 / 23, R117
+    // 160x44x1992 252 / 109, R1 177x768x160 44 / 19, R6 253x528x1504 36 / 24, R22 218x256x3864 125 / 95, R43 64x352x2156 98 / 70.  With at
+    // most 128 columns half of a tile is padding: then only while the single-CTA kernel's tiles are no more than one wave (R90
+    // 64x864x128 49 / 42, R2 40x764x64 41 / 19; R98 198x64x120 23.5 / 23.3, R77 576x124x72 32 / 38, R125 317x48x68 27 / 31).  One row block
+    // and a long launch keep the fused form that is documented for them.
+    const bool short_pair = precision == TRITURUS_B200_PRECISION_3XTF32 && stab_mode == 0 && J <= 1024 && (I > 128 || !big) &&
+                            (K > 128 || tile_count(R, I, K, 128, I > 128 ? 2 : 1) <= sm_count());
+    const bool want_pair = !b_km && !single_cta && (wide_pair || short_pair);
     // (long plain-TF32 contractions: 128 columns, so that the master copy fits beside the accumulator)
     // Plain TF32 on pairs: the TMEM-operand kernel, with the optimistic stabiliser unless a pre-pass was asked for.
     const int pair_variant = precision != TRITURUS_B200_PRECISION_TF32 || stab_mode == 4 ? 2564
@@ -765,17 +775,17 @@ static int direct_width(const float* base, int64_t n, int64_t inner, int64_t s0,
 
 // Does an automatic call of lm2exp run lm2exp_direct_kernel?  Estimates in us, of device time in a graph.  Direct: 3 and, per 32 x 32
 // tile, 5 ns and 0.034 per contraction value (more where shared memory leaves one or two blocks per SM, and with the third
-// product); else what one wave of the tcgen05 kernels takes, 2.5 times that where they fetch an operand element by
-// element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 512^3 24.0 / 11.2, 1 x 1024x128x1024 11.7 / 11.4,
+// product); else what one wave of the tcgen05 kernels takes (in 3xTF32 those of CTA pairs), or 2.5 times the single-CTA kernel's
+// where an operand is fetched element by element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 512^3 24.0 / 11.2, 1 x 1024x128x1024 11.7 / 11.4,
 // 16 x 256^3 15.8 / 17.0, 64 x 128x128x512 17.0 / 39.5; odd: 100 x 65x33x70 19.5 / 8.5, 64 x 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50.
-// 3xTF32: 1 x 64^3 11.1 / 3.2, 8 x 128^3 17.4 / 3.8, 1 x 512^3 33.3 / 13.6, 16 x 256^3 23.1 / 19.8, 32 x 256^3 23.4 / 36.3; odd: 24 x
+// 3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 / 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x
 // 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58.
 static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd) {
   if (J > 512 || R > 65535 || (I + 31) / 32 > 65535) return false;
   const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
   const double tiles = static_cast<double>(R) * ((I + 31) / 32) * ((K + 31) / 32);
   const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? 1.4 : 1.0) * (odd ? 1.3 : 1.0);
-  const double tcgen = (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
+  const double tcgen = x3 && !odd ? 14.0 + 0.014 * J : (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
   return direct <= tcgen;
 }
 
