@@ -912,3 +912,36 @@ def test_3xtf32_calls_of_up_to_1024_terms_run_on_pairs(shape):
         o = o.cpu()
         assert torch.equal(o == float("-inf"), want == float("-inf")) and not torch.isnan(o).any()
         assert ((o.double() - want).abs() <= tol)[fin].all()
+
+
+@pytest.mark.parametrize("shape", [
+    (1, 177, 768, 160),    # a single tile of each row block, 96 columns of padding
+    (8, 132, 288, 1000),   # four rows in the second row block, a slab with 24 columns of padding
+    (30, 253, 68, 1200),   # three k-blocks, the last with four rows; ragged rows
+    (1, 320, 4096, 260),   # the longest contraction of the rule, a second slab of four columns
+    (12, 512, 764, 96),    # fewer than 128 columns
+], ids=str)  # fmt: skip
+def test_tf32_calls_of_several_row_blocks_run_on_pairs(shape):
+    """Automatic calls in plain TF32 that the TMEM-operand pair kernel takes although they are short; and the same calls in
+    the forms that it does not take (a as a transposed view, column maxima of the result), which stay where they were."""
+    import triturus_b200 as tb
+    from triturus_b200 import _native
+
+    R, I, J, K = shape
+    assert _native.LIB.triturus_b200_lm2exp_plan(R, I, J, K, 0, 0) == 102566
+    assert _native.LIB.triturus_b200_lm2exp_direct(R, I, J, K, 0, 0, 0) == 0
+    g = torch.Generator().manual_seed(sum(shape))
+    a = torch.rand(R, I, J, generator=g)
+    b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)
+    b[torch.rand(R, J, K, generator=g) < 0.02] = float("-inf")
+    b[0, :, K - 1] = float("-inf")
+    want = orc.lm2exp_fp64(a, b)
+    ad, bd = a.cuda(), b.cuda()
+    outs = [tb.lm2exp(ad, bd, precision="tf32"), tb.lm2exp(ad.transpose(1, 2).contiguous().transpose(1, 2), bd, precision="tf32")]
+    out, m = tb.lm2exp(ad, bd, precision="tf32", return_colmax=True)
+    assert torch.equal(m, out.amax(1))
+    outs += [out, tb.lm2exp(ad, bd, precision="tf32", b_colmax=bd.amax(1))]
+    tb.check_status()
+    for o in outs:
+        assert torch.equal(o.cpu() == float("-inf"), want == float("-inf"))
+        _assert_close(o.cpu(), a, b, "tf32", want)

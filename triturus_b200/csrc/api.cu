@@ -552,8 +552,9 @@ constexpr int64_t kLongContraction = 32768;
 // have_m: the caller supplies the stabiliser, so the tile is chosen as usual but no max pass of either kind runs.
 // b_km: b is stored with j contiguous; only the single-CTA kernel takes it, with the pre-pass stabiliser.
 // single_cta: an operand is fetched element by element, which only the single-CTA kernel does.
+// plain_ts: the TMEM-operand pair kernel in plain TF32 takes the call (a with j contiguous, no column maxima of the result).
 static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, Lm2expPlan* out,
-                       bool have_m = false, bool b_km = false, bool single_cta = false) {
+                       bool have_m = false, bool b_km = false, bool single_cta = false, bool plain_ts = true) {
   if (variant < 0) return TRITURUS_B200_EINVAL;
   // 0 = automatic, 1 = pre-pass, 2 = fused max pass, 3 = fused max pass over the first k-block only (optimistic),
   // 4 = pre-pass over the first 32 rows only (optimistic; pair tile 2564)
@@ -587,7 +588,16 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
     // and a long launch keep the fused form that is documented for them.
     const bool short_pair = precision == TRITURUS_B200_PRECISION_3XTF32 && stab_mode == 0 && J <= 1024 && (I > 128 || !big) &&
                             (K > 128 || tile_count(R, I, K, 128, I > 128 ? 2 : 1) <= sm_count());
-    const bool want_pair = !b_km && !single_cta && (wide_pair || short_pair);
+    // Plain TF32, more than one row block, on the TMEM-operand pair kernel: the single-CTA kernel carries both operands and the
+    // exponentials through shared memory.  us, single-CTA / pairs: R1 177x768x160 32 / 15, R3 959x704x224 31 / 17, R30 201x800x276 38 /
+    // 24, R117 160x44x1992 96 / 65, R2 256x288x6720 20.5 / 14.2, R48 236x248x1236 54 / 43, R22 218x256x3864 63 / 55.  Up to 64 K values
+    // of b per entry the one fused launch stays, which counts for callers that are bound by the host.  So it does for long
+    // launches of more than 128 terms, where the epilogue of a pair's tile is not hidden (R84 252x144x1496 63 / 64), and where
+    // the other half of a tile is padding (R98 198x64x120 12.6 / 14.6).
+    const bool ts_pair = precision == TRITURUS_B200_PRECISION_TF32 && plain_ts && stab_mode == 0 && I > 128 && J <= 4096 && !big &&
+                         J * K > 65536 && (J <= 128 || tile_count(R, I, K, 256, 2) <= sm_count() / 2 * 5) &&
+                         (K > 128 || tile_count(R, I, K, 128, 2) <= sm_count());
+    const bool want_pair = !b_km && !single_cta && (wide_pair || short_pair || ts_pair);
     // (long plain-TF32 contractions: 128 columns, so that the master copy fits beside the accumulator)
     // Plain TF32 on pairs: the TMEM-operand kernel, with the optimistic stabiliser unless a pre-pass was asked for.
     const int pair_variant = precision != TRITURUS_B200_PRECISION_TF32 || stab_mode == 4 ? 2564
@@ -775,17 +785,19 @@ static int direct_width(const float* base, int64_t n, int64_t inner, int64_t s0,
 
 // Does an automatic call of lm2exp run lm2exp_direct_kernel?  Estimates in us, of device time in a graph.  Direct: 3 and, per 32 x 32
 // tile, 5 ns and 0.034 per contraction value (more where shared memory leaves one or two blocks per SM, and with the third
-// product); else what one wave of the tcgen05 kernels takes (in 3xTF32 those of CTA pairs), or 2.5 times the single-CTA kernel's
-// where an operand is fetched element by element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 512^3 24.0 / 11.2, 1 x 1024x128x1024 11.7 / 11.4,
-// 16 x 256^3 15.8 / 17.0, 64 x 128x128x512 17.0 / 39.5; odd: 100 x 65x33x70 19.5 / 8.5, 64 x 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50.
-// 3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 / 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x
-// 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58.
-static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd) {
+// product); else what one wave of the tcgen05 kernels takes: those of CTA pairs where plan_lm2exp chooses them (`pairs`: the layouts
+// and outputs of the call allow it), or the single-CTA kernel's, 2.5 times that where an operand is fetched element by
+// element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 1024x128x1024 11.7 / 11.4, 16 x 256^3 15.8 /
+// 17.0, 64 x 128x128x512 17.0 / 39.5, 4 x 136x216x868 11.2 / 11.0, 4 x 168x456x776 13.8 / 24.6; odd: 100 x 65x33x70 19.5 / 8.5, 64 x
+// 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50.  3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 /
+// 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58.
+static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd, bool pairs) {
   if (J > 512 || R > 65535 || (I + 31) / 32 > 65535) return false;
   const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
   const double tiles = static_cast<double>(R) * ((I + 31) / 32) * ((K + 31) / 32);
   const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? 1.4 : 1.0) * (odd ? 1.3 : 1.0);
-  const double tcgen = x3 && !odd ? 14.0 + 0.014 * J : (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
+  const double single = (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
+  const double tcgen = odd || !pairs ? single : x3 ? 14.0 + 0.014 * J : I > 128 && J * K > 65536 ? std::min(single, 11.0 + 0.005 * J) : single;
   return direct <= tcgen;
 }
 
@@ -883,16 +895,17 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   const int64_t as_raw[3] = {as0, as1, as2}, bs_raw[3] = {bs0, bs1, bs2};
   bool a_mn, b_km;
   const bool gen_a = !lm2exp_a_layout(a, R, I, J, as0, as1, as2, a_mn), gen_b = !lm2exp_b_layout(b, R, J, K, bs0, bs1, bs2, b_km);
+  const bool prec_3x = precision == TRITURUS_B200_PRECISION_3XTF32, plain_ts = !a_mn && out_colmax == nullptr;
   // (the element-wise loader takes the place of the warps that fold the column maxima of the result)
   if ((gen_a || gen_b) && out_colmax != nullptr) return TRITURUS_B200_EALIGN;
-  if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b))
+  if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b, !b_km && (prec_3x || plain_ts)))
     return lm2exp_direct(a, b, out, R, I, J, K, a_strides, b_strides, out_strides, precision, b_colmax, out_colmax,
                          static_cast<cudaStream_t>(stream));
 
   Lm2expPlan plan;
   {
     // A supplied stabiliser makes every max pass redundant (and a fused max pass cannot be requested as well).
-    const int prc = plan_lm2exp(R, I, J, K, precision, variant, &plan, b_colmax != nullptr, b_km, gen_a || gen_b);
+    const int prc = plan_lm2exp(R, I, J, K, precision, variant, &plan, b_colmax != nullptr, b_km, gen_a || gen_b, plain_ts);
     if (prc != TRITURUS_B200_OK) return prc;
   }
   const int bn = plan.bn, mt = plan.mt;
@@ -917,7 +930,6 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   const bool prepass = !fused && b_colmax == nullptr;
   // The TMEM-operand pair kernels in plain TF32 take a with j contiguous only and do not fold column maxima of the
   // result; other calls run on the pair kernel that keeps the operand in shared memory.
-  const bool prec_3x = precision == TRITURUS_B200_PRECISION_3XTF32;
   const bool use_ts = (plan.tspair && !a_mn && out_colmax == nullptr) || (pair && prec_3x);
   const bool ts_halves = use_ts && !prec_3x && J <= 32 * LmTsPair::NS;
   const bool pair3x = use_ts && prec_3x && pair3x_wins(R, I, J, K);
@@ -1135,7 +1147,7 @@ int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, i
   int64_t as[3] = {a_strides[0], a_strides[1], a_strides[2]}, bs[3] = {b_strides[0], b_strides[1], b_strides[2]};
   bool mn, km;
   const bool odd = !lm2exp_a_layout(a, R, I, J, as[0], as[1], as[2], mn) | !lm2exp_b_layout(b, R, J, K, bs[0], bs[1], bs[2], km);
-  const bool small = direct_lm_wins(R, I, J, K, precision, odd);
+  const bool small = direct_lm_wins(R, I, J, K, precision, odd, !km && (!mn || precision == TRITURUS_B200_PRECISION_3XTF32));
   if (out == nullptr) return small ? 1 : 0;
   if (!small || out_strides == nullptr) return TRITURUS_B200_EINVAL;
   if ((reinterpret_cast<uintptr_t>(out) & 3) != 0 || (K > 1 && out_strides[2] != 1) || (I > 1 && out_strides[1] <= 0) ||
@@ -1148,7 +1160,7 @@ int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, i
 int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd) {
   if (R <= 0 || I <= 0 || J <= 0 || K <= 0) return TRITURUS_B200_EINVAL;
   if (precision != TRITURUS_B200_PRECISION_TF32 && precision != TRITURUS_B200_PRECISION_3XTF32) return TRITURUS_B200_EINVAL;
-  return variant == 0 && direct_lm_wins(R, I, J, K, precision, odd != 0) ? 1 : 0;
+  return variant == 0 && direct_lm_wins(R, I, J, K, precision, odd != 0, true) ? 1 : 0;
 }
 
 int triturus_b200_mm_f32(const float* a, const float* b, float* out, int64_t M, int64_t K, int64_t N,
@@ -1235,7 +1247,7 @@ int triturus_b200_lm2exp_chain_launches(int64_t R, int64_t I, int64_t J, int64_t
   if (precision != TRITURUS_B200_PRECISION_TF32 && precision != TRITURUS_B200_PRECISION_3XTF32)
     return TRITURUS_B200_EINVAL;
   Lm2expPlan plan;
-  const int rc = plan_lm2exp(R, I, J, K, precision, variant, &plan, have_b_colmax != 0);
+  const int rc = plan_lm2exp(R, I, J, K, precision, variant, &plan, have_b_colmax != 0, false, false, !want_out_colmax);
   if (rc != TRITURUS_B200_OK) return rc;
   if ((plan.optimistic || plan.optimistic_fused) && !want_out_colmax) return 2;  // as triturus_b200_lm2exp_launches
   if (plan.optimistic_prepass && !want_out_colmax) return 4;
