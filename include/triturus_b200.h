@@ -150,8 +150,8 @@ int triturus_b200_lm2exp_chain_f32(const float* a, const float* b, float* out, i
  *            additionally, TF32 only, the generated operand kept in tensor memory instead of shared memory:
  *            1283 / 1284 = tile of 128 columns x 128 / 256 rows, 1285 = 256 columns x 128 rows, which the
  *            automatic choice uses where it would otherwise take 2561; in 3xTF32 the codes 1281, 1282, 2561 and 2562
- *            all run the one kernel of that precision, 128 columns x 128 rows with the generated operand in tensor
- *            memory, and plans name it 1281)
+ *            all run the kernels of that precision, the generated operand in tensor memory on 128 columns x 128 rows of a CTA
+ *            or 256 x up to 192 of a pair, whichever is estimated to be faster, and plans name them 1281)
  *            and SPLIT the number of slices the contraction over (i, j) of every output tile is cut into, the
  *            counterpart of the reference's NUM_SPLITS and mode argument (triturus/lt2exp.py:533-541):
  *            0 = automatic (slices when the output tiles would occupy fewer than half the SMs; when the last
@@ -199,7 +199,7 @@ int triturus_b200_lt2exp_f32(const float* w, const float* a, const float* b, flo
  * allocates for its split kernel (triturus/lt2exp.py:555-562).  With it the shared last wave (SPLIT 9998, and the
  * automatic choice for a ragged last wave) needs one launch and no atomics: a CTA that works on a later part of
  * a tile's contraction parks its raw partial sums in the workspace, and the CTA that holds the tile's first
- * k-blocks adds them to its own and writes the finished results.  The order of those additions is fixed, so
+ * k-blocks (in 3xTF32 the one that parks last) adds them up and writes the finished results.  The order of those additions is fixed, so
  * the results do not depend on timing.  triturus_b200_lt2exp_f32 (no workspace) never chooses the shared last
  * wave by itself and, when asked for it, falls back to additions into the zero-filled result.
  *   A contraction cut into slices takes the column maxima of a and b from it: 2 * R * K floats that its first launch writes.
