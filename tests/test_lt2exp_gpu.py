@@ -531,3 +531,22 @@ def test_3xtf32_on_pair_tiles(shape, split):
     assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
     fin = torch.isfinite(want)
     assert ((got.double() - want).abs() <= _tol_3xtf32(w, a, b, want))[fin].all()
+
+
+def test_rows_beyond_the_products_of_32_bits():
+    """3.7 million rows on pair tiles: tile times unit counts pass 2^31 at 3.57 million (see tests/test_row_tiles.py).  Tolerance:
+    _tol_3xtf32."""
+    import triturus_b200 as tb
+
+    S, J, K = 3_700_001, 32, 256
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w = torch.rand(1, S, 1, J, generator=g, device="cuda") + 1e-3
+    a = torch.randn(1, 1, K, generator=g, device="cuda")
+    b = torch.randn(1, J, K, generator=g, device="cuda") * 4.0
+    got = tb.lt2exp(w, a, b, precision="3xtf32")
+    tb.check_status()
+    assert got.isfinite().all()
+    rows = torch.tensor([*range(70), *range(3_565_900, 3_566_200), *range(S - 70, S)])
+    got, w, a, b = got[:, rows.cuda()].cpu(), w[:, rows.cuda()].cpu(), a.cpu(), b.cpu()
+    want = orc.lt2exp_fp64(w, a, b)
+    assert ((got.double() - want).abs() <= _tol_3xtf32(w, a, b, want)).all()

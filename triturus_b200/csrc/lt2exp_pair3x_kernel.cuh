@@ -24,6 +24,7 @@
 
 #include "lm2exp_tspair_kernel.cuh"
 #include "lt2exp_tmem_kernel.cuh"
+#include "row_tiles.cuh"
 
 namespace tb200 {
 
@@ -123,9 +124,9 @@ lt2exp_pair3x_kernel(const __grid_constant__ CUtensorMap tmap_w, const Lt2expPar
     const int tn = rest % p.tiles_n;
     r = rest / p.tiles_n;
     n0 = tn * 2 * BN + static_cast<int>(rank) * BN;
-    const int lo = tm * units / p.tiles_m;
-    s0 = lo * 32;
-    rows = ((tm + 1) * units / p.tiles_m - lo) * 32;
+    const RowTile t = row_tile(units, p.tiles_m, tm);
+    s0 = t.first * 32;
+    rows = t.units * 32;
   };
   // The commit of k-block `it - back`.
   auto wait_kb = [&](uint32_t it, uint32_t back, int code, bool warp_wide) -> bool {
