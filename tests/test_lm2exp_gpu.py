@@ -945,3 +945,21 @@ def test_tf32_calls_of_several_row_blocks_run_on_pairs(shape):
     for o in outs:
         assert torch.equal(o.cpu() == float("-inf"), want == float("-inf"))
         _assert_close(o.cpu(), a, b, "tf32", want)
+
+
+def test_rows_beyond_the_products_of_32_bits():
+    """3.7 million rows as pair tiles taken round robin: tile times unit counts pass 2^31 at 3.57 million (see
+    tests/test_row_tiles.py).  Tolerance: _tol_3xtf32."""
+    import triturus_b200 as tb
+
+    I, J, K = 3_700_001, 320, 516
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.rand(1, I, J, generator=g, device="cuda")
+    b = torch.randn(1, J, K, generator=g, device="cuda") * 4.0
+    got = tb.lm2exp(a, b, precision="3xtf32")
+    tb.check_status()
+    assert got.isfinite().all()
+    rows = torch.tensor([*range(70), *range(3_565_900, 3_566_200), *range(I - 70, I)])
+    got, a, b = got[:, rows.cuda()].cpu(), a[:, rows.cuda()].cpu(), b.cpu()
+    want = orc.lm2exp_fp64(a, b)
+    assert ((got.double() - want).abs() <= _tol_3xtf32(a, b, want)).all()

@@ -36,6 +36,7 @@
 #pragma once
 
 #include "lm2exp_tspair_kernel.cuh"
+#include "row_tiles.cuh"
 
 namespace tb200 {
 
@@ -94,8 +95,9 @@ struct PairWalk {
       const int tm = tile % nt, rest = tile / nt;
       r = rest / p.tiles_n;
       n0 = (rest % p.tiles_n) * (2 * Lm2expPair3xCfg::BM);
-      lo = tm * p.tiles_m / nt;
-      take = (tm + 1) * p.tiles_m / nt - lo;
+      const RowTile t = row_tile(p.tiles_m, nt, tm);
+      lo = t.first;
+      take = t.units;
       u += npairs;
     }
     i0 = lo * 32;
