@@ -104,6 +104,27 @@ def test_lt2exp(shape, precision):
     tb.check_status()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
+def test_lt2exp_weights_whose_row_sums_overflow(precision):
+    """sum_j w exp(b - mb) of one i is beyond fp32, the result is not: the factor exp(a - ma) belongs to the terms.  Impossible and
+    unlikely states, on every i that a warp takes."""
+    import triturus_b200 as tb
+
+    R, S, I, J, K = 1, 40, 20, 12, 33
+    assert _native.LIB.triturus_b200_lt2exp_direct(R, S, I, J, K, int(precision == "3xtf32"), 0, 0) == 1
+    w = torch.full((R, S, I, J), 3e38)
+    w[:, :, ::5] = 1.0  # the states of these i are the likely ones
+    a = torch.full((R, I, K), float("-inf"))
+    a[:, 1::5] = -60.0
+    a[:, ::5] = 0.0
+    b = torch.zeros(R, J, K)
+    want = orc.lt2exp_fp64(w, a, b)
+    assert want.isfinite().all()
+    _check(tb.lt2exp(w.cuda(), a.cuda(), b.cuda(), precision=precision), want, TOL[precision])
+    tb.check_status()
+
+
 def test_which_calls_are_small():
     """Explicit variants run what they name, and the rules keep to sizes that the kernels can hold."""
     lm, lt = _native.LIB.triturus_b200_lm2exp_direct, _native.LIB.triturus_b200_lt2exp_direct

@@ -120,15 +120,18 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 }
 
 // acc (32 rows x 32 columns over the warp) += a[32 rows][8] * e[8][32 columns]; a, e at the first of the 8 contraction values.
-// Lane 4 g + t holds rows g + 8 y and, of each group n of eight columns, columns 2 t and 2 t + 1.
-template <int PREC>
-__device__ __forceinline__ void direct_mma_step(float (&acc)[2][4][4], const float* a, int pitch, const float* e, int g, int t) {
+// Lane 4 g + t holds rows g + 8 y and, of each group n of eight columns, columns 2 t and 2 t + 1; of e column g of each group.
+// SCALED: column g of group n of e is multiplied with scale[n] first.
+template <int PREC, bool SCALED = false>
+__device__ __forceinline__ void direct_mma_step(float (&acc)[2][4][4], const float* a, int pitch, const float* e, int g, int t,
+                                                const float* scale = nullptr) {
   uint32_t bh[4][2], bl[4][2];
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float v = e[(t + 4 * h) * DIRECT_PITCH + n * 8 + g];
+      float v = e[(t + 4 * h) * DIRECT_PITCH + n * 8 + g];
+      if (SCALED) v *= scale[n];
       if (PREC) {
         float hi, lo;
         tf32_split_rn(v, hi, lo);
@@ -268,9 +271,10 @@ __host__ __device__ constexpr int direct_lt_smem(int I, int J, int nbuf) {
   return (need > red ? need : red) * 4;
 }
 
-// lt2exp as sum_i exp(a_i - ma) * (sum_j w[s, i, j] exp(b_j - mb)): the inner sums are products with the same exp(b - mb)
-// for all i, no product of the two exps is formed, and the sum over i is in fp32.  A warp takes one i at a time and fetches its 32
-// rows of w itself, one i ahead.  The blocks of a cluster share the i of a tile; each adds up a part of the tile's rows through
+// lt2exp as sum_i (sum_j w[s, i, j] (exp(a_i - ma) exp(b_j - mb))): the inner sums on the tensor cores, the sum over i in
+// fp32.  (exp(a_i - ma) as a factor of the inner sum instead of its terms would spare a product per term, but large
+// weights overflow an inner sum that the factor, zero for an impossible state, takes back.)  A warp takes one i at a time and
+// fetches its 32 rows of w itself, one i ahead.  The blocks of a cluster share the i of a tile; each adds up a part of the tile's rows through
 // distributed shared memory, in rank order.  Grid: (parts * K / 32, S / 32, R), clusters of `parts`.
 template <int PREC>
 __global__ void __launch_bounds__(DIRECT_THREADS, 2) lt2exp_direct_kernel(const DirectLtParams p) {
@@ -310,18 +314,17 @@ __global__ void __launch_bounds__(DIRECT_THREADS, 2) lt2exp_direct_kernel(const 
     fetch(i + 8, buf ^ 1);
     cp_async_wait<1>();
     __syncwarp();
-    float sum[2][4][4] = {};
+    float sum[2][4][4] = {}, scale[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) scale[n] = ea[i * DIRECT_PITCH + n * 8 + g];
     const float* wb = wt + buf * 32 * pitch;
-    for (int s = 0; s < J8 / 8; ++s) direct_mma_step<PREC>(sum, wb + 8 * s, pitch, eb + 8 * s * DIRECT_PITCH, g, t);
+    for (int s = 0; s < J8 / 8; ++s) direct_mma_step<PREC, true>(sum, wb + 8 * s, pitch, eb + 8 * s * DIRECT_PITCH, g, t, scale);
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const float2 x = *reinterpret_cast<const float2*>(ea + i * DIRECT_PITCH + n * 8 + 2 * t);
+    for (int y = 0; y < 2; ++y) {
 #pragma unroll
-      for (int y = 0; y < 2; ++y) {
-        acc[y][n][0] = fmaf(x.x, sum[y][n][0], acc[y][n][0]);
-        acc[y][n][1] = fmaf(x.y, sum[y][n][1], acc[y][n][1]);
-        acc[y][n][2] = fmaf(x.x, sum[y][n][2], acc[y][n][2]);
-        acc[y][n][3] = fmaf(x.y, sum[y][n][3], acc[y][n][3]);
+      for (int n = 0; n < 4; ++n) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[y][n][x] += sum[y][n][x];
       }
     }
     __syncwarp();  // every lane has read the buffer that the next fetch overwrites
