@@ -125,6 +125,23 @@ def test_lt2exp_weights_whose_row_sums_overflow(precision):
     tb.check_status()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
+def test_largest_weights(precision):
+    """Weights between the largest tf32 value and the largest float, which rounding to nearest would make infinite."""
+    import triturus_b200 as tb
+
+    top = torch.finfo(torch.float32).max
+    a = torch.zeros(1, 3, 9)
+    a[0, 0, 0], a[0, 1, 5], a[0, 2, 3] = top, top * (1 - 2.0**-13), float("inf")
+    b = torch.zeros(1, 9, 33)
+    w, x, y = a.view(1, 3, 3, 3), torch.zeros(1, 3, 33), torch.zeros(1, 3, 33)
+    for got in (tb.lm2exp(a.cuda(), b.cuda(), precision=precision), tb.lt2exp(w.cuda(), x.cuda(), y.cuda(), precision=precision)):
+        _check(got[:, :2], orc.lm2exp_fp64(a, b)[:, :2], TOL[precision])
+        assert not got[:, 2].isfinite().any()  # infinity stays what it is (3xTF32: no number, its low part is none)
+    tb.check_status()
+
+
 def test_which_calls_are_small():
     """Explicit variants run what they name, and the rules keep to sizes that the kernels can hold."""
     lm, lt = _native.LIB.triturus_b200_lm2exp_direct, _native.LIB.triturus_b200_lt2exp_direct

@@ -119,6 +119,13 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
   return r;
 }
 
+// The same of a weight, which may be as large as a float: what rounding would make infinite becomes the largest tf32 value, while
+// infinity and NaN stay.  (Low bits are left in place, the tensor core ignores them; a negative weight is truncated.)
+__device__ __forceinline__ uint32_t to_tf32_weight(float x) {
+  const uint32_t b = __float_as_uint(x);
+  return max(__viaddmin_u32(b, 0x1000u, 0x7f7fffffu), b);
+}
+
 // acc (32 rows x 32 columns over the warp) += a[32 rows][8] * e[8][32 columns]; a, e at the first of the 8 contraction values.
 // Lane 4 g + t holds rows g + 8 y and, of each group n of eight columns, columns 2 t and 2 t + 1; of e column g of each group.
 // SCALED: column g of group n of e is multiplied with scale[n] first.
@@ -152,7 +159,7 @@ __device__ __forceinline__ void direct_mma_step(float (&acc)[2][4][4], const flo
         tf32_split_trunc(v, hi, lo);
         ah[x] = __float_as_uint(hi), al[x] = __float_as_uint(lo);
       } else {
-        ah[x] = to_tf32(v);
+        ah[x] = to_tf32_weight(v);
       }
     }
     if (PREC) {
