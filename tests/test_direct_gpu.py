@@ -205,3 +205,42 @@ def test_calls_that_the_extension_leaves_to_python():
     torch.cuda.synchronize()
     assert torch.equal(held, out) and torch.equal(held_lt, lt)
     tb.check_status()
+
+
+@pytest.mark.gpu
+def test_threads_run_while_a_launch_waits_for_the_queue():
+    """More calls than the queue of a stream holds, behind a kernel of about a second: while a call waits in its launch another
+    Python thread goes on."""
+    import threading
+    import time
+
+    import triturus_b200 as tb
+
+    a, b = torch.rand(2, 40, 24, device="cuda"), torch.randn(2, 24, 50, device="cuda")
+    w, x, y = torch.rand(2, 20, 6, 7, device="cuda"), torch.randn(2, 6, 50, device="cuda"), torch.randn(2, 7, 50, device="cuda")
+    for call in (lambda: _native.HOST.lm2exp(a, b, 1, 0), lambda: _native.HOST.lt2exp(w, x, y, 1, 0)):
+        assert call() is not None
+        torch.cuda.synchronize()
+        gaps, stop = [0.0], threading.Event()
+
+        def ticks():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(1e-3)
+                now = time.perf_counter()
+                gaps.append(now - last)
+                last = now
+
+        other = threading.Thread(target=ticks)
+        other.start()
+        torch.cuda._sleep(int(1.5e9))  # 0.75 s at 2 GHz, at most twice that
+        start = time.perf_counter()
+        for _ in range(3000):
+            call()
+        waited = time.perf_counter() - start
+        stop.set()
+        other.join()
+        torch.cuda.synchronize()
+        assert waited > 0.4, waited  # (the launches did wait, or the test says nothing)
+        assert max(gaps) < 0.5 * waited, (max(gaps), waited)
+    tb.check_status()

@@ -52,6 +52,11 @@ bool int_arg(PyObject* o, int* v) {
   return *v == x;
 }
 
+struct ThreadsRun {  // without the interpreter lock, for the time of a launch: it waits where the queue of the stream is full
+  PyThreadState* state = PyEval_SaveThread();
+  ~ThreadsRun() { PyEval_RestoreThread(state); }
+};
+
 PyObject* none() { Py_RETURN_NONE; }
 
 at::Tensor new_result(const at::Tensor& like, int64_t r, int64_t i, int64_t k) {
@@ -81,8 +86,13 @@ PyObject* lm2exp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const float* bp = b->const_data_ptr<float>();
   if (triturus_b200_lm2exp_small_f32(ap, bp, nullptr, R, I, J, K, as, bs, nullptr, precision, nullptr) != 1) return none();
   at::Tensor out = new_result(*a, R, I, K);
-  const int rc = triturus_b200_lm2exp_small_f32(ap, bp, out.mutable_data_ptr<float>(), R, I, J, K, as, bs, out.strides().data(), precision,
-                                                c10::cuda::getCurrentCUDAStream(a->get_device()).stream());
+  float* op = out.mutable_data_ptr<float>();
+  const auto stream = c10::cuda::getCurrentCUDAStream(a->get_device()).stream();
+  int rc;
+  {
+    ThreadsRun unlocked;
+    rc = triturus_b200_lm2exp_small_f32(ap, bp, op, R, I, J, K, as, bs, out.strides().data(), precision, stream);
+  }
   if (rc != TRITURUS_B200_OK) return failed("triturus_b200_lm2exp_small_f32", rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -107,9 +117,15 @@ PyObject* lt2exp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int odd = ws[3] != 1 || (bits & 1) != 0;
   if (triturus_b200_lt2exp_direct(R, S, I, J, K, precision, variant, odd) != 1) return none();
   at::Tensor out = new_result(*a, R, S, K);
-  const int rc = triturus_b200_lt2exp_direct_f32(wp, a->const_data_ptr<float>(), b->const_data_ptr<float>(), out.mutable_data_ptr<float>(), R,
-                                                 S, I, J, K, ws, a->strides().data(), b->strides().data(), out.strides().data(), precision,
-                                                 nullptr, nullptr, nullptr, c10::cuda::getCurrentCUDAStream(a->get_device()).stream());
+  const float *ap = a->const_data_ptr<float>(), *bp = b->const_data_ptr<float>();
+  float* op = out.mutable_data_ptr<float>();
+  const auto stream = c10::cuda::getCurrentCUDAStream(a->get_device()).stream();
+  int rc;
+  {
+    ThreadsRun unlocked;
+    rc = triturus_b200_lt2exp_direct_f32(wp, ap, bp, op, R, S, I, J, K, ws, a->strides().data(), b->strides().data(), out.strides().data(),
+                                         precision, nullptr, nullptr, nullptr, stream);
+  }
   if (rc != TRITURUS_B200_OK) return failed("triturus_b200_lt2exp_direct_f32", rc);
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
