@@ -351,3 +351,22 @@ def test_plans_over_random_shapes_are_consistent():
         else:
             assert n == (1 if split == 1 else 3), (R, S, I, J, K, prec, code, n)
         assert lt_plan(R, S, I, J, K, prec, code) == code, (R, S, I, J, K, prec, code)
+
+
+def _cannot_build(force=False):
+    raise RuntimeError("no C++ compiler found")
+
+
+def test_import_without_the_extension_for_small_calls(monkeypatch, tmp_path):
+    """No _host.so and nothing to build it with: a warning, and every call goes through ctypes."""
+    monkeypatch.setattr(tb_build, "HOST_PATH", tmp_path / "_host.so")
+    monkeypatch.setattr(tb_build, "build_host", _cannot_build)
+    with pytest.warns(RuntimeWarning, match="no C.. compiler found"):
+        host = _native._load_host()
+    a, b = torch.rand(2, 4, 5), torch.rand(2, 5, 6)
+    assert host.lm2exp(a, b, 1, 0) is None and host.lt2exp(a[..., None], b, b, 1, 0) is None
+    monkeypatch.setattr(_native, "HOST", host)
+    with pytest.raises(AssertionError):
+        triturus_b200.lm2exp(a, a)
+    with pytest.raises(_native.NativeLibraryError):  # (CPU tensors)
+        triturus_b200.lm2exp(a, b)

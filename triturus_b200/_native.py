@@ -7,6 +7,7 @@ CUDA device raises.
 
 import ctypes
 import os
+import warnings
 from ctypes import POINTER, c_char_p, c_int, c_int32, c_int64, c_size_t, c_void_p
 
 import torch
@@ -158,21 +159,32 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
 LIB = _load()
 
 
+class _NoHost:
+    """In the place of the extension module where there is none: no call is a small one to it, all go through ctypes."""
+
+    lm2exp = lt2exp = staticmethod(lambda *args: None)
+
+
 def _load_host():
     """The extension module that makes small calls of the library (csrc/host.cpp), built first where it is missing or stale;
-    like the library, an existing one is used as it is where it cannot be rebuilt."""
-    if _build.host_is_stale():
-        try:
-            _build.build_host()
-        except Exception as exc:  # noqa: BLE001
-            if not _build.HOST_PATH.exists():
-                raise NativeLibraryError(f"{_build.HOST_PATH} is missing and could not be built ({exc})") from exc
+    like the library, an existing one is used as it is where it cannot be rebuilt.  Without one (no C++ compiler, no headers)
+    everything works, small calls some 12 us slower each."""
     try:
-        from . import _host
-    except ImportError:
-        # built against another torch or interpreter: once more from its source
-        _build.build_host(force=True)
-        from . import _host
+        if _build.host_is_stale():
+            try:
+                _build.build_host()
+            except Exception:  # noqa: BLE001
+                if not _build.HOST_PATH.exists():
+                    raise
+        try:
+            from . import _host
+        except ImportError:
+            # built against another torch or interpreter: once more from its source
+            _build.build_host(force=True)
+            from . import _host
+    except Exception as exc:  # noqa: BLE001
+        warnings.warn(f"triturus_b200: no {_build.HOST_PATH.name} ({exc}); small calls are slower without it", RuntimeWarning, stacklevel=2)
+        return _NoHost
     _host.set_error_class(NativeLibraryError)
     return _host
 
