@@ -370,3 +370,13 @@ def test_import_without_the_extension_for_small_calls(monkeypatch, tmp_path):
         triturus_b200.lm2exp(a, a)
     with pytest.raises(_native.NativeLibraryError):  # (CPU tensors)
         triturus_b200.lm2exp(a, b)
+
+
+def test_an_extension_of_another_torch_is_not_loaded(monkeypatch):
+    """_host.so is there, but not of this torch, and cannot be rebuilt."""
+    assert tb_build.HOST_PATH.exists() and not tb_build.host_is_stale()
+    monkeypatch.setattr(torch, "__version__", "9.9.9")
+    assert tb_build.host_is_stale()
+    monkeypatch.setenv("CXX", "/nonexistent/c++")
+    with pytest.warns(RuntimeWarning, match="_host.so"):
+        assert _native._load_host() is _native._NoHost

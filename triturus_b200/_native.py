@@ -166,22 +166,13 @@ class _NoHost:
 
 
 def _load_host():
-    """The extension module that makes small calls of the library (csrc/host.cpp), built first where it is missing or stale;
-    like the library, an existing one is used as it is where it cannot be rebuilt.  Without one (no C++ compiler, no headers)
+    """The extension module that makes small calls of the library (csrc/host.cpp), built first where it is missing or stale.
+    Unlike the library, which is plain C, one that is stale is never loaded: it has the layout of torch's objects compiled in,
+    so that one built against another torch may load and read them wrongly.  Without one (no C++ compiler, no headers)
     everything works, small calls some 12 us slower each."""
     try:
-        if _build.host_is_stale():
-            try:
-                _build.build_host()
-            except Exception:  # noqa: BLE001
-                if not _build.HOST_PATH.exists():
-                    raise
-        try:
-            from . import _host
-        except ImportError:
-            # built against another torch or interpreter: once more from its source
-            _build.build_host(force=True)
-            from . import _host
+        _build.build_host()  # (nothing to do where it was built from these sources, for this torch and interpreter)
+        from . import _host
     except Exception as exc:  # noqa: BLE001
         warnings.warn(f"triturus_b200: no {_build.HOST_PATH.name} ({exc}); small calls are slower without it", RuntimeWarning, stacklevel=2)
         return _NoHost
