@@ -103,7 +103,8 @@ int triturus_b200_lm2exp_launches(int64_t R, int64_t I, int64_t J, int64_t K, in
  * runs: 1 when a call with these arguments does (`odd`: a or b cannot be described by a tensor map), else 0; negative on invalid arguments.
  * Results agree with the plan's kernels to rounding.  Such a call touches neither the workspace nor the status word. */
 int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd);
-/* Such a call, and nothing else: out == NULL asks whether the call with these operands is small (1) or not (0; out_strides may be
+/* Such a call, and nothing else: out == NULL asks whether the call with these operands is small (1, plus 2 if no tensor map describes
+ * a, plus 4 if none describes b: a padded copy may then be faster from some 1e9 operations on) or not (0; out_strides may be
  * NULL too), else it is launched; TRITURUS_B200_EINVAL when it is not small. */
 int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, int64_t R, int64_t I, int64_t J, int64_t K,
                                    const int64_t a_strides[3], const int64_t b_strides[3], const int64_t out_strides[3],

@@ -159,6 +159,20 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
 LIB = _load()
 
 
+# Problems up to this many FLOP take operands that break the tensor-map rules in place (the single-CTA kernel then
+# fetches them element by element, about three times slower per k-block than through TMA); larger ones get the padded copy.
+# Rows of consecutive floats, which triturus_b200_pad_rows_f32 copies: from the line on no form was faster in place.
+# Microseconds per call of a loop, in place / with the copies, both operands odd: R24 150x101x203 (1.5e8 FLOP) 40 / 46 in
+# 3xTF32 and 33 / 46 in TF32; R64 the same (3.9e8) 61 / 46 and 45 / 47; R8 255x255x1001 (1.0e9) 66 / 47 and 54 / 47, but
+# with an odd a alone in TF32 31 / 33; R4 511^3 (1.1e9) 117 / 48 and 93 / 47, an odd a alone 50 / 34; R2 1001^3 (4.0e9)
+# 219 / 75 and 174 / 60.  Below the line the host's work for the copies (two allocations and launches, 12 us or
+# more) can be what counts.
+_IN_PLACE_MAX_FLOP = 1.1e9
+# Other views, which torch would copy: R64 64x64x8192 with a transposed b of odd pitch (4.3e9) 374 / 447 in 3xTF32, R128
+# 256x256x8190 (1.4e11) 1 200 / 1 600 in TF32 but 2 970 / 2 320 in 3xTF32.
+_IN_PLACE_MAX_FLOP_STRIDED = 8e9
+
+
 class _NoHost:
     """In the place of the extension module where there is none: no call is a small one to it, all go through ctypes."""
 
@@ -176,7 +190,7 @@ def _load_host():
     except Exception as exc:  # noqa: BLE001
         warnings.warn(f"triturus_b200: no {_build.HOST_PATH.name} ({exc}); small calls are slower without it", RuntimeWarning, stacklevel=2)
         return _NoHost
-    _host.set_error_class(NativeLibraryError)
+    _host.set_up(NativeLibraryError, _IN_PLACE_MAX_FLOP, _IN_PLACE_MAX_FLOP_STRIDED)
     return _host
 
 
@@ -299,20 +313,6 @@ def _pad_rows(t: torch.Tensor, buf: torch.Tensor) -> bool:
         rc = LIB.triturus_b200_pad_rows_f32(t.data_ptr(), buf.data_ptr(), R, rows, shape[-1], s0, s1, _raw_stream(idx))
     _check(rc, "triturus_b200_pad_rows_f32")
     return True
-
-
-# Problems up to this many FLOP take operands that break the tensor-map rules in place (the single-CTA kernel then
-# fetches them element by element, about three times slower per k-block than through TMA); larger ones get the padded copy.
-# Rows of consecutive floats, which triturus_b200_pad_rows_f32 copies: from the line on no form was faster in place.
-# Microseconds per call of a loop, in place / with the copies, both operands odd: R24 150x101x203 (1.5e8 FLOP) 40 / 46 in
-# 3xTF32 and 33 / 46 in TF32; R64 the same (3.9e8) 61 / 46 and 45 / 47; R8 255x255x1001 (1.0e9) 66 / 47 and 54 / 47, but
-# with an odd a alone in TF32 31 / 33; R4 511^3 (1.1e9) 117 / 48 and 93 / 47, an odd a alone 50 / 34; R2 1001^3 (4.0e9)
-# 219 / 75 and 174 / 60.  Below the line the host's work for the copies (two allocations and launches, 12 us or
-# more) can be what counts.
-_IN_PLACE_MAX_FLOP = 1.1e9
-# Other views, which torch would copy: R64 64x64x8192 with a transposed b of odd pitch (4.3e9) 374 / 447 in 3xTF32, R128
-# 256x256x8190 (1.4e11) 1 200 / 1 600 in TF32 but 2 970 / 2 320 in 3xTF32.
-_IN_PLACE_MAX_FLOP_STRIDED = 8e9
 
 
 def _in_place_small(t: torch.Tensor, flop: float, variant: int, want_colmax: bool) -> bool:

@@ -789,13 +789,15 @@ static int direct_width(const float* base, int64_t n, int64_t inner, int64_t s0,
 // and outputs of the call allow it), or the single-CTA kernel's, 2.5 times that where an operand is fetched element by
 // element (`odd`).  tcgen05 / direct, TF32: 1 x 64^3 7.8 / 3.1, 8 x 128^3 11.5 / 3.5, 1 x 1024x128x1024 11.7 / 11.4, 16 x 256^3 15.8 /
 // 17.0, 64 x 128x128x512 17.0 / 39.5, 4 x 136x216x868 11.2 / 11.0, 4 x 168x456x776 13.8 / 24.6; odd: 100 x 65x33x70 19.5 / 8.5, 64 x
-// 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50.  3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 /
-// 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58.
+// 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50, 5 x 511^3 with every second column of b 70 / 67.  3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 /
+// 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58; with every second column of b 5 x 511^3 93 / 78, 3 x
+// 500x511x1000 90 / 93.  (A caller that can make padded copies of odd operands does better with those from 1e9 operations on: see
+// triturus_b200_lm2exp_small_f32.)
 static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd, bool pairs) {
   if (J > 512 || R > 65535 || (I + 31) / 32 > 65535) return false;
   const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
   const double tiles = static_cast<double>(R) * ((I + 31) / 32) * ((K + 31) / 32);
-  const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? 1.4 : 1.0) * (odd ? 1.3 : 1.0);
+  const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? (odd ? 1.7 : 1.4) : 1.0) * (odd ? 1.3 : 1.0);
   const double single = (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
   const double tcgen = odd || !pairs ? single : x3 ? 14.0 + 0.014 * J : I > 128 && J * K > 65536 ? std::min(single, 11.0 + 0.005 * J) : single;
   return direct <= tcgen;
@@ -1146,9 +1148,9 @@ int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, i
   if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 3) != 0) return TRITURUS_B200_EALIGN;
   int64_t as[3] = {a_strides[0], a_strides[1], a_strides[2]}, bs[3] = {b_strides[0], b_strides[1], b_strides[2]};
   bool mn, km;
-  const bool odd = !lm2exp_a_layout(a, R, I, J, as[0], as[1], as[2], mn) | !lm2exp_b_layout(b, R, J, K, bs[0], bs[1], bs[2], km);
-  const bool small = direct_lm_wins(R, I, J, K, precision, odd, !km && (!mn || precision == TRITURUS_B200_PRECISION_3XTF32));
-  if (out == nullptr) return small ? 1 : 0;
+  const bool odd_a = !lm2exp_a_layout(a, R, I, J, as[0], as[1], as[2], mn), odd_b = !lm2exp_b_layout(b, R, J, K, bs[0], bs[1], bs[2], km);
+  const bool small = direct_lm_wins(R, I, J, K, precision, odd_a || odd_b, !km && (!mn || precision == TRITURUS_B200_PRECISION_3XTF32));
+  if (out == nullptr) return small ? 1 + (odd_a ? 2 : 0) + (odd_b ? 4 : 0) : 0;
   if (!small || out_strides == nullptr) return TRITURUS_B200_EINVAL;
   if ((reinterpret_cast<uintptr_t>(out) & 3) != 0 || (K > 1 && out_strides[2] != 1) || (I > 1 && out_strides[1] <= 0) ||
       (R > 1 && out_strides[0] <= 0))

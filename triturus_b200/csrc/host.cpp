@@ -63,7 +63,10 @@ at::Tensor new_result(const at::Tensor& like, int64_t r, int64_t i, int64_t k) {
   return at::empty({r, i, k}, at::TensorOptions().dtype(at::kFloat).device(like.device()));
 }
 
-PyObject* error_class = nullptr;  // what the Python side raises for a code of the library
+// Set by the Python side.
+PyObject* error_class = nullptr;  // what it raises for a code of the library
+double copy_flop_rows = 0.0;      // problems of more operations than this get a padded copy of an operand that no tensor map
+double copy_flop_strided = 0.0;   // describes: of rows of consecutive floats, and of other views
 
 PyObject* failed(const char* what, int rc) {
   PyErr_Format(error_class != nullptr ? error_class : PyExc_RuntimeError, "%s failed with code %d: %s", what, rc, triturus_b200_strerror(rc));
@@ -84,7 +87,12 @@ PyObject* lm2exp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t* bs = b->strides().data();
   const float* ap = a->const_data_ptr<float>();
   const float* bp = b->const_data_ptr<float>();
-  if (triturus_b200_lm2exp_small_f32(ap, bp, nullptr, R, I, J, K, as, bs, nullptr, precision, nullptr) != 1) return none();
+  const int small = triturus_b200_lm2exp_small_f32(ap, bp, nullptr, R, I, J, K, as, bs, nullptr, precision, nullptr);
+  if (small <= 0) return none();
+  // (the copies are the Python side's; with them the call is one of the large kernels)
+  const double flop = 2.0 * static_cast<double>(R) * static_cast<double>(I) * static_cast<double>(J) * static_cast<double>(K);
+  if ((small & 2) != 0 && flop > (as[2] == 1 ? copy_flop_rows : copy_flop_strided)) return none();
+  if ((small & 4) != 0 && flop > (bs[2] == 1 ? copy_flop_rows : copy_flop_strided)) return none();
   at::Tensor out = new_result(*a, R, I, K);
   float* op = out.mutable_data_ptr<float>();
   const auto stream = c10::cuda::getCurrentCUDAStream(a->get_device()).stream();
@@ -131,14 +139,17 @@ PyObject* lt2exp(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-PyObject* set_error_class(PyObject*, PyObject* cls) {
+// set_up(error_class, copy_flop_rows, copy_flop_strided)
+PyObject* set_up(PyObject*, PyObject* args) {
+  PyObject* cls;
+  if (!PyArg_ParseTuple(args, "Odd", &cls, &copy_flop_rows, &copy_flop_strided)) return nullptr;
   Py_XDECREF(error_class);
   error_class = Py_NewRef(cls);
   Py_RETURN_NONE;
 }
 
 PyMethodDef methods[] = {
-    {"set_error_class", set_error_class, METH_O, "The exception class for error codes of the library."},
+    {"set_up", set_up, METH_VARARGS, "set_up(error_class, copy_flop_rows, copy_flop_strided)"},
     {"lm2exp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(lm2exp)), METH_FASTCALL, "lm2exp(a, b, precision, variant) -> Tensor or None"},
     {"lt2exp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(lt2exp)), METH_FASTCALL, "lt2exp(w, a, b, precision, variant) -> Tensor or None"},
     {nullptr, nullptr, 0, nullptr}};
