@@ -213,17 +213,17 @@ def test_odd_operands_of_larger_calls_are_copied(precision):
     """Above the line of operations where padded copies are faster the extension leaves a call with operands that no tensor map
     describes to Python, which makes them (R6 511^3 in 3xTF32: 43 us with them, 90 without); below it, and for views that
     torch would have to copy, it takes the call."""
-    for R, small in ((2, True), (5, False)):  # 5.3e8 and 1.3e9 operations
-        assert _native.LIB.triturus_b200_lm2exp_direct(R, 511, 511, 511, precision, 0, 1) == 1
-        a, b = torch.rand(R, 511, 511, device="cuda"), torch.randn(R, 511, 511, device="cuda")
-        a4, b4 = (torch.zeros(R, 511, 512, device="cuda")[..., :511] for _ in range(2))
+    I, J, K = 320, 301, 511
+    for R, small in ((4, True), (12, False)):  # 3.9e8 and 1.2e9 operations
+        assert _native.LIB.triturus_b200_lm2exp_direct(R, I, J, K, precision, 0, 1) == 1
+        a, b = torch.rand(R, I, J, device="cuda"), torch.randn(R, J, K, device="cuda")
+        a4, b4 = torch.zeros(R, I, J + 3, device="cuda")[..., :J], torch.zeros(R, J, K + 1, device="cuda")[..., :K]
         a4.copy_(a), b4.copy_(b)
-        want = _native.HOST.lm2exp(a, b, precision, 0)
-        assert (want is not None) == small
-        assert (_native.HOST.lm2exp(a, b4, precision, 0) is not None) == small and (_native.HOST.lm2exp(a4, b, precision, 0) is not None) == small
+        for x, y in ((a, b), (a, b4), (a4, b)):
+            assert (_native.HOST.lm2exp(x, y, precision, 0) is not None) == small
         out = _native._lm2exp_impl(a, b, precision, 0)
         assert torch.allclose(out, torch.log(torch.bmm(a.double(), b.double().exp())).float(), rtol=0, atol=2e-3)
-    wide = torch.randn(5, 511, 1022, device="cuda")[..., ::2]
+    wide = torch.randn(R, J, 2 * K, device="cuda")[..., ::2]
     assert _native.HOST.lm2exp(a4, wide, precision, 0) is not None
 
 
