@@ -792,12 +792,15 @@ static int direct_width(const float* base, int64_t n, int64_t inner, int64_t s0,
 // 150x101x203 43.2 / 26.5, 4 x 511^3 91 / 50, 5 x 511^3 with every second column of b 70 / 67.  3xTF32: 9 x 292x88x328 17.4 / 12.1, 20 x 40x260x404 16.9 / 13.4, 26 x 160x204x204 17.8 /
 // 18.6, 7 x 408x376x288 18.9 / 25.6; odd: 24 x 150x101x203 37.3 / 12.1, 4 x 511^3 114 / 58; with every second column of b 5 x 511^3 93 / 78, 3 x
 // 500x511x1000 90 / 93.  (A caller that can make padded copies of odd operands does better with those from 1e9 operations on: see
-// triturus_b200_lm2exp_small_f32.)
-static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd, bool pairs) {
+// triturus_b200_lm2exp_small_f32.)  Transposed views (a with i contiguous, b with j), which the tensor maps of the single-CTA kernel
+// take, a / b / both, TF32: 4 x 256^3 single-CTA 16.8 / 12.7 / 13.4, direct 8.0 / 7.7 / 9.1; 8 x 256^3 16.7 / 13.3 / 14.1, 13.8 / 13.7 /
+// 16.4; 12 x 256^3, a, 16.7, 19.0; 3xTF32 12 x 256^3, b / both, 21.3 / 21.5, 20.7 / 24.8.
+static bool direct_lm_wins(int64_t R, int64_t I, int64_t J, int64_t K, int precision, bool odd, bool pairs, bool a_mn = false, bool b_km = false) {
   if (J > 512 || R > 65535 || (I + 31) / 32 > 65535) return false;
   const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
   const double tiles = static_cast<double>(R) * ((I + 31) / 32) * ((K + 31) / 32);
-  const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? (odd ? 1.7 : 1.4) : 1.0) * (odd ? 1.3 : 1.0);
+  const double copies = (odd ? 1.3 : 1.0) * (a_mn ? 1.5 : 1.0) * (b_km ? 1.55 : 1.0);  // of 4 bytes
+  const double direct = 3.0 + tiles * (0.005 + 0.034e-3 * J) * (x3 ? 1.15 : 1.0) * (J > 320 ? (odd ? 1.7 : 1.4) : 1.0) * copies;
   const double single = (x3 ? 10.0 + 0.048 * J : 8.0 + 0.032 * J) * (odd ? 2.5 : 1.0);
   const double tcgen = odd || !pairs ? single : x3 ? 14.0 + 0.014 * J : I > 128 && J * K > 65536 ? std::min(single, 11.0 + 0.005 * J) : single;
   return direct <= tcgen;
@@ -900,7 +903,7 @@ static int lm2exp_run_block(const float* a, const float* b, float* out, int64_t 
   const bool prec_3x = precision == TRITURUS_B200_PRECISION_3XTF32, plain_ts = !a_mn && out_colmax == nullptr;
   // (the element-wise loader takes the place of the warps that fold the column maxima of the result)
   if ((gen_a || gen_b) && out_colmax != nullptr) return TRITURUS_B200_EALIGN;
-  if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b, !b_km && (prec_3x || plain_ts)))
+  if (variant == 0 && direct_lm_wins(R, I, J, K, precision, gen_a || gen_b, !b_km && (prec_3x || plain_ts), a_mn, b_km))
     return lm2exp_direct(a, b, out, R, I, J, K, a_strides, b_strides, out_strides, precision, b_colmax, out_colmax,
                          static_cast<cudaStream_t>(stream));
 
@@ -1149,7 +1152,7 @@ int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, i
   int64_t as[3] = {a_strides[0], a_strides[1], a_strides[2]}, bs[3] = {b_strides[0], b_strides[1], b_strides[2]};
   bool mn, km;
   const bool odd_a = !lm2exp_a_layout(a, R, I, J, as[0], as[1], as[2], mn), odd_b = !lm2exp_b_layout(b, R, J, K, bs[0], bs[1], bs[2], km);
-  const bool small = direct_lm_wins(R, I, J, K, precision, odd_a || odd_b, !km && (!mn || precision == TRITURUS_B200_PRECISION_3XTF32));
+  const bool small = direct_lm_wins(R, I, J, K, precision, odd_a || odd_b, !km && (!mn || precision == TRITURUS_B200_PRECISION_3XTF32), mn, km);
   if (out == nullptr) return small ? 1 + (odd_a ? 2 : 0) + (odd_b ? 4 : 0) : 0;
   if (!small || out_strides == nullptr) return TRITURUS_B200_EINVAL;
   if ((reinterpret_cast<uintptr_t>(out) & 3) != 0 || (K > 1 && out_strides[2] != 1) || (I > 1 && out_strides[1] <= 0) ||
