@@ -282,12 +282,14 @@ def _tma_ok(t: torch.Tensor) -> bool:
 
 def _tma_ready(t: torch.Tensor) -> torch.Tensor:
     """Return `t` or a padded copy that meets `_tma_ok`.  The logical shape is unchanged."""
-    if _tma_ok(t):
-        return t
-    inner = t.shape[-1]
-    padded = (inner + 3) // 4 * 4
-    buf = torch.empty(*t.shape[:-1], padded, dtype=t.dtype, device=t.device)
-    view = buf[..., :inner]
+    return t if _tma_ok(t) else _padded_copy(t)
+
+
+def _padded_copy(t: torch.Tensor) -> torch.Tensor:
+    shape = t.shape
+    inner = shape[-1]
+    buf = torch.empty((*shape[:-1], (inner + 3) // 4 * 4), dtype=t.dtype, device=t.device)
+    view = buf.narrow(-1, 0, inner)
     if not _pad_rows(t, buf):
         view.copy_(t)
     return view
@@ -296,18 +298,19 @@ def _tma_ready(t: torch.Tensor) -> torch.Tensor:
 def _pad_rows(t: torch.Tensor, buf: torch.Tensor) -> bool:
     """Fill `buf` with the rows of `t` through the library's own kernel, which streams rows of consecutive floats whatever
     their pitch and base; False where it does not apply (the caller then copies with torch)."""
-    if not t.is_cuda or t.dtype != torch.float32 or t.stride(-1) != 1 or t.data_ptr() % 4 or not 2 <= t.dim() <= 4:
-        return False
     shape, stride = t.shape, t.stride()
-    if t.dim() == 4:  # the two middle dimensions as one sequence of rows
+    ndim = len(shape)
+    if not 2 <= ndim <= 4 or stride[-1] != 1 or not t.is_cuda or t.dtype != torch.float32 or t.data_ptr() % 4:
+        return False
+    if ndim == 4:  # the two middle dimensions as one sequence of rows
         if shape[1] > 1 and stride[1] != shape[2] * stride[2]:
             return False
         R, rows, s0, s1 = shape[0], shape[1] * shape[2], stride[0], stride[2]
-    elif t.dim() == 3:
+    elif ndim == 3:
         R, rows, s0, s1 = shape[0], shape[1], stride[0], stride[1]
     else:
         R, rows, s0, s1 = 1, shape[0], 0, stride[0]
-    if buf.numel() == 0 or buf.numel() >= 1 << 33:
+    if not 0 < buf.numel() < 1 << 33:
         return False
     with _on_device(t.device) as idx:
         rc = LIB.triturus_b200_pad_rows_f32(t.data_ptr(), buf.data_ptr(), R, rows, shape[-1], s0, s1, _raw_stream(idx))
@@ -439,13 +442,12 @@ def _lm2exp_chain_impl(
         if b_colmax.shape != (R, K) or b_colmax.dtype != torch.float32 or b_colmax.device != b.device:
             raise ValueError(f"b_colmax must be a float32 [{R}, {K}] tensor on {b.device}")
         b_colmax = b_colmax.contiguous()
-        ws_ptr, ws_bytes, ws = None, 0, None
-    else:
-        ws_bytes = int(LIB.triturus_b200_lm2exp_workspace_bytes(R, I, J, K))
-        with _on_device(a.device):
-            ws = _lm2exp_workspace(a.device, ws_bytes)
-        ws_ptr = ws.data_ptr()
     with _on_device(a.device) as idx:
+        ws, ws_ptr, ws_bytes = None, None, 0  # (ws: held until the launch)
+        if b_colmax is None:
+            ws_bytes = int(LIB.triturus_b200_lm2exp_workspace_bytes(R, I, J, K))
+            ws = _lm2exp_workspace(a.device, ws_bytes)
+            ws_ptr = ws.data_ptr()
         rc = LIB.triturus_b200_lm2exp_chain_f32(
             a.data_ptr(), b.data_ptr(), out.data_ptr(), R, I, J, K,
             _i64(a.stride()), _i64(b.stride()), _i64(out.stride()),
@@ -461,7 +463,10 @@ def _lm2exp_chain_impl(
 def _lt2exp_direct_odd(w: torch.Tensor, K: int, precision: int, variant: int) -> bool:
     """True when a call with a w that breaks the tensor-map rules is small enough for the kernel that takes any strides."""
     R, S, I, J = w.shape
-    odd = (w.data_ptr() // 4 | J | w.stride(0) | w.stride(1) | w.stride(2)) & 1 != 0 or w.stride(3) != 1
+    if I > 128 or J > 128 or variant not in (0, 10000):
+        return False
+    s0, s1, s2, s3 = w.stride()
+    odd = (w.data_ptr() // 4 | J | s0 | s1 | s2) & 1 != 0 or s3 != 1
     return LIB.triturus_b200_lt2exp_direct(R, S, I, J, K, int(precision), int(variant), int(odd)) == 1
 
 
@@ -486,7 +491,7 @@ def _lt2exp_impl(w: torch.Tensor, a: torch.Tensor, b: torch.Tensor, precision: i
     if not _tma_ok(w):
         if _lt2exp_direct_odd(w, K, precision, variant):
             return _lt2exp_direct(w, a, b, None, None, None, precision)
-        w = _tma_ready(w)
+        w = _padded_copy(w)
     # a and b are read with ordinary loads and go in as they are, whatever their strides (16-byte loads when they
     # allow it; a view with a k stride other than 1 is read 4 bytes at a time, uncoalesced but without a copy)
     out = torch.empty((R, S, K), dtype=torch.float32, device=a.device)
@@ -546,7 +551,7 @@ def _lt2exp_chain_impl(
         if _lt2exp_direct_odd(w, K, precision, variant):
             out_colmax = torch.empty((R, K) if want_colmax else (0,), dtype=torch.float32, device=a.device)
             return _lt2exp_direct(w, a, b, a_colmax, b_colmax, out_colmax if want_colmax else None, precision), out_colmax
-        w = _tma_ready(w)
+        w = _padded_copy(w)
     out = torch.empty((R, S, K), dtype=torch.float32, device=a.device)
     out_colmax = torch.empty((R, K) if want_colmax else (0,), dtype=torch.float32, device=a.device)
     with _on_device(a.device) as idx:

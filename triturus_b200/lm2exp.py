@@ -34,9 +34,10 @@ def lm2exp(
         out = _native.HOST.lm2exp(a, b, precision_code(precision), variant)  # None: not an ordinary call of a small problem
         if out is not None:
             return out
-    assert len(a.shape) == len(b.shape) == 3
-    assert a.shape[0] == b.shape[0]
-    assert a.shape[2] == b.shape[1]
+    sa, sb = a.shape, b.shape
+    assert len(sa) == len(sb) == 3
+    assert sa[0] == sb[0]
+    assert sa[2] == sb[1]
     assert a.dtype == b.dtype == torch.float32
     assert a.device == b.device
     _native._require_cuda(a, b)

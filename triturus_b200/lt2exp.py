@@ -44,19 +44,21 @@ def lt2exp(
         out = _native.HOST.lt2exp(w, a, b, precision_code(precision), variant)
         if out is not None:
             return out
-    assert len(w.shape) == 4
-    assert len(a.shape) == len(b.shape) == 3
-    assert w.shape[0] == a.shape[0] == b.shape[0]
-    assert w.shape[2] == a.shape[1]
-    assert w.shape[3] == b.shape[1]
-    assert a.shape[2] == b.shape[2]
+    sw, sa, sb = w.shape, a.shape, b.shape
+    assert len(sw) == 4
+    assert len(sa) == len(sb) == 3
+    assert sw[0] == sa[0] == sb[0]
+    assert sw[2] == sa[1]
+    assert sw[3] == sb[1]
+    assert sa[2] == sb[2]
     assert w.dtype == a.dtype == b.dtype == torch.float32
     assert w.device == a.device == b.device
     if mode not in _MODES:
         raise ValueError(f"Uknown mode '{mode}' for the l2exp kernel")
     # The reference flattens the last two dimensions of w with .view (triturus/lt2exp.py:549), which
     # raises when they are not jointly contiguous; keep that contract.
-    w.view(w.shape[0], w.shape[1], -1)
+    if not w.is_contiguous():
+        w.view(sw[0], sw[1], -1)
     _native._require_cuda(w, a, b)
     prec = resolve_precision(precision)
     if w.numel() == 0 or a.numel() == 0 or b.numel() == 0:
