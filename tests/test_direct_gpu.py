@@ -151,6 +151,10 @@ def test_which_calls_are_small():
     assert lt(3, 75, 50, 50, 100, 1, 0, 1) == 1 and lt(3, 75, 50, 50, 100, 1, 10000, 1) == 1
     assert lt(3, 75, 50, 50, 100, 1, 99990000, 1) == 0 and lt(3, 75, 50, 50, 100, 1, 11281, 1) == 0
     assert lt(1, 256, 256, 256, 256, 1, 0, 0) == 0 and lt(1, 1, 128, 128, 1, 0, 0, 0) == 0
+    # several waves of blocks, one per SM, and contractions of few k-blocks: the tcgen05 kernels are faster
+    for shape, precision in (((4, 259, 112, 36, 44), 0), ((34, 2, 37, 60, 108), 1), ((64, 56, 4, 32, 148), 0), ((16, 97, 3, 4, 460), 0)):
+        assert lt(*shape, precision, 0, 0) == 0
+    assert lt(4, 259, 112, 36, 44, 0, 10000, 0) == 1  # (never split)
     for shape in ((1, 1, 129, 1, 1), (1, 1, 1, 129, 1)):
         assert lt(*shape, 0, 0, 0) == 0
 

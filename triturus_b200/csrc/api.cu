@@ -1652,13 +1652,45 @@ extern "C" size_t triturus_b200_lt2exp_workspace_bytes(int64_t R, int64_t S, int
 // such calls in TF32 and 29 - 35 in 3xTF32.  tcgen05 / direct, TF32: 1 x 32 32x32x64 19.9 / 5.7, 1 x 128 64x64x256 22.8 / 8.9, 16 x 32
 // 32x32x512 20.8 / 18.6, 8 x 128 32x32x512 22.2 / 27.0; 3xTF32: 1 x 64 64x64x128 29.8 / 7.7, 3 x 75 50x50x100 34.7 / 17.0, 16 x 32 32x32x512
 // 29.2 / 21.7, 8 x 128 32x32x512 32.6 / 35.1.
+//
+// That line is far from what runs where a launch is several waves of blocks, each with the columns of a and b to fetch and
+// exponentiate, or the contraction so short that the tcgen05 kernel has little to do.  Second estimate: a wave of blocks (one per SM where
+// the tiles of w are large) 4 and, per i of a warp, 1.4 and 0.18 per eight j; a wave of tcgen05 tiles 9.5 and 0.36 per k-block of a
+// slice, 5 for the launches of a split contraction, 3 for a padded copy of w.  Of 600 shapes around the line the first alone gives
+// 28 to the direct kernel that it is slower for, by 3.3 us on average, up to 2 times (4 x 259 112x36x44 36.8 / 18.7 in TF32, 34 x 2
+// 37x60x108 40 / 28.5 in 3xTF32, 64 x 56 4x32x148 17.4 / 10.9 in TF32); both 19, by 1.4.
+struct DirectLtShape {
+  int parts;  // blocks that share a tile's rows i: enough to fill the GPU, each with at least one row per warp
+  int nbuf;
+};
+static DirectLtShape direct_lt_shape(int64_t tiles, int64_t I) {
+  int parts = 1;
+  while (parts < 8 && tiles * parts < 2 * sm_count() && I > 8 * parts) parts *= 2;
+  return {parts, I > 8 * parts ? 2 : 1};
+}
+
 static bool direct_lt_wins(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant, bool odd) {
   if ((variant != 0 && variant != 10000) || R > 65535 || (S + 31) / 32 > 65535 || J > 128 || I > 128) return false;
   if (tb200::direct_lt_smem(static_cast<int>(I), static_cast<int>(J), 2) > 200 * 1024) return false;
   const bool x3 = precision == TRITURUS_B200_PRECISION_3XTF32;
-  const double tiles = std::max(static_cast<double>(R) * ((S + 31) / 32) * ((K + 31) / 32), 37.0);
-  const double terms = static_cast<double>(I) * ((J + 7) / 8 * 8);
-  return (4.0 + tiles * (0.012 + 0.035e-3 * terms * (odd ? 1.6 : 1.0))) * (x3 ? 1.25 : 1.0) <= (x3 ? 27.0 : 17.0);
+  const int64_t all = R * ((S + 31) / 32) * ((K + 31) / 32), steps = (J + 7) / 8;
+  const double tiles = std::max(static_cast<double>(all), 37.0);
+  const double terms = static_cast<double>(I * steps * 8);
+  if ((4.0 + tiles * (0.012 + 0.035e-3 * terms * (odd ? 1.6 : 1.0))) * (x3 ? 1.25 : 1.0) > (x3 ? 27.0 : 17.0)) return false;
+
+  const DirectLtShape sh = direct_lt_shape(all, I);
+  const int smem = tb200::direct_lt_smem(static_cast<int>(I), static_cast<int>(J), sh.nbuf) + 5 * 1024;  // (and the static arrays)
+  const double slots = static_cast<double>(sm_count()) * (2 * smem <= 227 * 1024 ? 2 : 1);
+  const double waves = std::max(static_cast<double>(all) * sh.parts / slots, 1.0);
+  const double rounds = static_cast<double>(((I + sh.parts - 1) / sh.parts + 7) / 8);
+  const double direct = x3 ? waves * (4.6 + rounds * (1.45 + (odd ? 0.42 : 0.30) * steps))
+                           : 1.0 + waves * (3.8 + rounds * (1.4 + (odd ? 0.22 : 0.175) * steps));
+  const int64_t kb = I * ((J + 31) / 32), nt = R * ((S + 127) / 128) * ((K + 127) / 128);
+  const int64_t slices = variant == 0 && 2 * nt <= sm_count() && kb >= 64 ? std::max<int64_t>(std::min(sm_count() / nt, kb / 4), 1) : 1;
+  const double slice = static_cast<double>((kb + slices - 1) / slices), tile_waves = std::max(static_cast<double>(nt) / sm_count(), 1.0);
+  const double tcgen = x3 ? (15.5 + 0.55 * slice) * tile_waves + (slices > 1 ? 6.0 : 0.0) + ((J & 3) != 0 ? 6.0 : 0.0)
+                          : (9.5 + 0.36 * slice) * tile_waves + (slices > 1 ? 5.0 : 0.0) + ((J & 3) != 0 ? 3.0 : 0.0);
+  return direct <= 1.1 * tcgen;
 }
 
 template <int PREC>
@@ -1694,12 +1726,9 @@ static int lt2exp_direct(const float* w, const float* a, const float* b, float* 
   p.width_w = direct_width(w, J, ws[3], ws[0], ws[1], ws[2]);
   p.width_a = direct_width(a, K, as[2], as[0], as[1]);
   p.width_b = direct_width(b, K, bs[2], bs[0], bs[1]);
-  // Blocks that share a tile's rows i: enough to fill the GPU, each with at least one row per warp.
-  const int64_t tiles = R * ((S + 31) / 32) * ((K + 31) / 32);
-  int parts = 1;
-  while (parts < 8 && tiles * parts < 2 * sm_count() && I > 8 * parts) parts *= 2;
-  p.parts = parts;
-  p.nbuf = I > 8 * parts ? 2 : 1;
+  const DirectLtShape sh = direct_lt_shape(R * ((S + 31) / 32) * ((K + 31) / 32), I);
+  p.parts = sh.parts;
+  p.nbuf = sh.nbuf;
   if (out_colmax != nullptr) {
     const int64_t blocks = (R * K + 255) / 256;
     fill_neg_inf_kernel<<<static_cast<int>(blocks < 1184 ? blocks : 1184), 256, 0, stream>>>(out_colmax, R * K);
