@@ -187,6 +187,9 @@ int triturus_b200_lt2exp_direct_f32(const float* w, const float* a, const float*
  * wave shared).  The counterpart of reading the reference's autotuner choice (triturus/lt2exp.py:9-75,78-222); negative
  * on invalid arguments. */
 int triturus_b200_lt2exp_plan(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant);
+/* Which kernel the tile code 1281 of a 3xTF32 call runs (the plan's, whatever triturus_b200_lt2exp_direct says): 1 = CTA pairs, 0 = CTAs on
+ * 128 x 128; negative on invalid arguments.  `workspace`: the call comes with the workspace of triturus_b200_lt2exp_ws_f32. */
+int triturus_b200_lt2exp_pairs(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int variant, int workspace);
 /* The same for triturus_b200_lm2exp_f32: STAB * 100000 + BN * 10 + MT with STAB = 1 (pre-pass), 2 (fused max
  * pass), 3 or 4 (their optimistic forms); the tile code 2567 stands by itself (its stabiliser is part of the
  * tile).  Negative on invalid arguments. */

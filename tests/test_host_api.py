@@ -2,6 +2,8 @@
 the reference's argument checks; nothing here launches a kernel."""
 
 import ctypes
+import math
+import random
 import re
 from pathlib import Path
 
@@ -380,3 +382,21 @@ def test_an_extension_of_another_torch_is_not_loaded(monkeypatch):
     monkeypatch.setenv("CXX", "/nonexistent/c++")
     with pytest.warns(RuntimeWarning, match="_host.so"):
         assert _native._load_host() is _native._NoHost
+
+
+def test_3xtf32_kernels_of_lt2exp():
+    """CTA pairs or 128 x 128 tiles: whole tiles are chosen as whole tiles where a call never splits or has no workspace to share a
+    last wave in, and a plan's own code runs the kernel of the plan."""
+    lib = _native.LIB
+    pairs = lib.triturus_b200_lt2exp_pairs
+    assert pairs(32, 256, 256, 256, 256, 0, 1) == 1 and pairs(90, 128, 128, 32, 128, 0, 1) == 0 and pairs(0, 1, 1, 1, 1, 0, 1) < 0
+    for shape in ((1, 334, 157, 24, 1574), (5, 173, 25, 135, 188)):  # unsplit: 93 us on 128 x 128, 124 on pairs; 83, 112
+        assert pairs(*shape, 0, 1) == 1 and pairs(*shape, 10000, 1) == 0
+    rng = random.Random(0)
+    park = 4096 + 148 * 2 * 128 * 128 * 4  # what the parts of a shared last wave of 128 x 128 tiles need
+    for _ in range(3000):
+        shape = tuple(round(math.exp(rng.uniform(0, math.log(x)))) for x in (128, 600, 256, 256, 4096))
+        code = lib.triturus_b200_lt2exp_plan(*shape, 1, 0)
+        ws = lib.triturus_b200_lt2exp_workspace_bytes(*shape, 1, 0)
+        assert lib.triturus_b200_lt2exp_plan(*shape, 1, code) == code and lib.triturus_b200_lt2exp_workspace_bytes(*shape, 1, code) == ws
+        assert pairs(*shape, 0, ws >= park) == pairs(*shape, code, ws >= park) == pairs(*shape, 0, 1)

@@ -1384,6 +1384,13 @@ struct LtCtas<Cfg, std::void_t<decltype(Cfg::CTAS)>> {
   static constexpr int value = Cfg::CTAS;
 };
 
+// Scratch memory for the end-to-end form: one parked tile per CTA behind the flags.  (3xTF32: every part parks, up to two per
+// tile of a last wave that fills more than half of the SMs.)
+template <class Cfg>
+static size_t lt2exp_park_bytes() {
+  return kParkHeader + static_cast<size_t>(sm_count() / LtCtas<Cfg>::value) * (Cfg::PREC ? 2 : 1) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
+}
+
 template <class Cfg, void (*Kern)(const CUtensorMap, const Lt2expParams), bool CAN_PARK>
 static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLaunch& L) {
   auto kern = Kern;
@@ -1399,9 +1406,7 @@ static int launch_lt2exp_with(const CUtensorMap& tw, Lt2expParams p, const LtLau
   p.num_tiles = static_cast<int>(nt);
   constexpr int CTAS = LtCtas<Cfg>::value;
   const int workers = sm_count() / CTAS;  // CTAs, or pairs of them
-  // Scratch memory for the end-to-end form: one parked tile per CTA behind the flags.
-  // (3xTF32: every part parks, up to two per tile of a last wave that fills more than half of the SMs.)
-  const size_t park_need = kParkHeader + static_cast<size_t>(workers) * (Cfg::PREC ? 2 : 1) * Cfg::MT * Cfg::BM * Cfg::BN * sizeof(float);
+  const size_t park_need = lt2exp_park_bytes<Cfg>();
   const bool have_ws = CAN_PARK && sm_count() * sizeof(int) * (Cfg::PREC ? 4 : 1) <= kParkHeader &&
                        (L.query != nullptr || (L.ws != nullptr && L.ws_bytes >= park_need &&
                                                (reinterpret_cast<uintptr_t>(L.ws) & 255) == 0));
@@ -1496,13 +1501,14 @@ using LtM_2 = Lt2expTmemCfg<2, 6>;
 using LtMX_1 = Lt2expTmemCfg<1, 4, 1>;  // 3xTF32, 128 x 128
 
 // Cycles of the busiest of `workers` CTAs (or pairs of them) over `nt` tiles in 3xTF32, as launch_lt2exp_with shares them out.  A
-// slice costs 39 000 besides its k-blocks, the launches before and after among them.
-static double lt2exp_busiest(int64_t nt, int I, int J, int workers, double per_kb, double per_item) {
+// slice costs 39 000 besides its k-blocks, the launches before and after among them.  whole: tiles are neither cut nor shared;
+// can_share: there is a workspace for a shared last wave.
+static double lt2exp_busiest(int64_t nt, int I, int J, int workers, double per_kb, double per_item, bool whole, bool can_share) {
   const int64_t kbt = static_cast<int64_t>((J + 31) / 32) * I, waves = (nt + workers - 1) / workers;
-  const int64_t nsplit = lt2exp_split(nt, I, J, 0, false, workers).nsplit;
+  const int64_t nsplit = whole ? 1 : lt2exp_split(nt, I, J, 0, false, workers).nsplit;
   if (nsplit > 1) return static_cast<double>((kbt + nsplit - 1) / nsplit) * per_kb + 39000.0;
   const double item = static_cast<double>(kbt) * per_kb + per_item;
-  if (!lt2exp_share_wins(nt, kbt, workers)) return static_cast<double>(waves) * item;
+  if (whole || !can_share || !lt2exp_share_wins(nt, kbt, workers)) return static_cast<double>(waves) * item;
   const LtShare sh = lt2exp_share(nt, kbt, workers);
   const int64_t longest = sh.parts > 0 ? kbt / sh.parts : sh.main;
   return static_cast<double>(waves - 1) * item + static_cast<double>(longest) * per_kb + per_item + 28000.0;
@@ -1514,14 +1520,21 @@ static double lt2exp_busiest(int64_t nt, int I, int J, int workers, double per_k
 // / pairs: R15 160x126x163x480 458 / 315, R148 192x8x32x256 76.3 / 50.3, R64 32x64x64x1024 262 / 211, R40 64x90x200x500 407 / 341, R32
 // 256^4 1 105 / 1 044, R1 256^4 65.9 / 59.3; and where pairs would have columns of padding or fill the GPU unevenly, R90
 // 128x128x32x128 92.3 / 130, R25 92x155x80x524 254 / 285, R2 384x128x128x384 62.3 / 67.4.
-static bool lt2exp_pair3x_wins(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K) {
+// Calls that never split, and calls without a workspace, are estimated as such (R1 334x157x24x1574 unsplit 93 / 124).  Such
+// an estimate only takes pairs back, and not where the free one is already of whole tiles: the code of a plan, which may say that
+// they are whole, or come with no more workspace than the plan wants, runs the kernel of the plan.
+static bool lt2exp_pair3x_wins(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, bool whole, bool can_share) {
   const int64_t units = (S + 31) / 32, row_tiles = (units + Lt2expPair3xCfg::UNITS - 1) / Lt2expPair3xCfg::UNITS;
   const double per_kb = std::max(192.0 * static_cast<double>((units + row_tiles - 1) / row_tiles), 700.0);
-  const double one = lt2exp_busiest(R * ((S + 127) / 128) * ((K + 127) / 128), static_cast<int>(I), static_cast<int>(J), sm_count(), 1000.0,
-                                    25000.0);
-  const double two = lt2exp_busiest(R * row_tiles * ((K + 255) / 256), static_cast<int>(I), static_cast<int>(J), sm_count() / 2, per_kb,
-                                    30000.0);
-  return two < 0.92 * one;
+  auto one = [&](bool w, bool s) {
+    return lt2exp_busiest(R * ((S + 127) / 128) * ((K + 127) / 128), static_cast<int>(I), static_cast<int>(J), sm_count(), 1000.0, 25000.0, w, s);
+  };
+  auto two = [&](bool w, bool s) {
+    return lt2exp_busiest(R * row_tiles * ((K + 255) / 256), static_cast<int>(I), static_cast<int>(J), sm_count() / 2, per_kb, 30000.0, w, s);
+  };
+  const double any = one(false, true);
+  if (two(false, true) >= 0.92 * any) return false;
+  return (!whole && can_share) || two(whole, can_share) < 0.92 * std::max(one(whole, can_share), any);
 }
 
 //                          BN   MT NS NTW
@@ -1542,7 +1555,8 @@ constexpr int kPair3xTile = 9;  // (`mt` of lt2exp_pair3x_kernel; plans name 3xT
 // *promote: plain TF32 over a contraction of more than kLongContraction terms on a tile whose accumulator
 // leaves room for a master copy in TMEM (the automatic choice is restricted to such tiles; an explicit
 // 256 x 256 tile or TMEM-operand variant is honoured and runs without the re-summation).
-static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int* bn,
+// can_share: the workspace of the call holds the tiles of a shared last wave.
+static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, bool can_share, int* bn,
                           int* mt, int* split, bool* promote) {
   if (variant < 0) return TRITURUS_B200_EINVAL;
   *split = variant / 10000;
@@ -1564,7 +1578,7 @@ static int lt2exp_variant(int variant, int precision, int64_t R, int64_t S, int6
   *bn = tile / 10;
   *mt = tile % 10;
   *promote = long_tf && (tile == 1281 || tile == 1282 || tile == 2561);
-  if (precision == TRITURUS_B200_PRECISION_3XTF32 && tile == 1281 && tb200::lt2exp_pair3x_wins(R, S, I, J, K)) {
+  if (precision == TRITURUS_B200_PRECISION_3XTF32 && tile == 1281 && tb200::lt2exp_pair3x_wins(R, S, I, J, K, *split == 1, can_share)) {
     *mt = kPair3xTile;
     return TRITURUS_B200_OK;
   }
@@ -1607,7 +1621,7 @@ static int lt2exp_query(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, i
   if (rc != TRITURUS_B200_OK) return rc;
   int bn, mt, split;
   bool promote;
-  rc = lt2exp_variant(variant, precision, R, S, I, J, K, &bn, &mt, &split, &promote);
+  rc = lt2exp_variant(variant, precision, R, S, I, J, K, true, &bn, &mt, &split, &promote);
   if (rc != TRITURUS_B200_OK) return rc;
   tb200::Lt2expParams p{};
   p.R = static_cast<int>(R);
@@ -1636,6 +1650,15 @@ extern "C" int triturus_b200_lt2exp_plan(int64_t R, int64_t S, int64_t I, int64_
   int tile = 0;
   const int rc = lt2exp_query(R, S, I, J, K, precision, variant, &q, &tile);
   return rc == TRITURUS_B200_OK ? q.split_code * 10000 + tile : rc;
+}
+
+extern "C" int triturus_b200_lt2exp_pairs(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int variant, int workspace) {
+  int bn, mt, split;
+  bool promote;
+  int rc = lt2exp_check_dims(R, S, I, J, K, TRITURUS_B200_PRECISION_3XTF32);
+  if (rc == TRITURUS_B200_OK)
+    rc = lt2exp_variant(variant, TRITURUS_B200_PRECISION_3XTF32, R, S, I, J, K, workspace != 0, &bn, &mt, &split, &promote);
+  return rc == TRITURUS_B200_OK ? mt == kPair3xTile : rc;
 }
 
 extern "C" size_t triturus_b200_lt2exp_workspace_bytes(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K,
@@ -1775,7 +1798,7 @@ static int lt2exp_run_block(const float* w, const float* a, const float* b, floa
   int bn, mt, split;
   bool promote;
   {
-    const int rc = lt2exp_variant(variant, precision, R, S, I, J, K, &bn, &mt, &split, &promote);
+    const int rc = lt2exp_variant(variant, precision, R, S, I, J, K, true, &bn, &mt, &split, &promote);
     if (rc != TRITURUS_B200_OK) return rc;
   }
 
