@@ -392,6 +392,8 @@ def test_3xtf32_kernels_of_lt2exp():
     assert pairs(32, 256, 256, 256, 256, 0, 1) == 1 and pairs(90, 128, 128, 32, 128, 0, 1) == 0 and pairs(0, 1, 1, 1, 1, 0, 1) < 0
     for shape in ((1, 334, 157, 24, 1574), (5, 173, 25, 135, 188)):  # unsplit: 93 us on 128 x 128, 124 on pairs; 83, 112
         assert pairs(*shape, 0, 1) == 1 and pairs(*shape, 10000, 1) == 0
+    # a last wave shared by many is not worth their parking: whole tiles (35 us, shared 43)
+    assert lib.triturus_b200_lt2exp_plan(14, 235, 39, 32, 67, 1, 0) == 11281 and lib.triturus_b200_lt2exp_plan(32, 256, 256, 256, 256, 1, 0) == 99981281
     rng = random.Random(0)
     park = 4096 + 148 * 2 * 128 * 128 * 4  # what the parts of a shared last wave of 128 x 128 tiles need
     for _ in range(3000):

@@ -1346,8 +1346,9 @@ static LtShare lt2exp_share(int64_t nt, int64_t kbt, int G) {
   return sh;
 }
 
-// 3xTF32: is sharing the last wave worth it?  By at least 3 % of the launch, counting the parking and adding up of a part as 28
-// k-blocks more than an item's own.  us, whole / shared: R10 128x128x128x2048 538 / 360, R40 64x90x200x500 669 / 409, R6
+// 3xTF32: is sharing the last wave worth it?  By at least 3 % of the launch, counting the parking and adding up of two parts as 28
+// k-blocks more than an item's own and of every further one as 3 (without those, 38 of 220 shapes that it chose to share were slower
+// than with whole tiles, R14 235x39x32x67 43 / 35; now 11, by 15 % at most).  us, whole / shared: R10 128x128x128x2048 538 / 360, R40 64x90x200x500 669 / 409, R6
 // 200x100x100x1000 225 / 178, R30 60x100x100x1000 420 / 365, R8 256x128x128x4096 1 136 / 1 068, R32 256^4 1 320 / 1 249; R90
 // 128x128x32x128 88.9 / 91.6 and R128 128x100x100x128 334 / 341, which the estimate leaves whole.
 static bool lt2exp_share_wins(int64_t nt, int64_t kbt, int G) {
@@ -1355,7 +1356,8 @@ static bool lt2exp_share_wins(int64_t nt, int64_t kbt, int G) {
   const LtShare sh = lt2exp_share(nt, kbt, G);
   if (waves > 8 || sh.parts == 1) return false;
   const int64_t longest = sh.parts > 0 ? kbt / sh.parts : sh.main;
-  return static_cast<double>((waves - 1) * item + longest + kItemBlocks + 28) < 0.97 * static_cast<double>(waves * item);
+  const int64_t more = std::max(sh.parts - 2, 0);
+  return static_cast<double>((waves - 1) * item + longest + kItemBlocks + 28 + 3 * more) < 0.97 * static_cast<double>(waves * item);
 }
 
 // What a launch function is asked to do: launch, or (query != nullptr) only report what it would launch.
