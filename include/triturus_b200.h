@@ -93,14 +93,16 @@ const char* triturus_b200_strerror(int code);
  * maximum in a first loop over j inside its kernel (triturus/lm2exp.py:124-127).
  */
 size_t triturus_b200_lm2exp_workspace_bytes(int64_t R, int64_t I, int64_t J, int64_t K);
-/* Number of kernels one triturus_b200_lm2exp_f32 call launches for these arguments on the current device:
+/* Number of kernels one triturus_b200_lm2exp_f32 call launches for these arguments on the current device, unless it is a small
+ * one (triturus_b200_lm2exp_direct, below: one kernel):
  * 2 (stabiliser pre-pass + contraction; or an optimistic kernel + its conditional launch), 1 (fused max pass) or
  * 4 (optimistic 32-row pre-pass, contraction, and two conditional launches; a with j contiguous and a full-size
  * workspace assumed); negative on invalid arguments.  The reference has no counterpart (its launch count is Triton's business, triturus/lm2exp.py:186-205). */
 int triturus_b200_lm2exp_launches(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant);
 /* Small calls.  An automatic call (variant 0) whose time would be latency runs one launch of lm2exp_direct_kernel (mma.sync
  * on 32 x 32 tiles) instead of the plan that triturus_b200_lm2exp_plan and _launches name, which an explicit variant still
- * runs: 1 when a call with these arguments does (`odd`: a or b cannot be described by a tensor map), else 0; negative on invalid arguments.
+ * runs: 1 when a call with these arguments does (`odd`: a or b cannot be described by a tensor map; else a with j and b with k
+ * contiguous), else 0; negative on invalid arguments.  With out_colmax a fill launch comes before it.
  * Results agree with the plan's kernels to rounding.  Such a call touches neither the workspace nor the status word. */
 int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd);
 /* Such a call, and nothing else: out == NULL asks whether the call with these operands is small (1, plus 2 if no tensor map describes
@@ -168,32 +170,35 @@ int triturus_b200_lm2exp_chain_f32(const float* a, const float* b, float* out, i
  *            and the in-place log pass.  Unsplit results are deterministic.
  *   No workspace is needed.
  */
-/* Number of kernels one triturus_b200_lt2exp_f32 call launches for these arguments on the current device
- * (1, or 3 when the contraction is split); negative on invalid arguments. */
+/* Number of kernels one triturus_b200_lt2exp_f32 call launches for these arguments on the current device, unless it is a small one
+ * (triturus_b200_lt2exp_direct, below: one kernel): 1, or 3 when the contraction is split; negative on invalid arguments. */
 int triturus_b200_lt2exp_launches(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant);
 /* Small calls, as for lm2exp: 1 when an automatic or unsplit call (variant 0 or 10000) with these arguments runs one launch of
  * lt2exp_direct_kernel instead of its plan (`odd_w`: the rows of w can only be fetched 4 bytes at a time: J odd, or strides or base odd).
  * Deterministic, also where the plan would split the contraction. */
 int triturus_b200_lt2exp_direct(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd_w);
 /* That kernel by itself, for w of any strides as well: the other entry points want w to meet the tensor-map rules.
- * I and J at most 128 each and (I + J) * 160 + J * 2048 bytes of shared memory within 200 KB (TRITURUS_B200_EINVAL else).
+ * I and J at most 128 each and, with J rounded up to a multiple of 8, (I + J) * 160 + J * 2048 + 8192 bytes of shared memory within
+ * 200 KB (TRITURUS_B200_EINVAL else).
  * a_colmax, b_colmax, out_colmax as in triturus_b200_lt2exp_chain_f32 (all may be NULL). */
 int triturus_b200_lt2exp_direct_f32(const float* w, const float* a, const float* b, float* out, int64_t R, int64_t S, int64_t I,
                                     int64_t J, int64_t K, const int64_t w_strides[4], const int64_t a_strides[3],
                                     const int64_t b_strides[3], const int64_t out_strides[3], int precision, const float* a_colmax,
                                     const float* b_colmax, float* out_colmax, void* stream);
-/* What a triturus_b200_lt2exp_f32 call with these arguments runs on the current device, as the explicit variant
- * code that pins it: SPLIT * 10000 + BN * 10 + MT with SPLIT = 1 (whole tiles), the slice count, or 9998 (last
+/* What a triturus_b200_lt2exp_f32 call with these arguments runs on the current device, unless it is a small one, as the explicit
+ * variant code that pins it: SPLIT * 10000 + BN * 10 + MT with SPLIT = 1 (whole tiles), the slice count, or 9998 (last
  * wave shared).  The counterpart of reading the reference's autotuner choice (triturus/lt2exp.py:9-75,78-222); negative
  * on invalid arguments. */
 int triturus_b200_lt2exp_plan(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int precision, int variant);
-/* Which kernel the tile code 1281 of a 3xTF32 call runs (the plan's, whatever triturus_b200_lt2exp_direct says): 1 = CTA pairs, 0 = CTAs on
- * 128 x 128; negative on invalid arguments.  `workspace`: the call comes with the workspace of triturus_b200_lt2exp_ws_f32. */
-int triturus_b200_lt2exp_pairs(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int variant, int workspace);
 /* The same for triturus_b200_lm2exp_f32: STAB * 100000 + BN * 10 + MT with STAB = 1 (pre-pass), 2 (fused max
  * pass), 3 or 4 (their optimistic forms); the tile code 2567 stands by itself (its stabiliser is part of the
  * tile).  Negative on invalid arguments. */
 int triturus_b200_lm2exp_plan(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant);
+/* Which kernel the tile code 1281 of a 3xTF32 call runs (the plan's, whatever triturus_b200_lt2exp_direct says): 1 = CTA pairs, 0 = CTAs on
+ * 128 x 128; negative on invalid arguments.  `workspace`: the call comes with the workspace of triturus_b200_lt2exp_ws_f32. */
+int triturus_b200_lt2exp_pairs(int64_t R, int64_t S, int64_t I, int64_t J, int64_t K, int variant, int workspace);
+/* Rows of the tiles that the pair code 2564 of a 3xTF32 call runs on: 192 (two accumulators) or 256 (one); negative on invalid arguments. */
+int triturus_b200_lm2exp_pair_rows(int64_t R, int64_t I, int64_t J, int64_t K);
 int triturus_b200_lt2exp_f32(const float* w, const float* a, const float* b, float* out, int64_t R, int64_t S,
                              int64_t I, int64_t J, int64_t K, const int64_t w_strides[4], const int64_t a_strides[3],
                              const int64_t b_strides[3], const int64_t out_strides[3], int precision, int variant,

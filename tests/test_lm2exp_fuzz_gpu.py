@@ -83,9 +83,10 @@ def test_random_views_are_read_without_error(seed):
         bv, b = bv * 4.0, b * 4.0
         want = orc.lm2exp_fp64(a, b)
         for precision in ("tf32", "3xtf32"):
-            got = tb.lm2exp(av, bv, precision=precision)
-            tb.check_status()
-            res = orc.compare_logspace(got.cpu(), want, ATOL[precision])
-            if not res["ok"]:
-                failures.append(((R, I, J, K), ka, kb, precision, res))
+            for variant in (0, 1281):  # (many of these are small calls; 1281: the single-CTA kernel, which larger ones run)
+                got = tb.lm2exp(av, bv, precision=precision, variant=variant)
+                tb.check_status()
+                res = orc.compare_logspace(got.cpu(), want, ATOL[precision])
+                if not res["ok"]:
+                    failures.append(((R, I, J, K), ka, kb, precision, variant, res))
     assert not failures, failures[:3]

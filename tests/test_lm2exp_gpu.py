@@ -611,7 +611,7 @@ def test_operands_that_break_the_tensor_map_rules_are_read_in_place(shape, preci
 def test_strided_and_broadcast_views_in_place(precision):
     """Every third row and every second column of a, every second column of b, a b broadcast over the batch
     (stride 0) and a base that is only 4-byte aligned: through the wrapper, which for problems of this size makes
-    no copy, and through the C ABI; a pair tile asked for with such operands is refused by the C ABI."""
+    no copy, and through the C ABI, on the direct kernel and on the single-CTA one; a pair tile asked for with such operands is refused by the C ABI."""
     import triturus_b200 as tb
     from triturus_b200 import _native
 
@@ -630,6 +630,11 @@ def test_strided_and_broadcast_views_in_place(precision):
     assert rc == 0
     tb.check_status()
     _assert_close(got.cpu(), a_v.cpu().contiguous(), b_b.cpu().contiguous(), precision)
+    # (calls of this size run the direct kernel; larger ones the element-wise loader of the single-CTA kernel)
+    for b_x in (b_v, b_b):
+        got = tb.lm2exp(a_v, b_x, precision=precision, variant=1281)
+        tb.check_status()
+        _assert_close(got.cpu(), a_v.cpu().contiguous(), b_x.cpu().contiguous(), precision)
     rc, _ = _raw_lm2exp(a_v, b_v, "tf32", 2564)
     assert rc == -1  # TRITURUS_B200_EINVAL
     # a large problem with an odd extent still gets the padded copy from the wrapper (faster there)
@@ -853,8 +858,10 @@ def test_3xtf32_pair_tiles_with_two_accumulators(shape, variant):
     padding): at the edges of its tiles, row units and shares, for both layouts of a, with impossible states, and with the
     column maxima of the result."""
     import triturus_b200 as tb
+    from triturus_b200 import _native
 
     R, I, J, K = shape
+    assert _native.LIB.triturus_b200_lm2exp_pair_rows(*shape) == 192
     g = torch.Generator().manual_seed(sum(shape))
     a = torch.rand(R, I, J, generator=g)
     b = torch.randn(R, J, K, generator=g) * 4.0 + 100.0 * torch.randn(R, 1, K, generator=g)

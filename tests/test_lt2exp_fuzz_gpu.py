@@ -1,5 +1,5 @@
 """GPU: lt2exp on random shapes with a and b given as random views (transposed, strided, shifted by one element,
-broadcast over the batch), all three modes, against the float64 oracle."""
+broadcast over the batch), all three modes and whole tiles, against the float64 oracle."""
 
 import random
 
@@ -29,10 +29,11 @@ def test_random_shapes_and_views(seed):
         av, a, bv, b = av * 3.0, a * 3.0, bv * 3.0, b * 3.0
         want = orc.lt2exp_fp64(w, a, b)
         for precision in ("tf32", "3xtf32"):
-            for mode in ("auto", "unsplit", "split"):
-                got = tb.lt2exp(w.cuda(), av, bv, mode=mode, precision=precision)
+            # (automatic and unsplit calls that are small run the direct kernel; 11281 whole tiles of the tcgen05 kernels)
+            for mode, variant in (("auto", 0), ("unsplit", 0), ("split", 0), ("auto", 11281)):
+                got = tb.lt2exp(w.cuda(), av, bv, mode=mode, precision=precision, variant=variant)
                 tb.check_status()
                 res = orc.compare_logspace(got.cpu(), want, ATOL[precision])
                 if not res["ok"]:
-                    failures.append(((R, S, I, J, K), ka, kb, precision, mode, res))
+                    failures.append(((R, S, I, J, K), ka, kb, precision, mode, variant, res))
     assert not failures, failures[:3]

@@ -505,16 +505,20 @@ def test_3xtf32_sums_of_one_term(I, J, variant):
     ((80, 190, 2, 20, 256), 1),     # a second tile for a few pairs, two k-blocks each
     ((1, 385, 128, 64, 512), 0),    # tiles of four, four and five row units; slices that begin and end inside a row of k-blocks
     ((1, 385, 128, 64, 512), 7),
-    ((1, 64, 60, 70, 1000), 9998),  # parts of four column tiles, parked and added up; the last tile has 24 columns in its second half
+    ((3, 64, 60, 70, 904), 9998),   # parts of twelve tiles, parked and added up; the last of an entry has 8 columns in its second half
     ((40, 60, 50, 50, 512), 0),     # a last wave of few tiles: equal parts
     ((60, 60, 100, 100, 512), 0),   # ... of more: mains and tails
 ], ids=str)  # fmt: skip
 def test_3xtf32_on_pair_tiles(shape, split):
     """Shapes that the 3xTF32 kernel of CTA pairs takes (tiles of 256 columns and up to six units of 32 rows), at the edges of its
-    tiles and work items, with impossible states and the column maxima of the result.  Tolerance: _tol_3xtf32."""
+    tiles and work items, with impossible states; with the workspace that parked parts need, and with the column maxima of the
+    result (a chain, which has none: parts are added into the result).  Tolerance: _tol_3xtf32."""
     import triturus_b200 as tb
+    from triturus_b200 import _native
 
     R, S, I, J, K = shape
+    for workspace in (0, 1):
+        assert _native.LIB.triturus_b200_lt2exp_pairs(*shape, split * 10000 + 1281, workspace) == 1
     g = torch.Generator().manual_seed(sum(shape))
     w = torch.rand(R, S, I, J, generator=g) + 1e-3
     a = torch.randn(R, I, K, generator=g) * 4.0 + 50.0 * torch.randn(R, 1, K, generator=g)
@@ -522,15 +526,17 @@ def test_3xtf32_on_pair_tiles(shape, split):
     a[torch.rand(R, I, K, generator=g) < 0.02] = float("-inf")
     b[0, :, K // 2] = float("-inf")
     variant = split * 10000 + 1281
+    out = tb.lt2exp(w.cuda(), a.cuda(), b.cuda(), precision="3xtf32", variant=variant)
     got, m = tb.lt2exp(w.cuda(), a.cuda(), b.cuda(), precision="3xtf32", variant=variant, return_colmax=True)
     tb.check_status()
     assert torch.equal(m, got.amax(1))
     some = sorted({0, R // 2, R - 1})
-    got, w, a, b = got[some].cpu(), w[some], a[some], b[some]
+    out, got, w, a, b = out[some].cpu(), got[some].cpu(), w[some], a[some], b[some]
     want = orc.lt2exp_fp64(w, a, b, chunk=1)
-    assert torch.equal(got == float("-inf"), want == float("-inf")) and not torch.isnan(got).any()
     fin = torch.isfinite(want)
-    assert ((got.double() - want).abs() <= _tol_3xtf32(w, a, b, want))[fin].all()
+    for o in (out, got):
+        assert torch.equal(o == float("-inf"), want == float("-inf")) and not torch.isnan(o).any()
+        assert ((o.double() - want).abs() <= _tol_3xtf32(w, a, b, want))[fin].all()
 
 
 def test_rows_beyond_the_products_of_32_bits():

@@ -25,6 +25,7 @@ EXPORTED_SYMBOLS = (
     "triturus_b200_lt2exp_launches",
     "triturus_b200_lt2exp_plan",
     "triturus_b200_lt2exp_pairs",
+    "triturus_b200_lm2exp_pair_rows",
     "triturus_b200_lm2exp_direct",
     "triturus_b200_lm2exp_small_f32",
     "triturus_b200_lt2exp_direct",
@@ -100,6 +101,8 @@ def _bind(lib: ctypes.CDLL) -> ctypes.CDLL:
     lib.triturus_b200_lt2exp_plan.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int]
     lib.triturus_b200_lt2exp_pairs.restype = c_int
     lib.triturus_b200_lt2exp_pairs.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int64, c_int, c_int]
+    lib.triturus_b200_lm2exp_pair_rows.restype = c_int
+    lib.triturus_b200_lm2exp_pair_rows.argtypes = [c_int64] * 4
     lib.triturus_b200_lm2exp_direct.restype = c_int
     lib.triturus_b200_lm2exp_direct.argtypes = [c_int64, c_int64, c_int64, c_int64, c_int, c_int, c_int]
     lib.triturus_b200_lt2exp_direct.restype = c_int

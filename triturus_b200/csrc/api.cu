@@ -1162,6 +1162,11 @@ int triturus_b200_lm2exp_small_f32(const float* a, const float* b, float* out, i
                        static_cast<cudaStream_t>(stream));
 }
 
+int triturus_b200_lm2exp_pair_rows(int64_t R, int64_t I, int64_t J, int64_t K) {
+  if (R <= 0 || I <= 0 || J <= 0 || K <= 0) return TRITURUS_B200_EINVAL;
+  return pair3x_wins(R, I, J, K) ? Lm2expPair3xCfg::BN : 256;
+}
+
 int triturus_b200_lm2exp_direct(int64_t R, int64_t I, int64_t J, int64_t K, int precision, int variant, int odd) {
   if (R <= 0 || I <= 0 || J <= 0 || K <= 0) return TRITURUS_B200_EINVAL;
   if (precision != TRITURUS_B200_PRECISION_TF32 && precision != TRITURUS_B200_PRECISION_3XTF32) return TRITURUS_B200_EINVAL;
