@@ -74,14 +74,29 @@ def workload_string(wl, custom: bool = False) -> str:
     return f"{wl.name}{' (custom dims)' if custom else ''}: {wl.op} fp32 {wl.dims}"
 
 
-def launches_per_step(wl, precision: str, variant: int, chain: bool = False) -> int:
-    """Kernels of this library launched per step, asked from the library: lm2exp is the contraction kernel
-    plus, unless the max pass is fused into it, the stabiliser pre-pass; lt2exp is one kernel, or three
-    (zero-fill, contraction, log pass) when the contraction is split over the SMs."""
+def runs_direct(wl, precision: str, variant: int) -> bool:
+    """Whether a step is a small call, which one launch of the direct kernel does instead of the plan."""
     from triturus_b200 import _native
 
     d = wl.dims
     prec = 0 if precision == "tf32" else 1
+    if wl.op == "lt2exp":
+        return _native.LIB.triturus_b200_lt2exp_direct(d["R"], d["S"], d["I"], d["J"], d["K"], prec, variant, d["J"] % 2) == 1
+    odd = int(d["J"] % 4 != 0 or d["K"] % 4 != 0)
+    return _native.LIB.triturus_b200_lm2exp_direct(d["R"], d["I"], d["J"], d["K"], prec, variant, odd) == 1
+
+
+def launches_per_step(wl, precision: str, variant: int, chain: bool = False) -> int:
+    """Kernels of this library launched per step, asked from the library: lm2exp is the contraction kernel
+    plus, unless the max pass is fused into it, the stabiliser pre-pass; lt2exp is one kernel, or three
+    (zero-fill, contraction, log pass) when the contraction is split over the SMs.  A small call is one, and a fill
+    of the column maxima where they are returned."""
+    from triturus_b200 import _native
+
+    d = wl.dims
+    prec = 0 if precision == "tf32" else 1
+    if runs_direct(wl, precision, variant):
+        return 2 if chain else 1
     if wl.op == "lt2exp":
         n = _native.LIB.triturus_b200_lt2exp_launches(d["R"], d["S"], d["I"], d["J"], d["K"], prec, variant)
     elif chain:
@@ -93,12 +108,15 @@ def launches_per_step(wl, precision: str, variant: int, chain: bool = False) -> 
     return int(n)
 
 
-def plan_code(wl, precision: str, variant: int) -> int:
-    """The explicit variant code of what the library runs for this workload (tile shape, stabiliser / split form)."""
+def plan_code(wl, precision: str, variant: int):
+    """The explicit variant code of what the library runs for this workload (tile shape, stabiliser / split form), or "direct"
+    for a small call."""
     from triturus_b200 import _native
 
     d = wl.dims
     prec = 0 if precision == "tf32" else 1
+    if runs_direct(wl, precision, variant):
+        return "direct"
     if wl.op == "lt2exp":
         return int(_native.LIB.triturus_b200_lt2exp_plan(d["R"], d["S"], d["I"], d["J"], d["K"], prec, variant))
     return int(_native.LIB.triturus_b200_lm2exp_plan(d["R"], d["I"], d["J"], d["K"], prec, variant))
@@ -627,7 +645,7 @@ def main() -> None:
     kernel_ms = prepass_ms = None
     pcode = plan_code(wl, args.precision, args.variant)
     # 0 optimistic TMEM-operand pair kernel, 1 pre-pass, 2 / 3 fused max pass, 4 optimistic 32-row pre-pass
-    stab = pcode // 100000 if wl.op == "lm2exp" else -1
+    stab = pcode // 100000 if wl.op == "lm2exp" and pcode != "direct" else -1
     if stab in (0, 1, 4) and not args.chain and not args.profile_mode:
         m_pre = tb.colmax(inputs[1])
         kern = lambda: tb.lm2exp(*inputs, precision=args.precision, variant=args.variant, b_colmax=m_pre)  # noqa: E731

@@ -287,13 +287,15 @@ def test_odd_operands_are_read_in_place_only_where_that_is_faster():
 
 
 def test_automatic_plans_of_lm2exp():
-    """What a call runs for the benchmark shapes and around the size rule of the optimistic stabilisers (the plan
-    queries need no GPU: without one they assume 148 SMs)."""
+    """The plans of the benchmark shapes and around the size rule of the optimistic stabilisers (the queries need no GPU:
+    without one they assume 148 SMs).  A call of cfg1 is a small one, which runs the direct kernel instead of its plan."""
     plan, launches = _native.LIB.triturus_b200_lm2exp_plan, _native.LIB.triturus_b200_lm2exp_launches
     assert plan(32, 1024, 1024, 1024, 0, 0) == 2567 and launches(32, 1024, 1024, 1024, 0, 0) == 2      # cfg2, TF32
     assert plan(32, 1024, 1024, 1024, 1, 0) == 402564 and launches(32, 1024, 1024, 1024, 1, 0) == 4    # cfg2, 3xTF32
     assert plan(128, 256, 256, 8192, 0, 0) == 2567                                                      # cfg3
     assert plan(4, 256, 256, 256, 0, 0) == 201281 and launches(4, 256, 256, 256, 0, 0) == 1             # cfg1
+    assert _native.LIB.triturus_b200_lm2exp_direct(4, 256, 256, 256, 0, 0, 0) == 1
+    assert _native.LIB.triturus_b200_lm2exp_direct(32, 1024, 1024, 1024, 0, 0, 0) == 0
     assert plan(64, 256, 256, 256, 0, 0) // 100000 == 2      # two row blocks but under 2e10 FLOP: one fused launch
     assert plan(256, 128, 256, 8192, 0, 0) // 100000 == 3    # one row block, long launch: optimistic fused max pass
     assert plan(4, 1024, 1024, 1024, 0, 0) == 102566         # a chunk of the host pipeline: pre-pass + pair kernel
