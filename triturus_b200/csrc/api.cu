@@ -439,7 +439,7 @@ struct Pair3xPlan {
   int64_t busiest;  // cost of the busiest pair
 };
 
-// Shares or round robin: whichever keeps the busiest pair busy for less.  (R32 1024^3: 58 units against 66.)
+// Shares or round robin: whichever keeps the busiest pair busy for less.  (R32 1024^3: 60 units against 66.)
 static Pair3xPlan pair3x_plan(int64_t R, int64_t I, int64_t K, int64_t pairs) {
   const int64_t units = (I + 31) / 32, tiles_n = (K + 2 * Lm2expPair3xCfg::BM - 1) / (2 * Lm2expPair3xCfg::BM);
   const int64_t nt = (units + Lm2expPair3xCfg::UNITS - 1) / Lm2expPair3xCfg::UNITS;
@@ -460,10 +460,10 @@ static Pair3xPlan pair3x_plan(int64_t R, int64_t I, int64_t K, int64_t pairs) {
 
 // Tiles of 192 rows with two accumulators, or of 256 with one?  Cycles of the busiest pair: the second leaves 14 400 of every
 // tile to the epilogue and its tiles come in whole waves; in the first a unit takes 1.1 times its MMAs, or the 2 500 of its
-// epilogue where the contraction is short, and the last epilogue 8 000 alone.  us, one / two accumulators: R48 260x1000x300 129 /
+// epilogue where the contraction is short, and the last epilogue 8 000 alone.  us in a loop, one / two accumulators: R48 260x1000x300 129 /
 // 82, R40 1000x700x700 212 / 175, R12 768^3 75 / 58, R64 320x128x512 57 / 40, R8 384x256x2048 39.6 / 30.1, R64 512x512x256 62.6 / 55.8,
-// R24 512x256x1024 59.2 / 52.9, R16 1024x1024x512 95 / 87; R1 2048^3 89 / 91 and R100 512x64x256 38.3 / 39.6, which the
-// estimate leaves to one accumulator.
+// R24 512x256x1024 59.2 / 52.9, R16 1024x1024x512 95 / 87; level for R1 2048^3 and R100 512x64x256, which the estimate leaves to one
+// accumulator.
 // A launch of more than about 130 us runs at the power limit, where regenerating the operand for more tiles costs what the
 // overlap gains (R32 1024^3 316 / 324): there only a quarter less of cycles counts.
 static bool pair3x_wins(int64_t R, int64_t I, int64_t J, int64_t K) {
@@ -591,7 +591,9 @@ static int plan_lm2exp(int64_t R, int64_t I, int64_t J, int64_t K, int precision
     // Plain TF32, more than one row block, on the TMEM-operand pair kernel: the single-CTA kernel carries both operands and the
     // exponentials through shared memory.  us, single-CTA / pairs: R1 177x768x160 32 / 15, R3 959x704x224 31 / 17, R30 201x800x276 38 /
     // 24, R117 160x44x1992 96 / 65, R2 256x288x6720 20.5 / 14.2, R48 236x248x1236 54 / 43, R22 218x256x3864 63 / 55.  Up to 64 K values
-    // of b per entry the one fused launch stays, which counts for callers that are bound by the host.  So it does for long
+    // of b per entry the one fused launch stays, whose plan code callers may have saved.  That is right for loops that the
+    // host bounds (R32 256^3 fused 18.6 us per call in a loop, pairs 20.1; 16.4 and 15.5 on the device) and gives away time
+    // above some 20 us (R64 256^3 19.6 / 15.3 on the device, 22.7 / 19.5 in a loop; R96 256x128x512 30.4 / 26.6).  So it does for long
     // launches of more than 128 terms, where the epilogue of a pair's tile is not hidden (R84 252x144x1496 63 / 64), and where
     // the other half of a tile is padding (R98 198x64x120 12.6 / 14.6).
     const bool ts_pair = precision == TRITURUS_B200_PRECISION_TF32 && plain_ts && stab_mode == 0 && I > 128 && J <= 4096 && !big &&

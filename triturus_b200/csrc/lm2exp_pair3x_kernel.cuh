@@ -19,8 +19,8 @@
 // units each; as 720 equal tiles round robin some pairs would have ten of them, 60 units.  Where the groups would leave more
 // pairs idle than equal tiles do, tiles go round robin.
 //
-// Measured against 256-row tiles with one accumulator, us per call: R40 1000x700x700 212 -> 175, R48 260x1000x300 129 -> 82, R64
-// 512x512x256 63.3 -> 59.5; which of the two a call takes is pair3x_wins in api.cu.
+// Measured against 256-row tiles with one accumulator, us per call in a loop: R40 1000x700x700 206 -> 180, R48 260x1000x300 128 -> 82,
+// R64 512x512x256 62.7 -> 55.8 (with other inputs in every pass 63.2 -> 59.3); which of the two a call takes is pair3x_wins in api.cu.
 //
 // Rings.  The barriers of k-blocks are rings of eight (index = k-block counter `it` % 8, phase it / 8), whatever the number
 // of stages that the memory allows: TMEM stage it % 2, shared-memory stage of a it % 4.  Who wants to overwrite a stage waits

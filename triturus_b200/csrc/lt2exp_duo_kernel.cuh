@@ -6,8 +6,8 @@
 // election, the descriptors), and the tensor core, which queues no more than an MMA or two, stands still meanwhile.  Here a
 // stage holds the k-blocks of two consecutive rows i, the issuer asks for the next stage in the middle of one, and the
 // tiles of w have a ring of their own, four stages deep, beside the two operand stages that tensor memory has room for:
-// 1 075 to 1 160 cycles per stage of 1 024.  R16 128x64x64x2048 69.6 -> 57.7 us, R8 100x100x100x3000 165 -> 139, R30
-// 128x64x64x2048 131 -> 110.  What is left of the first (102 000 cycles): 13 300 before the first MMA, which are HBM's (a, b and the first
+// 1 075 to 1 160 cycles per stage of 1 024.  us in a loop: R16 128x64x64x2048 74.8 -> 61.6, R8 100x100x100x3000 167 -> 142, R30
+// 128x64x64x2048 132 -> 108; with other inputs in every pass the first 71.9 -> 63.8.  What is left of the first (102 000 cycles): 13 300 before the first MMA, which are HBM's (a, b and the first
 // tiles of w of all SMs at once), 2 900 where the j-chunk changes, 7 900 in the epilogue.
 //
 // TMEM: [0, 256) accumulators of the two blocks, then two operand stages of [block][row of the pair][32 j] = 128 columns.
